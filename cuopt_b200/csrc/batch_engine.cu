@@ -201,42 +201,6 @@ struct b_term_dual_epi {
   }
 };
 
-// Power iteration sweeps: out = A^T q (store) and z = A (A^T q) with rowbuf = q z.
-template <typename TX>
-struct b_store_epi {
-  static constexpr int kRed = 0;
-  TX* out;
-  inst_ctx ctx;
-  struct pre_t {};
-  __device__ bool skip() const { return false; }
-  __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
-  __device__ __forceinline__ pre_t load(int) const { return pre_t{}; }
-  __device__ __forceinline__ void operator()(int r, double acc, const pre_t&, red_t<0>&) const
-  {
-    out[r] = (TX)acc;
-  }
-};
-struct b_power_z_epi {
-  static constexpr int kRed = 0;
-  double* z;
-  const double* q;
-  double* rowbuf;
-  inst_ctx ctx;
-  struct pre_t {
-    double q;
-    int b;
-  };
-  __device__ bool skip() const { return false; }
-  __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
-  __device__ __forceinline__ pre_t load(int i) const { return pre_t{q[i], ctx.inst[i]}; }
-  __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<0>&) const
-  {
-    if (!ctx.active[p.b]) return;
-    z[i]      = acc;
-    rowbuf[i] = p.q * acc;
-  }
-};
-
 // Rows of an instance are processed in chunks of at most kChunkRows (each inside one instance), so
 // a large instance does not serialise a kernel on one block.
 constexpr int kChunkRows = 2048;
@@ -458,14 +422,6 @@ __global__ void b_advance_kernel(pdlp_scalars* sc, const int* active, int count,
     if (active[b]) sc[b].t0 += steps;
 }
 
-// Power iteration per instance (reference pdlp.cu:2620-2731), one block per instance.
-struct b_power_state {
-  double s2;
-  double resid;
-  int iters;
-  int pad;
-};
-
 // Fixed-order block sum of per-thread values (compensated per thread, then a fixed tree).
 __device__ __forceinline__ double block_sum(const ksum& acc, double* sm)
 {
@@ -480,134 +436,15 @@ __device__ __forceinline__ double block_sum(const ksum& acc, double* sm)
   return v;
 }
 
-// The power iteration's vector work runs on the same row chunks; chunk partial sums are combined
-// per instance in chunk order (deterministic).
-
-// Thread 0's fixed-order sum of the partials of instance b's chunks, shared with the block.
-__device__ __forceinline__ double instance_total(const double* part, const int* chunk_off, int b,
-                                                 double* slot)
-{
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int c = chunk_off[b]; c < chunk_off[b + 1]; ++c) t += part[c];
-    *slot = t;
-  }
-  __syncthreads();
-  return *slot;
-}
-
-// part[c] = sum of z^2 over chunk c.
-__global__ void __launch_bounds__(kBlock) b_chunk_sumsq_kernel(const int4* chunks, const int* pactive,
-                                                               const double* z, double* part)
-{
-  const int4 ch = chunks[blockIdx.x];
-  if (!pactive[ch.x]) return;
-  __shared__ double sm[kBlock];
-  ksum acc;
-  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) acc.add(z[i] * z[i]);
-  const double v = block_sum(acc, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = v;
-}
-
-// q = z / |z| over chunk c (|z| of its instance).
-__global__ void __launch_bounds__(kBlock)
-  b_chunk_normalize_kernel(const int4* chunks, const int* chunk_off, const int* pactive,
-                           const double* part, const double* z, double* q)
-{
-  const int4 ch = chunks[blockIdx.x];
-  if (!pactive[ch.x]) return;
-  __shared__ double slot;
-  const double nq = sqrt(instance_total(part, chunk_off, ch.x, &slot));
-  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) q[i] = z[i] / nq;
-}
-
-// part[c] = sum of rowbuf (q_i z_i) over chunk c.
-__global__ void __launch_bounds__(kBlock) b_chunk_sum_kernel(const int4* chunks, const int* pactive,
-                                                             const double* v, double* part)
-{
-  const int4 ch = chunks[blockIdx.x];
-  if (!pactive[ch.x]) return;
-  __shared__ double sm[kBlock];
-  ksum acc;
-  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) acc.add(v[i]);
-  const double t = block_sum(acc, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = t;
-}
-
-// The power iteration's step folds the next step's norm and normalisation into this step's
-// chunk kernels (same values as the separate kernels above, two launches fewer per step):
-// part[c] = sum of rowbuf (q_i z_i) over chunk c and part_z[c] = sum of z_i^2 over chunk c.
-__global__ void __launch_bounds__(kBlock)
-  b_chunk_sum_sumsq_kernel(const int4* chunks, const int* pactive, const double* v,
-                           const double* z, double* part, double* part_z)
-{
-  const int4 ch = chunks[blockIdx.x];
-  if (!pactive[ch.x]) return;
-  __shared__ double sm[kBlock];
-  ksum acc, acc_z;
-  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) {
-    acc.add(v[i]);
-    acc_z.add(z[i] * z[i]);
-  }
-  const double t   = block_sum(acc, sm);
-  const double t_z = block_sum(acc_z, sm);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x]   = t;
-    part_z[blockIdx.x] = t_z;
-  }
-}
-
-// s2 = q . z of the instance;  part_r[c] = sum over chunk c of (z - s2 q)^2;  then q <- z / |z|,
-// the next step's normalised vector.
-__global__ void __launch_bounds__(kBlock)
-  b_chunk_residual_next_kernel(const int4* chunks, const int* chunk_off, const int* pactive,
-                               const double* part_s2, const double* part_z, const double* z,
-                               double* q, double* part_r)
-{
-  const int4 ch = chunks[blockIdx.x];
-  if (!pactive[ch.x]) return;
-  __shared__ double slot, slot_z;
-  __shared__ double sm[kBlock];
-  const double s2 = instance_total(part_s2, chunk_off, ch.x, &slot);
-  const double nq = sqrt(instance_total(part_z, chunk_off, ch.x, &slot_z));
-  ksum acc;
-  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) {
-    const double v = q[i] * -s2 + z[i];
-    acc.add(v * v);
-    q[i] = z[i] / nq;
-  }
-  const double t = block_sum(acc, sm);
-  if (threadIdx.x == 0) part_r[blockIdx.x] = t;
-}
-
-// Per instance: record sigma^2 and the residual, test convergence.
-__global__ void b_power_check_kernel(const int* chunk_off, int count, const double* part_s2,
-                                     const double* part_r, int* pactive, b_power_state* ps,
-                                     double tol, int* remaining)
-{
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < count; b += gridDim.x * blockDim.x) {
-    if (!pactive[b]) continue;
-    double s2 = 0.0, r = 0.0;
-    for (int c = chunk_off[b]; c < chunk_off[b + 1]; ++c) {
-      s2 += part_s2[c];
-      r += part_r[c];
-    }
-    ps[b].s2    = s2;
-    ps[b].resid = sqrt(r);
-    ps[b].iters += 1;
-    if (ps[b].resid < tol) {
-      pactive[b] = 0;
-      atomicSub(remaining, 1);
-    }
-  }
-}
-
-// Golub-Kahan-Lanczos step size per instance (mixed precision), the single engine's
-// lanczos_step_size run on every instance at once: u and v hold the unnormalised Lanczos vectors,
-// st[b] their norms, and rowbuf the squares of the new vector for the per-instance norms.
+// Golub-Kahan-Lanczos bidiagonalisation per instance (the step size), the single engine's
+// run on every instance at once: u and v hold the unnormalised Lanczos vectors, st[b] their
+// norms (and the row chunks of the running sum that have been added), and rowbuf the squares of
+// the new vector for the per-instance norms.
 struct b_gk_state {
   double beta;
   double alpha;
+  unsigned arrived;
+  unsigned pad;
 };
 
 // Row j of A^T applied to u:  p_j = (A^T u)_j / beta - beta v_j / alpha  (written over v_j).
@@ -658,25 +495,39 @@ struct b_gk_dual_epi {
   }
 };
 
-// Per iterating instance b, the norm of its new vector from the chunk sums: FIELD 0 sets alpha
-// (hist[k * count + b]), FIELD 1 sets beta (hist[(k + 1) * count + b]).
-template <int FIELD>
-__global__ void b_gk_record_kernel(const int* chunk_off, int count, const double* part,
-                                   const int* active, b_gk_state* st, double* hist, int k)
+// The norm of each iterating instance's new vector: block c sums its chunk of `v` (the squares in
+// the row buffer, or with SQUARE the vector itself), and the block that finishes last of its
+// instance adds the instance's chunks in chunk order.  FIELD 0 sets alpha (hist[k * count + b]),
+// FIELD 1 sets beta (hist[(k + 1) * count + b]).
+template <int FIELD, bool SQUARE = false>
+__global__ void __launch_bounds__(kBlock)
+  b_gk_norm_kernel(const int4* chunks, const int* chunk_off, int count, const int* active,
+                   const double* v, double* part, b_gk_state* st, double* hist, int k)
 {
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < count; b += gridDim.x * blockDim.x) {
-    if (!active[b]) continue;
-    double t = 0.0;
-    for (int c = chunk_off[b]; c < chunk_off[b + 1]; ++c) t += part[c];
-    const double v = sqrt(t);
-    if (FIELD == 0) {
-      st[b].alpha                     = v;
-      hist[(size_t)k * count + b]     = v;
-    } else {
-      st[b].beta                      = v;
-      hist[(size_t)(k + 1) * count + b] = v;
-    }
+  const int4 ch = chunks[blockIdx.x];
+  const int b   = ch.x;
+  if (!active[b]) return;
+  __shared__ double sm[kBlock];
+  ksum acc;
+  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock) acc.add(SQUARE ? v[i] * v[i] : v[i]);
+  const double t = block_sum(acc, sm);
+  if (threadIdx.x != 0) return;
+  const int c0 = chunk_off[b], c1 = chunk_off[b + 1];
+  part[blockIdx.x] = t;
+  __threadfence();
+  if (atomicAdd(&st[b].arrived, 1u) != (unsigned)(c1 - c0 - 1)) return;
+  __threadfence();
+  double sum = 0.0;
+  for (int c = c0; c < c1; ++c) sum += __ldcg(part + c);
+  const double norm = sqrt(sum);
+  if (FIELD == 0) {
+    st[b].alpha                 = norm;
+    hist[(size_t)k * count + b] = norm;
+  } else {
+    st[b].beta                        = norm;
+    hist[(size_t)(k + 1) * count + b] = norm;
   }
+  st[b].arrived = 0;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1077,117 +928,53 @@ class batch_engine {
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
   }
 
-  // Power iteration of every instance (graph chunks of 32 iterations; converged instances freeze).
+  // The reference's power iteration of every instance (pdlp.cu:2620-2731) in the Krylov space of
+  // its start vector, as in single solves.  On 64 LPs of 200 to 20 000 rows, whose iterations take
+  // up to 2 800 products with A A^T, the step sizes took 164 of 264 ms with the iteration itself.
   void power_iteration()
   {
-    const int m = in_.m, n = in_.n;
-    // Every instance starts from the first m_b values of the std::mt19937(1) normal sequence.
-    std::vector<double> z0(m);
-    int max_rows = 0;
-    for (int b = 0; b < B_; ++b) max_rows = std::max(max_rows, in_.row_start[b + 1] - in_.row_start[b]);
-    const auto seq = power_start_sequence(max_rows);
-    for (int b = 0; b < B_; ++b)
-      std::copy(seq->begin(), seq->begin() + (in_.row_start[b + 1] - in_.row_start[b]),
-                z0.begin() + in_.row_start[b]);
-    dbuf<double> dz(m), dq(m), datq(n);
-    dq.upload(z0.data(), m, s_);
-    permute_gather(dq.data(), L_.row_new2old.data(), m, 1.0, dz.data(), s_);
-    dbuf<b_power_state> ps(B_);
-    ps.zero(s_);
-    dbuf<int> pact(B_), remaining(1);
-    std::vector<int> pact_h(B_, 1);
-    pact.upload(pact_h.data(), B_, s_);
-    remaining.upload(&B_, 1, s_);
-    const inst_ctx rctx{rinst_.data(), pact.data(), nullptr};
-    const inst_ctx cctx{cinst_.data(), pact.data(), nullptr};
-    const int nchunks = rows_.count;
-    dbuf<double> part_z(std::max(nchunks, 1)), part_s2(std::max(nchunks, 1)),
-      part_r(std::max(nchunks, 1));
-    const int4* dchunks_p   = rows_.chunks.data();
-    const int* dchunk_off_p = rows_.offsets.data();
-    // q = z0 / |z0| once; every step then ends with the next step's q (z / |z|).
-    b_chunk_sumsq_kernel<<<nchunks, kBlock, 0, s_>>>(dchunks_p, pact.data(), dz.data(),
-                                                     part_z.data());
-    b_chunk_normalize_kernel<<<nchunks, kBlock, 0, s_>>>(dchunks_p, dchunk_off_p, pact.data(),
-                                                         part_z.data(), dz.data(), dq.data());
-    launches_ += 2;
-    B200_LAUNCH_CHECK();
-    auto one_iteration = [&]() {
-      const auto As  = wview<TX>(true, As_.data());
-      const auto ATs = wview<TX>(false, ATs_.data());
-      sell_map_kernel<TX, double, b_store_epi<double>><<<sell_grid(ATs), kBlock, 0, s_>>>(
-        ATs, dq.data(), b_store_epi<double>{datq.data(), cctx}, partials_.data());
-      sell_map_kernel<TX, double, b_power_z_epi><<<sell_grid(As), kBlock, 0, s_>>>(
-        As, datq.data(), b_power_z_epi{dz.data(), dq.data(), rowbuf_.data(), rctx},
-        partials_.data());
-      b_chunk_sum_sumsq_kernel<<<nchunks, kBlock, 0, s_>>>(dchunks_p, pact.data(),
-                                                           rowbuf_.data(), dz.data(),
-                                                           part_s2.data(), part_z.data());
-      b_chunk_residual_next_kernel<<<nchunks, kBlock, 0, s_>>>(
-        dchunks_p, dchunk_off_p, pact.data(), part_s2.data(), part_z.data(), dz.data(),
-        dq.data(), part_r.data());
-      b_power_check_kernel<<<ceil_div(B_, kBlock), kBlock, 0, s_>>>(
-        dchunk_off_p, B_, part_s2.data(), part_r.data(), pact.data(), ps.data(), kPowerTol,
-        remaining.data());
-    };
-    // Chunks of 32 iterations are captured into a graph.  When the instances still iterating are
-    // at most half of those the sweeps were last restricted to, the work lists shrink to them and
-    // the chunk is captured again.
-    cudaGraphExec_t exec = nullptr;
-    auto capture = [&]() {
-      if (exec) cudaGraphExecDestroy(exec);
-      cudaGraph_t graph;
-      B200_CUDA_CHECK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
-      for (int i = 0; i < 32; ++i) one_iteration();
-      B200_CUDA_CHECK(cudaStreamEndCapture(s_, &graph));
-      B200_CUDA_CHECK(cudaGraphInstantiate(&exec, graph, 0));
-      cudaGraphDestroy(graph);
-    };
-    capture();
-    int left = B_, listed = B_;
-    for (int done_iters = 0; done_iters < kPowerMaxIters; done_iters += 32) {
-      if (kPowerMaxIters - done_iters < 32) {
-        for (int i = 0; i < kPowerMaxIters - done_iters; ++i) one_iteration();
-      } else {
-        B200_CUDA_CHECK(cudaGraphLaunch(exec, s_));
-      }
-      launches_ += 5.0 * std::min(32, kPowerMaxIters - done_iters);
-      remaining.download(&left, 1, s_);
-      B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      if (left == 0) break;
-      if (2 * left <= listed) {
-        pact.download(pact_h.data(), B_, s_);
-        B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-        rebuild_work(pact_h);
-        listed = left;
-        capture();
-        char what[96];
-        std::snprintf(what, sizeof what, "batch: power to %d its, %d instances left",
-                      done_iters + 32, left);
-        trace(what);
-      }
-    }
-    cudaGraphExecDestroy(exec);
-    clear_work();
-    std::vector<b_power_state> h(B_);
-    ps.download(h.data(), B_, s_);
-    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    eta_.resize(B_);
-    power_iters_.resize(B_);
-    for (int b = 0; b < B_; ++b) {
-      eta_[b]         = kStepScaling / std::sqrt(h[b].s2);
-      power_iters_[b] = h[b].iters;
-    }
+    std::vector<krylov_power_iteration> power(B_);
+    bidiagonalise(kKrylovMaxSteps, [&](int b, int k, const double* a, const double* bb) {
+      const bool done = power[b].advance(a, bb, k);
+      power_iters_[b] = power[b].iterations();
+      return done;
+    });
+    for (int b = 0; b < B_; ++b) eta_[b] = kStepScaling / std::sqrt(power[b].sigma2());
   }
 
-  // Golub-Kahan-Lanczos on every instance (the single engine's lanczos_step_size, per instance):
-  // chunks of kLanczosChunk steps; after each chunk an instance whose sigma_max^2 estimate moved by
-  // at most kLanczosTol (relative), or whose recurrence broke down, stops, and the sweeps shrink
-  // to the instances still iterating once they are at most half of those listed.
+  // The largest singular value of every instance (the single engine's lanczos_step_size): an
+  // instance stops when its estimate moved by at most kLanczosTol (relative) over a chunk of
+  // steps, or its recurrence broke down.
   void lanczos_step_size()
   {
+    std::vector<double> prev(B_, -1.0), sigma2(B_, 0.0);
+    bidiagonalise(kLanczosMaxSteps, [&](int b, int k, const double* a, const double* bb) {
+      bool breakdown = false;
+      int used       = k;
+      for (int j = 0; j < k; ++j)
+        if (!(a[j] > 0.0) || !(bb[j] > 0.0) || !std::isfinite(a[j]) || !std::isfinite(bb[j])) {
+          used      = j + 1;
+          breakdown = true;
+          break;
+        }
+      sigma2[b]       = largest_bidiagonal_sigma2(a, bb, used);
+      power_iters_[b] = used;
+      const bool done = breakdown || (prev[b] > 0.0 && std::fabs(sigma2[b] - prev[b]) <=
+                                                         kLanczosTol * sigma2[b]);
+      prev[b] = sigma2[b];
+      return done;
+    });
+    for (int b = 0; b < B_; ++b) eta_[b] = kStepScaling / std::sqrt(sigma2[b]);
+  }
+
+  // Golub-Kahan bidiagonalisation of every instance, in chunks of kLanczosChunk steps: after each,
+  // test(instance, steps, diagonal, subdiagonal) tells which instances are done, and the sweeps
+  // shrink to the others once these are at most half of those listed.
+  template <class Test>
+  void bidiagonalise(int max_steps, Test&& test)
+  {
     const int m = in_.m, n = in_.n;
-    const int ld = kLanczosMaxSteps + 2;  // history rows (steps), each B_ wide
+    const int ld = max_steps + 2;  // history rows (steps), each B_ wide
     // Every instance starts from the first m_b values of the std::mt19937(1) normal sequence.
     std::vector<double> z0(m);
     int max_rows = 0;
@@ -1202,18 +989,19 @@ class batch_engine {
     permute_gather(tmp.data(), L_.row_new2old.data(), m, 1.0, u.data(), s_);
     v.zero(s_);
     st.zero(s_);
+    alphas.zero(s_);  // an instance without rows or columns records nothing
+    betas.zero(s_);
     dbuf<int> pact(B_);
     std::vector<int> pact_h(B_, 1);
     pact.upload(pact_h.data(), B_, s_);
     const inst_ctx rctx{rinst_.data(), pact.data(), nullptr};
     const inst_ctx cctx{cinst_.data(), pact.data(), nullptr};
-    dbuf<double> part_r(std::max(rows_.count, 1)), part_c(std::max(cols_.count, 1));
-    // beta_0 = |z0| per instance (betas[b * ld + 0])
-    b_chunk_sumsq_kernel<<<rows_.count, kBlock, 0, s_>>>(rows_.chunks.data(), pact.data(),
-                                                        u.data(), part_r.data());
-    b_gk_record_kernel<1><<<ceil_div(B_, kBlock), kBlock, 0, s_>>>(
-      rows_.offsets.data(), B_, part_r.data(), pact.data(), st.data(), betas.data(), -1);
-    launches_ += 2;
+    dbuf<double> part(std::max({rows_.count, cols_.count, 1}));
+    // beta_0 = |z0| per instance
+    b_gk_norm_kernel<1, true><<<rows_.count, kBlock, 0, s_>>>(
+      rows_.chunks.data(), rows_.offsets.data(), B_, pact.data(), u.data(), part.data(), st.data(),
+      betas.data(), -1);
+    ++launches_;
     B200_LAUNCH_CHECK();
     auto step = [&](int k) {
       const auto As  = wview<TX>(true, As_.data());
@@ -1221,63 +1009,52 @@ class batch_engine {
       sell_map_kernel<TX, double, b_gk_primal_epi><<<sell_grid(ATs), kBlock, 0, s_>>>(
         ATs, u.data(), b_gk_primal_epi{v.data(), rowbuf_.data(), st.data(), cctx},
         partials_.data());
-      b_chunk_sum_kernel<<<cols_.count, kBlock, 0, s_>>>(cols_.chunks.data(), pact.data(),
-                                                         rowbuf_.data(), part_c.data());
-      b_gk_record_kernel<0><<<ceil_div(B_, kBlock), kBlock, 0, s_>>>(
-        cols_.offsets.data(), B_, part_c.data(), pact.data(), st.data(), alphas.data(), k);
+      b_gk_norm_kernel<0><<<cols_.count, kBlock, 0, s_>>>(
+        cols_.chunks.data(), cols_.offsets.data(), B_, pact.data(), rowbuf_.data(), part.data(),
+        st.data(), alphas.data(), k);
       sell_map_kernel<TX, double, b_gk_dual_epi><<<sell_grid(As), kBlock, 0, s_>>>(
         As, v.data(), b_gk_dual_epi{u.data(), rowbuf_.data(), st.data(), rctx},
         partials_.data());
-      b_chunk_sum_kernel<<<rows_.count, kBlock, 0, s_>>>(rows_.chunks.data(), pact.data(),
-                                                         rowbuf_.data(), part_r.data());
-      b_gk_record_kernel<1><<<ceil_div(B_, kBlock), kBlock, 0, s_>>>(
-        rows_.offsets.data(), B_, part_r.data(), pact.data(), st.data(), betas.data(), k);
+      b_gk_norm_kernel<1><<<rows_.count, kBlock, 0, s_>>>(
+        rows_.chunks.data(), rows_.offsets.data(), B_, pact.data(), rowbuf_.data(), part.data(),
+        st.data(), betas.data(), k);
     };
-    std::vector<double> ha((size_t)B_ * ld), hb((size_t)B_ * ld), prev(B_, -1.0), sigma2(B_, 0.0);
+    std::vector<double> ha((size_t)B_ * ld), hb((size_t)B_ * ld);
     std::vector<char> done(B_, 0);
-    std::vector<int> used_steps(B_, 0);
     eta_.assign(B_, 0.0);
     power_iters_.assign(B_, 0);
     int left = B_, listed = B_, k = 0;
-    while (left > 0 && k < kLanczosMaxSteps) {
-      const int c = std::min(kLanczosChunk, kLanczosMaxSteps - k);
+    while (left > 0 && k < max_steps) {
+      const int c = std::min(kLanczosChunk, max_steps - k);
       for (int i = 0; i < c; ++i) step(k + i);
-      launches_ += 6.0 * c;
+      launches_ += 4.0 * c;
       B200_LAUNCH_CHECK();
-      k += c;
-      alphas.download(ha.data(), (size_t)k * B_, s_);
-      betas.download(hb.data(), (size_t)(k + 1) * B_, s_);
+      // The new rows of the histories.
+      B200_CUDA_CHECK(cudaMemcpyAsync(ha.data() + (size_t)k * B_, alphas.data() + (size_t)k * B_,
+                                      (size_t)c * B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
+      B200_CUDA_CHECK(cudaMemcpyAsync(hb.data() + (size_t)(k + 1) * B_,
+                                      betas.data() + (size_t)(k + 1) * B_,
+                                      (size_t)c * B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
       B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      // Each instance's estimate (a Sturm bisection per instance, the host's share of the step)
-      // is independent of the others: instances are split over host threads, each writing only
-      // its own entries, so the results do not depend on the split.
+      k += c;
+      // Each instance's test (the host's share of the step) is independent of the others:
+      // instances are split over host threads, each writing only its own entries, so the results
+      // do not depend on the split.
       parallel_ranges(B_, [&](int b0, int b1) {
-        std::vector<double> a(ld), bb(ld);
+        std::vector<double> a(k), bb(k);
         for (int b = b0; b < b1; ++b) {
           if (!pact_h[b]) continue;
           // betas[0] holds |z0|; the recurrence coefficients are betas[1..].
-          for (int j = 0; j < k; ++j) a[j] = ha[(size_t)j * B_ + b];
-          for (int j = 0; j <= k; ++j) bb[j] = hb[(size_t)j * B_ + b];
-          bool breakdown = false;
-          int used       = k;
-          for (int j = 0; j < k; ++j)
-            if (!(a[j] > 0.0) || !(bb[j + 1] > 0.0) || !std::isfinite(a[j]) ||
-                !std::isfinite(bb[j + 1])) {
-              used      = j + 1;
-              breakdown = true;
-              break;
-            }
-          sigma2[b]     = largest_bidiagonal_sigma2(a.data(), bb.data() + 1, used);
-          done[b]       = breakdown || k >= kLanczosMaxSteps ||
-                    (prev[b] > 0.0 && std::fabs(sigma2[b] - prev[b]) <= kLanczosTol * sigma2[b]);
-          used_steps[b] = used;
-          prev[b]       = sigma2[b];
+          for (int j = 0; j < k; ++j) {
+            a[j]  = ha[(size_t)j * B_ + b];
+            bb[j] = hb[(size_t)(j + 1) * B_ + b];
+          }
+          done[b] = test(b, k, a.data(), bb.data());
         }
       });
       for (int b = 0; b < B_; ++b)
         if (pact_h[b] && done[b]) {
-          pact_h[b]       = 0;
-          power_iters_[b] = used_steps[b];
+          pact_h[b] = 0;
           --left;
         }
       if (left == 0) break;
@@ -1286,16 +1063,12 @@ class batch_engine {
         rebuild_work(pact_h);
         listed = left;
         char what[96];
-        std::snprintf(what, sizeof what, "batch: lanczos to %d steps, %d instances left", k,
+        std::snprintf(what, sizeof what, "batch: bidiagonal to %d steps, %d instances left", k,
                       left);
         trace(what);
       }
     }
     clear_work();
-    for (int b = 0; b < B_; ++b) {
-      if (pact_h[b]) power_iters_[b] = k;  // step limit reached
-      eta_[b] = kStepScaling / std::sqrt(sigma2[b]);
-    }
   }
 
   // ---------------------------------------------------------------- work lists

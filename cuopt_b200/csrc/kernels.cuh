@@ -102,14 +102,18 @@ struct has_max_red : std::false_type {};
 template <class E>
 struct has_max_red<E, std::void_t<decltype(E::kMaxRed)>> : std::bool_constant<E::kMaxRed> {};
 
-// out[q] = sum over blocks of partials[b*K+q], summed by one block (ordered, compensated).
-template <int K>
+// out[q] = sum over blocks of partials[b*K+q], summed by one block (ordered, compensated).  L2: the
+// partials were written by other blocks of the same launch, so they are read through L2.
+template <int K, bool L2 = false>
 __device__ __forceinline__ void ordered_block_sum(const double* partials, int nblocks, double* out)
 {
   __shared__ double sm[kBlock];
   for (int q = 0; q < K; ++q) {
     ksum acc;
-    for (int b = threadIdx.x; b < nblocks; b += kBlock) acc.add(partials[(size_t)b * K + q]);
+    for (int b = threadIdx.x; b < nblocks; b += kBlock) {
+      const double* p = partials + (size_t)b * K + q;
+      acc.add(L2 ? __ldcg(p) : *p);
+    }
     sm[threadIdx.x] = acc.value();
     __syncthreads();
     for (int s = kBlock / 2; s > 0; s >>= 1) {
@@ -211,60 +215,11 @@ __device__ __forceinline__ T gather_load(const T* __restrict__ g, int i)
     return g[i];
 }
 
-// Where a sweep reads the matrix's values and indices from: global memory with evict-first loads
-// (every sweep but one), or a copy of the block's own virtual blocks in shared memory (the
-// cluster power iteration), whose element k of the view's arrays sits at k - shift.
-struct global_matrix {
-  static constexpr int64_t shift = 0;
-  template <typename T>
-  __device__ __forceinline__ T ld(const T* p) const
-  {
-    return ld_stream(p);
-  }
-  template <typename T>
-  __device__ __forceinline__ void chunk(const T* p, double (&v)[4]) const
-  {
-    load_chunk(p, v);
-  }
-  __device__ __forceinline__ int4 idx_chunk(const int* p) const { return load_idx_chunk(p); }
-};
-struct shared_matrix {
-  int64_t shift;
-  template <typename T>
-  __device__ __forceinline__ T ld(const T* p) const
-  {
-    return *p;
-  }
-  __device__ __forceinline__ void chunk(const float* p, double (&v)[4]) const
-  {
-    const float4 t = *reinterpret_cast<const float4*>(p);
-    v[0]           = t.x;
-    v[1]           = t.y;
-    v[2]           = t.z;
-    v[3]           = t.w;
-  }
-  __device__ __forceinline__ void chunk(const double* p, double (&v)[4]) const
-  {
-    const double2 a = reinterpret_cast<const double2*>(p)[0];
-    const double2 b = reinterpret_cast<const double2*>(p)[1];
-    v[0]            = a.x;
-    v[1]            = a.y;
-    v[2]            = b.x;
-    v[3]            = b.y;
-  }
-  __device__ __forceinline__ int4 idx_chunk(const int* p) const
-  {
-    return *reinterpret_cast<const int4*>(p);
-  }
-};
-
 // WPB: warps (rows or slices) per block.  Only the grouping of warps into blocks depends on it,
 // not any row's arithmetic; sweeps with block reductions (kRed > 0) use kWarpsPerBlock.
-template <typename TM, typename TG, class Epi, bool COH = false, int WPB = kWarpsPerBlock,
-          class MS = global_matrix>
+template <typename TM, typename TG, class Epi, bool COH = false, int WPB = kWarpsPerBlock>
 __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* __restrict__ g,
-                                               const Epi& epi, double* partials, int vb,
-                                               const MS& ms = MS{})
+                                               const Epi& epi, double* partials, int vb)
 {
   constexpr int K = Epi::kRed;
   static_assert(K == 0 || WPB == kWarpsPerBlock, "block reductions assume kWarpsPerBlock warps");
@@ -283,10 +238,10 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
     const int row = q < A.long_count() ? (A.long_list ? A.long_list[q] : q) : 0;
     if (q < A.long_count() && !skip_rows(epi, row, row)) {
       const auto pre  = epi.load(row);
-      const int64_t b = A.long_off[row] - ms.shift, e = A.long_off[row + 1] - ms.shift;
+      const int64_t b = A.long_off[row], e = A.long_off[row + 1];
       double acc      = 0.0;
       for (int64_t k = b + lane; k < e; k += kWarp)
-        acc += (double)ms.ld(A.val + k) * (double)gather_load<COH>(g, ms.ld(A.idx + k));
+        acc += (double)ld_stream(A.val + k) * (double)gather_load<COH>(g, ld_stream(A.idx + k));
       acc = warp_sum(acc);
       if (lane == 0) epi(row, acc, pre, red);
     }
@@ -300,15 +255,15 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
       const auto pre     = epi.load(valid ? row : A.rows - 1);
       const int64_t base = A.slice_off[s];
       const int nchunk   = (int)((A.slice_off[s + 1] - base) >> 7);  // 32 lanes x 4 elements
-      const TM* v        = A.val + (base - ms.shift) + lane * kChunk;
-      const int* ix      = A.idx + (base - ms.shift) + lane * kChunk;
+      const TM* v        = A.val + base + lane * kChunk;
+      const int* ix      = A.idx + base + lane * kChunk;
       double acc         = 0.0;
       int q              = 0;
       for (; q + 2 <= nchunk; q += 2) {
-        const int4 i0 = ms.idx_chunk(ix), i1 = ms.idx_chunk(ix + 32 * kChunk);
+        const int4 i0 = load_idx_chunk(ix), i1 = load_idx_chunk(ix + 32 * kChunk);
         double v0[4], v1[4];
-        ms.chunk(v, v0);
-        ms.chunk(v + 32 * kChunk, v1);
+        load_chunk(v, v0);
+        load_chunk(v + 32 * kChunk, v1);
         const TG g0 = gather_load<COH>(g, i0.x), g1 = gather_load<COH>(g, i0.y);
         const TG g2 = gather_load<COH>(g, i0.z), g3 = gather_load<COH>(g, i0.w);
         const TG g4 = gather_load<COH>(g, i1.x), g5 = gather_load<COH>(g, i1.y);
@@ -325,9 +280,9 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
         ix += 64 * kChunk;
       }
       if (q < nchunk) {
-        const int4 i0 = ms.idx_chunk(ix);
+        const int4 i0 = load_idx_chunk(ix);
         double v0[4];
-        ms.chunk(v, v0);
+        load_chunk(v, v0);
         const TG g0 = gather_load<COH>(g, i0.x), g1 = gather_load<COH>(g, i0.y);
         const TG g2 = gather_load<COH>(g, i0.z), g3 = gather_load<COH>(g, i0.w);
         acc += v0[0] * (double)g0;
@@ -941,39 +896,6 @@ struct term_linf_dual_epi {
   }
 };
 
-// Plain sweep epilogues.
-template <typename TX>
-struct store_epi {  // out[r] = acc
-  static constexpr int kRed = 0;
-  TX* out;
-  const int* done;  // optional early-exit flag
-  struct pre_t {};
-  __device__ bool skip() const { return done && *done; }
-  __device__ __forceinline__ pre_t load(int) const { return pre_t{}; }
-  __device__ __forceinline__ void operator()(int r, double acc, const pre_t&, red_t<0>&) const
-  {
-    out[r] = (TX)acc;
-  }
-};
-
-// Power iteration z = A (A^T q) with q . z accumulated (reference pdlp.cu:2664-2711).
-struct power_z_epi {
-  static constexpr int kRed = 1;
-  double* z;
-  const double* q;
-  const int* done;
-  struct pre_t {
-    double q;
-  };
-  __device__ bool skip() const { return *done != 0; }
-  __device__ __forceinline__ pre_t load(int i) const { return pre_t{q[i]}; }
-  __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<1>& r) const
-  {
-    z[i] = acc;
-    r.v[0] += p.q * acc;
-  }
-};
-
 // ---------------------------------------------------------------------------------------------
 // Reductions over plain vectors (block partials; finalize with finalize_sum_kernel).
 
@@ -1005,316 +927,15 @@ __global__ void __launch_bounds__(kBlock) vec_reduce_kernel(const TA* a, const T
 }
 
 // ---------------------------------------------------------------------------------------------
-// Power iteration helpers (reference pdlp.cu:2620-2731).  State on device:
-//   pi[0] = |z|, pi[1] = sigma_max^2, pi[2] = |residual|, done flag, iteration counter.
-struct power_state {
-  double norm_z;
-  double s2;
-  double resid;
-  int done;
-  int iters;
-};
-
-// The power iteration's vector steps.  Each scalar a step needs is summed by the consuming block
-// itself from the producer's block partials (ordered_block_sum, as finalize_sum_kernel does, so
-// every block gets the value finalize_sum_kernel would store): no separate finalize launches.
-//   q = z / |z|, |z|^2 from the vec_reduce partials (nz blocks).
-static __global__ void __launch_bounds__(kBlock)
-  power_normalize_sum_kernel(const double* z, double* q, int m, const double* part_z, int nz,
-                             power_state* ps)
-{
-  if (ps->done) return;
-  __shared__ double total;
-  ordered_block_sum<1>(part_z, nz, &total);
-  const double nq = sqrt(total);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-    q[i] = z[i] / nq;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ps->norm_z = nq;
-}
-//   s2 = q . z from the power_z sweep's partials (ns blocks); q <- q (-s2) + z; partial sums of
-//   squares of the result in part_r.
-static __global__ void __launch_bounds__(kBlock)
-  power_residual_sum_kernel(double* q, const double* z, int m, const double* part_s, int ns,
-                            const power_state* ps, double* part_r)
-{
-  red_t<1> r;
-  r.v[0] = 0.0;
-  if (!ps->done) {
-    __shared__ double s2;
-    ordered_block_sum<1>(part_s, ns, &s2);
-    const double s = s2;
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < m; i += gridDim.x * kBlock) {
-      const double v = q[i] * -s + z[i];
-      q[i]           = v;
-      r.v[0] += v * v;
-    }
-  }
-  block_reduce_store<1>(r, part_r);
-}
-//   Record s2 and the residual (one block); done once the residual is below tol.
-static __global__ void __launch_bounds__(kBlock)
-  power_check_sum_kernel(power_state* ps, const double* part_s, int ns, const double* part_r,
-                         int nr, double tol)
-{
-  if (ps->done) return;
-  __shared__ double s2, rsq;
-  ordered_block_sum<1>(part_s, ns, &s2);
-  ordered_block_sum<1>(part_r, nr, &rsq);
-  if (threadIdx.x == 0) {
-    ps->s2    = s2;
-    ps->resid = sqrt(rsq);
-    ps->iters += 1;
-    if (ps->resid < tol) ps->done = 1;
-  }
-}
-
-// The power iteration of a small LP in one thread-block cluster of C blocks of kBlock threads, all
-// steps up to convergence (or max_iters) in one launch.  Every block keeps full copies of z, q and
-// A^T q in its shared memory: the vector steps (normalisation, residual, and their sums) run on
-// the local copies in every block at once, the two sweeps are split over the blocks (virtual
-// blocks rank, rank + C, ...) and send each new entry of A^T q and z, and each q . z block
-// partial, to every block's copy through distributed shared memory, so a step needs two cluster
-// barriers.  Every sum is formed exactly as in the multi-kernel form: the vector steps emulate
-// its pg blocks of kBlock threads (grid stride pg * kBlock, one block reduction each), the sweeps
-// are its virtual blocks, and every scalar is ordered_block_sum of the same block partials, so
-// both forms give the same step size bit for bit.
-template <typename TX>
-struct cluster_atq_epi {  // (A^T q)_j to every block's copy
-  static constexpr int kRed = 0;
-  dsmem_sink<double> sink;
-  struct pre_t {};
-  __device__ bool skip() const { return false; }
-  __device__ __forceinline__ pre_t load(int) const { return pre_t{}; }
-  __device__ __forceinline__ void operator()(int j, double acc, const pre_t&, red_t<0>&) const
-  {
-    sink(j, acc);
-  }
-};
-struct cluster_z_epi {  // z_i = (A atq)_i to every block's copy; q . z block partial
-  static constexpr int kRed = 1;
-  dsmem_sink<double> sink;
-  const double* q;  // this block's copy of q
-  struct pre_t {
-    double q;
-  };
-  __device__ bool skip() const { return false; }
-  __device__ __forceinline__ pre_t load(int i) const { return pre_t{q[i]}; }
-  __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<1>& r) const
-  {
-    sink(i, acc);
-    r.v[0] += p.q * acc;
-  }
-};
-
-// Largest m (constraints) the cluster power iteration takes: its vector steps run pg = m / kBlock
-// emulated block reductions in every block.
-constexpr int kClusterPowerMaxRows = 8192;
-
-// Dynamic shared memory (doubles): z (m_pad), q (m_pad), A^T q (n_pad), the q . z partials of the
-// sweep's ga virtual blocks (ga_pad, a copy in every block), their local staging (ga_pad), and
-// the |z|^2 and residual partials of the pg emulated blocks (pg_pad each, local).
-inline size_t cluster_power_smem(int m, int n, int pg, int ga)
-{
-  auto pad = [](int v) { return (size_t)((v + 15) & ~15); };
-  return (2 * pad(m) + pad(n) + 2 * pad(ga) + 2 * pad(pg)) * sizeof(double);
-}
-
-// ordered_block_sum<1> of nb <= 32 partials, formed by warp 0: each thread's compensated sum of a
-// single partial is that partial, and the block tree's levels above 16 only add zeros, so the
-// warp's shuffle tree of the same pairs gives the same value.  Result in *out for the block.
-__device__ __forceinline__ void small_ordered_sum(const double* p, int nb, double* out)
-{
-  if (threadIdx.x < kWarp) {
-    double v = (int)threadIdx.x < nb ? p[threadIdx.x] : 0.0;
-#pragma unroll
-    for (int h = 16; h > 0; h >>= 1) v += __shfl_down_sync(0xffffffffu, v, h);
-    if (threadIdx.x == 0) *out = v;
-  }
-  __syncthreads();
-}
-
-// Largest emulated block count of the cluster power iteration's vector steps and sums, and the
-// largest number of virtual blocks of one sweep that one block of the cluster takes.
-constexpr int kClusterPowerMaxBlocks = 32;
-constexpr int kClusterPowerMaxOwn    = 16;
-
-// Element range [lo, hi) of virtual block vb (8 warps) of a sweep's matrix: its long rows, or its
-// slices, are contiguous in the matrix's arrays.
-template <typename TX>
-__device__ __forceinline__ void vb_range(const dev_sell<TX>& M, int vb, int64_t& lo, int64_t& hi)
-{
-  const int lb = long_blocks(M.long_count());
-  if (vb < lb) {
-    const int q0 = vb * kWarpsPerBlock, q1 = min(q0 + kWarpsPerBlock, M.long_count());
-    lo           = M.long_off[q0];
-    hi           = M.long_off[q1];
-  } else {
-    const int s0 = (vb - lb) * kWarpsPerBlock, s1 = min(s0 + kWarpsPerBlock, M.slice_count());
-    lo           = M.slice_off[s0];
-    hi           = M.slice_off[s1];
-  }
-}
-
-// With `cache`, each block first copies the values and indices of its own virtual blocks of both
-// sweeps into shared memory after the vectors (each range 16-byte aligned) and reads them there.
-template <typename TX>
-__global__ void __launch_bounds__(kBlock)
-  cluster_power_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, const double* z0, int m, int n,
-                       int pg, int gt, int ga, power_state* ps, double tol, int max_iters,
-                       int cache)
-{
-  extern __shared__ __align__(16) unsigned char cp_smem[];
-  auto pad     = [](int v) { return (v + 15) & ~15; };
-  double* zc   = reinterpret_cast<double*>(cp_smem);
-  double* qc   = zc + pad(m);
-  double* atqc = qc + pad(m);
-  double* sc   = atqc + pad(n);  // q . z partials (every block's copy)
-  double* st   = sc + pad(ga);   // this block's partials before they are sent
-  double* pz   = st + pad(ga);   // |z|^2 partials
-  double* pr   = pz + pad(pg);   // residual partials
-  __shared__ double scalar;
-  const unsigned rank = cluster_rank(), C = cluster_size();
-  const int lane = threadIdx.x & (kWarp - 1), warp = threadIdx.x / kWarp;
-  const dsmem_sink<double> to_z{(unsigned)__cvta_generic_to_shared(zc), C};
-  const dsmem_sink<double> to_atq{(unsigned)__cvta_generic_to_shared(atqc), C};
-  const unsigned sc_addr = (unsigned)__cvta_generic_to_shared(sc);
-
-  for (int i = threadIdx.x; i < m; i += kBlock) zc[i] = z0[i];
-  // The matrix copy: per sweep (0: A^T, 1: A) and own virtual block k, the range's start and the
-  // byte offsets of its values and indices in the copy.
-  __shared__ long long own_lo[2][kClusterPowerMaxOwn];
-  __shared__ unsigned own_val[2][kClusterPowerMaxOwn], own_idx[2][kClusterPowerMaxOwn];
-  unsigned char* mat = reinterpret_cast<unsigned char*>(pr + pad(pg));
-  if (cache) {
-    unsigned used = 0;
-    for (int w = 0; w < 2; ++w) {
-      const dev_sell<TX>& M = w == 0 ? AT : A;
-      const int g           = w == 0 ? gt : ga;
-      int k                 = 0;
-      for (int vb = (int)rank; vb < g; vb += (int)C, ++k) {
-        int64_t lo, hi;
-        vb_range(M, vb, lo, hi);
-        const unsigned vbytes = (unsigned)(((hi - lo) * (int64_t)sizeof(TX) + 15) & ~15);
-        const unsigned ibytes = (unsigned)(((hi - lo) * (int64_t)sizeof(int) + 15) & ~15);
-        TX* dv                = reinterpret_cast<TX*>(mat + used);
-        int* di               = reinterpret_cast<int*>(mat + used + vbytes);
-        for (int64_t e = lo + threadIdx.x; e < hi; e += kBlock) {
-          dv[e - lo] = M.val[e];
-          di[e - lo] = M.idx[e];
-        }
-        if (threadIdx.x == 0) {
-          own_lo[w][k]  = lo;
-          own_val[w][k] = used;
-          own_idx[w][k] = used + vbytes;
-        }
-        used += vbytes + ibytes;
-      }
-    }
-  }
-  __syncthreads();
-  // Sweep w's virtual block vb (the k-th of this block) from the copy or from global memory.
-  auto sweep = [&](int w, int vb, int k, const double* gv, auto epi, double* partials) {
-    const dev_sell<TX>& M = w == 0 ? AT : A;
-    if (cache) {
-      dev_sell<TX> V = M;
-      V.val          = reinterpret_cast<const TX*>(mat + own_val[w][k]);
-      V.idx          = reinterpret_cast<const int*>(mat + own_idx[w][k]);
-      sell_map_block<TX, double, decltype(epi), false, kWarpsPerBlock, shared_matrix>(
-        V, gv, epi, partials, vb, shared_matrix{own_lo[w][k]});
-    } else {
-      sell_map_block<TX, double, decltype(epi)>(M, gv, epi, partials, vb);
-    }
-  };
-  // An emulated block's partial is formed by one warp: for each of the block's 8 warps w, the
-  // warp's lanes take the sums of threads 32 w + lane, warp_sum pairs them as warp w's own
-  // warp_sum would, and the 8 results are added in order from 0.0 (block_reduce_store's two
-  // stages).  Warp k of this block forms the partials of emulated blocks k, k + 8, ...
-  // |z|^2 partials of the pg emulated blocks (vec_reduce_kernel<0>).
-  auto sumsq = [&]() {
-    for (int b = warp; b < pg; b += kWarpsPerBlock) {
-      double s = 0.0;
-      for (int w = 0; w < kWarpsPerBlock; ++w) {
-        double r = 0.0;
-        for (int i = b * kBlock + w * kWarp + lane; i < m; i += pg * kBlock) {
-          const double v = zc[i];
-          r += v * v;
-        }
-        s += warp_sum(r);
-      }
-      if (lane == 0) pz[b] = s;
-    }
-    __syncthreads();
-  };
-  sumsq();
-  // Every block of the cluster is running before any block stores into another's memory.
-  cluster_barrier();
-  int it = 0, done = 0;
-  double nq = 0.0, s2 = 0.0, resid = 0.0;
-  while (it < max_iters && !done) {
-    // q = z / |z|  (power_normalize_sum_kernel), on the local copies.
-    small_ordered_sum(pz, pg, &scalar);
-    nq = sqrt(scalar);
-    for (int i = threadIdx.x; i < m; i += kBlock) qc[i] = zc[i] / nq;
-    __syncthreads();
-    // A^T q over this block's virtual blocks, entries sent to every copy.
-    for (int vb = (int)rank, k = 0; vb < gt; vb += (int)C, ++k)
-      sweep(0, vb, k, qc, cluster_atq_epi<TX>{to_atq}, nullptr);
-    cluster_barrier();
-    // z = A (A^T q) with the q . z partial of each virtual block, both sent to every copy.
-    for (int vb = (int)rank, k = 0; vb < ga; vb += (int)C, ++k) {
-      sweep(1, vb, k, atqc, cluster_z_epi{to_z, qc}, st);
-      if (threadIdx.x == 0)
-        for (unsigned c = 0; c < C; ++c)
-          dsmem_store(sc_addr + (unsigned)vb * (unsigned)sizeof(double), c, st[vb]);
-    }
-    cluster_barrier();
-    // q <- q (-s2) + z with its squares' partials (power_residual_sum_kernel) and the next |z|^2
-    // partials, then the test of power_check_sum_kernel, all on the local copies.
-    small_ordered_sum(sc, ga, &scalar);
-    s2 = scalar;
-    for (int b = warp; b < pg; b += kWarpsPerBlock) {
-      double sr = 0.0, sz = 0.0;
-      for (int w = 0; w < kWarpsPerBlock; ++w) {
-        double rr = 0.0, rz = 0.0;
-        for (int i = b * kBlock + w * kWarp + lane; i < m; i += pg * kBlock) {
-          const double zi = zc[i];
-          const double v  = qc[i] * -s2 + zi;
-          qc[i]           = v;
-          rr += v * v;
-          rz += zi * zi;
-        }
-        sr += warp_sum(rr);
-        sz += warp_sum(rz);
-      }
-      if (lane == 0) {
-        pr[b] = sr;
-        pz[b] = sz;
-      }
-    }
-    __syncthreads();
-    small_ordered_sum(pr, pg, &scalar);
-    resid = sqrt(scalar);
-    ++it;
-    done = resid < tol;
-  }
-  if (rank == 0 && threadIdx.x == 0) {
-    ps->norm_z = nq;
-    ps->s2     = s2;
-    ps->resid  = resid;
-    ps->iters  = it;
-    ps->done   = done;
-  }
-  // No block leaves while another may still store into its shared memory.
-  cluster_barrier();
-}
-
-
-// Golub-Kahan-Lanczos bidiagonalisation of the scaled A (the mixed-precision step size).  The
-// vectors are stored unnormalised; gk_state holds their norms: u has norm beta (beta_k), v has
-// norm alpha (alpha_{k-1}, or 0 before the first step).
+// Golub-Kahan-Lanczos bidiagonalisation of the scaled A (the step size).  The vectors are stored
+// unnormalised; gk_state holds their norms: u has norm beta (beta_k), v has norm alpha
+// (alpha_{k-1}, or 0 before the first step), the steps done, and the blocks of the running sweep
+// that have finished.
 struct gk_state {
   double beta;
   double alpha;
+  int step;
+  unsigned arrived;
 };
 
 // Row j of A^T applied to u:  p_j = (A^T u)_j / beta - beta v_j / alpha  (written over v_j).
@@ -1355,17 +976,46 @@ struct gk_dual_epi {
   }
 };
 
-// Records a new norm: FIELD 0 sets alpha (history alphas[k]), FIELD 1 sets beta (betas[k + 1]).
-template <int FIELD>
-static __global__ void gk_record_kernel(gk_state* st, const double* sumsq, double* hist, int k)
+// The norm |z0| that the recurrence starts from: beta and the first entry of its history.
+static __global__ void gk_start_kernel(gk_state* st, const double* sumsq, double* betas)
 {
-  const double v = sqrt(*sumsq);
-  if (FIELD == 0) {
-    st->alpha = v;
-    hist[k]   = v;
-  } else {
-    st->beta    = v;
-    hist[k + 1] = v;
+  st->beta = betas[0] = sqrt(*sumsq);
+}
+
+// One half step: the sweep with its fused recurrence, and the norm of the new vector, which the
+// block that finishes last sums from the block partials (in the order of finalize_sum_kernel).
+// FIELD 0 (rows of A^T) records alpha of the step, FIELD 1 (rows of A) beta, and moves the step on.
+// A step is two launches; with the sum and its recording as kernels of their own it was six, and
+// on a 12k x 30k LP those four one-block kernels were the larger part of it.
+template <int FIELD, typename TM, class Epi>
+__global__ void __launch_bounds__(kBlock) gk_sweep_kernel(const dev_sell<TM> A,
+                                                          const double* __restrict__ g, Epi epi,
+                                                          double* partials, gk_state* st,
+                                                          double* hist)
+{
+  sell_map_block(A, g, epi, partials, (int)blockIdx.x);
+  __shared__ int last;
+  if (threadIdx.x == 0) {  // the thread that wrote this block's partial
+    __threadfence();
+    last = atomicAdd(&st->arrived, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double total;
+  ordered_block_sum<1, true>(partials, (int)gridDim.x, &total);
+  if (threadIdx.x == 0) {
+    const double v = sqrt(total);
+    const int k    = st->step;
+    if (FIELD == 0) {
+      st->alpha = v;
+      hist[k]   = v;
+    } else {
+      st->beta    = v;
+      hist[k + 1] = v;
+      st->step    = k + 1;
+    }
+    st->arrived = 0;
   }
 }
 

@@ -426,172 +426,19 @@ class engine {
     return hres_[0];
   }
 
+  // Step size from the reference's power iteration (start vector std::mt19937(1) normals in the
+  // user's constraint order, pdlp.cu:2632-2638), carried out in the Krylov space of its start
+  // vector: krylov_power_iteration on the Golub-Kahan coefficients.  Every product with A and
+  // its transpose counts, and it needs about a tenth of them: on a 200k x 500k LP (FP64) the step
+  // size took 243 ms with the iteration itself.
   void power_iteration()
   {
-    const int m = in_.m, n = in_.n;
-    // Start vector: std::mt19937(1) normals in the user's constraint order (pdlp.cu:2632-2638).
-    const auto seq          = power_start_sequence(m);
-    const std::vector<double>& z0 = *seq;
-    dbuf<double> dz(m), dq(m), datq(n);
-    dbuf<power_state> ps(1);
-    ps.zero(s_);
-    dq.upload(z0.data(), m, s_);
-    permute_gather(dq.data(), L_.row_new2old.data(), m, 1.0, dz.data(), s_);
-    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    dbuf<TX> q_tx, atq_tx;
-    const auto As  = view_of<TX>(L_.A, As_.data());
-    const auto ATs = view_of<TX>(L_.AT, ATs_.data());
-    const int ga = sell_grid(As), gt = sell_grid(ATs);
-    // Block partials: |z|^2 and q . z in the first half of partials_ (the second overwrites the
-    // first once it is consumed), the residual's in the second half.
-    double* part   = partials_.data();
-    double* part_r = partials_.data() + partials_.size() / 2;
-    // The vector steps run on a grid sized to the m entries (at most vgrid_ blocks): small LPs
-    // launch a few blocks instead of vgrid_ mostly idle ones.
-    const int pg = std::max(1, std::min(vgrid_, ceil_div(m, kBlock)));
-    if (cluster_power(As, ATs, dz.data(), ps.data(), pg, ga, gt)) return;
-    auto one_iteration = [&]() {
-      vec_reduce_kernel<0, double><<<pg, kBlock, 0, s_>>>(dz.data(), nullptr, m, part,
-                                                          &ps.data()->done);
-      power_normalize_sum_kernel<<<pg, kBlock, 0, s_>>>(dz.data(), dq.data(), m, part, pg,
-                                                        ps.data());
-      sell_map_kernel<TX, double, store_epi<double>><<<gt, kBlock, 0, s_>>>(
-        ATs, dq.data(), store_epi<double>{datq.data(), &ps.data()->done}, part);
-      sell_map_kernel<TX, double, power_z_epi><<<ga, kBlock, 0, s_>>>(
-        As, datq.data(), power_z_epi{dz.data(), dq.data(), &ps.data()->done}, part);
-      power_residual_sum_kernel<<<pg, kBlock, 0, s_>>>(dq.data(), dz.data(), m, part, ga,
-                                                       ps.data(), part_r);
-      power_check_sum_kernel<<<1, kBlock, 0, s_>>>(ps.data(), part, ga, part_r, pg, kPowerTol);
-    };
-    // Chunks of 32 iterations are captured once into a graph and replayed until convergence.
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-    B200_CUDA_CHECK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
-    for (int i = 0; i < 32; ++i) one_iteration();
-    B200_CUDA_CHECK(cudaStreamEndCapture(s_, &graph));
-    B200_CUDA_CHECK(cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
-    power_state h{};
-    for (int done_iters = 0; done_iters < kPowerMaxIters; done_iters += 32) {
-      if (kPowerMaxIters - done_iters < 32) {
-        for (int i = 0; i < kPowerMaxIters - done_iters; ++i) one_iteration();
-      } else {
-        B200_CUDA_CHECK(cudaGraphLaunch(exec, s_));
-      }
-      launches_ += 6.0 * std::min(32, kPowerMaxIters - done_iters);
-      B200_CUDA_CHECK(cudaMemcpyAsync(&h, ps.data(), sizeof(h), cudaMemcpyDeviceToHost, s_));
-      B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      if (h.done) break;
-    }
-    cudaGraphExecDestroy(exec);
-    power_iters_ = h.iters;
-    eta_         = kStepScaling / std::sqrt(h.s2);
-  }
-
-  // Small LPs (at most kClusterPowerNnz non-zeros and kClusterPowerMaxRows rows, z, q and A^T q
-  // within one block's shared memory, and unless CUDA graphs are asked for with
-  // pdlp_persistent_iterations = 0): the whole power iteration in one launch of
-  // cluster_power_kernel, which forms every sum as the multi-kernel form does (same step size bit
-  // for bit) with two cluster barriers per step in place of six kernel boundaries.  Returns false
-  // where it does not apply.
-  static constexpr int64_t kClusterPowerNnz = 262144;
-  bool cluster_power(const dev_sell<TX>& As, const dev_sell<TX>& ATs, const double* z0,
-                     power_state* ps, int pg, int ga, int gt)
-  {
-    if (p_.persistent == 0 || L_.nnz > kClusterPowerNnz || in_.m > kClusterPowerMaxRows ||
-        pg > kClusterPowerMaxBlocks || ga > kClusterPowerMaxBlocks)
-      return false;
-    int dev = 0, optin = 0;
-    B200_CUDA_CHECK(cudaGetDevice(&dev));
-    B200_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    const size_t vec_smem = cluster_power_smem(in_.m, in_.n, pg, ga);
-    const size_t limit = max_dynamic_smem((const void*)cluster_power_kernel<TX>);
-    if (vec_smem > limit) return false;
-    // Shared memory a block needs to hold its own virtual blocks of both sweeps (cluster size c).
-    auto ranges = [&](const dev_matrix& M) {
-      std::vector<int64_t> lo(M.n_long + 1), so(M.n_slices + 1);
-      B200_CUDA_CHECK(cudaMemcpyAsync(lo.data(), M.long_off.data(), lo.size() * sizeof(int64_t),
-                                      cudaMemcpyDeviceToHost, s_));
-      B200_CUDA_CHECK(cudaMemcpyAsync(so.data(), M.slice_off.data(),
-                                      so.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s_));
-      B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      std::vector<int64_t> count;  // elements of each virtual block
-      const int lb = long_blocks(M.n_long);
-      for (int vb = 0; vb < lb; ++vb)
-        count.push_back(lo[std::min((vb + 1) * kWarpsPerBlock, M.n_long)] - lo[vb * kWarpsPerBlock]);
-      for (int s0 = 0; s0 < M.n_slices; s0 += kWarpsPerBlock)
-        count.push_back(so[std::min(s0 + kWarpsPerBlock, M.n_slices)] - so[s0]);
-      return count;
-    };
-    const std::vector<int64_t> cnt_t = ranges(L_.AT), cnt_a = ranges(L_.A);
-    auto copy_smem = [&](int c) -> size_t {
-      size_t worst = 0;
-      for (int r = 0; r < c; ++r) {
-        size_t bytes = 0;
-        int own      = 0;
-        for (const auto* cnt : {&cnt_t, &cnt_a}) {
-          int k = 0;
-          for (size_t vb = r; vb < cnt->size(); vb += c, ++k)
-            bytes += (((*cnt)[vb] * sizeof(TX) + 15) & ~size_t(15)) +
-                     (((*cnt)[vb] * sizeof(int) + 15) & ~size_t(15));
-          own = std::max(own, k);
-        }
-        if (own > kClusterPowerMaxOwn) return SIZE_MAX;
-        worst = std::max(worst, bytes);
-      }
-      return worst;
-    };
-    const void* fn = (const void*)cluster_power_kernel<TX>;
-    int blocks = 0, cache = 0;
-    size_t smem = vec_smem;
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    // 16 blocks where the device allows clusters of that size, else the portable 8; the matrix
-    // copy where it fits beside the vectors.
-    for (int c : {16, 8}) {
-      if (c > 8)
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess) {
-          (void)cudaGetLastError();
-          continue;
-        }
-      const size_t mat = copy_smem(c);
-      cache            = mat != SIZE_MAX && vec_smem + mat <= limit;
-      smem             = vec_smem + (cache ? mat : 0);
-      allow_max_dynamic_smem(fn);
-      cfg                      = cudaLaunchConfig_t{};
-      cfg.gridDim              = dim3(c);
-      cfg.blockDim             = dim3(kBlock);
-      cfg.dynamicSmemBytes     = smem;
-      cfg.stream               = s_;
-      attr[0].id               = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = c;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs                = attr;
-      cfg.numAttrs             = 1;
-      int clusters             = 0;
-      if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0) {
-        blocks = c;
-        break;
-      }
-      (void)cudaGetLastError();
-    }
-    if (blocks == 0) return false;
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_power_kernel<TX>, ATs, As, z0, in_.m, in_.n,
-                                       pg, gt, ga, ps, kPowerTol, kPowerMaxIters, cache));
-    ++launches_;
-    power_state h{};
-    B200_CUDA_CHECK(cudaMemcpyAsync(&h, ps, sizeof(h), cudaMemcpyDeviceToHost, s_));
-    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    power_iters_    = h.iters;
-    eta_            = kStepScaling / std::sqrt(h.s2);
-    cluster_blocks_ = blocks;
-    if (std::getenv("CUOPT_B200_TRACE"))
-      std::fprintf(stderr, "[cuopt_b200] cluster power iteration: %d blocks, %zu bytes of shared "
-                           "memory each, matrix copy %s\n",
-                   blocks, smem, cache ? "on" : "off");
-    return true;
+    krylov_power_iteration power;
+    bidiagonalise(kKrylovMaxSteps, [&](int k, const double* a, const double* b) {
+      return power.advance(a, b, k);
+    });
+    power_iters_ = power.iterations();
+    eta_         = kStepScaling / std::sqrt(power.sigma2());
   }
 
   // Largest singular value of the scaled A by Golub-Kahan-Lanczos bidiagonalisation, used in
@@ -601,71 +448,67 @@ class engine {
   // as the power iteration; stops when the estimate changes by less than 1e-10 relative.
   void lanczos_step_size()
   {
+    double sigma2 = 0.0, prev = -1.0;
+    bidiagonalise(kLanczosMaxSteps, [&](int& k, const double* a, const double* b) {
+      bool breakdown = false;
+      int used       = k;
+      for (int j = 0; j < k; ++j)
+        if (!(a[j] > 0.0) || !(b[j] > 0.0) || !std::isfinite(a[j]) || !std::isfinite(b[j])) {
+          used      = j + 1;
+          breakdown = true;
+          break;
+        }
+      sigma2          = largest_bidiagonal_sigma2(a, b, used);
+      const bool done = breakdown ||
+                        (prev > 0.0 && std::fabs(sigma2 - prev) <= kLanczosTol * sigma2);
+      if (done) k = used;
+      power_iters_ = k;
+      prev         = sigma2;
+      return done;
+    });
+    eta_ = kStepScaling / std::sqrt(sigma2);
+  }
+
+  // Golub-Kahan-Lanczos bidiagonalisation from the power iteration's start vector, in chunks of
+  // kLanczosChunk steps, until test(steps, diagonal, subdiagonal) holds or max_steps are done.
+  template <class Test>
+  void bidiagonalise(int max_steps, Test&& test)
+  {
     const int m = in_.m, n = in_.n;
-    const auto seq          = power_start_sequence(m);
+    const auto seq                = power_start_sequence(m);
     const std::vector<double>& z0 = *seq;
-    constexpr int kChunk = kLanczosChunk, kMaxSteps = kLanczosMaxSteps;
-    dbuf<double> u(m), v(n), tmp(m), alphas(kMaxSteps + 1), betas(kMaxSteps + 2);
+    dbuf<double> u(m), v(n), tmp(m), alphas(max_steps + 1), betas(max_steps + 2);
     dbuf<gk_state> st(1);
     tmp.upload(z0.data(), m, s_);
     permute_gather(tmp.data(), L_.row_new2old.data(), m, 1.0, u.data(), s_);
     v.zero(s_);
     st.zero(s_);
-    double beta0 = 0.0;
-    {
-      vec_reduce_kernel<0, double><<<vgrid_, kBlock, 0, s_>>>(u.data(), nullptr, m,
-                                                              partials_.data(), nullptr);
-      finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), vgrid_, dres_.data());
-      gk_record_kernel<1><<<1, 1, 0, s_>>>(st.data(), dres_.data(), betas.data(), -1);
-      launches_ += 3;
-      B200_LAUNCH_CHECK();
-      betas.download(&beta0, 1, s_);
-      B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    }
+    vec_reduce_kernel<0, double><<<vgrid_, kBlock, 0, s_>>>(u.data(), nullptr, m,
+                                                            partials_.data(), nullptr);
+    finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), vgrid_, dres_.data());
+    gk_start_kernel<<<1, 1, 0, s_>>>(st.data(), dres_.data(), betas.data());
+    launches_ += 3;
     const auto As = view_of<TX>(L_.A, As_.data()), ATs = view_of<TX>(L_.AT, ATs_.data());
-    auto step = [&](int k) {
-      sell_map_kernel<TX, double, gk_primal_epi><<<sell_grid(ATs), kBlock, 0, s_>>>(
-        ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data());
-      finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(ATs),
-                                                   dres_.data());
-      gk_record_kernel<0><<<1, 1, 0, s_>>>(st.data(), dres_.data(), alphas.data(), k);
-      sell_map_kernel<TX, double, gk_dual_epi><<<sell_grid(As), kBlock, 0, s_>>>(
-        As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data());
-      finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(As),
-                                                   dres_.data() + 1);
-      gk_record_kernel<1><<<1, 1, 0, s_>>>(st.data(), dres_.data() + 1, betas.data(), k);
-    };
-    std::vector<double> ha(kMaxSteps + 1), hb(kMaxSteps + 2);
-    double sigma2 = 0.0, prev = -1.0;
-    int k = 0;
-    while (k < kMaxSteps) {
-      const int c = std::min(kChunk, kMaxSteps - k);
-      for (int i = 0; i < c; ++i) step(k + i);
-      launches_ += 6.0 * c;
+    std::vector<double> ha(max_steps + 1), hb(max_steps + 2);
+    for (int k = 0; k < max_steps;) {
+      const int c = std::min(kLanczosChunk, max_steps - k);
+      for (int i = 0; i < c; ++i) {
+        gk_sweep_kernel<0, TX, gk_primal_epi><<<sell_grid(ATs), kBlock, 0, s_>>>(
+          ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data(), st.data(),
+          alphas.data());
+        gk_sweep_kernel<1, TX, gk_dual_epi><<<sell_grid(As), kBlock, 0, s_>>>(
+          As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data(), st.data(),
+          betas.data());
+      }
+      launches_ += 2.0 * c;
       B200_LAUNCH_CHECK();
       k += c;
       alphas.download(ha.data(), k, s_);
       betas.download(hb.data(), k + 1, s_);
       B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      // betas[0] holds |z0| (written at index -1 + 1); the recurrence coefficients are betas[1..].
-      bool breakdown = false;
-      int used = k;
-      for (int j = 0; j < k; ++j)
-        if (!(ha[j] > 0.0) || !(hb[j + 1] > 0.0) || !std::isfinite(ha[j]) || !std::isfinite(hb[j + 1])) {
-          used      = j + 1;
-          breakdown = true;
-          break;
-        }
-      sigma2 = largest_bidiagonal_sigma2(ha.data(), hb.data() + 1, used);
-      if (breakdown || (prev > 0.0 && std::fabs(sigma2 - prev) <= kLanczosTol * sigma2)) {
-        k = used;
-        break;
-      }
-      prev = sigma2;
+      // betas[0] holds |z0|; the recurrence coefficients are betas[1..].
+      if (test(k, ha.data(), hb.data() + 1)) break;
     }
-    (void)beta0;
-    power_iters_ = k;
-    eta_         = kStepScaling / std::sqrt(sigma2);
   }
 
   // ------------------------------------------------------------------ iteration kernels
@@ -1574,7 +1417,6 @@ class engine {
   form_key form_key_{};
   double form_us_[3] = {0, 0, 0};  // the timings behind the choice (this solve's or cached)
   size_t cluster_smem_ = 0;         // dynamic shared memory of the cluster form
-  int cluster_blocks_  = 0;         // blocks of the cluster power iteration (0: not used)
   long cluster_launches_ = 0;
   // Warps per block of the plain sweeps and the timings they were chosen by.
   int wpb_primal_ = kWarpsPerBlock, wpb_dual_ = kWarpsPerBlock;
