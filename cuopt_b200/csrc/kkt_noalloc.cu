@@ -3,7 +3,7 @@
 // Computes, for (x, y, reduced costs) of an LP held in device memory in the user's CSR order, the
 // same quantities the solver reports for its own solution (the reference's
 // convergence_information_t::compute_convergence_information, cpp/src/pdlp/termination_strategy/
-// convergence_information.cu:327-489, restated by evaluate_unscaled in pdlp_engine.cu):
+// convergence_information.cu:327-489, restated by term_kernel in kernels.cuh):
 //   l2 primal residual  |A x - clamp(A x, lc, uc)|_2
 //   l2 dual residual    |c - A^T y - rc|_2
 //   primal / dual objective, gap, and the three relative errors.
@@ -14,13 +14,13 @@
 // latency-bound loops (heuristics testing many candidate points) where cudaMalloc / cudaFree would
 // add an implicit device synchronisation on every call.  The solver's own evaluation builds a
 // relabelled matrix layout and per-solve buffers; this variant reads the user's CSR directly and
-// keeps its scratch in fixed-size device globals instead:
-//   g_na_aty      A^T y accumulator, kNaMaxCols doubles (4 MiB): bounds num_variables;
-//                 must be zero before the row pass (cleared by a memset on every call);
-//   g_na_partials per-block partial sums of the two passes, written in full before they are read;
-//   g_na_bad      count of malformed entries (column indices outside [0, n), rows whose offsets
-//                 decrease or start below 0); must be zero before the row pass (cleared on every
-//                 call).
+// keeps its scratch in fixed-size device globals instead (g_na):
+//   aty           A^T y accumulator, kNaMaxCols doubles (4 MiB): bounds num_variables; must be zero
+//                 before the row pass (cleared on every call);
+//   partials      per-block partial sums of the two passes, written in full before they are read;
+//   bad, arrived  count of malformed entries (column indices outside [0, n), rows whose offsets
+//                 decrease or start below 0), and the blocks of the column pass that have
+//                 finished; zero before the row pass (cleared on every call).
 // Because the scratch is one static copy per device, calls that overlap in time on the same
 // device (different streams or host threads without ordering between them) race on it and give
 // wrong results; callers must order them.  A^T y is accumulated with double-precision atomics, so
@@ -30,6 +30,8 @@
 // their device memory.
 #include <math_constants.h>
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdio>
 
 #include <cuopt_b200.h>
@@ -39,30 +41,43 @@
 namespace cuopt_b200 {
 namespace {
 
-constexpr int kBlock         = 256;
-constexpr int kWarpsPerBlock = kBlock / kWarp;
-constexpr int kNaMaxCols     = 1 << 19;  // 524,288 columns
-constexpr int kNaBlocks  = 592;      // 148 SMs x 4 resident blocks; fixed so partials fit
+constexpr int kBlock     = 256;
+constexpr int kNaMaxCols = 1 << 19;  // 524,288 columns
+constexpr int kNaBlocks  = 1184;     // 148 SMs x 8 resident blocks of 256 threads
 constexpr int kNaRowRed  = 3;        // row pass: |r_p|^2, dual row term, |b|^2
 constexpr int kNaColRed  = 4;        // column pass: |r_d|^2, c.x, rc.x, |c|^2
+// Small LPs run in one cluster of kNaClusterBlocks blocks: one launch in place of a memset and two
+// kernels (300 x 700: see na_small_kernel).  The line is drawn on m n, which bounds the non-zeros
+// (the host does not know them), so that a dense LP does not end up on 8 SMs with more than 2^20.
+constexpr int kNaClusterBlocks  = 8;
+constexpr int kNaClusterThreads = 1024;
+constexpr int64_t kNaClusterArea = 1 << 20;
 
-static __device__ __align__(256) double g_na_aty[kNaMaxCols];
-static __device__ __align__(256) double g_na_partials[kNaBlocks * (kNaRowRed + kNaColRed)];
-static __device__ __align__(256) unsigned int g_na_bad;
+struct na_globals {
+  unsigned bad, arrived;  // the clear of a call covers these and the first n entries of aty
+  double aty[kNaMaxCols];
+  double partials[kNaBlocks * (kNaRowRed + kNaColRed)];
+};
+static __device__ __align__(256) na_globals g_na;
 
-struct na_scratch {
-  double* aty;
-  double* partials;
-  unsigned int* bad;
+struct na_problem {
+  int m, n;
+  const int* off;
+  const int* idx;
+  const double* val;
+  const double *c, *lo, *up, *x, *y, *rc;
+  double sgn, offset;
+  double* out;
 };
 
 __device__ __forceinline__ double fin0(double v) { return isfinite(v) ? v : 0.0; }
 
-// Block sum of K per-thread values (fixed order); thread q < K writes partials[blockIdx.x*K + q].
-template <int K>
-__device__ __forceinline__ void block_sum_store(const double (&v)[K], double* partials)
+// Block sum of K per-thread values (fixed order); thread q < K writes partials[block * K + q].
+template <int K, int THREADS>
+__device__ __forceinline__ void block_sum_store(const double (&v)[K], double* partials, int block)
 {
-  __shared__ double sm[kWarpsPerBlock][K];
+  constexpr int W = THREADS / kWarp;
+  __shared__ double sm[W][K];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < K; ++q) {
@@ -73,119 +88,172 @@ __device__ __forceinline__ void block_sum_store(const double (&v)[K], double* pa
   if (threadIdx.x < K) {
     double t = 0.0;
 #pragma unroll
-    for (int w = 0; w < kWarpsPerBlock; ++w) t += sm[w][threadIdx.x];
-    partials[(size_t)blockIdx.x * K + threadIdx.x] = t;
+    for (int w = 0; w < W; ++w) t += sm[w][threadIdx.x];
+    partials[(size_t)block * K + threadIdx.x] = t;
   }
 }
 
-// Warp per constraint row: A x and the row's residual / dual-objective / |b| terms, and the
-// scatter of y_i A[i, :] into the A^T y accumulator.
-__global__ void __launch_bounds__(kBlock)
-  na_rows_kernel(int m, int n, const int* __restrict__ off, const int* __restrict__ idx,
-                 const double* __restrict__ val, const double* __restrict__ x,
-                 const double* __restrict__ y, const double* __restrict__ lo,
-                 const double* __restrict__ up, double sgn, na_scratch s)
+// G lanes per constraint row: A x and the row's residual / dual-objective / |b| terms, and the
+// scatter of y_i A[i, :] into the A^T y accumulator.  Bound by the L1 request rate (one gather and
+// one reduction per non-zero), so rows shorter than a warp share one: with a whole warp per row of
+// 20 non-zeros 12 of 32 lanes issued nothing.
+template <int G>
+__device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwarps,
+                                        double (&r)[kNaRowRed])
 {
-  double r[kNaRowRed] = {};
-  const int lane = threadIdx.x & 31;
-  const int nw   = gridDim.x * kWarpsPerBlock;
-  for (int i = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); i < m; i += nw) {
-    const int b = off[i], e = off[i + 1];
-    if (b < 0 || e < b) {  // malformed offsets: counted, the row is skipped
-      if (lane == 0) atomicAdd(s.bad, 1u);
-      continue;
-    }
-    const double yi = y[i];
-    double ax       = 0.0;
-    for (int k = b + lane; k < e; k += kWarp) {
-      const int j = idx[k];
-      if ((unsigned)j >= (unsigned)n) {
-        atomicAdd(s.bad, 1u);
-        continue;
+  constexpr int kRows = kWarp / G;  // rows per warp
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
+  for (int i0 = warp0 * kRows; i0 < p.m; i0 += nwarps * kRows) {
+    const int i = i0 + grp;
+    int b = 0, e = 0;
+    double yi = 0.0, l = 0.0, u = 0.0;
+    if (i < p.m) {
+      b  = p.off[i];
+      e  = p.off[i + 1];
+      yi = p.y[i];
+      l  = p.lo[i];
+      u  = p.up[i];
+      if (b < 0 || e < b) {  // malformed offsets: counted, the row's entries are skipped
+        if (sub == 0) atomicAdd(&g_na.bad, 1u);
+        b = e = 0;
+        l = u = CUDART_NAN;  // and it contributes nothing (below)
       }
-      const double a = val[k];
-      ax += a * x[j];
-      atomicAdd(s.aty + j, a * yi);
     }
-    ax = warp_sum(ax);
-    if (lane == 0) {
-      const double l = lo[i], u = up[i];
+    double ax = 0.0;
+#pragma unroll 2
+    for (int k = b + sub; k < e; k += G) {
+      const int j    = p.idx[k];
+      const double a = p.val[k];
+      if ((unsigned)j >= (unsigned)p.n) {
+        atomicAdd(&g_na.bad, 1u);
+      } else {
+        ax += a * p.x[j];
+        atomicAdd(g_na.aty + j, a * yi);
+      }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
+    if (sub == 0 && i < p.m && !(isnan(l) && isnan(u))) {
       const double rp   = ax - fmax(l, fmin(ax, u));
-      const double yint = sgn * yi;  // the dual in minimisation form
+      const double yint = p.sgn * yi;  // the dual in minimisation form
       r[0] += rp * rp;
       r[1] += fmax(yint, 0.0) * fin0(l) + fmin(yint, 0.0) * fin0(u);
       r[2] += ((isfinite(l) && l != u) ? l * l : 0.0) + (isfinite(u) ? u * u : 0.0);
     }
   }
-  block_sum_store<kNaRowRed>(r, s.partials);
+}
+
+// The row pass of block `block` of `nblocks`; the lanes per row follow the mean row length.
+template <int THREADS>
+__device__ __forceinline__ void na_row_pass(const na_problem& p, int block, int nblocks)
+{
+  double r[kNaRowRed] = {};
+  const int warp0 = block * (THREADS / kWarp) + (threadIdx.x >> 5);
+  const int nw    = nblocks * (THREADS / kWarp);
+  const int mean  = p.off[p.m] / p.m;
+  if (mean <= 12)
+    na_rows<4>(p, warp0, nw, r);
+  else if (mean <= 48)
+    na_rows<8>(p, warp0, nw, r);
+  else
+    na_rows<32>(p, warp0, nw, r);
+  block_sum_store<kNaRowRed, THREADS>(r, g_na.partials, block);
 }
 
 // Thread per variable: dual residual and objective terms.
-__global__ void __launch_bounds__(kBlock)
-  na_cols_kernel(int n, const double* __restrict__ c, const double* __restrict__ x,
-                 const double* __restrict__ rc, na_scratch s)
+template <int THREADS>
+__device__ __forceinline__ void na_col_pass(const na_problem& p, int block, int nblocks)
 {
   double r[kNaColRed] = {};
-  for (int j = blockIdx.x * kBlock + threadIdx.x; j < n; j += gridDim.x * kBlock) {
-    const double cj = c[j], xj = x[j], sj = rc[j];
-    const double rd = (cj - s.aty[j]) - sj;
+  for (int j = block * THREADS + threadIdx.x; j < p.n; j += nblocks * THREADS) {
+    const double cj = p.c[j], xj = p.x[j], sj = p.rc[j];
+    const double rd = (cj - __ldcg(g_na.aty + j)) - sj;
     r[0] += rd * rd;
     r[1] += cj * xj;
     r[2] += sj * xj;
     r[3] += cj * cj;
   }
-  block_sum_store<kNaColRed>(r, s.partials + kNaBlocks * kNaRowRed);
+  block_sum_store<kNaColRed, THREADS>(r, g_na.partials + kNaBlocks * kNaRowRed, block);
 }
 
-// One block: ordered, compensated sums over the block partials, then the reported quantities.
-__global__ void __launch_bounds__(kBlock)
-  na_finish_kernel(double sgn, double offset, na_scratch s, double* __restrict__ out)
+// One block: ordered, compensated sums over the block partials (a warp for each quantity), then
+// the reported quantities.  The partials come from other blocks of the launch: read through L2.
+__device__ __forceinline__ void na_finish(const na_problem& p, int row_blocks, int col_blocks)
 {
-  __shared__ double sm[kBlock];
   __shared__ double tot[kNaRowRed + kNaColRed];
-  for (int q = 0; q < kNaRowRed + kNaColRed; ++q) {
-    const bool row_q    = q < kNaRowRed;
-    const int K         = row_q ? kNaRowRed : kNaColRed;
-    const double* base  = row_q ? s.partials : s.partials + kNaBlocks * kNaRowRed;
-    const int qq        = row_q ? q : q - kNaRowRed;
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (q < kNaRowRed + kNaColRed) {
+    const bool row_q   = q < kNaRowRed;
+    const int K        = row_q ? kNaRowRed : kNaColRed;
+    const int nb       = row_q ? row_blocks : col_blocks;
+    const double* base = g_na.partials + (row_q ? q : kNaBlocks * kNaRowRed + q - kNaRowRed);
     ksum acc;
-    for (int b = threadIdx.x; b < kNaBlocks; b += kBlock) acc.add(base[(size_t)b * K + qq]);
-    sm[threadIdx.x] = acc.value();
-    __syncthreads();
-    for (int h = kBlock / 2; h > 0; h >>= 1) {
-      if (threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) tot[q] = sm[0];
-    __syncthreads();
+#pragma unroll 4
+    for (int b = lane; b < nb; b += kWarp) acc.add(__ldcg(base + (size_t)b * K));
+    const double t = warp_sum(acc.value());
+    if (lane == 0) tot[q] = t;
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
     const double rp2 = tot[0], drow = tot[1], b2 = tot[2];
     const double rd2 = tot[3], cx = tot[4], sx = tot[5], c2 = tot[6];
     const double l2p = sqrt(rp2), l2d = sqrt(rd2);
-    const double primal = cx + offset;
-    const double dual   = sgn * (drow + sgn * sx) + offset;
+    const double primal = cx + p.offset;
+    const double dual   = p.sgn * (drow + p.sgn * sx) + p.offset;
     const double gap    = fabs(primal - dual);
-    const unsigned bad  = *s.bad;
+    const unsigned bad  = __ldcg(&g_na.bad);
     const double vals[8] = {l2p, l2d, primal, dual, gap, l2p / (1.0 + sqrt(b2)),
                             l2d / (1.0 + sqrt(c2)), gap / (1.0 + fabs(primal) + fabs(dual))};
-    for (int q = 0; q < 8; ++q) out[q] = bad ? CUDART_NAN : vals[q];
-    out[8] = (double)bad;
+    for (int k = 0; k < 8; ++k) p.out[k] = bad ? CUDART_NAN : vals[k];
+    p.out[8] = (double)bad;
   }
 }
 
-// Device addresses of the static scratch on the current device.  Looked up on every call (a host
-// query that allocates nothing), so that a device reset or a new primary context, after which the
-// module is loaded again at new addresses, never leaves a stale address behind.
-bool scratch_for_current_device(na_scratch& out, int& dev)
+__global__ void __launch_bounds__(kBlock) na_rows_kernel(const na_problem p)
 {
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  na_scratch s{};
-  if (cudaGetSymbolAddress((void**)&s.aty, g_na_aty) != cudaSuccess) return false;
-  if (cudaGetSymbolAddress((void**)&s.partials, g_na_partials) != cudaSuccess) return false;
-  if (cudaGetSymbolAddress((void**)&s.bad, g_na_bad) != cudaSuccess) return false;
-  out = s;
-  return true;
+  na_row_pass<kBlock>(p, (int)blockIdx.x, (int)gridDim.x);
+}
+
+// The column pass; the block that finishes last forms the results.
+__global__ void __launch_bounds__(kBlock) na_cols_kernel(const na_problem p, int row_blocks)
+{
+  na_col_pass<kBlock>(p, (int)blockIdx.x, (int)gridDim.x);
+  __shared__ int last;
+  __syncthreads();  // threads 0 .. kNaColRed - 1 wrote the block's partials
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&g_na.arrived, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  na_finish(p, row_blocks, (int)gridDim.x);
+}
+
+// The whole evaluation in one cluster: clear, row pass, column pass, results, a cluster barrier
+// (hardware, no polling) between them.
+__device__ __forceinline__ void na_cluster_barrier()
+{
+  __threadfence();
+  asm volatile(
+    "barrier.cluster.arrive.release;\n"
+    "barrier.cluster.wait.acquire;\n" ::
+      : "memory");
+}
+__global__ void __cluster_dims__(kNaClusterBlocks, 1, 1) __launch_bounds__(kNaClusterThreads)
+  na_small_kernel(const na_problem p)
+{
+  const int block = (int)blockIdx.x;
+  for (int j = block * kNaClusterThreads + threadIdx.x; j < p.n;
+       j += kNaClusterBlocks * kNaClusterThreads)
+    g_na.aty[j] = 0.0;
+  if (block == 0 && threadIdx.x == 0) g_na.bad = 0;
+  na_cluster_barrier();
+  na_row_pass<kNaClusterThreads>(p, block, kNaClusterBlocks);
+  na_cluster_barrier();
+  na_col_pass<kNaClusterThreads>(p, block, kNaClusterBlocks);
+  na_cluster_barrier();
+  if (block == 0) na_finish(p, kNaClusterBlocks, kNaClusterBlocks);
 }
 
 }  // namespace
@@ -209,21 +277,28 @@ extern "C" cuopt_int_t cuOptComputeKKTErrorsNoAlloc(
                  (int)n, kNaMaxCols);
     return CUOPT_INVALID_ARGUMENT;
   }
-  na_scratch s{};
-  int dev = 0;
-  if (!scratch_for_current_device(s, dev)) {
-    std::fprintf(stderr, "cuOptComputeKKTErrorsNoAlloc: scratch lookup failed on device %d\n", dev);
-    return CUOPT_RUNTIME_ERROR;
-  }
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const double sgn      = sense == CUOPT_MAXIMIZE ? -1.0 : 1.0;
-  if (cudaMemsetAsync(s.aty, 0, (size_t)n * sizeof(double), st) != cudaSuccess ||
-      cudaMemsetAsync(s.bad, 0, sizeof(unsigned int), st) != cudaSuccess)
-    return CUOPT_RUNTIME_ERROR;
-  na_rows_kernel<<<kNaBlocks, kBlock, 0, st>>>(m, n, d_off, d_idx, d_val, d_x, d_y, d_lo, d_up, sgn,
-                                               s);
-  na_cols_kernel<<<kNaBlocks, kBlock, 0, st>>>(n, d_c, d_x, d_rc, s);
-  na_finish_kernel<<<1, kBlock, 0, st>>>(sgn, offset, s, d_out);
+  const na_problem p{m, n, d_off, d_idx, d_val, d_c, d_lo, d_up, d_x, d_y, d_rc, sgn, offset, d_out};
+  if ((int64_t)m * n <= kNaClusterArea) {
+    na_small_kernel<<<kNaClusterBlocks, kNaClusterThreads, 0, st>>>(p);
+  } else {
+    // The scratch's address is looked up on every call (a host query that allocates nothing), so
+    // that a device reset or a new primary context, after which the module is loaded again at a
+    // new address, never leaves a stale one behind.
+    void* scratch = nullptr;
+    if (cudaGetSymbolAddress(&scratch, g_na) != cudaSuccess) {
+      std::fprintf(stderr, "cuOptComputeKKTErrorsNoAlloc: scratch lookup failed\n");
+      return CUOPT_RUNTIME_ERROR;
+    }
+    if (cudaMemsetAsync(scratch, 0, offsetof(na_globals, aty) + (size_t)n * sizeof(double), st) !=
+        cudaSuccess)
+      return CUOPT_RUNTIME_ERROR;
+    const int row_blocks = std::min(kNaBlocks, ceil_div(m, kBlock / kWarp));
+    const int col_blocks = std::min(kNaBlocks, ceil_div(n, kBlock));
+    na_rows_kernel<<<row_blocks, kBlock, 0, st>>>(p);
+    na_cols_kernel<<<col_blocks, kBlock, 0, st>>>(p, row_blocks);
+  }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     std::fprintf(stderr, "cuOptComputeKKTErrorsNoAlloc: %s\n", cudaGetErrorString(e));

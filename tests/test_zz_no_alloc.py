@@ -187,3 +187,56 @@ def test_no_alloc_leaves_free_memory_unchanged():
     free_after, _ = torch.cuda.mem_get_info()
     assert free_after == free_before
     _check(st, res)
+
+
+@pytest.mark.parametrize("m,n,length", [
+    (1, 1, 1), (1, 700, 700), (700, 1, 1), (1024, 1024, 5), (1024, 1025, 5),  # around m n = 2^20
+    (3001, 5003, 12), (3001, 5003, 13), (1200, 5003, 48), (1200, 5003, 49),   # lanes per row
+    (37, 900, 900), (9001, 400, 33)])
+def test_no_alloc_sizes_against_numpy(m, n, length):
+    """The evaluation of an arbitrary point at the edges of its forms (one cluster or two kernels,
+    4, 8 or 32 lanes per row) against numpy; a row of every size down to empty, infinite bounds,
+    an equality, and the second call after one on other sizes."""
+    torch = pytest.importorskip("torch")
+    L = lib()
+    rng = np.random.default_rng(m + 7 * n + length)
+    lens = np.full(m, min(length, n))
+    lens[rng.random(m) < 0.1] = 0
+    lens[0] = min(n, length + 40)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    idx = rng.integers(0, n, off[-1]).astype(np.int32)
+    val = rng.standard_normal(off[-1])
+    x, rc, c = (rng.standard_normal(n) for _ in range(3))
+    y = rng.standard_normal(m)
+    lo = np.where(rng.random(m) < 0.3, -np.inf, rng.standard_normal(m))
+    up = np.where(rng.random(m) < 0.3, np.inf, np.where(np.isfinite(lo), lo, 0.0) + 0.5)
+    up[m // 2] = lo[m // 2] = 0.25
+    rows = np.repeat(np.arange(m), lens)
+    ax = np.bincount(rows, weights=val * x[idx], minlength=m)
+    aty = np.bincount(idx, weights=val * y[rows], minlength=n)
+    fin = lambda v: np.where(np.isfinite(v), v, 0.0)
+    b2 = (np.where(lo != up, fin(lo), 0.0) ** 2).sum() + (fin(up) ** 2).sum()
+    l2p, l2d = (np.linalg.norm(v) for v in (ax - np.clip(ax, lo, up), c - aty - rc))
+    primal = c @ x + 2.5
+    dual = np.maximum(y, 0) @ fin(lo) + np.minimum(y, 0) @ fin(up) + rc @ x + 2.5
+    gap = abs(primal - dual)
+    want = [l2p, l2d, primal, dual, gap, l2p / (1 + np.sqrt(b2)), l2d / (1 + np.linalg.norm(c)),
+            gap / (1 + abs(primal) + abs(dual))]
+    t = lambda a, dt=torch.float64: torch.as_tensor(a, device="cuda", dtype=dt)
+    d = {"c": t(c), "off": t(off, torch.int32), "idx": t(idx, torch.int32), "val": t(val),
+         "lo": t(lo), "up": t(up), "x": t(x), "y": t(y), "rc": t(rc)}
+    lp = type("Sizes", (), {"m": m, "n": n})
+    for _ in range(2):
+        code, got = _no_alloc(L, torch, d, lp, 1, 2.5)
+        assert code == 0 and got[8] == 0
+        # Sums of at most a million terms of order 1 in FP64; the objectives are sums with
+        # cancellation, so they are held relative to the size of their terms.
+        size = 1 + np.abs(c * x).sum() + np.abs(rc * x).sum() + np.abs(y * fin(lo)).sum() + \
+            np.abs(y * fin(up)).sum()
+        for q in (0, 1, 5, 6):
+            assert abs(got[q] - want[q]) <= 1e-12 * (1 + abs(want[q]))
+        for q in (2, 3, 4, 7):
+            assert abs(got[q] - want[q]) <= 1e-13 * size
+    other = {**d, "off": t([0] * (m + 1), torch.int32)}
+    code, got = _no_alloc(L, torch, other, lp, 1, 0.0)  # no entries: A x = 0, A^T y = 0
+    assert code == 0 and abs(got[1] - np.linalg.norm(c - rc)) <= 1e-12 * (1 + got[1])
