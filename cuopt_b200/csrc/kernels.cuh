@@ -854,6 +854,44 @@ struct term_dual_epi {
   }
 };
 
+// Both termination sweeps in one launch (blocks [0, gp) the rows of A, the others the rows of A^T),
+// and their sums by the block that finishes last, in finalize_sum_kernel's order, written to device
+// memory and to the pinned host buffer that the host reads once the launch's event has completed
+// (with the two error flags behind them, see enqueue_conv).  As two sweeps, two one-block sums and
+// a copy this took five stream operations per check; on a 2000 x 5000 LP they were the longer part
+// of it.  arrived must be 0 before the launch and is 0 after it.
+static __global__ void __launch_bounds__(kBlock)
+  term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
+              const double* __restrict__ yu, term_primal_epi ep, term_dual_epi ed, int gp, int gd,
+              double* partials, unsigned* arrived, double* out, double* host, const int* flag_a,
+              const int* flag_b)
+{
+  double* part_d = partials + 2 * (size_t)gp;
+  if ((int)blockIdx.x < gp)
+    sell_map_block(A, xu, ep, partials, (int)blockIdx.x);
+  else
+    sell_map_block(AT, yu, ed, part_d, (int)blockIdx.x - gp);
+  __shared__ int last;
+  __syncthreads();  // threads 0 .. 2 wrote the block's partials
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double sums[5];
+  ordered_block_sum<2, true>(partials, gp, sums);
+  ordered_block_sum<3, true>(part_d, gd, sums + 2);
+  if (threadIdx.x < 5) out[threadIdx.x] = host[threadIdx.x] = sums[threadIdx.x];
+  if (threadIdx.x == 0) {
+    int* flags = reinterpret_cast<int*>(host + 8);
+    flags[0]   = *flag_a;
+    flags[1]   = flag_b ? *flag_b : 0;
+    *arrived   = 0;
+  }
+}
+
 // Per-constraint forms of the residuals (per_constraint_residual; reference
 // convergence_information.cu:390-420, 453-470 with relative_residual_t, utils.cuh:578-590):
 // max(0, max_i r_p,i - rel * max(|l_i|, |u_i|) over the finite bounds (combine_finite_abs_bounds,

@@ -120,10 +120,20 @@ class engine {
     B200_CUDA_CHECK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
     configure_pool_once();
     hres_ = pinned_scratch();
+    B200_CUDA_CHECK(cudaStreamCreateWithFlags(&es_, cudaStreamNonBlocking));
+    B200_CUDA_CHECK(cudaEventCreateWithFlags(&kept_, cudaEventDisableTiming));
+    B200_CUDA_CHECK(cudaEventCreateWithFlags(&checked_, cudaEventDisableTiming));
   }
+  engine(const engine&)            = delete;
+  engine& operator=(const engine&) = delete;
   ~engine()
   {
+    // A check may still read buffers that are released, in the order of s_, after this.
+    if (es_) cudaStreamSynchronize(es_);
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
+    if (kept_) cudaEventDestroy(kept_);
+    if (checked_) cudaEventDestroy(checked_);
+    if (es_) cudaStreamDestroy(es_);
   }
 
   // Setup only (layout, scaling, step size): the base of a climber batch.
@@ -192,6 +202,7 @@ class engine {
     const int g = std::max({sell_grid(view64(L_.A)), sell_grid(view64(L_.AT)), vgrid_});
     partials_.resize((size_t)g * 4);
     dres_.resize(64);
+    prepare_checks();
 
     // Unscaled vectors in internal order; objective negated for maximisation
     // (reference problem_helpers.cuh:132-151).
@@ -265,6 +276,14 @@ class engine {
     init_plain_form();
   }
 
+  void prepare_checks()
+  {
+    tpartials_.resize(2 * (size_t)sell_grid(view64(L_.A)) + 3 * (size_t)sell_grid(view64(L_.AT)));
+    tres_.resize(8);
+    tarrived_.resize(1);
+    tarrived_.zero(s_);
+  }
+
   // Takes the precision-independent state of another engine over (see continue_from).
   template <typename TM>
   void adopt(engine<TM>& o)
@@ -297,6 +316,7 @@ class engine {
     restarts_    = o.restarts_;
     launches_    = o.launches_;
     sched_       = o.sched_;
+    prepare_checks();
     // Scaled matrices and vectors in FP64, from the unscaled data and the shared scaling.
     As_.resize(L_.A.stored());
     ATs_.resize(L_.AT.stored());
@@ -984,69 +1004,57 @@ class engine {
   }
 
   // ------------------------------------------------------------------ termination
-  conv_info evaluate()
+  // A termination check runs on its own stream beside the plain iterations that follow the step it
+  // looks at: it reads x_hat, y_hat and the slack, which only the next step that keeps them
+  // overwrites, and that step is not launched before the check's results are in (resolve).
+  void post_check()
   {
     const int m = in_.m, n = in_.n;
-    unscale_kernel<TX><<<vgrid_, kBlock, 0, s_>>>(xhat_.data(), yhat_.data(), slack_.data(),
-                                                  dc_.data(), dr_.data(), 1.0 / beta_,
-                                                  1.0 / gamma_, n, m, xu_.data(), yu_.data(),
-                                                  su_.data());
+    B200_CUDA_CHECK(cudaStreamWaitEvent(es_, kept_, 0));
+    unscale_kernel<TX><<<std::min(vgrid_, ceil_div((long)n + m, kBlock)), kBlock, 0, es_>>>(
+      xhat_.data(), yhat_.data(), slack_.data(), dc_.data(), dr_.data(), 1.0 / beta_, 1.0 / gamma_,
+      n, m, xu_.data(), yu_.data(), su_.data());
     ++launches_;
-    return evaluate_unscaled();
-  }
-
-  // Residuals and objectives of (xu_, yu_, su_) on the unscaled problem (c64_, lc64_, uc64_).
-  conv_info evaluate_unscaled()
-  {
     enqueue_conv(hres_);
-    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
+    B200_CUDA_CHECK(cudaEventRecord(checked_, es_));
+  }
+  conv_info wait_check()
+  {
+    B200_CUDA_CHECK(cudaEventSynchronize(checked_));
     collect_form_timing();
     return read_conv(hres_);
   }
 
-  // The kernels of a termination check on (xu_, yu_, su_) and the copy of their results to the
-  // pinned host buffer h: h[0..6] the sums, h[8] two error flags (the persistent kernel's barrier
-  // status and the tiled sweeps' bounded-wait flag).
+  // The kernels of a termination check on (xu_, yu_, su_), which leave their results in the pinned
+  // host buffer h: h[0..6] the sums, h[8] two error flags (the persistent kernel's barrier status
+  // and the tiled sweeps' bounded-wait flag).
   void enqueue_conv(double* h)
   {
     const auto A = view64(L_.A), AT = view64(L_.AT);
-    sell_map_kernel<double, double, term_primal_epi><<<sell_grid(A), kBlock, 0, s_>>>(
-      A, xu_.data(), term_primal_epi{lc64_.data(), uc64_.data(), yu_.data()}, partials_.data());
-    finalize_sum_kernel<2><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(A), dres_.data());
-    sell_map_kernel<double, double, term_dual_epi><<<sell_grid(AT), kBlock, 0, s_>>>(
-      AT, yu_.data(), term_dual_epi{c64_.data(), xu_.data(), su_.data()}, partials_.data());
-    finalize_sum_kernel<3><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(AT),
-                                                 dres_.data() + 2);
-    launches_ += 4;
-    int nres = 5;
+    const int gp = sell_grid(A), gd = sell_grid(AT);
+    term_kernel<<<gp + gd, kBlock, 0, es_>>>(
+      A, AT, xu_.data(), yu_.data(), term_primal_epi{lc64_.data(), uc64_.data(), yu_.data()},
+      term_dual_epi{c64_.data(), xu_.data(), su_.data()}, gp, gd, tpartials_.data(),
+      tarrived_.data(), tres_.data(), h, &pctl_.data()->status,
+      tile_primal_ || tile_dual_ ? terr_.data() : nullptr);
+    ++launches_;
     if (p_.per_constraint_residual) {
-      sell_map_kernel<double, double, term_linf_primal_epi><<<sell_grid(A), kBlock, 0, s_>>>(
+      sell_map_kernel<double, double, term_linf_primal_epi><<<gp, kBlock, 0, es_>>>(
         A, xu_.data(), term_linf_primal_epi{lc64_.data(), uc64_.data(), p_.rel_primal},
-        partials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(A),
-                                                   dres_.data() + 5);
-      sell_map_kernel<double, double, term_linf_dual_epi><<<sell_grid(AT), kBlock, 0, s_>>>(
+        tpartials_.data());
+      finalize_max_kernel<1><<<1, kBlock, 0, es_>>>(tpartials_.data(), gp, tres_.data() + 5);
+      sell_map_kernel<double, double, term_linf_dual_epi><<<gd, kBlock, 0, es_>>>(
         AT, yu_.data(), term_linf_dual_epi{c64_.data(), su_.data(), p_.rel_dual},
-        partials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(AT),
-                                                   dres_.data() + 6);
+        tpartials_.data());
+      finalize_max_kernel<1><<<1, kBlock, 0, es_>>>(tpartials_.data(), gd, tres_.data() + 6);
       launches_ += 4;
-      nres = 7;
+      B200_CUDA_CHECK(cudaMemcpyAsync(h + 5, tres_.data() + 5, 2 * sizeof(double),
+                                      cudaMemcpyDeviceToHost, es_));
     }
     B200_LAUNCH_CHECK();
-    B200_CUDA_CHECK(
-      cudaMemcpyAsync(h, dres_.data(), nres * sizeof(double), cudaMemcpyDeviceToHost, s_));
-    int* flags = reinterpret_cast<int*>(h + 8);
-    flags[0] = flags[1] = 0;
-    if (persist_launches_ > 0)
-      B200_CUDA_CHECK(cudaMemcpyAsync(flags, &pctl_.data()->status, sizeof(int),
-                                      cudaMemcpyDeviceToHost, s_));
-    if ((tile_primal_ || tile_dual_) && terr_.size() > 0)
-      B200_CUDA_CHECK(
-        cudaMemcpyAsync(flags + 1, terr_.data(), sizeof(int), cudaMemcpyDeviceToHost, s_));
   }
 
-  // The check's results from h once the copies have completed.  Throws when a persistent launch's
+  // The check's results from h once its event has completed.  Throws when a persistent launch's
   // barrier or a tiled sweep's panel copy gave up its wait since the solve began.
   conv_info read_conv(const double* h)
   {
@@ -1205,6 +1213,12 @@ class engine {
     double& best_gap   = sched_.best_gap;
     if (sched_.fresh) set_scalars(0);
     sched_.fresh = false;
+    B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
+    // An iteration takes about 9 us plus a gather per non-zero and sweep at 250 G/s, and a check
+    // about 40 us from its launch to the host's decision; the 8 iterations of a run between two
+    // checks are launched in one piece while that wastes little.
+    const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
+    ahead_ = est_us <= 16.0 ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
     const auto A = As_view(), AT = ATs_view();
 
     for (;;) {
@@ -1213,9 +1227,10 @@ class engine {
       bool restarted   = false;
       if (major || cond) {
         close_cycle(k);
-        const conv_info cv = evaluate();
-        const int st       = decide(cv, k);
-        if (st != kKeepGoing) return finish(r, st, cv, k);
+        post_check();
+        posted_ = k;
+        conv_info cv;
+        if ((major || !may_run_ahead(k)) && !resolve(r, cv)) return;
 
         if (major) {
           // should_cupdlpx_restart (reference pdlp_restart_strategy.cu:689-754)
@@ -1282,10 +1297,21 @@ class engine {
           if (is_check(kk) || is_major_step(kk) || ((kk + 1) % kMajor == 0)) break;
           ++R;
         }
+        // With a check outstanding, the first iterations are launched before its results are
+        // waited for, enough of them to cover its latency; when it ends the solve, they go to waste.
+        if (posted_ >= 0) R = std::min(R, ahead_);
         run_plain(R, k);
         k += R;
         since += R;
+        if (posted_ >= 0) {
+          conv_info cv;
+          if (!resolve(r, cv)) return;
+        }
         continue;
+      }
+      if (posted_ >= 0) {
+        conv_info cv;
+        if (!resolve(r, cv)) return;
       }
 
       // A step that keeps x_hat / y_hat / slack (major) and/or measures the fixed-point error.
@@ -1297,6 +1323,7 @@ class engine {
           launch_primal<false, false, true>(0);
           launch_dual<false, false, true>(0);
         }
+        if (mstep) B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
         finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(A),
                                                      dres_.data() + 8);
         // compute_fixed_error (reference pdlp.cu:1749-1857)
@@ -1324,6 +1351,7 @@ class engine {
       } else {
         launch_primal<true, true, false>(0);
         launch_dual<true, true, false>(0);
+        B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
         advance_kernel<<<1, 1, 0, s_>>>(scalars_.data(), 1);
         ++launches_;
         B200_LAUNCH_CHECK();
@@ -1331,6 +1359,28 @@ class engine {
       ++k;
       ++since;
     }
+  }
+
+  // Waits for the outstanding check; false when it ends the loop (r is then filled in).
+  bool resolve(pdlp_result& r, conv_info& cv)
+  {
+    const long k = posted_;
+    posted_      = -1;
+    cv           = wait_check();
+    const int st = decide(cv, k);
+    if (st == kKeepGoing) return true;
+    finish(r, st, cv, k);
+    return false;
+  }
+
+  // Whether iterations may be launched before the results of the check at k are in: not where the
+  // FP64 continuation of a mixed solve, which starts from the iterates of the check that ended it,
+  // may follow.
+  bool may_run_ahead(long k) const
+  {
+    if constexpr (std::is_same_v<TX, float>)
+      return p_.refinement_passes <= 0 && k - sched_.stall_k < kStallWindow;
+    return true;
   }
 
   // Termination decision of the check at iteration k on its results cv (reference
@@ -1384,6 +1434,14 @@ class engine {
   const lp_device_input& in_;
   const pdlp_params& p_;
   cudaStream_t s_ = nullptr;
+  // Termination checks: their stream, the event of the last step that kept x_hat / y_hat / slack,
+  // the event of the last check's end, and the check that has been launched but not read yet.
+  cudaStream_t es_     = nullptr;
+  cudaEvent_t kept_    = nullptr;
+  cudaEvent_t checked_ = nullptr;
+  long posted_         = -1;
+  dbuf<double> tpartials_, tres_;
+  dbuf<unsigned> tarrived_;
   double *x_out_ = nullptr, *y_out_ = nullptr, *rc_out_ = nullptr;
   int sms_ = 148, vgrid_ = 592;
   double* hres_ = nullptr;
@@ -1425,6 +1483,7 @@ class engine {
   double obj_scale_ = 1.0, obj_offset_ = 0.0;
   double c_norm_ = 0, b_norm_ = 0, beta_ = 1, gamma_ = 1;
   loop_state sched_;
+  long ahead_ = 1;  // plain iterations launched before a check's results are waited for
   double eta_ = 0, omega_ = 1, best_omega_ = 1;
   int power_iters_ = 0, restarts_ = 0;
   double launches_ = 0;
