@@ -372,12 +372,12 @@ __global__ void b_halpern_kernel(TX* x, const TX* xbar, const TX* xa, int n, TX*
       const int b = cinst[i];
       if (!active[b]) continue;
       const double w = halpern_weight(sc + b, 0);
-      x[i]           = (TX)(w * (double)xbar[i] + (1.0 - w) * (double)xa[i]);
+      x[i]           = (TX)halpern_mix(w, (double)xbar[i], (double)xa[i]);
     } else {
       const int r = i - n, b = rinst[r];
       if (!active[b]) continue;
       const double w = halpern_weight(sc + b, 0);
-      y[r]           = (TX)(w * (double)ybar[r] + (1.0 - w) * (double)ya[r]);
+      y[r]           = (TX)halpern_mix(w, (double)ybar[r], (double)ya[r]);
     }
   }
 }

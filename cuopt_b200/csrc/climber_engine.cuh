@@ -300,9 +300,9 @@ __global__ void mm_halpern_kernel(double* x, const double* xbar, const double* x
     if (!active[b]) continue;
     const double w = halpern_weight(sc + b, 0);
     if (is_x)
-      x[k] = w * xbar[k] + (1.0 - w) * xa[k];
+      x[k] = halpern_mix(w, xbar[k], xa[k]);
     else
-      y[k] = w * ybar[k] + (1.0 - w) * ya[k];
+      y[k] = halpern_mix(w, ybar[k], ya[k]);
   }
 }
 

@@ -38,6 +38,11 @@ struct dev_sell {
 };
 
 B200_HD inline int long_blocks(int n_long, int wpb = kWarpsPerBlock) { return ceil_div(n_long, wpb); }
+template <typename T>
+__device__ __forceinline__ int sell_grid_device(const dev_sell<T>& a)
+{
+  return long_blocks(a.long_count()) + ceil_div(a.slice_count(), kWarpsPerBlock);
+}
 // Grid of sell_map_kernel (and of the setup kernels, which always see full views).
 template <typename T>
 inline int sell_grid(const dev_sell<T>& a, int wpb = kWarpsPerBlock)
@@ -59,6 +64,13 @@ __device__ __forceinline__ double halpern_weight(const pdlp_scalars* st, int it_
 {
   const double t = (double)(st->t0 + it_off);
   return (t + 1.0) / (t + 2.0);
+}
+
+// The Halpern step w v + (1 - w) anchor, rounded the same way in every form of the iterations (left
+// to the compiler, which of the two products was fused depended on the kernel).
+__device__ __forceinline__ double halpern_mix(double w, double v, double anchor)
+{
+  return fma(w, v, (1.0 - w) * anchor);
 }
 
 template <int K>
@@ -509,7 +521,7 @@ __device__ __forceinline__ void primal_row_step(int j, double acc, const P& p,
   if constexpr (HALPERN) {
     const double w = halpern_weight(st, it_off);
     xbar[j]        = (TX)xb;
-    xout[j]        = (TX)(w * xb + (1.0 - w) * (double)p.xa);
+    xout[j]        = (TX)halpern_mix(w, xb, (double)p.xa);
   } else {
     xbar[j] = (TX)xb;
   }
@@ -531,7 +543,7 @@ __device__ __forceinline__ double dual_row_step(int i, double acc, const P& p,
   const double yb = 2.0 * ny - yi;
   if constexpr (HALPERN) {
     const double w  = halpern_weight(st, it_off);
-    const TX y_next = (TX)(w * yb + (1.0 - w) * (double)p.ya);
+    const TX y_next = (TX)halpern_mix(w, yb, (double)p.ya);
     yout[i]         = y_next;
     sink(i, (double)y_next);
   } else {
@@ -605,15 +617,22 @@ struct dual_epi {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Cluster-resident plain iterations for small LPs: one thread-block cluster of C blocks runs a run
-// of L plain iterations.  Every block keeps a full copy of both gathered vectors (y for the primal
-// sweep, x_bar for the dual sweep) in its shared memory, so the sweeps gather from shared memory;
-// a row's new value is written to global memory by its epilogue, as in the other forms, and
-// stored into every block's copy through distributed shared memory (mapa + st.shared::cluster).
-// A cluster barrier (arrive.release / wait.acquire: hardware, no spin loop) follows every sweep.
-// Every row is computed by one warp exactly as in sell_map_kernel.
-constexpr int kClusterThreads = 1024;
-constexpr int kClusterGroups  = kClusterThreads / kBlock;  // 8-warp groups per block
+// Cluster-resident plain iterations for small LPs: one thread-block cluster of C blocks runs L plain
+// iterations, the last of which may be one that keeps x_hat, y_hat and the slack for a termination
+// check.  Every block holds a full copy of both gathered vectors (y for the primal sweep, x_bar for
+// the dual sweep) in its shared memory and sends each new entry to every block's copy through
+// distributed shared memory (mapa + st.shared::cluster: posted, only the barrier waits for them).  A
+// cluster barrier (arrive.release / wait.acquire: hardware, no spin loop) follows every sweep.
+// Every row is computed by one warp exactly as in sell_map_kernel: same products, same order.
+//
+// With CACHED, each block also keeps its share of A and A^T and its rows' operands and iterates in
+// shared memory (16-bit column indices), so an iteration touches no global memory: what bounds it
+// is the shared-memory requests of the products, the broadcasts and two cluster barriers.  Without
+// (the shares do not fit), the matrices and operands are read from L2 every iteration, as the
+// only form of this kernel once did: its iteration is bound by the latency of those dependent reads
+// (2000 x 5000 LP, FP64: 8.95 us an iteration).
+constexpr int kResidentThreads = 512;
+constexpr int kResidentWarps   = kResidentThreads / kWarp;
 
 __device__ __forceinline__ unsigned cluster_rank()
 {
@@ -629,6 +648,7 @@ __device__ __forceinline__ unsigned cluster_size()
 }
 __device__ __forceinline__ void cluster_barrier()
 {
+  __syncwarp();
   asm volatile(
     "barrier.cluster.arrive.release.aligned;\n"
     "barrier.cluster.wait.acquire.aligned;\n" ::
@@ -649,93 +669,372 @@ __device__ __forceinline__ void dsmem_store(unsigned saddr, unsigned rank, float
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-// Copies a row's new value into every block's shared-memory copy of its vector (base: the
-// shared-memory address of the copy in this block's window).
+// Copies a row's new value into every block's shared-memory copy of its vector (at: the
+// shared-memory address of the entry in this block's copy).
 template <typename TX>
 struct dsmem_sink {
-  unsigned base;
+  unsigned at;
   unsigned blocks;
-  __device__ __forceinline__ void operator()(int r, double v) const
+  __device__ __forceinline__ void operator()(int, double v) const
   {
-    const unsigned target = base + (unsigned)r * (unsigned)sizeof(TX);
-    for (unsigned c = 0; c < blocks; ++c) dsmem_store(target, c, (TX)v);
+    for (unsigned c = 0; c < blocks; ++c) dsmem_store(at, c, (TX)v);
   }
 };
 
-// The plain epilogues (primal_epi / dual_epi with the Halpern step fused) with the new x_bar_j,
-// or y_i, also sent to the cluster's copies.
+// Shares of a matrix: units are its long rows, then its slices; unit u belongs to block u % C as
+// its unit u / C.  Capacities of a block's share: units, and elements (each unit's start is padded
+// to 4, so that chunk loads are aligned).
+struct resident_dims {
+  int blocks = 0;       // C
+  int units[2] = {0, 0};     // A^T, A
+  int elems[2] = {0, 0};
+  B200_HD static size_t pad(size_t b) { return (b + 15) & ~(size_t)15; }
+  // The image of a block's constant data (device memory, copied to shared memory by each launch):
+  // {start, length} of the units of A^T and A, the operands c, l, u and l_c, u_c per unit lane,
+  // values and indices of A^T and A.
+  template <typename TX>
+  B200_HD size_t image_at(int part) const
+  {
+    const size_t bytes[9] = {(size_t)units[0] * 8,
+                             (size_t)units[1] * 8,
+                             (size_t)units[0] * 3 * kWarp * sizeof(TX),
+                             (size_t)units[1] * 2 * kWarp * sizeof(TX),
+                             (size_t)elems[0] * sizeof(TX),
+                             (size_t)elems[1] * sizeof(TX),
+                             (size_t)elems[0] * 2,
+                             (size_t)elems[1] * 2,
+                             0};
+    size_t at = 0;
+    for (int q = 0; q < part; ++q) at += pad(bytes[q]);
+    return at;
+  }
+  template <typename TX>
+  B200_HD size_t image_bytes() const
+  {
+    return image_at<TX>(8);
+  }
+  // Shared memory of a launch: y, x_bar, then (CACHED) the iterates x, x_anchor, y, y_anchor per
+  // unit lane and the image.
+  template <typename TX>
+  B200_HD static size_t vector_bytes(int m, int n)
+  {
+    return pad((size_t)m * sizeof(TX)) + pad((size_t)n * sizeof(TX));
+  }
+  template <typename TX>
+  B200_HD size_t state_bytes() const
+  {
+    return (size_t)(units[0] + units[1]) * 2 * kWarp * sizeof(TX);
+  }
+  template <typename TX>
+  size_t smem(int m, int n) const
+  {
+    return vector_bytes<TX>(m, n) + state_bytes<TX>() + image_bytes<TX>();
+  }
+};
+
 template <typename TX>
+__device__ __forceinline__ void unit_range(const dev_sell<TX>& M, int u, int64_t& lo, int64_t& hi)
+{
+  if (u < M.n_long) {
+    lo = M.long_off[u];
+    hi = M.long_off[u + 1];
+  } else {
+    lo = M.slice_off[u - M.n_long];
+    hi = M.slice_off[u - M.n_long + 1];
+  }
+}
+
+// Builds the image of block blockIdx.x (once per solve).
+template <typename TX>
+__global__ void __launch_bounds__(kResidentThreads)
+  resident_image_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, const TX* c, const TX* lo,
+                        const TX* up, const TX* lc, const TX* uc, resident_dims D,
+                        unsigned char* images)
+{
+  unsigned char* img = images + blockIdx.x * D.image_bytes<TX>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int w = 0; w < 2; ++w) {
+    const dev_sell<TX>& M = w == 0 ? AT : A;
+    const int total       = M.n_long + M.n_slices;
+    int2* table           = reinterpret_cast<int2*>(img + D.image_at<TX>(w));
+    if (threadIdx.x == 0) {
+      int at = 0;
+      for (int i = 0; i < D.units[w]; ++i) {
+        const int u = (int)blockIdx.x + D.blocks * i;
+        int64_t b = 0, e = 0;
+        if (u < total) unit_range(M, u, b, e);
+        table[i] = make_int2(at, (int)(e - b));
+        at += ((int)(e - b) + 3) & ~3;
+      }
+    }
+    __syncthreads();
+    TX* ops           = reinterpret_cast<TX*>(img + D.image_at<TX>(2 + w));
+    TX* val           = reinterpret_cast<TX*>(img + D.image_at<TX>(4 + w));
+    unsigned short* x = reinterpret_cast<unsigned short*>(img + D.image_at<TX>(6 + w));
+    const int slots   = D.units[w] * kWarp;
+    for (int i = warp; i < D.units[w]; i += kResidentWarps) {
+      const int u  = (int)blockIdx.x + D.blocks * i;
+      const int2 t = table[i];
+      int row      = -1;
+      if (u < M.n_long) {
+        if (lane == 0) row = u;
+      } else if (u < total) {
+        row = M.n_long + (u - M.n_long) * kWarp + lane;
+        if (row >= M.rows) row = -1;
+      }
+      const int s = i * kWarp + lane;
+      if (w == 0) {
+        ops[s]             = row >= 0 ? c[row] : TX(0);
+        ops[slots + s]     = row >= 0 ? lo[row] : TX(0);
+        ops[2 * slots + s] = row >= 0 ? up[row] : TX(0);
+      } else {
+        ops[s]         = row >= 0 ? lc[row] : TX(0);
+        ops[slots + s] = row >= 0 ? uc[row] : TX(0);
+      }
+      int64_t b = 0, e = 0;
+      if (u < total) unit_range(M, u, b, e);
+      for (int k = lane; k < t.y; k += kWarp) {
+        val[t.x + k] = M.val[b + k];
+        x[t.x + k]   = (unsigned short)M.idx[b + k];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ void shared_chunk(const float* p, double (&v)[4])
+{
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0]           = t.x;
+  v[1]           = t.y;
+  v[2]           = t.z;
+  v[3]           = t.w;
+}
+__device__ __forceinline__ void shared_chunk(const double* p, double (&v)[4])
+{
+  const double2 a = reinterpret_cast<const double2*>(p)[0];
+  const double2 b = reinterpret_cast<const double2*>(p)[1];
+  v[0]            = a.x;
+  v[1]            = a.y;
+  v[2]            = b.x;
+  v[3]            = b.y;
+}
+
+// The product of a slice's row (this lane's) from shared memory, in sell_map_block's order.
+template <typename TX>
+__device__ __forceinline__ double resident_slice(const TX* v, const unsigned short* x, int nchunk,
+                                                 const TX* g)
+{
+  double acc = 0.0;
+#pragma unroll 2
+  for (int q = 0; q < nchunk; ++q) {
+    const ushort4 i = *reinterpret_cast<const ushort4*>(x);
+    double w[4];
+    shared_chunk(v, w);
+    const TX g0 = g[i.x], g1 = g[i.y], g2 = g[i.z], g3 = g[i.w];
+    acc += w[0] * (double)g0;
+    acc += w[1] * (double)g1;
+    acc += w[2] * (double)g2;
+    acc += w[3] * (double)g3;
+    v += kWarp * kChunk;
+    x += kWarp * kChunk;
+  }
+  return acc;
+}
+template <typename TX>
+__device__ __forceinline__ double resident_long(const TX* v, const unsigned short* x, int len,
+                                                const TX* g)
+{
+  double acc = 0.0;
+  for (int k = threadIdx.x & 31; k < len; k += kWarp) acc += (double)v[k] * (double)g[x[k]];
+  return warp_sum(acc);
+}
+
+// The plain epilogues with the new x_bar_j, or y_i, also sent to the cluster's copies.
+template <typename TX, bool MAJOR>
 struct cluster_primal_epi {
   static constexpr int kRed = 0;
   using base_t              = primal_epi<TX, false, true, false>;
   using pre_t               = typename base_t::pre_t;
   base_t base;
-  dsmem_sink<TX> sink;
+  unsigned copy, blocks;
   __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return base.load(j); }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<0>&) const
   {
-    primal_row_step<TX, false, true, false>(j, acc, p, base.st, base.it_off, base.xbar, base.xout,
+    const dsmem_sink<TX> sink{copy + (unsigned)j * (unsigned)sizeof(TX), blocks};
+    primal_row_step<TX, MAJOR, true, false>(j, acc, p, base.st, base.it_off, base.xbar, base.xout,
                                             base.xhat, base.slack, base.aty, sink);
   }
 };
-template <typename TX>
+template <typename TX, bool MAJOR>
 struct cluster_dual_epi {
   static constexpr int kRed = 0;
   using base_t              = dual_epi<TX, false, true, false>;
   using pre_t               = typename base_t::pre_t;
   base_t base;
-  dsmem_sink<TX> sink;
+  unsigned copy, blocks;
   __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const { return base.load(i); }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<0>&) const
   {
-    dual_row_step<TX, false, true>(i, acc, p, base.st, base.it_off, base.ybar, base.yout,
+    const dsmem_sink<TX> sink{copy + (unsigned)i * (unsigned)sizeof(TX), blocks};
+    dual_row_step<TX, MAJOR, true>(i, acc, p, base.st, base.it_off, base.ybar, base.yout,
                                    base.yhat, sink);
   }
 };
 
-// Dynamic shared memory: the copy of y (m elements, padded to 16), then the copy of x_bar (n
-// elements).  pe / de: the plain primal / dual epilogues (it_off set per iteration), whose gathered
-// vectors are y (de.y = de.yout) and x_bar (pe.xbar).  Each block runs kClusterGroups groups of
-// kWarpsPerBlock warps; group g of block `rank` takes the sweep's 8-warp virtual blocks
-// rank + C g, rank + C g + C kClusterGroups, ... (gp / gd of them), so small sweeps spread over
-// every block of the cluster.
-template <typename TX>
-__global__ void __launch_bounds__(kClusterThreads)
-  cluster_plain_kernel(const dev_sell<TX> AT, const dev_sell<TX> A,
-                       primal_epi<TX, false, true, false> pe, dual_epi<TX, false, true, false> de,
-                       int L, int m, int gp, int gd, pdlp_scalars* st)
+// L plain iterations, the last one a keeping one when `keep`.  pe / de: the plain primal / dual
+// epilogues (it_off set per iteration), whose gathered vectors are y (de.y = de.yout) and x_bar
+// (pe.xbar).  Without CACHED a block runs kResidentWarps / kWarpsPerBlock groups of kWarpsPerBlock
+// warps, which take the sweep's 8-warp virtual blocks in turn.
+template <typename TX, bool CACHED>
+__global__ void __launch_bounds__(kResidentThreads)
+  resident_plain_kernel(const dev_sell<TX> AT, const dev_sell<TX> A,
+                        primal_epi<TX, false, true, false> pe, dual_epi<TX, false, true, false> de,
+                        int L, int keep, int m, int n, resident_dims D,
+                        const unsigned char* images, pdlp_scalars* st)
 {
   extern __shared__ __align__(16) unsigned char cl_smem[];
-  TX* ys          = reinterpret_cast<TX*>(cl_smem);
-  const int m_pad = (m + 15) & ~15;
-  TX* xbs         = ys + m_pad;
+  TX* ys  = reinterpret_cast<TX*>(cl_smem);
+  TX* xbs = reinterpret_cast<TX*>(cl_smem + resident_dims::pad((size_t)m * sizeof(TX)));
   const unsigned rank = cluster_rank(), blocks = cluster_size();
-  for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = de.y[i];
-  // Every block of the cluster is running (and has its copy of y) before any block stores into
-  // another's shared memory.
-  cluster_barrier();
-  const dsmem_sink<TX> to_xbs{(unsigned)__cvta_generic_to_shared(xbs), blocks};
-  const dsmem_sink<TX> to_ys{(unsigned)__cvta_generic_to_shared(ys), blocks};
-  const int group  = threadIdx.x / (kWarpsPerBlock * kWarp);
-  const int first  = (int)rank + (int)blocks * group;
-  const int stride = (int)blocks * kClusterGroups;
-  for (int it = 0; it < L; ++it) {
-    pe.it_off = it;
-    de.it_off = it;
-    const cluster_primal_epi<TX> bp{pe, to_xbs};
-    for (int vb = first; vb < gp; vb += stride)
-      sell_map_block<TX, TX, cluster_primal_epi<TX>>(AT, ys, bp, nullptr, vb);
+  const unsigned y_copy  = (unsigned)__cvta_generic_to_shared(ys);
+  const unsigned xb_copy = (unsigned)__cvta_generic_to_shared(xbs);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < m; i += kResidentThreads) ys[i] = de.y[i];
+
+  if constexpr (CACHED) {
+    const int ut = AT.n_long + AT.n_slices, ua = A.n_long + A.n_slices;
+    const int sp = D.units[0] * kWarp, sd = D.units[1] * kWarp;
+    TX* xs             = reinterpret_cast<TX*>(cl_smem + resident_dims::vector_bytes<TX>(m, n));
+    TX *xas = xs + sp, *yis = xas + sp, *yas = yis + sd;
+    unsigned char* img = reinterpret_cast<unsigned char*>(yas + sd);
+    {
+      const size_t bytes       = D.image_bytes<TX>();
+      const unsigned char* src = images + rank * bytes;
+      for (size_t b = (size_t)threadIdx.x * 16; b < bytes; b += kResidentThreads * 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(img + b)),
+                     "l"(src + b)
+                     : "memory");
+    }
+    // The row of this lane in the block's unit i of the sweep (-1: none).
+    auto row_of = [&](const dev_sell<TX>& M, int total, int i) {
+      const int u = (int)rank + D.blocks * i;
+      if (u < M.n_long) return lane == 0 ? u : -1;
+      if (u >= total) return -1;
+      const int r = M.n_long + (u - M.n_long) * kWarp + lane;
+      return r < M.rows ? r : -1;
+    };
+    for (int i = warp; i < D.units[0]; i += kResidentWarps) {
+      const int j = row_of(AT, ut, i);
+      if (j >= 0) {
+        xs[i * kWarp + lane]  = pe.x[j];
+        xas[i * kWarp + lane] = pe.xa[j];
+      }
+    }
+    for (int i = warp; i < D.units[1]; i += kResidentWarps) {
+      const int r = row_of(A, ua, i);
+      if (r >= 0) {
+        yis[i * kWarp + lane] = de.y[r];
+        yas[i * kWarp + lane] = de.ya[r];
+      }
+    }
+    const pdlp_scalars sc = *st;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int2* tab_p           = reinterpret_cast<const int2*>(img + D.image_at<TX>(0));
+    const int2* tab_d           = reinterpret_cast<const int2*>(img + D.image_at<TX>(1));
+    const TX* op_p              = reinterpret_cast<const TX*>(img + D.image_at<TX>(2));
+    const TX* op_d              = reinterpret_cast<const TX*>(img + D.image_at<TX>(3));
+    const TX* val_p             = reinterpret_cast<const TX*>(img + D.image_at<TX>(4));
+    const TX* val_d             = reinterpret_cast<const TX*>(img + D.image_at<TX>(5));
+    const unsigned short* idx_p = reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(6));
+    const unsigned short* idx_d = reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(7));
+    // Every block of the cluster is running (and has its copy of y) before any block stores into
+    // another's shared memory.
     cluster_barrier();
-    const cluster_dual_epi<TX> bd{de, to_ys};
-    for (int vb = first; vb < gd; vb += stride)
-      sell_map_block<TX, TX, cluster_dual_epi<TX>>(A, xbs, bd, nullptr, vb);
+    for (int it = 0; it < L; ++it) {
+      const bool last = it == L - 1;
+      for (int i = warp; i < D.units[0]; i += kResidentWarps) {
+        const int u = (int)rank + D.blocks * i;
+        if (u >= ut) break;
+        const int2 t     = tab_p[i];
+        const int s      = i * kWarp + lane;
+        const int j      = row_of(AT, ut, i);
+        const double acc = u < AT.n_long
+                             ? resident_long(val_p + t.x, idx_p + t.x, t.y, ys)
+                             : resident_slice(val_p + t.x + lane * kChunk,
+                                              idx_p + t.x + lane * kChunk, t.y >> 7, ys);
+        if (j >= 0) {
+          const typename primal_epi<TX, false, true, false>::pre_t p{
+            xs[s], op_p[s], op_p[sp + s], op_p[2 * sp + s], xas[s]};
+          const dsmem_sink<TX> sink{xb_copy + (unsigned)j * (unsigned)sizeof(TX), blocks};
+          TX xb;
+          if (last && keep)
+            primal_row_step<TX, true, true, false>(0, acc, p, &sc, it, &xb, xs + s, pe.xhat + j,
+                                                   pe.slack + j, (TX*)nullptr, sink);
+          else
+            primal_row_step<TX, false, true, false>(0, acc, p, &sc, it, &xb, xs + s, (TX*)nullptr,
+                                                    (TX*)nullptr, (TX*)nullptr, sink);
+          if (last) {
+            pe.xout[j] = xs[s];
+            pe.xbar[j] = xb;
+          }
+        }
+      }
+      cluster_barrier();
+      for (int i = warp; i < D.units[1]; i += kResidentWarps) {
+        const int u = (int)rank + D.blocks * i;
+        if (u >= ua) break;
+        const int2 t     = tab_d[i];
+        const int s      = i * kWarp + lane;
+        const int r      = row_of(A, ua, i);
+        const double acc = u < A.n_long
+                             ? resident_long(val_d + t.x, idx_d + t.x, t.y, xbs)
+                             : resident_slice(val_d + t.x + lane * kChunk,
+                                              idx_d + t.x + lane * kChunk, t.y >> 7, xbs);
+        if (r >= 0) {
+          const typename dual_epi<TX, false, true, false>::pre_t p{yis[s], op_d[s], op_d[sd + s],
+                                                                   yas[s]};
+          const dsmem_sink<TX> sink{y_copy + (unsigned)r * (unsigned)sizeof(TX), blocks};
+          if (last && keep)
+            dual_row_step<TX, true, true>(0, acc, p, &sc, it, (TX*)nullptr, yis + s, de.yhat + r,
+                                          sink);
+          else
+            dual_row_step<TX, false, true>(0, acc, p, &sc, it, (TX*)nullptr, yis + s,
+                                           (TX*)nullptr, sink);
+          if (last) de.yout[r] = yis[s];
+        }
+      }
+      cluster_barrier();
+    }
+  } else {
     cluster_barrier();
+    const int gp = sell_grid_device(AT), gd = sell_grid_device(A);
+    const int group  = warp / kWarpsPerBlock;
+    const int first  = (int)rank + (int)blocks * group;
+    const int stride = (int)blocks * (kResidentWarps / kWarpsPerBlock);
+    for (int it = 0; it < L; ++it) {
+      pe.it_off = de.it_off = it;
+      const bool kept       = keep && it == L - 1;
+      for (int vb = first; vb < gp; vb += stride)
+        if (kept)
+          sell_map_block<TX, TX>(AT, ys, cluster_primal_epi<TX, true>{pe, xb_copy, blocks}, nullptr, vb);
+        else
+          sell_map_block<TX, TX>(AT, ys, cluster_primal_epi<TX, false>{pe, xb_copy, blocks}, nullptr, vb);
+      cluster_barrier();
+      for (int vb = first; vb < gd; vb += stride)
+        if (kept)
+          sell_map_block<TX, TX>(A, xbs, cluster_dual_epi<TX, true>{de, y_copy, blocks}, nullptr, vb);
+        else
+          sell_map_block<TX, TX>(A, xbs, cluster_dual_epi<TX, false>{de, y_copy, blocks}, nullptr, vb);
+      cluster_barrier();
+    }
   }
   if (rank == 0 && threadIdx.x == 0) st->t0 += L;
 }
-
 
 // Row j of A^T applied to y_bar: interaction (A^T y_bar - A^T y) . (x_bar - x) and |x_bar - x|^2
 // (reference adaptive_step_size_strategy.cu:352-518).
@@ -767,10 +1066,10 @@ __global__ void halpern_kernel(TX* x, const TX* xbar, const TX* xa, int n, TX* y
   const double w = halpern_weight(st, 0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n + m; i += gridDim.x * blockDim.x) {
     if (i < n)
-      x[i] = (TX)(w * (double)xbar[i] + (1.0 - w) * (double)xa[i]);
+      x[i] = (TX)halpern_mix(w, (double)xbar[i], (double)xa[i]);
     else {
       const int r = i - n;
-      y[r]        = (TX)(w * (double)ybar[r] + (1.0 - w) * (double)ya[r]);
+      y[r]        = (TX)halpern_mix(w, (double)ybar[r], (double)ya[r]);
     }
   }
 }

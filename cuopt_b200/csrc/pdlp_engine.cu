@@ -337,11 +337,11 @@ class engine {
     }
     copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(x_.data(), o.x_.data(), n);
     copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(xa_.data(), o.xa_.data(), n);
-    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(xhat_.data(), o.xhat_.data(), n);
-    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(slack_.data(), o.slack_.data(), n);
+    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(xhat_.data(), o.kept_xhat(), n);
+    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(slack_.data(), o.kept_slack(), n);
     copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(y_.data(), o.y_.data(), m);
     copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(ya_.data(), o.ya_.data(), m);
-    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(yhat_.data(), o.yhat_.data(), m);
+    copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(yhat_.data(), o.kept_yhat(), m);
     launches_ += 7;
     B200_LAUNCH_CHECK();
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
@@ -827,21 +827,7 @@ class engine {
     const bool ok   = coop && persist_grid_ > 0 && sell;
     pctl_.resize(1);
     pctl_.zero(s_);
-    // The cluster form where both gathered vectors fit in one block's shared memory.
-    int optin = 0;
-    B200_CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cluster_smem_ = ((size_t)((in_.m + 15) & ~15) + (size_t)in_.n) * sizeof(TX);
-    bool cl_ok    = sell && cluster_smem_ <= max_dynamic_smem(cluster_fn());
-    if (cl_ok) {
-      allow_max_dynamic_smem(cluster_fn());
-      cudaLaunchConfig_t cfg{};
-      cudaLaunchAttribute attr[1];
-      cluster_config(cfg, attr);
-      int clusters = 0;
-      cl_ok = cudaOccupancyMaxActiveClusters(&clusters, cluster_fn(), &cfg) == cudaSuccess &&
-              clusters > 0;
-      (void)cudaGetLastError();
-    }
+    const bool cl_ok = p_.persistent != 0 && sell && prepare_resident();
     form_key_ = form_key{in_.m, in_.n, L_.nnz, dev, (int)sizeof(TX)};
     int known = -1;
     for (double& u : form_us_) u = 0.0;
@@ -859,41 +845,152 @@ class engine {
   }
 
   // ------------------------------------------------------------------ cluster plain iterations
-  static constexpr int kClusterBlocks = 8;  // blocks per cluster (the portable maximum)
-  static const void* cluster_fn()
+  static const void* resident_fn(bool cached)
   {
-    return (const void*)cluster_plain_kernel<TX>;
+    return cached ? (const void*)resident_plain_kernel<TX, true>
+                  : (const void*)resident_plain_kernel<TX, false>;
   }
   void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1]) const
   {
     cfg                              = cudaLaunchConfig_t{};
-    cfg.gridDim                      = dim3(kClusterBlocks);
-    cfg.blockDim                     = dim3(kClusterThreads);
+    cfg.gridDim                      = dim3(resident_.blocks);
+    cfg.blockDim                     = dim3(kResidentThreads);
     cfg.dynamicSmemBytes             = cluster_smem_;
     cfg.stream                       = s_;
     attr[0].id                       = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x         = kClusterBlocks;
+    attr[0].val.clusterDim.x         = resident_.blocks;
     attr[0].val.clusterDim.y         = 1;
     attr[0].val.clusterDim.z         = 1;
     cfg.attrs                        = attr;
     cfg.numAttrs                     = 1;
   }
-  // Returns true for the first launch of the engine (which may include loading the kernel).
-  bool launch_cluster(int L)
+  // Sizes the cluster form, where both gathered vectors fit in one block's shared memory: 16 blocks
+  // where the device allows clusters of that size, else the portable 8, with the matrices' shares in
+  // shared memory where they fit beside the vectors.  Builds the blocks' images in that case.
+  bool prepare_resident()
+  {
+    const int m = in_.m, n = in_.n;
+    if (resident_dims::vector_bytes<TX>(m, n) > max_dynamic_smem(resident_fn(true))) return false;
+    const auto AT = ATs_view(), A = As_view();
+    std::vector<int64_t> off[4];
+    const dbuf<int64_t>* src[4] = {&L_.AT.long_off, &L_.AT.slice_off, &L_.A.long_off,
+                                   &L_.A.slice_off};
+    for (int q = 0; q < 4; ++q) {
+      off[q].resize(src[q]->size());
+      src[q]->download(off[q].data(), off[q].size(), s_);
+    }
+    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
+    for (const bool cached : {true, false})
+      for (const int c : {16, 8}) {
+        resident_dims d;
+        d.blocks = c;
+        for (int w = 0; cached && w < 2; ++w) {
+          const int longs = w == 0 ? AT.n_long : A.n_long, slices = w == 0 ? AT.n_slices : A.n_slices;
+          const auto &lo = off[2 * w], &so = off[2 * w + 1];
+          std::vector<int64_t> share(c, 0);
+          for (int u = 0; u < longs + slices; ++u) {
+            const int64_t e = u < longs ? lo[u + 1] - lo[u] : so[u - longs + 1] - so[u - longs];
+            share[u % c] += (e + 3) & ~int64_t(3);
+          }
+          const int64_t most = *std::max_element(share.begin(), share.end());
+          d.units[w]         = ceil_div(longs + slices, c);
+          if (most > INT_MAX / 2) return false;
+          d.elems[w] = (int)((most + 7) & ~int64_t(7));
+        }
+        const void* fn    = resident_fn(cached);
+        const size_t smem = cached ? d.smem<TX>(m, n) : resident_dims::vector_bytes<TX>(m, n);
+        if (smem > max_dynamic_smem(fn)) continue;
+        if (c > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                       cudaSuccess) {
+          (void)cudaGetLastError();
+          continue;
+        }
+        allow_max_dynamic_smem(fn);
+        resident_        = d;
+        resident_cached_ = cached;
+        cluster_smem_    = smem;
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[1];
+        cluster_config(cfg, attr);
+        int clusters  = 0;
+        const bool ok = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
+                        clusters > 0;
+        (void)cudaGetLastError();
+        if (!ok) continue;
+        if (cached) {
+          images_.resize(c * d.image_bytes<TX>());
+          resident_image_kernel<TX><<<c, kResidentThreads, 0, s_>>>(
+            AT, A, cs_.data(), ls_.data(), us_.data(), lcs_.data(), ucs_.data(), d, images_.data());
+          ++launches_;
+          B200_LAUNCH_CHECK();
+        }
+        for (auto* v : {&xhat2_, &slack2_}) v->resize(n);
+        yhat2_.resize(m);
+        return true;
+      }
+    return false;
+  }
+  // L plain iterations; with keep, the last one keeps x_hat, y_hat and the slack (in buffer kept_in_
+  // of the two).  Returns true for the first launch of the engine (which may include loading the
+  // kernel).
+  bool launch_cluster(int L, bool keep = false)
   {
     const auto AT = ATs_view(), A = As_view();
     persist_pe pe{x_.data(),   cs_.data(),   ls_.data(),    us_.data(),  xa_.data(),
-                  xbar_.data(), x_.data(),   xhat_.data(),  slack_.data(), aty_.data(),
+                  xbar_.data(), x_.data(),   kept_xhat(),   kept_slack(), aty_.data(),
                   scalars_.data(), 0};
     persist_de de{y_.data(),    lcs_.data(), ucs_.data(),  ya_.data(),      ybar_.data(),
-                  y_.data(),    yhat_.data(), scalars_.data(), 0};
+                  y_.data(),    kept_yhat(), scalars_.data(), 0};
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     cluster_config(cfg, attr);
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_plain_kernel<TX>, AT, A, pe, de, L, in_.m,
-                                       sell_grid(AT), sell_grid(A), scalars_.data()));
+    auto* fn = resident_cached_ ? resident_plain_kernel<TX, true> : resident_plain_kernel<TX, false>;
+    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, AT, A, pe, de, L, (int)keep, in_.m, in_.n,
+                                       resident_, (const unsigned char*)images_.data(),
+                                       scalars_.data()));
     ++launches_;
     return cluster_launches_++ == 0;
+  }
+  TX* kept_xhat() { return kept_in_ ? xhat2_.data() : xhat_.data(); }
+  TX* kept_slack() { return kept_in_ ? slack2_.data() : slack_.data(); }
+  TX* kept_yhat() { return kept_in_ ? yhat2_.data() : yhat_.data(); }
+
+  // The iterations up to the next fixed-point-error step in the cluster form, once it is chosen:
+  // one launch from each keeping step to the next, that step included, and the check on what it
+  // kept beside the launch after it (the two buffers take turns: a launch writes one while the
+  // check on the other is outstanding, and a check is read before the launch after next).  Returns
+  // false when a check ended the loop.
+  bool run_resident(pdlp_result& r)
+  {
+    long &k = sched_.k, &since = sched_.since;
+    auto launch = [&](long L, bool keep) {
+      if (L <= 0) return;
+      launch_cluster((int)L, keep);
+      if (keep) B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
+      k += L;
+      since += L;
+    };
+    conv_info cv;
+    for (;;) {
+      long step = k;
+      while (!is_major_step(step)) ++step;
+      // The fixed-point-error step keeps too and is not a plain one; what the step before it would
+      // keep is never checked.
+      const long error_step = (k / kMajor + 1) * kMajor - 1;
+      if (step >= error_step - 1) {
+        launch(error_step - k, false);
+        return posted_ < 0 || resolve(r, cv);
+      }
+      const bool ahead = may_run_ahead(step + 2);
+      if (!ahead && posted_ >= 0 && !resolve(r, cv)) return false;
+      kept_in_ = 1 - kept_in_;
+      launch(step + 1 - k, true);
+      if (!ahead) launch(1, false);  // the check is read at its own iterates
+      if (posted_ >= 0 && !resolve(r, cv)) return false;
+      post_check();
+      posted_ = step + 2;
+      if (!ahead && !resolve(r, cv)) return false;
+    }
   }
 
   // Returns true for the first launch of the engine (which may include loading the kernel).
@@ -1012,8 +1109,8 @@ class engine {
     const int m = in_.m, n = in_.n;
     B200_CUDA_CHECK(cudaStreamWaitEvent(es_, kept_, 0));
     unscale_kernel<TX><<<std::min(vgrid_, ceil_div((long)n + m, kBlock)), kBlock, 0, es_>>>(
-      xhat_.data(), yhat_.data(), slack_.data(), dc_.data(), dr_.data(), 1.0 / beta_, 1.0 / gamma_,
-      n, m, xu_.data(), yu_.data(), su_.data());
+      kept_xhat(), kept_yhat(), kept_slack(), dc_.data(), dr_.data(), 1.0 / beta_, 1.0 / gamma_, n,
+      m, xu_.data(), yu_.data(), su_.data());
     ++launches_;
     enqueue_conv(hres_);
     B200_CUDA_CHECK(cudaEventRecord(checked_, es_));
@@ -1290,6 +1387,10 @@ class engine {
 
       const bool mstep = is_major_step(k);
       const bool fpe_it = ((k + 1) % kMajor == 0) || restarted;
+      if (!mstep && !fpe_it && form_.decided() && form_.chosen() == 2) {
+        if (!run_resident(r)) return;
+        continue;
+      }
       if (!mstep && !fpe_it) {
         long R = 1;
         while (R < 255) {
@@ -1313,6 +1414,7 @@ class engine {
         conv_info cv;
         if (!resolve(r, cv)) return;
       }
+      if (mstep) kept_in_ = 0;
 
       // A step that keeps x_hat / y_hat / slack (major) and/or measures the fixed-point error.
       if (fpe_it) {
@@ -1475,6 +1577,13 @@ class engine {
   form_key form_key_{};
   double form_us_[3] = {0, 0, 0};  // the timings behind the choice (this solve's or cached)
   size_t cluster_smem_ = 0;         // dynamic shared memory of the cluster form
+  resident_dims resident_;          // its blocks and their shares (none without resident_cached_)
+  bool resident_cached_ = false;
+  dbuf<unsigned char> images_;
+  // x_hat, y_hat and the slack of the last keeping step are in buffer kept_in_: 0 is xhat_, yhat_,
+  // slack_; the cluster form alternates with these.
+  int kept_in_ = 0;
+  dbuf<TX> xhat2_, slack2_, yhat2_;
   long cluster_launches_ = 0;
   // Warps per block of the plain sweeps and the timings they were chosen by.
   int wpb_primal_ = kWarpsPerBlock, wpb_dual_ = kWarpsPerBlock;

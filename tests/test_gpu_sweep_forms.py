@@ -1,0 +1,74 @@
+"""Edges of the sweeps' forms: every form of the plain iterations and every block shape computes the
+same iterates bit for bit, at the sizes where slices, wide rows and cluster shares begin and end,
+and the oracle's to its parity tolerance."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from cuopt_b200 import generators as gen
+from cuopt_b200 import linear_programming as lpm
+from .helpers import datamodel_from_lp, settings
+
+pytestmark = pytest.mark.gpu
+
+GRAPHS, PERSISTENT, CLUSTER = 0, 1, 2
+ITERATE_RTOL = 1e-9  # the repository's parity tolerance for iterates against the oracle
+
+
+def _solve(lp, form, limit, precision=0, wpb=0, refine=False):
+    s = settings(tol=1e-13, iteration_limit=limit, precision=precision)
+    s.set_parameter(lpm.CUOPT_PDLP_PERSISTENT_ITERATIONS, form)
+    if wpb:
+        s.set_parameter(lpm.CUOPT_PDLP_SWEEP_WARPS_PER_BLOCK, wpb)
+    return lpm.Solve(datamodel_from_lp(lp), s)
+
+
+def _same(a, b):
+    assert a.get_lp_stats()["nb_iterations"] == b.get_lp_stats()["nb_iterations"]
+    for f in ("get_primal_solution", "get_dual_solution", "get_reduced_cost"):
+        assert np.array_equal(getattr(a, f)(), getattr(b, f)())
+
+
+def _lp(kind, m, n, k):
+    if kind == "wide":  # rows on both sides of 512 elements, and of several thousand
+        return gen.skewed_lp(m, n, seed=m + n, zipf_a=0.7, cap=k)
+    return gen.constructed_lp(m, n, k, seed=m + n)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("kind,m,n,k", [
+    ("plain", 1, 2, 1), ("plain", 31, 64, 3), ("plain", 32, 65, 3), ("plain", 33, 96, 5),
+    ("plain", 511, 1025, 4), ("plain", 1500, 3601, 13),  # shares of more than one unit a warp
+    ("wide", 60, 2500, 2500), ("wide", 37, 520, 520)])
+def test_forms_are_bit_identical(kind, m, n, k, precision):
+    """230 iterations: checks every 10, a restart at 200 (so that the anchor is not zero)."""
+    lp = _lp(kind, m, n, k)
+    ref = _solve(lp, GRAPHS, 230, precision)
+    _same(ref, _solve(lp, PERSISTENT, 230, precision))
+    c = _solve(lp, CLUSTER, 230, precision)
+    assert c.stats["plain_iteration_form"] == CLUSTER
+    _same(ref, c)
+    for wpb in (4, 16):
+        _same(ref, _solve(lp, GRAPHS, 230, precision, wpb))
+
+
+@pytest.mark.parametrize("limit", [1200, 1300])
+def test_cluster_form_checks_every_hundred_iterations(limit):
+    lp = gen.constructed_lp(150, 333, 5, seed=4)
+    _same(_solve(lp, GRAPHS, limit), _solve(lp, CLUSTER, limit))
+
+
+@pytest.mark.parametrize("form", [GRAPHS, CLUSTER])
+def test_refined_mixed_solve_takes_over_the_kept_iterates(form):
+    """The FP64 continuation starts from the iterates of the check that ended the mixed solve."""
+    lp = gen.constructed_lp(300, 700, 6, seed=12)
+    out = []
+    for f in (GRAPHS, form):
+        s = settings(tol=1e-5, precision=1)
+        s.set_parameter(lpm.CUOPT_PDLP_PERSISTENT_ITERATIONS, f)
+        s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_PASSES, 1)
+        s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_TOLERANCE, 1e-8)
+        out.append(lpm.Solve(datamodel_from_lp(lp), s))
+    assert out[0].stats["refinement_passes"] == 1
+    _same(out[0], out[1])
