@@ -259,6 +259,8 @@ B200_HD inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 // chunk of every row with a single 128-bit load per lane (512 contiguous bytes for 32-bit data).
 // Slice lengths are multiples of 4 and slice bases multiples of 4 elements (16-byte aligned).
 constexpr int kChunk = 4;
+// Long rows above this many elements are taken by several warps in the sweeps (see kernels.cuh).
+constexpr int kWideRow = 512;
 B200_HD inline int64_t sell_pos(int64_t base, int k, int lane)
 {
   return base + ((int64_t)(k >> 2) * 32 + lane) * kChunk + (k & 3);

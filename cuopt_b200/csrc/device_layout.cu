@@ -6,6 +6,7 @@
 
 #include <climits>
 #include <stdexcept>
+#include <utility>
 
 namespace cuopt_b200 {
 
@@ -38,8 +39,9 @@ __global__ void col_count_kernel(const int* idx, int64_t nnz, int n, int* cnt, i
 // block-diagonal batch, so every instance's items stay contiguous inside each class; without it
 // all items are instance 0.  A stable radix sort on these keys with values 0..count-1 keeps
 // original order on ties, which makes the permutation deterministic.
-__global__ void make_keys_kernel(const int* len, const int* inst, int count, int thr, int window,
-                                 uint64_t* keys, int* ids, int* nlong)
+// counts[0], counts[1] <- the long items, and those above `wide`.
+__global__ void make_keys_kernel(const int* len, const int* inst, int count, int thr, int wide,
+                                 int window, uint64_t* keys, int* ids, int* counts)
 {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     const int l      = len[i];
@@ -47,7 +49,8 @@ __global__ void make_keys_kernel(const int* len, const int* inst, int count, int
     uint64_t k;
     if (l > thr) {
       k = (b << 31) | (uint64_t)(INT_MAX - l);
-      atomicAdd(nlong, 1);
+      atomicAdd(counts, 1);
+      if (l > wide) atomicAdd(counts + 1, 1);
     } else {
       k = (1ull << 63) | (b << 47) | ((uint64_t)(i / window) << 31) | (uint64_t)(thr - l);
     }
@@ -193,8 +196,9 @@ struct temp_store {
   }
 };
 
-// Relabelling of `count` items with lengths `len` (device).  Returns the number of long items.
-int order_items(const int* len, const int* inst, int count, const layout_params& p,
+// Relabelling of `count` items with lengths `len` (device).  Returns the number of long items, and
+// of wide ones (which come first of these without instances; 0 with).
+std::pair<int, int> order_items(const int* len, const int* inst, int count, const layout_params& p,
                 cudaStream_t s, temp_store& tmp, dbuf<int>& new2old, dbuf<int>& old2new,
                 int* d_counter, int* h_counter)
 {
@@ -202,9 +206,9 @@ int order_items(const int* len, const int* inst, int count, const layout_params&
   dbuf<int> ids(count);
   new2old.resize(count);
   old2new.resize(count);
-  B200_CUDA_CHECK(cudaMemsetAsync(d_counter, 0, sizeof(int), s));
-  make_keys_kernel<<<grid_for(count), kT, 0, s>>>(len, inst, count, p.long_threshold, p.window,
-                                                  keys.data(), ids.data(), d_counter);
+  B200_CUDA_CHECK(cudaMemsetAsync(d_counter, 0, 2 * sizeof(int), s));
+  make_keys_kernel<<<grid_for(count), kT, 0, s>>>(
+    len, inst, count, p.long_threshold, kWideRow, p.window, keys.data(), ids.data(), d_counter);
   B200_LAUNCH_CHECK();
   size_t bytes = 0;
   B200_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys.data(), keys_out.data(),
@@ -213,18 +217,20 @@ int order_items(const int* len, const int* inst, int count, const layout_params&
                                                   keys_out.data(), ids.data(), new2old.data(),
                                                   count, 0, 64, s));
   invert_perm_kernel<<<grid_for(count), kT, 0, s>>>(new2old.data(), count, old2new.data());
-  B200_CUDA_CHECK(cudaMemcpyAsync(h_counter, d_counter, sizeof(int), cudaMemcpyDeviceToHost, s));
+  B200_CUDA_CHECK(
+    cudaMemcpyAsync(h_counter, d_counter, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
-  return *h_counter;
+  return {h_counter[0], inst ? 0 : h_counter[1]};
 }
 
 // Internal CSR (offsets int32 rows+1, idx, val, src) -> dev_matrix
-void to_sell(int rows, int cols, int n_long, const int* off, const int* idx, const double* val,
+void to_sell(int rows, int cols, int n_long, int n_wide, const int* off, const int* idx, const double* val,
              const int* src, int64_t nnz, cudaStream_t s, temp_store& tmp, dev_matrix& M)
 {
   M.rows     = rows;
   M.cols     = cols;
   M.n_long   = n_long;
+  M.n_wide   = n_wide;
   M.n_slices = (rows - n_long + 31) / 32;
   M.long_off.resize(n_long + 1);
   long_off_kernel<<<grid_for(n_long + 1), kT, 0, s>>>(off, n_long, M.long_off.data());
@@ -283,7 +289,7 @@ void build_device_layout(int m, int n, const int* d_off, const int* d_idx, const
   const int64_t nnz = nnz32;
   out.nnz           = nnz;
   temp_store tmp;
-  dbuf<int> counters(2);
+  dbuf<int> counters(3);
   int* hcount = reinterpret_cast<int*>(pinned_scratch() + 32);
 
   dbuf<int> rlen(std::max(m, 1)), clen(std::max(n, 1));
@@ -291,17 +297,17 @@ void build_device_layout(int m, int n, const int* d_off, const int* d_idx, const
   clen.zero(s);
   counters.zero(s);
   if (nnz > 0)
-    col_count_kernel<<<grid_for(nnz), kT, 0, s>>>(d_idx, nnz, n, clen.data(), counters.data() + 1);
+    col_count_kernel<<<grid_for(nnz), kT, 0, s>>>(d_idx, nnz, n, clen.data(), counters.data() + 2);
   B200_LAUNCH_CHECK();
-  B200_CUDA_CHECK(cudaMemcpyAsync(hcount + 1, counters.data() + 1, sizeof(int),
+  B200_CUDA_CHECK(cudaMemcpyAsync(hcount + 2, counters.data() + 2, sizeof(int),
                                   cudaMemcpyDeviceToHost, s));
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
-  if (hcount[1]) throw std::invalid_argument("constraint matrix column index out of range");
+  if (hcount[2]) throw std::invalid_argument("constraint matrix column index out of range");
   trace_sync(s, "layout: lengths");
 
-  const int a_long = order_items(rlen.data(), p.row_inst, m, p, s, tmp, out.row_new2old,
+  const auto [a_long, a_wide] = order_items(rlen.data(), p.row_inst, m, p, s, tmp, out.row_new2old,
                                  out.row_old2new, counters.data(), hcount);
-  const int t_long = order_items(clen.data(), p.col_inst, n, p, s, tmp, out.col_new2old,
+  const auto [t_long, t_wide] = order_items(clen.data(), p.col_inst, n, p, s, tmp, out.col_new2old,
                                  out.col_old2new, counters.data(), hcount);
   trace_sync(s, "layout: relabelling");
 
@@ -348,9 +354,9 @@ void build_device_layout(int m, int n, const int* d_off, const int* d_idx, const
   }
 
   trace_sync(s, "layout: internal A^T");
-  to_sell(m, n, a_long, aoff.data(), aidx.data(), aval.data(), asrc.data(), nnz, s, tmp, out.A);
+  to_sell(m, n, a_long, a_wide, aoff.data(), aidx.data(), aval.data(), asrc.data(), nnz, s, tmp, out.A);
   trace_sync(s, "layout: sliced A");
-  to_sell(n, m, t_long, toff.data(), tidx.data(), tval.data(), tsrc.data(), nnz, s, tmp, out.AT);
+  to_sell(n, m, t_long, t_wide, toff.data(), tidx.data(), tval.data(), tsrc.data(), nnz, s, tmp, out.AT);
   trace_sync(s, "layout: sliced A^T");
   B200_CUDA_CHECK(cudaStreamSynchronize(s));
 }

@@ -25,6 +25,7 @@ struct dev_sell;
 
 struct dev_matrix {
   int rows = 0, cols = 0, n_long = 0, n_slices = 0;
+  int n_wide = 0;  // long rows above kWideRow elements (first of all rows; 0 in batches)
   int64_t stored_count = 0;
   dbuf<int64_t> long_off, slice_off;
   dbuf<int> idx;

@@ -33,22 +33,42 @@ struct dev_sell {
   const int* slice_list = nullptr;
   int work_long         = 0;
   int work_slices       = 0;
+  int n_wide            = 0;  // the first n_wide long rows are taken by kWideStrands warps each
   B200_HD int long_count() const { return long_list ? work_long : n_long; }
+  B200_HD int wide_count() const { return long_list ? 0 : n_wide; }
   B200_HD int slice_count() const { return slice_list ? work_slices : n_slices; }
 };
 
 B200_HD inline int long_blocks(int n_long, int wpb = kWarpsPerBlock) { return ceil_div(n_long, wpb); }
-template <typename T>
-__device__ __forceinline__ int sell_grid_device(const dev_sell<T>& a)
-{
-  return long_blocks(a.long_count()) + ceil_div(a.slice_count(), kWarpsPerBlock);
-}
-// Grid of sell_map_kernel (and of the setup kernels, which always see full views).
+// Grid of the kernels that take every long row with one warp (setup, climbers).
 template <typename T>
 inline int sell_grid(const dev_sell<T>& a, int wpb = kWarpsPerBlock)
 {
   const int g = long_blocks(a.long_count(), wpb) + ceil_div(a.slice_count(), wpb);
   return g > 0 ? g : 1;  // an empty work list still launches one (idle) block
+}
+// Wide rows: a row of a few thousand elements on one warp is a chain of some 150 dependent load
+// rounds, which a sweep waits for when the rest of it is done (20k x 60k LP, Zipf rows up to 5000
+// long: 38 of 50 us an iteration).  So rows longer than kWideRow elements (a sixteenth of such a
+// chain) are cut into kWideStrands strands, lane l of strand s taking elements 256 t + 32 s + l,
+// whose sums are added in strand order: by the 8 warps of a block (or half block of 16 warps), or
+// by one warp where a block has fewer.  Every form of the sweeps adds them in the same order.
+constexpr int kWideStrands = 8;
+B200_HD inline int wide_blocks(int n_wide, int wpb = kWarpsPerBlock)
+{
+  return wpb >= kWideStrands ? ceil_div(n_wide, wpb / kWideStrands) : ceil_div(n_wide, wpb);
+}
+// Blocks of a sweep (sell_map_block) before its slices, and all of them.
+template <typename T>
+B200_HD inline int row_blocks(const dev_sell<T>& a, int wpb = kWarpsPerBlock)
+{
+  return wide_blocks(a.wide_count(), wpb) + long_blocks(a.long_count() - a.wide_count(), wpb);
+}
+template <typename T>
+B200_HD inline int sweep_grid(const dev_sell<T>& a, int wpb = kWarpsPerBlock)
+{
+  const int g = row_blocks(a, wpb) + ceil_div(a.slice_count(), wpb);
+  return g > 0 ? g : 1;
 }
 
 // Scalars that change between iterations live on the device so captured graphs stay valid.
@@ -227,6 +247,38 @@ __device__ __forceinline__ T gather_load(const T* __restrict__ g, int i)
     return g[i];
 }
 
+// The strands of a wide row (elements [b, e)): this warp's, and all of them on one warp.
+template <bool COH, typename TM, typename TG>
+__device__ __forceinline__ double wide_strand(const dev_sell<TM>& A, const TG* __restrict__ g,
+                                              int64_t b, int64_t e, int strand)
+{
+  double acc = 0.0;
+#pragma unroll 4
+  for (int64_t k = b + strand * kWarp + (threadIdx.x & 31); k < e; k += kWideStrands * kWarp)
+    acc += (double)ld_stream(A.val + k) * (double)gather_load<COH>(g, ld_stream(A.idx + k));
+  return warp_sum(acc);
+}
+template <class Load>
+__device__ __forceinline__ double wide_row_by_warp(int len, Load&& term)
+{
+  double acc[kWideStrands];
+#pragma unroll
+  for (int q = 0; q < kWideStrands; ++q) acc[q] = 0.0;
+  for (int k = threadIdx.x & 31; k < len; k += kWideStrands * kWarp)
+#pragma unroll
+    for (int q = 0; q < kWideStrands; ++q)
+      if (k + q * kWarp < len) term(k + q * kWarp, acc[q]);
+  double sum = 0.0;
+#pragma unroll
+  for (int q = 0; q < kWideStrands; ++q) sum += warp_sum(acc[q]);
+  return sum;
+}
+// Barrier of one group of kWideStrands warps of the block (group g of up to 15).
+__device__ __forceinline__ void wide_barrier(int g)
+{
+  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kWideStrands* kWarp) : "memory");
+}
+
 // WPB: warps (rows or slices) per block.  Only the grouping of warps into blocks depends on it,
 // not any row's arithmetic; sweeps with block reductions (kRed > 0) use kWarpsPerBlock.
 template <typename TM, typename TG, class Epi, bool COH = false, int WPB = kWarpsPerBlock>
@@ -244,9 +296,42 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
     return;
   }
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & (WPB - 1);
-  const int lb   = long_blocks(A.long_count(), WPB);
-  if (vb < lb) {
-    const int q   = vb * WPB + warp;
+  const int wb   = wide_blocks(A.wide_count(), WPB);
+  const int lb   = row_blocks(A, WPB);
+  if (vb < wb) {
+    if constexpr (WPB >= kWideStrands) {
+      __shared__ double strands[2][kWideStrands];
+      static_assert(WPB <= 2 * kWideStrands, "two groups of strands");
+      const int group = threadIdx.x / (kWideStrands * kWarp), strand = warp & (kWideStrands - 1);
+      const int row   = vb * (WPB / kWideStrands) + warp / kWideStrands;
+      if (row < A.wide_count()) {
+        const auto pre = epi.load(row);
+        const double t = wide_strand<COH>(A, g, A.long_off[row], A.long_off[row + 1], strand);
+        wide_barrier(group);  // the sums of the group's row before have been read
+        if (lane == 0) strands[group][strand] = t;
+        wide_barrier(group);
+        if (strand == 0 && lane == 0) {
+          double acc = 0.0;
+#pragma unroll
+          for (int q = 0; q < kWideStrands; ++q) acc += strands[group][q];
+          epi(row, acc, pre, red);
+        }
+      }
+    } else {
+      const int row = vb * WPB + warp;
+      if (row < A.wide_count()) {
+        const auto pre  = epi.load(row);
+        const int64_t b = A.long_off[row];
+        const double acc =
+          wide_row_by_warp((int)(A.long_off[row + 1] - b), [&](int k, double& a) {
+            a += (double)ld_stream(A.val + b + k) *
+                 (double)gather_load<COH>(g, ld_stream(A.idx + b + k));
+          });
+        if (lane == 0) epi(row, acc, pre, red);
+      }
+    }
+  } else if (vb < lb) {
+    const int q   = A.wide_count() + (vb - wb) * WPB + warp;
     const int row = q < A.long_count() ? (A.long_list ? A.long_list[q] : q) : 0;
     if (q < A.long_count() && !skip_rows(epi, row, row)) {
       const auto pre  = epi.load(row);
@@ -340,7 +425,7 @@ template <typename TM, typename TG, class Epi>
 void launch_sell_wpb(int wpb, const dev_sell<TM>& A, const TG* g, const Epi& epi,
                      double* partials, cudaStream_t s)
 {
-  const int grid = sell_grid(A, wpb);
+  const int grid = sweep_grid(A, wpb);
   switch (wpb) {
     case 4:
       sell_map_wpb_kernel<TM, TG, Epi, 4><<<grid, 4 * kWarp, 0, s>>>(A, g, epi, partials);
@@ -349,7 +434,7 @@ void launch_sell_wpb(int wpb, const dev_sell<TM>& A, const TG* g, const Epi& epi
       sell_map_wpb_kernel<TM, TG, Epi, 16><<<grid, 16 * kWarp, 0, s>>>(A, g, epi, partials);
       break;
     default:
-      sell_map_kernel<TM, TG, Epi><<<sell_grid(A), kBlock, 0, s>>>(A, g, epi, partials);
+      sell_map_kernel<TM, TG, Epi><<<grid, kBlock, 0, s>>>(A, g, epi, partials);
   }
 }
 
@@ -843,8 +928,11 @@ __device__ __forceinline__ double resident_slice(const TX* v, const unsigned sho
 }
 template <typename TX>
 __device__ __forceinline__ double resident_long(const TX* v, const unsigned short* x, int len,
-                                                const TX* g)
+                                                const TX* g, bool wide)
 {
+  if (wide)
+    return wide_row_by_warp(
+      len, [&](int k, double& a) { a += (double)v[k] * (double)g[x[k]]; });
   double acc = 0.0;
   for (int k = threadIdx.x & 31; k < len; k += kWarp) acc += (double)v[k] * (double)g[x[k]];
   return warp_sum(acc);
@@ -964,7 +1052,7 @@ __global__ void __launch_bounds__(kResidentThreads)
         const int s      = i * kWarp + lane;
         const int j      = row_of(AT, ut, i);
         const double acc = u < AT.n_long
-                             ? resident_long(val_p + t.x, idx_p + t.x, t.y, ys)
+                             ? resident_long(val_p + t.x, idx_p + t.x, t.y, ys, u < AT.n_wide)
                              : resident_slice(val_p + t.x + lane * kChunk,
                                               idx_p + t.x + lane * kChunk, t.y >> 7, ys);
         if (j >= 0) {
@@ -992,7 +1080,7 @@ __global__ void __launch_bounds__(kResidentThreads)
         const int s      = i * kWarp + lane;
         const int r      = row_of(A, ua, i);
         const double acc = u < A.n_long
-                             ? resident_long(val_d + t.x, idx_d + t.x, t.y, xbs)
+                             ? resident_long(val_d + t.x, idx_d + t.x, t.y, xbs, u < A.n_wide)
                              : resident_slice(val_d + t.x + lane * kChunk,
                                               idx_d + t.x + lane * kChunk, t.y >> 7, xbs);
         if (r >= 0) {
@@ -1012,7 +1100,7 @@ __global__ void __launch_bounds__(kResidentThreads)
     }
   } else {
     cluster_barrier();
-    const int gp = sell_grid_device(AT), gd = sell_grid_device(A);
+    const int gp = sweep_grid(AT), gd = sweep_grid(A);
     const int group  = warp / kWarpsPerBlock;
     const int first  = (int)rank + (int)blocks * group;
     const int stride = (int)blocks * (kResidentWarps / kWarpsPerBlock);

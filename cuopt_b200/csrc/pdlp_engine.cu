@@ -38,8 +38,10 @@ double now_s()
 template <typename T>
 dev_sell<T> view_of(const dev_matrix& M, const T* v)
 {
-  return dev_sell<T>{M.rows, M.n_long, M.n_slices, M.long_off.data(), M.slice_off.data(),
-                     M.idx.data(), v};
+  dev_sell<T> s{M.rows, M.n_long, M.n_slices, M.long_off.data(), M.slice_off.data(), M.idx.data(),
+                v};
+  s.n_wide = M.n_wide;
+  return s;
 }
 inline dev_sell<double> view64(const dev_matrix& M) { return view_of<double>(M, M.val.data()); }
 
@@ -199,7 +201,7 @@ class engine {
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
     trace("engine: layout");
     vgrid_ = sms_ * 4;
-    const int g = std::max({sell_grid(view64(L_.A)), sell_grid(view64(L_.AT)), vgrid_});
+    const int g = std::max({sweep_grid(view64(L_.A)), sweep_grid(view64(L_.AT)), vgrid_});
     partials_.resize((size_t)g * 4);
     dres_.resize(64);
     prepare_checks();
@@ -278,7 +280,7 @@ class engine {
 
   void prepare_checks()
   {
-    tpartials_.resize(2 * (size_t)sell_grid(view64(L_.A)) + 3 * (size_t)sell_grid(view64(L_.AT)));
+    tpartials_.resize(2 * (size_t)sweep_grid(view64(L_.A)) + 3 * (size_t)sweep_grid(view64(L_.AT)));
     tres_.resize(8);
     tarrived_.resize(1);
     tarrived_.zero(s_);
@@ -513,10 +515,10 @@ class engine {
     for (int k = 0; k < max_steps;) {
       const int c = std::min(kLanczosChunk, max_steps - k);
       for (int i = 0; i < c; ++i) {
-        gk_sweep_kernel<0, TX, gk_primal_epi><<<sell_grid(ATs), kBlock, 0, s_>>>(
+        gk_sweep_kernel<0, TX, gk_primal_epi><<<sweep_grid(ATs), kBlock, 0, s_>>>(
           ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data(), st.data(),
           alphas.data());
-        gk_sweep_kernel<1, TX, gk_dual_epi><<<sell_grid(As), kBlock, 0, s_>>>(
+        gk_sweep_kernel<1, TX, gk_dual_epi><<<sweep_grid(As), kBlock, 0, s_>>>(
           As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data(), st.data(),
           betas.data());
       }
@@ -548,7 +550,7 @@ class engine {
     if constexpr (!MAJOR && HALPERN && !SAVE_ATY)
       launch_sell_wpb(wpb ? wpb : wpb_primal_, A, y_.data(), e, partials_.data(), s_);
     else
-      sell_map_kernel<TX, TX, decltype(e)><<<sell_grid(A), kBlock, 0, s_>>>(A, y_.data(), e,
+      sell_map_kernel<TX, TX, decltype(e)><<<sweep_grid(A), kBlock, 0, s_>>>(A, y_.data(), e,
                                                                            partials_.data());
     ++launches_;
   }
@@ -562,7 +564,7 @@ class engine {
     if constexpr (!MAJOR && HALPERN && !FPE)
       launch_sell_wpb(wpb ? wpb : wpb_dual_, A, xbar_.data(), e, partials_.data(), s_);
     else
-      sell_map_kernel<TX, TX, decltype(e)><<<sell_grid(A), kBlock, 0, s_>>>(A, xbar_.data(), e,
+      sell_map_kernel<TX, TX, decltype(e)><<<sweep_grid(A), kBlock, 0, s_>>>(A, xbar_.data(), e,
                                                                            partials_.data());
     ++launches_;
   }
@@ -820,7 +822,7 @@ class engine {
     B200_CUDA_CHECK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     B200_CUDA_CHECK(
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_fn(), kBlock, 0));
-    const int need = std::max(sell_grid(ATs_view()), sell_grid(As_view()));
+    const int need = std::max(sweep_grid(ATs_view()), sweep_grid(As_view()));
     persist_grid_  = std::min(need, per_sm * sms_);
     // The persistent and cluster kernels run the sliced-ELL sweeps only.
     const bool sell = !tile_primal_ && !tile_dual_;
@@ -1003,7 +1005,7 @@ class engine {
     persist_de de{y_.data(),    lcs_.data(), ucs_.data(),  ya_.data(),      ybar_.data(),
                   y_.data(),    yhat_.data(), scalars_.data(), 0};
     advance_one adv{scalars_.data()};
-    int gp = sell_grid(AT), gd = sell_grid(A);
+    int gp = sweep_grid(AT), gd = sweep_grid(A);
     const TX* y    = y_.data();
     const TX* xb   = xbar_.data();
     persist_ctl* c = pctl_.data();
@@ -1128,7 +1130,7 @@ class engine {
   void enqueue_conv(double* h)
   {
     const auto A = view64(L_.A), AT = view64(L_.AT);
-    const int gp = sell_grid(A), gd = sell_grid(AT);
+    const int gp = sweep_grid(A), gd = sweep_grid(AT);
     term_kernel<<<gp + gd, kBlock, 0, es_>>>(
       A, AT, xu_.data(), yu_.data(), term_primal_epi{lc64_.data(), uc64_.data(), yu_.data()},
       term_dual_epi{c64_.data(), xu_.data(), su_.data()}, gp, gd, tpartials_.data(),
@@ -1274,12 +1276,12 @@ class engine {
     const double nd = stat<true>(d.data(), n), ne = stat<true>(e.data(), m);
     const double sum_cd = stat<false>(cd.data(), n), sum_ps = stat<false>(pe.data(), m);
     const auto A = As_view(), AT = ATs_view();
-    sell_map_kernel<TX, double, ray_primal_epi<TX>><<<sell_grid(A), kBlock, 0, s_>>>(
+    sell_map_kernel<TX, double, ray_primal_epi<TX>><<<sweep_grid(A), kBlock, 0, s_>>>(
       A, d.data(),
       ray_primal_epi<TX>{lcs_.data(), ucs_.data(), dr_.data(), nd > 0.0 ? 1.0 / nd : 1.0,
                          vm.data()},
       partials_.data());
-    sell_map_kernel<TX, double, ray_dual_epi<TX>><<<sell_grid(AT), kBlock, 0, s_>>>(
+    sell_map_kernel<TX, double, ray_dual_epi<TX>><<<sweep_grid(AT), kBlock, 0, s_>>>(
       AT, e.data(), ray_dual_epi<TX>{ls_.data(), us_.data(), dc_.data(), sn.data(), vn.data()},
       partials_.data());
     launches_ += 2;
@@ -1426,12 +1428,12 @@ class engine {
           launch_dual<false, false, true>(0);
         }
         if (mstep) B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
-        finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(A),
+        finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), sweep_grid(A),
                                                      dres_.data() + 8);
         // compute_fixed_error (reference pdlp.cu:1749-1857)
-        sell_map_kernel<TX, TX, fpe_epi<TX>><<<sell_grid(AT), kBlock, 0, s_>>>(
+        sell_map_kernel<TX, TX, fpe_epi<TX>><<<sweep_grid(AT), kBlock, 0, s_>>>(
           AT, ybar_.data(), fpe_epi<TX>{aty_.data(), xbar_.data(), x_.data()}, partials_.data());
-        finalize_sum_kernel<2><<<1, kBlock, 0, s_>>>(partials_.data(), sell_grid(AT),
+        finalize_sum_kernel<2><<<1, kBlock, 0, s_>>>(partials_.data(), sweep_grid(AT),
                                                      dres_.data() + 9);
         // Infeasibility information from this step's deltas, for the checks at iterations 200
         // and 400 only (reference termination_strategy.cu:187-199).
@@ -1626,7 +1628,7 @@ class engine {
       B200_CUDA_CHECK(cudaMemcpyAsync(&long_nnz, M.long_off.data() + M.n_long, sizeof(int64_t),
                                       cudaMemcpyDeviceToHost, s_));
       B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      const int lb = long_blocks(V.long_count()), g = sell_grid(V);
+      const int lb = row_blocks(V), g = sweep_grid(V);
       out[0] = M.n_long;
       out[1] = (double)long_nnz;
       out[2] = lb > 0 ? time_of([&] { launch(lb, 0); }) : 0.0;

@@ -72,3 +72,17 @@ def test_refined_mixed_solve_takes_over_the_kept_iterates(form):
         out.append(lpm.Solve(datamodel_from_lp(lp), s))
     assert out[0].stats["refinement_passes"] == 1
     _same(out[0], out[1])
+
+
+@pytest.mark.parametrize("m,n,cap", [(400, 7000, 5000), (2500, 9000, 1200)])
+def test_wide_rows_follow_the_oracle(m, n, cap):
+    from oracle import oracle as O
+
+    lp = gen.skewed_lp(m, n, seed=m, cap=cap)
+    assert np.diff(lp.row_off).max() > 512
+    for limit in (10, 200, 210):
+        res, x, y, _ = O.solve(lp, tol=1e-13, iteration_limit=limit)
+        sol = _solve(lp, GRAPHS, limit)
+        assert sol.get_lp_stats()["nb_iterations"] == res["iterations"]
+        for got, want in ((sol.get_primal_solution(), x), (sol.get_dual_solution(), y)):
+            assert np.max(np.abs(got - want)) <= ITERATE_RTOL * (1 + np.abs(want).max())
