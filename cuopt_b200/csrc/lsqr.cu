@@ -6,19 +6,24 @@
 // 5000 x 5000 bases of the 64-LP adjoint workload), where restarted GMRES and BiCGStab stall and
 // LSQR converges in 7 000 - 11 000 iterations.  A batch of such systems would need two kernel
 // boundaries and a reduction per system per iteration if each iteration were a grid-wide launch,
-// so instead every system gets one thread block that runs its whole LSQR loop:
-//   * the iterate vectors u (rows), v, x and w (cols) live in shared memory when they fit
-//     (rows + 3 cols doubles <= kSmemBudget), else in a global scratch slice of the block's own;
+// so instead every system gets one thread-block cluster that runs its whole LSQR loop:
+//   * every block of the cluster holds a copy of u (rows) and v (cols) in shared memory, gathers
+//     from it, and sends each new entry to every block's copy through distributed shared memory;
+//     x and w are kept by the block that owns their column;
 //   * the operator and its transpose are stored as 32-row sliced ELL (lane t of a warp owns row t
-//     of a slice and reads element k at base + 32 k + t, so a warp reads 32 contiguous values per
-//     step), rows sorted by length, so each product is a coalesced stream from L2 with gathers
-//     from shared memory;
-//   * the two norms of an iteration are block reductions in a fixed order, computed identically by
-//     every thread, so the scalar recurrence and the stopping decision are uniform and the result
-//     is deterministic;
+//     of a slice and reads element k at base + 32 k + t), rows sorted by length; slice s belongs to
+//     block s % C, whose share is copied into its shared memory (16-bit indices) where it fits, so
+//     that an iteration reads no global memory;
+//   * the two norms of an iteration are sums of per-warp sums, sent to every block with the vector
+//     entries and added in a fixed order by every warp, so the scalar recurrence and the stopping
+//     decision are uniform, the result is deterministic, and an iteration costs two products and
+//     two cluster barriers (hardware, no spin loop);
 //   * the x / w update of an iteration is applied in the next transpose product by the thread that
-//     owns the row, so an iteration costs two products and two block synchronisations.
-// Each block stops at LSQR's tests or at its iteration limit: there are no waits between blocks.
+//     owns the row.
+// One block per system, reading the operator from L2, took 33 us an iteration on the 5000 x 5000
+// systems.  Systems whose vectors do not fit (some 14 000 rows and columns) still run in one block
+// each, with u, v, x and w in global memory.
+// Each cluster stops at LSQR's tests or at its iteration limit: none waits for another.
 #include "common.cuh"
 #include "lsqr.hpp"
 
@@ -34,7 +39,6 @@ namespace {
 
 constexpr int kLsqrThreads = 512;
 constexpr int kLsqrWarps   = kLsqrThreads / kWarp;
-constexpr size_t kSmemBudget = 200 * 1024;
 constexpr int kEquilibrationPasses = 10;
 
 struct lsqr_desc {
@@ -48,7 +52,8 @@ struct lsqr_desc {
   const double* q_val;
   const double* b;          // rows (sorted, equilibrated)
   double* z;                // cols (sorted, equilibrated)
-  double* scratch;          // rows + 3 cols doubles when the vectors are not in shared memory
+  double* scratch;          // rows + 3 cols doubles (systems that run in one block each)
+  int64_t share_p, share_q; // most elements of P and Q that one block of a cluster holds
   int max_iter;
   double tol;
 };
@@ -107,14 +112,12 @@ __device__ __forceinline__ void slice_products(int slices, int rows, const int64
   }
 }
 
-template <bool SMEM>
-__global__ void __launch_bounds__(kLsqrThreads) lsqr_kernel(const lsqr_desc* __restrict__ descs,
+__global__ void __launch_bounds__(kLsqrThreads, 1) lsqr_kernel(const lsqr_desc* __restrict__ descs,
                                                             lsqr_out* __restrict__ outs)
 {
-  extern __shared__ double dyn[];
   __shared__ double part_a[kLsqrWarps * 2], part_b[kLsqrWarps * 2];
   const lsqr_desc d = descs[blockIdx.x];
-  double* u = SMEM ? dyn : d.scratch;
+  double* u = d.scratch;
   double* v = u + d.rows;
   double* x = v + d.cols;
   double* w = x + d.cols;
@@ -215,6 +218,273 @@ __global__ void __launch_bounds__(kLsqrThreads) lsqr_kernel(const lsqr_desc* __r
   // The last pending x update, then the result.
   for (int j = threadIdx.x; j < d.cols; j += T) d.z[j] = x[j] + c1 * w[j];
   if (threadIdx.x == 0) outs[blockIdx.x] = lsqr_out{it, flag, rnorm, arnorm};
+}
+
+// Shared memory of one block of a cluster of C for a system: u, v, the x and w of the block's
+// columns, the per-warp sums of the two norms from every block, and with `cached` the block's
+// shares of P and Q: {start, length} per slice, values, 16-bit indices.
+struct lsqr_smem {
+  size_t v, x, w, part_a, part_b, tab[2], val[2], idx[2], bytes;
+  static B200_HD size_t pad(size_t b) { return (b + 15) & ~(size_t)15; }
+  B200_HD lsqr_smem(int rows, int cols, int slices_p, int slices_q, int64_t elems_p,
+                    int64_t elems_q, int C, bool cached)
+  {
+    size_t at    = pad((size_t)rows * 8);
+    auto take    = [&](size_t b) {
+      const size_t here = at;
+      at += pad(b);
+      return here;
+    };
+    const size_t np = (size_t)(slices_p + C - 1) / C, nq = (size_t)(slices_q + C - 1) / C;
+    v      = take((size_t)cols * 8);
+    x      = take(nq * kWarp * 8);
+    w      = take(nq * kWarp * 8);
+    part_a = take((size_t)C * kLsqrWarps * 8);
+    part_b = take((size_t)C * kLsqrWarps * 16);
+    tab[0] = take(cached ? np * 8 : 0);
+    tab[1] = take(cached ? nq * 8 : 0);
+    val[0] = take(cached ? (size_t)elems_p * 8 : 0);
+    val[1] = take(cached ? (size_t)elems_q * 8 : 0);
+    idx[0] = take(cached ? (size_t)elems_p * 2 : 0);
+    idx[1] = take(cached ? (size_t)elems_q * 2 : 0);
+    bytes  = at;
+  }
+};
+
+__device__ __forceinline__ unsigned lsqr_rank()
+{
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void lsqr_barrier()
+{
+  __syncwarp();
+  asm volatile(
+    "barrier.cluster.arrive.release.aligned;\n"
+    "barrier.cluster.wait.acquire.aligned;\n" ::
+      : "memory");
+}
+// Stores v at `p`'s place in block c of the cluster.
+__device__ __forceinline__ void send(const double* p, unsigned c, double v)
+{
+  unsigned remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+               : "=r"(remote)
+               : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(c));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+}
+
+// Sends this warp's sums of K per-thread values to every block (lane c to block c of C <= 16); after
+// the next cluster barrier, cluster_totals adds them in one order everywhere.
+template <int K>
+__device__ __forceinline__ void send_sums(const double (&v)[K], const double* part, unsigned rank,
+                                          int C)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    const double s = warp_sum(v[q]);
+    if (lane < C) send(part + ((size_t)q * C + rank) * kLsqrWarps + warp, lane, s);
+  }
+}
+template <int K>
+__device__ __forceinline__ void cluster_totals(const double* part, int C, double (&out)[K])
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    double s = 0.0;
+    for (int i = lane; i < C * kLsqrWarps; i += kWarp) s += part[q * C * kLsqrWarps + i];
+    out[q] = warp_sum(s);
+  }
+}
+
+template <bool CACHED>
+__global__ void __launch_bounds__(kLsqrThreads, 1)
+  lsqr_cluster_kernel(const lsqr_desc* __restrict__ descs, lsqr_out* __restrict__ outs, int C)
+{
+  extern __shared__ __align__(16) unsigned char dyn[];
+  const unsigned rank = lsqr_rank();
+  const int system    = (int)blockIdx.x / C;
+  const lsqr_desc d   = descs[system];
+  const lsqr_smem S(d.rows, d.cols, d.slices_p, d.slices_q, d.share_p, d.share_q, C, CACHED);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = kLsqrThreads;
+  auto at        = [&](size_t o) { return reinterpret_cast<double*>(dyn + o); };
+  double *u = at(0), *v = at(S.v), *x = at(S.x), *w = at(S.w);
+  double *part_a = at(S.part_a), *part_b = at(S.part_b);
+  const int np = (d.slices_p + C - 1) / C, nq = (d.slices_q + C - 1) / C;
+
+  if constexpr (CACHED) {
+    for (int m = 0; m < 2; ++m) {
+      const int n           = m == 0 ? np : nq, slices = m == 0 ? d.slices_p : d.slices_q;
+      const int64_t* so     = m == 0 ? d.p_slice : d.q_slice;
+      const int* gi         = m == 0 ? d.p_idx : d.q_idx;
+      const double* gv      = m == 0 ? d.p_val : d.q_val;
+      int2* tab             = reinterpret_cast<int2*>(dyn + S.tab[m]);
+      double* val           = at(S.val[m]);
+      unsigned short* idx   = reinterpret_cast<unsigned short*>(dyn + S.idx[m]);
+      if (threadIdx.x == 0) {
+        int start = 0;
+        for (int i = 0; i < n; ++i) {
+          const int s   = (int)rank + C * i;
+          const int len = s < slices ? (int)(so[s + 1] - so[s]) : 0;
+          tab[i]        = make_int2(start, len >> 5);
+          start += len;
+        }
+      }
+      __syncthreads();
+      for (int i = warp; i < n; i += kLsqrWarps) {
+        const int s = (int)rank + C * i;
+        if (s >= slices) break;
+        const int64_t base = so[s];
+        const int2 t       = tab[i];
+        for (int k = lane; k < t.y * kWarp; k += kWarp) {
+          val[t.x + k] = gv[base + k];
+          idx[t.x + k] = (unsigned short)gi[base + k];
+        }
+      }
+    }
+  }
+  // The products of this block's rows of P (m = 0) or Q (m = 1) with `vec`: f(unit, row, product).
+  auto products = [&](int m, const double* vec, auto&& f) {
+    const int n = m == 0 ? np : nq, slices = m == 0 ? d.slices_p : d.slices_q;
+    const int rows = m == 0 ? d.rows : d.cols;
+    for (int i = warp; i < n; i += kLsqrWarps) {
+      const int s = (int)rank + C * i;
+      if (s >= slices) break;
+      double acc = 0.0;
+      if constexpr (CACHED) {
+        const int2 t             = reinterpret_cast<const int2*>(dyn + S.tab[m])[i];
+        const double* vp         = at(S.val[m]) + t.x + lane;
+        const unsigned short* ip = reinterpret_cast<const unsigned short*>(dyn + S.idx[m]) + t.x +
+                                   lane;
+#pragma unroll 4
+        for (int k = 0; k < t.y; ++k) acc += vp[kWarp * k] * vec[ip[kWarp * k]];
+      } else {
+        const int64_t* so  = m == 0 ? d.p_slice : d.q_slice;
+        const int64_t base = so[s];
+        const int len      = (int)((so[s + 1] - base) >> 5);
+        const int* ip      = (m == 0 ? d.p_idx : d.q_idx) + base + lane;
+        const double* vp   = (m == 0 ? d.p_val : d.q_val) + base + lane;
+#pragma unroll 4
+        for (int k = 0; k < len; ++k) acc += vp[kWarp * k] * vec[ip[kWarp * k]];
+      }
+      const int r = s * kWarp + lane;
+      if (r < rows) f(i, r, acc);
+    }
+  };
+
+  // u = b, beta = |b| (every block sums its whole copy)
+  double t1[1] = {0.0}, r1[1];
+  for (int r = threadIdx.x; r < d.rows; r += T) {
+    const double bv = d.b[r];
+    u[r]            = bv;
+    t1[0] += bv * bv;
+  }
+  block_sums<1>(t1, part_a, r1);
+  __syncthreads();  // part_a is read before other blocks write it
+  double beta        = sqrt(r1[0]);
+  const double bnorm = beta;
+  if (!(beta > 0.0) || !isfinite(beta)) {  // in every block of the cluster
+    if (rank == 0) {
+      for (int j = threadIdx.x; j < d.cols; j += T) d.z[j] = 0.0;
+      if (threadIdx.x == 0) outs[system] = lsqr_out{0, 0, beta, 0.0};
+    }
+    return;
+  }
+  // Every block of the cluster is running before any stores into another's shared memory.
+  lsqr_barrier();
+  double us = 1.0 / beta;  // the normalised u is u * us
+  // v = Op^T u / beta, alpha = |v|; x = w = 0 (w becomes v_1 in the first transpose product)
+  t1[0] = 0.0;
+  products(1, u, [&](int i, int j, double acc) {
+    const double vj = acc * us;
+    for (int c = 0; c < C; ++c) send(v + j, c, vj);
+    x[i * kWarp + lane] = 0.0;
+    w[i * kWarp + lane] = 0.0;
+    t1[0] += vj * vj;
+  });
+  send_sums<1>(t1, part_b, rank, C);
+  lsqr_barrier();
+  cluster_totals<1>(part_b, C, r1);
+  double alpha  = sqrt(r1[0]);
+  double vs     = alpha > 0.0 ? 1.0 / alpha : 0.0;
+  double rhobar = alpha, phibar = beta, anorm2 = 0.0, xnorm = 0.0;
+  double c1 = 0.0, c2 = 0.0;  // pending update: x += c1 w; w = v - c2 w
+  double rnorm = beta, arnorm = alpha * beta;
+  int flag = 3, it = 0;
+  if (!(alpha > 0.0)) {
+    flag = 2;  // Op^T b = 0: z = 0 is the least-squares solution
+  } else {
+    for (it = 1; it <= d.max_iter; ++it) {
+      // u <- Op v - alpha u  (normalised v = v * vs, normalised u = u * us)
+      t1[0] = 0.0;
+      products(0, v, [&](int, int r, double acc) {
+        const double un = acc * vs - alpha * (u[r] * us);
+        for (int c = 0; c < C; ++c) send(u + r, c, un);
+        t1[0] += un * un;
+      });
+      send_sums<1>(t1, part_a, rank, C);
+      lsqr_barrier();
+      cluster_totals<1>(part_a, C, r1);
+      beta = sqrt(r1[0]);
+      us   = beta > 0.0 ? 1.0 / beta : 0.0;
+      anorm2 += alpha * alpha + beta * beta;
+      // pending x / w update, then v <- Op^T u - beta v
+      double t2[2] = {0.0, 0.0}, r2[2];
+      products(1, u, [&](int i, int j, double acc) {
+        const int q     = i * kWarp + lane;
+        const double vo = v[j] * vs;
+        double wj       = w[q];
+        const double xj = x[q] + c1 * wj;
+        wj              = vo - c2 * wj;
+        x[q]            = xj;
+        w[q]            = wj;
+        const double vn = acc * us - beta * vo;
+        for (int c = 0; c < C; ++c) send(v + j, c, vn);
+        t2[0] += vn * vn;
+        t2[1] += xj * xj;
+      });
+      send_sums<2>(t2, part_b, rank, C);
+      lsqr_barrier();
+      cluster_totals<2>(part_b, C, r2);
+      alpha = sqrt(r2[0]);
+      vs    = alpha > 0.0 ? 1.0 / alpha : 0.0;
+      xnorm = sqrt(r2[1]);
+      // Plane rotation (no damping) and the new pending update.
+      const double rho = sqrt(rhobar * rhobar + beta * beta);
+      const double cs = rhobar / rho, sn = beta / rho;
+      const double theta = sn * alpha;
+      rhobar             = -cs * alpha;
+      const double phi   = cs * phibar;
+      phibar             = sn * phibar;
+      c1                 = phi / rho;
+      c2                 = theta / rho;
+      rnorm              = phibar;
+      arnorm             = alpha * fabs(sn * phi);
+      const double anorm = sqrt(anorm2);
+      if (rnorm <= d.tol * bnorm + d.tol * anorm * xnorm) {
+        flag = 1;
+        break;
+      }
+      if (arnorm <= d.tol * anorm * rnorm) {
+        flag = 2;
+        break;
+      }
+      if (!(alpha > 0.0) || !(beta > 0.0)) {  // exact breakdown: the Krylov space is exhausted
+        flag = 1;
+        break;
+      }
+    }
+    if (it > d.max_iter) it = d.max_iter;
+  }
+  // The last pending x update, then the result.
+  for (int i = warp; i < nq; i += kLsqrWarps) {
+    const int j = ((int)rank + C * i) * kWarp + lane, q = i * kWarp + lane;
+    if (j < d.cols) d.z[j] = x[q] + c1 * w[q];
+  }
+  if (rank == 0 && threadIdx.x == 0) outs[system] = lsqr_out{it, flag, rnorm, arnorm};
 }
 
 // Host-side packing of one problem: equilibration, transposition, row sorting, sliced ELL.
@@ -347,6 +617,86 @@ void parallel_for(int count, F&& f)
   for (auto& th : pool) th.join();
 }
 
+// Most elements that one of C blocks holds of a sliced matrix (slice s in block s % C).
+int64_t most_elements(const std::vector<int64_t>& slice, int C)
+{
+  std::vector<int64_t> share(C, 0);
+  for (size_t s = 0; s + 1 < slice.size(); ++s) share[s % C] += slice[s + 1] - slice[s];
+  return *std::max_element(share.begin(), share.end());
+}
+size_t cluster_smem(const packed& q, int C, bool cached)
+{
+  return lsqr_smem(q.rows, q.cols, (int)q.p_slice.size() - 1, (int)q.q_slice.size() - 1,
+                   cached ? most_elements(q.p_slice, C) : 0,
+                   cached ? most_elements(q.q_slice, C) : 0, C, cached)
+    .bytes;
+}
+
+// Blocks per cluster and whether their shares of the operators are cached.
+struct cluster_plan {
+  int blocks   = 1;
+  bool cached  = false;
+  size_t smem  = 0;
+  void configure(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1], int systems,
+                 cudaStream_t s) const
+  {
+    cfg                      = cudaLaunchConfig_t{};
+    cfg.gridDim              = dim3(systems * blocks);
+    cfg.blockDim             = dim3(kLsqrThreads);
+    cfg.dynamicSmemBytes     = smem;
+    cfg.stream               = s;
+    attr[0].id               = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs                = attr;
+    cfg.numAttrs             = 1;
+  }
+};
+
+// The plan with the least estimated time: waves of clusters, each iteration of one taking about
+// 1.2 us for its barriers and sums plus the products, shared by its blocks (0.16 ns per non-zero
+// and product from shared memory, 0.4 ns from L2).
+cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>& ids, size_t limit)
+{
+  cluster_plan best;
+  if (ids.empty()) return best;
+  double nnz = 0.0, best_us = 0.0;
+  for (int i : ids) nnz += (double)(pk[i].p_val.size() + pk[i].q_val.size()) / ids.size();
+  for (const bool cached : {true, false})
+    for (const int c : {16, 8, 4, 2, 1}) {
+      cluster_plan p;
+      p.blocks = c;
+      p.cached = cached;
+      for (int i : ids) p.smem = std::max(p.smem, cluster_smem(pk[i], c, cached));
+      const void* fn = cached ? (const void*)lsqr_cluster_kernel<true>
+                              : (const void*)lsqr_cluster_kernel<false>;
+      if (p.smem > limit) continue;
+      if (c > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                     cudaSuccess) {
+        (void)cudaGetLastError();
+        continue;
+      }
+      allow_max_dynamic_smem(fn);
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute attr[1];
+      p.configure(cfg, attr, (int)ids.size(), nullptr);
+      int active = 0;
+      if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) {
+        (void)cudaGetLastError();
+        continue;
+      }
+      const double waves = std::ceil((double)ids.size() / active);
+      const double us    = waves * (1.2 + nnz * (cached ? 1.6e-4 : 4e-4) / c);
+      if (best.smem == 0 || us < best_us) {
+        best    = p;
+        best_us = us;
+      }
+    }
+  if (best.smem == 0) throw cuda_error("lsqr: no cluster shape can be launched");
+  return best;
+}
+
 }  // namespace
 
 std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>& ps,
@@ -365,26 +715,27 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   }
   parallel_for(count, [&](int i) { pack(*ps[i], pk[i]); });
 
-  // Systems with work go to the device, split by where their vectors fit.
-  std::vector<int> smem_ids, glob_ids;
-  size_t smem_bytes = 0, scratch_doubles = 0;
+  // Systems with work go to the device: those whose vectors fit in a cluster's blocks, and the rest.
+  const size_t limit = std::min(max_dynamic_smem((const void*)lsqr_cluster_kernel<true>),
+                                max_dynamic_smem((const void*)lsqr_cluster_kernel<false>));
+  std::vector<int> clus_ids, glob_ids;
+  size_t scratch_doubles = 0;
   for (int i = 0; i < count; ++i) {
     res[i].z.assign(ps[i]->cols, 0.0);
     if (pk[i].rows == 0 || pk[i].cols == 0) continue;
-    const size_t need = ((size_t)pk[i].rows + 3 * (size_t)pk[i].cols) * sizeof(double);
-    if (need <= kSmemBudget) {
-      smem_ids.push_back(i);
-      smem_bytes = std::max(smem_bytes, need);
+    if (cluster_smem(pk[i], 1, false) <= limit) {
+      clus_ids.push_back(i);
     } else {
       glob_ids.push_back(i);
       scratch_doubles += (size_t)pk[i].rows + 3 * (size_t)pk[i].cols;
     }
   }
-  if (smem_ids.empty() && glob_ids.empty()) return res;
+  if (clus_ids.empty() && glob_ids.empty()) return res;
+  const cluster_plan plan = plan_clusters(pk, clus_ids, limit);
 
   // One upload of every array: offsets, indices, values, right-hand sides; outputs z.
   size_t n_off = 0, n_idx = 0, n_val = 0, n_b = 0, n_z = 0;
-  auto order = smem_ids;
+  auto order = clus_ids;
   order.insert(order.end(), glob_ids.begin(), glob_ids.end());
   for (int i : order) {
     n_off += pk[i].p_slice.size() + pk[i].q_slice.size();
@@ -457,6 +808,8 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
     d.b        = d_b.data() + w.b;
     d.z        = d_z.data() + w.z;
     d.scratch  = d_scratch.data() + w.scratch;
+    d.share_p  = most_elements(q.p_slice, plan.blocks);
+    d.share_q  = most_elements(q.q_slice, plan.blocks);
     d.tol      = tol;
     d.max_iter = default_iter > 0 ? default_iter
                                   : (int)std::min<long long>(200000, 20LL * (q.rows + q.cols));
@@ -465,15 +818,17 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   dbuf<lsqr_desc> d_desc(h_desc.size());
   dbuf<lsqr_out> d_out(h_desc.size());
   d_desc.upload(h_desc.data(), h_desc.size(), s);
-  const int n_smem = (int)smem_ids.size(), n_glob = (int)glob_ids.size();
-  if (n_smem > 0) {
-    allow_max_dynamic_smem((const void*)lsqr_kernel<true>);
-    lsqr_kernel<true><<<n_smem, kLsqrThreads, smem_bytes, s>>>(d_desc.data(), d_out.data());
-    B200_LAUNCH_CHECK();
+  const int n_clus = (int)clus_ids.size(), n_glob = (int)glob_ids.size();
+  if (n_clus > 0) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    plan.configure(cfg, attr, n_clus, s);
+    auto* fn = plan.cached ? lsqr_cluster_kernel<true> : lsqr_cluster_kernel<false>;
+    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, (const lsqr_desc*)d_desc.data(), d_out.data(),
+                                       plan.blocks));
   }
   if (n_glob > 0) {
-    lsqr_kernel<false><<<n_glob, kLsqrThreads, 0, s>>>(d_desc.data() + n_smem,
-                                                       d_out.data() + n_smem);
+    lsqr_kernel<<<n_glob, kLsqrThreads, 0, s>>>(d_desc.data() + n_clus, d_out.data() + n_clus);
     B200_LAUNCH_CHECK();
   }
   std::vector<double> h_z(n_z);
