@@ -464,8 +464,7 @@ struct b_gk_primal_epi {
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<0>&) const
   {
     if (!ctx.active[p.b]) return;
-    const double b = st[p.b].beta, a = st[p.b].alpha;
-    const double pj = acc / b - (a > 0.0 ? b * (p.v / a) : 0.0);
+    const double pj = gk_next_v(acc, p.v, st[p.b].beta, st[p.b].alpha);
     v[j]            = pj;
     rowbuf[j]       = pj * pj;
   }
@@ -488,8 +487,7 @@ struct b_gk_dual_epi {
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<0>&) const
   {
     if (!ctx.active[p.b]) return;
-    const double a = st[p.b].alpha, b = st[p.b].beta;
-    const double qi = acc / a - a * (p.u / b);
+    const double qi = gk_next_u(acc, p.u, st[p.b].alpha, st[p.b].beta);
     u[i]            = qi;
     rowbuf[i]       = qi * qi;
   }

@@ -906,9 +906,9 @@ __device__ __forceinline__ void shared_chunk(const double* p, double (&v)[4])
 }
 
 // The product of a slice's row (this lane's) from shared memory, in sell_map_block's order.
-template <typename TX>
+template <typename TX, typename TG>
 __device__ __forceinline__ double resident_slice(const TX* v, const unsigned short* x, int nchunk,
-                                                 const TX* g)
+                                                 const TG* g)
 {
   double acc = 0.0;
 #pragma unroll 2
@@ -916,7 +916,7 @@ __device__ __forceinline__ double resident_slice(const TX* v, const unsigned sho
     const ushort4 i = *reinterpret_cast<const ushort4*>(x);
     double w[4];
     shared_chunk(v, w);
-    const TX g0 = g[i.x], g1 = g[i.y], g2 = g[i.z], g3 = g[i.w];
+    const TG g0 = g[i.x], g1 = g[i.y], g2 = g[i.z], g3 = g[i.w];
     acc += w[0] * (double)g0;
     acc += w[1] * (double)g1;
     acc += w[2] * (double)g2;
@@ -926,9 +926,9 @@ __device__ __forceinline__ double resident_slice(const TX* v, const unsigned sho
   }
   return acc;
 }
-template <typename TX>
+template <typename TX, typename TG>
 __device__ __forceinline__ double resident_long(const TX* v, const unsigned short* x, int len,
-                                                const TX* g, bool wide)
+                                                const TG* g, bool wide)
 {
   if (wide)
     return wide_row_by_warp(
@@ -1363,6 +1363,17 @@ struct gk_state {
   unsigned arrived;
 };
 
+// p_j = (A^T u)_j / beta - beta v_j / alpha (no second term before the first step), and
+// q_i = (A v)_i / alpha - alpha u_i / beta, rounded the same way in every kernel.
+__device__ __forceinline__ double gk_next_v(double acc, double v, double beta, double alpha)
+{
+  return alpha > 0.0 ? __dsub_rn(acc / beta, __dmul_rn(beta, v / alpha)) : acc / beta;
+}
+__device__ __forceinline__ double gk_next_u(double acc, double u, double alpha, double beta)
+{
+  return fma(-alpha, u / beta, acc / alpha);
+}
+
 // Row j of A^T applied to u:  p_j = (A^T u)_j / beta - beta v_j / alpha  (written over v_j).
 struct gk_primal_epi {
   static constexpr int kRed = 1;
@@ -1375,8 +1386,7 @@ struct gk_primal_epi {
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{v[j]}; }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<1>& r) const
   {
-    const double b = st->beta, a = st->alpha;
-    const double pj = acc / b - (a > 0.0 ? b * (p.v / a) : 0.0);
+    const double pj = gk_next_v(acc, p.v, st->beta, st->alpha);
     v[j]            = pj;
     r.v[0] += pj * pj;
   }
@@ -1394,8 +1404,7 @@ struct gk_dual_epi {
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{u[i]}; }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<1>& r) const
   {
-    const double a = st->alpha, b = st->beta;
-    const double qi = acc / a - a * (p.u / b);
+    const double qi = gk_next_u(acc, p.u, st->alpha, st->beta);
     u[i]            = qi;
     r.v[0] += qi * qi;
   }
@@ -1441,6 +1450,139 @@ __global__ void __launch_bounds__(kBlock) gk_sweep_kernel(const dev_sell<TM> A,
       st->step    = k + 1;
     }
     st->arrived = 0;
+  }
+}
+
+// `steps` steps of the recurrence for a small LP in one launch: a cluster of C blocks whose blocks
+// keep copies of u and v and their shares of the matrices (the images of the resident form) in
+// shared memory.  A half step is this block's products, its new entries sent to every copy, one
+// cluster barrier and the norm, formed as gk_sweep_kernel forms it: the sum of every warp goes to
+// its place in ws (8 per block of the sweep's grid, in every copy), each block's 8 are added in order,
+// and the blocks' in ordered_block_sum's tree (at most kBlock blocks: one partial a thread), so both
+// forms give the same coefficients bit for bit.  Two launches a step took 22 us on a 2000 x 5000 LP.
+constexpr int kClusterGkSums = kBlock * kWarpsPerBlock;  // most entries of ws per sweep
+template <typename TX>
+B200_HD inline size_t cluster_gk_smem(int m, int n, int gt, int ga, const resident_dims& D)
+{
+  return resident_dims::vector_bytes<double>(m, n) +
+         (size_t)(gt + ga) * kWarpsPerBlock * sizeof(double) + D.image_bytes<TX>();
+}
+// The place in ws of the sum of the warp that takes unit u of M.
+template <typename TX>
+__device__ __forceinline__ int unit_sum(const dev_sell<TX>& M, int u)
+{
+  if (u < M.n_wide) return u * kWarpsPerBlock;
+  const int q = u < M.n_long ? u - M.n_wide : u - M.n_long;
+  return (u < M.n_long ? M.n_wide : row_blocks(M)) * kWarpsPerBlock + q;
+}
+__device__ __forceinline__ double cluster_gk_norm(const double* ws, int blocks)
+{
+  const int lane = threadIdx.x & 31;
+  double e[kBlock / kWarp];
+#pragma unroll
+  for (int j = 0; j < kBlock / kWarp; ++j) {
+    const int b = lane + j * kWarp;
+    double t    = 0.0;
+    if (b < blocks)
+      for (int w = 0; w < kWarpsPerBlock; ++w) t += ws[b * kWarpsPerBlock + w];
+    e[j] = t;
+  }
+#pragma unroll
+  for (int h = kBlock / kWarp / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; ++j) e[j] += e[j + h];
+#pragma unroll
+  for (int h = kWarp / 2; h > 0; h >>= 1) e[0] += __shfl_down_sync(0xffffffffu, e[0], h);
+  return sqrt(__shfl_sync(0xffffffffu, e[0], 0));
+}
+
+template <typename TX>
+__global__ void __launch_bounds__(kResidentThreads, 1)
+  cluster_gk_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, double* u_out, double* v_out,
+                    gk_state* st, double* alphas, double* betas, int steps, int m, int n,
+                    resident_dims D, const unsigned char* images)
+{
+  extern __shared__ __align__(16) unsigned char gk_smem[];
+  const unsigned rank = cluster_rank(), blocks = cluster_size();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int grid[2] = {sweep_grid(AT), sweep_grid(A)};
+  double* u  = reinterpret_cast<double*>(gk_smem);
+  double* v  = reinterpret_cast<double*>(gk_smem + resident_dims::pad((size_t)m * 8));
+  double* ws = reinterpret_cast<double*>(gk_smem + resident_dims::vector_bytes<double>(m, n));
+  unsigned char* img = reinterpret_cast<unsigned char*>(ws + (grid[0] + grid[1]) * kWarpsPerBlock);
+  {
+    const size_t bytes       = D.image_bytes<TX>();
+    const unsigned char* src = images + rank * bytes;
+    for (size_t b = (size_t)threadIdx.x * 16; b < bytes; b += kResidentThreads * 16)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(img + b)),
+                   "l"(src + b)
+                   : "memory");
+  }
+  for (int i = threadIdx.x; i < m; i += kResidentThreads) u[i] = u_out[i];
+  for (int i = threadIdx.x; i < n; i += kResidentThreads) v[i] = v_out[i];
+  for (int i = threadIdx.x; i < (grid[0] + grid[1]) * kWarpsPerBlock; i += kResidentThreads)
+    ws[i] = 0.0;
+  double beta = st->beta, alpha = st->alpha;
+  const int k0 = st->step;
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  // Every block is running, with its copies, before any stores into another's shared memory (and
+  // has read the state before block 0 writes it).
+  cluster_barrier();
+  // The half step of matrix M (w = 0: rows of A^T from u to v, w = 1: rows of A from v to u).
+  auto half = [&](const dev_sell<TX>& M, int w, const double* g, double* own, double nrm,
+                  double other) {
+    const int total             = M.n_long + M.n_slices;
+    const int2* tab             = reinterpret_cast<const int2*>(img + D.image_at<TX>(w));
+    const TX* val               = reinterpret_cast<const TX*>(img + D.image_at<TX>(4 + w));
+    const unsigned short* idx   = reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(6 + w));
+    double* sums                = ws + (w == 0 ? 0 : grid[0] * kWarpsPerBlock);
+    for (int i = warp; i < D.units[w]; i += kResidentWarps) {
+      const int q = (int)rank + D.blocks * i;
+      if (q >= total) break;
+      const int2 t = tab[i];
+      int row      = -1;
+      double acc;
+      if (q < M.n_long) {
+        if (lane == 0) row = q;
+        acc = resident_long(val + t.x, idx + t.x, t.y, g, q < M.n_wide);
+      } else {
+        row = M.n_long + (q - M.n_long) * kWarp + lane;
+        if (row >= M.rows) row = -1;
+        acc = resident_slice(val + t.x + lane * kChunk, idx + t.x + lane * kChunk, t.y >> 7, g);
+      }
+      double sq = 0.0;
+      if (row >= 0) {
+        const double e = w == 0 ? gk_next_v(acc, own[row], nrm, other)
+                                : gk_next_u(acc, own[row], nrm, other);
+        const unsigned at = (unsigned)__cvta_generic_to_shared(own + row);
+        for (unsigned c = 0; c < blocks; ++c) dsmem_store(at, c, e);
+        sq = e * e;
+      }
+      sq = warp_sum(sq);
+      if (lane < (int)blocks)
+        dsmem_store((unsigned)__cvta_generic_to_shared(sums + unit_sum(M, q)), lane, sq);
+    }
+    cluster_barrier();
+    return cluster_gk_norm(sums, grid[w]);
+  };
+  for (int k = 0; k < steps; ++k) {
+    alpha = half(AT, 0, u, v, beta, alpha);
+    beta  = half(A, 1, v, u, alpha, beta);
+    if (rank == 0 && threadIdx.x == 0) {
+      alphas[k0 + k]    = alpha;
+      betas[k0 + k + 1] = beta;
+    }
+  }
+  if (rank == 0) {
+    for (int i = threadIdx.x; i < m; i += kResidentThreads) u_out[i] = u[i];
+    for (int i = threadIdx.x; i < n; i += kResidentThreads) v_out[i] = v[i];
+    if (threadIdx.x == 0) {
+      st->beta  = beta;
+      st->alpha = alpha;
+      st->step  = k0 + steps;
+    }
   }
 }
 

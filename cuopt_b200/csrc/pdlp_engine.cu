@@ -253,6 +253,7 @@ class engine {
       view64(L_.AT), dr_.data(), dc_.data(), ATs_.data());
 
     prepare_vectors();
+    resident_ok_ = p_.persistent != 0 && prepare_resident();
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
     trace("engine: scaling");
     // Step size from the largest singular value of the scaled A (reference pdlp.cu:2620-2731),
@@ -346,6 +347,7 @@ class engine {
     copy_convert_kernel<TM, TX><<<vgrid_, kBlock, 0, s_>>>(yhat_.data(), o.kept_yhat(), m);
     launches_ += 7;
     B200_LAUNCH_CHECK();
+    resident_ok_ = p_.persistent != 0 && prepare_resident();
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
     init_plain_form();
   }
@@ -512,25 +514,64 @@ class engine {
     launches_ += 3;
     const auto As = view_of<TX>(L_.A, As_.data()), ATs = view_of<TX>(L_.AT, ATs_.data());
     std::vector<double> ha(max_steps + 1), hb(max_steps + 2);
-    for (int k = 0; k < max_steps;) {
-      const int c = std::min(kLanczosChunk, max_steps - k);
-      for (int i = 0; i < c; ++i) {
-        gk_sweep_kernel<0, TX, gk_primal_epi><<<sweep_grid(ATs), kBlock, 0, s_>>>(
-          ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data(), st.data(),
-          alphas.data());
-        gk_sweep_kernel<1, TX, gk_dual_epi><<<sweep_grid(As), kBlock, 0, s_>>>(
-          As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data(), st.data(),
-          betas.data());
+    const size_t smem  = cluster_gk_smem<TX>(m, n, sweep_grid(ATs), sweep_grid(As), resident_);
+    const bool cluster = resident_ok_ && resident_cached_ && sweep_grid(ATs) <= kBlock &&
+                         sweep_grid(As) <= kBlock && allow_cluster_gk(smem);
+    for (int k = 0, tested = 0; k < max_steps;) {
+      // One cluster launch takes the steps that most small LPs need, then two chunks at a time.
+      const int want = !cluster ? kLanczosChunk : k == 0 ? 6 * kLanczosChunk : 2 * kLanczosChunk;
+      const int c    = std::min(want, max_steps - k);
+      if (cluster) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[1];
+        cluster_config(cfg, attr, smem);
+        B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_gk_kernel<TX>, ATs, As, u.data(), v.data(),
+                                           st.data(), alphas.data(), betas.data(), c, m, n,
+                                           resident_, (const unsigned char*)images_.data()));
+        ++launches_;
+      } else {
+        for (int i = 0; i < c; ++i) {
+          gk_sweep_kernel<0, TX, gk_primal_epi><<<sweep_grid(ATs), kBlock, 0, s_>>>(
+            ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data(), st.data(),
+            alphas.data());
+          gk_sweep_kernel<1, TX, gk_dual_epi><<<sweep_grid(As), kBlock, 0, s_>>>(
+            As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data(), st.data(),
+            betas.data());
+        }
+        launches_ += 2.0 * c;
       }
-      launches_ += 2.0 * c;
       B200_LAUNCH_CHECK();
       k += c;
       alphas.download(ha.data(), k, s_);
       betas.download(hb.data(), k + 1, s_);
       B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-      // betas[0] holds |z0|; the recurrence coefficients are betas[1..].
-      if (test(k, ha.data(), hb.data() + 1)) break;
+      // betas[0] holds |z0|; the recurrence coefficients are betas[1..].  Tested at every chunk,
+      // however many a launch took.
+      while (tested < k) {
+        tested      = std::min(tested + kLanczosChunk, k);
+        int at      = tested;
+        if (test(at, ha.data(), hb.data() + 1)) return;
+      }
     }
+  }
+  bool allow_cluster_gk(size_t smem)
+  {
+    const void* fn = (const void*)cluster_gk_kernel<TX>;
+    if (smem > max_dynamic_smem(fn)) return false;
+    if (resident_.blocks > 8 &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    allow_max_dynamic_smem(fn);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    cluster_config(cfg, attr, smem);
+    int clusters  = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
+                    clusters > 0;
+    (void)cudaGetLastError();
+    return ok;
   }
 
   // ------------------------------------------------------------------ iteration kernels
@@ -829,7 +870,7 @@ class engine {
     const bool ok   = coop && persist_grid_ > 0 && sell;
     pctl_.resize(1);
     pctl_.zero(s_);
-    const bool cl_ok = p_.persistent != 0 && sell && prepare_resident();
+    const bool cl_ok = sell && resident_ok_;
     form_key_ = form_key{in_.m, in_.n, L_.nnz, dev, (int)sizeof(TX)};
     int known = -1;
     for (double& u : form_us_) u = 0.0;
@@ -852,12 +893,12 @@ class engine {
     return cached ? (const void*)resident_plain_kernel<TX, true>
                   : (const void*)resident_plain_kernel<TX, false>;
   }
-  void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1]) const
+  void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1], size_t smem) const
   {
     cfg                              = cudaLaunchConfig_t{};
     cfg.gridDim                      = dim3(resident_.blocks);
     cfg.blockDim                     = dim3(kResidentThreads);
-    cfg.dynamicSmemBytes             = cluster_smem_;
+    cfg.dynamicSmemBytes             = smem;
     cfg.stream                       = s_;
     attr[0].id                       = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x         = resident_.blocks;
@@ -913,7 +954,7 @@ class engine {
         cluster_smem_    = smem;
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
-        cluster_config(cfg, attr);
+        cluster_config(cfg, attr, smem);
         int clusters  = 0;
         const bool ok = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
                         clusters > 0;
@@ -945,7 +986,7 @@ class engine {
                   y_.data(),    kept_yhat(), scalars_.data(), 0};
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
-    cluster_config(cfg, attr);
+    cluster_config(cfg, attr, cluster_smem_);
     auto* fn = resident_cached_ ? resident_plain_kernel<TX, true> : resident_plain_kernel<TX, false>;
     B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, AT, A, pe, de, L, (int)keep, in_.m, in_.n,
                                        resident_, (const unsigned char*)images_.data(),
@@ -1580,7 +1621,7 @@ class engine {
   double form_us_[3] = {0, 0, 0};  // the timings behind the choice (this solve's or cached)
   size_t cluster_smem_ = 0;         // dynamic shared memory of the cluster form
   resident_dims resident_;          // its blocks and their shares (none without resident_cached_)
-  bool resident_cached_ = false;
+  bool resident_ok_ = false, resident_cached_ = false;
   dbuf<unsigned char> images_;
   // x_hat, y_hat and the slack of the last keeping step are in buffer kept_in_: 0 is xhat_, yhat_,
   // slack_; the cluster form alternates with these.
