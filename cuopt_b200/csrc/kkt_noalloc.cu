@@ -119,16 +119,25 @@ __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwar
         l = u = CUDART_NAN;  // and it contributes nothing (below)
       }
     }
+    // Four elements a lane at a time, so that their loads, then their gathers, are in flight together.
     double ax = 0.0;
-#pragma unroll 2
-    for (int k = b + sub; k < e; k += G) {
-      const int j    = p.idx[k];
-      const double a = p.val[k];
-      if ((unsigned)j >= (unsigned)p.n) {
-        atomicAdd(&g_na.bad, 1u);
-      } else {
-        ax += a * p.x[j];
-        atomicAdd(g_na.aty + j, a * yi);
+    for (int k = b + sub; k < e; k += 4 * G) {
+      int j[4];
+      double a[4], xj[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) j[q] = k + q * G < e ? p.idx[k + q * G] : -1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = k + q * G < e ? p.val[k + q * G] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) xj[q] = (unsigned)j[q] < (unsigned)p.n ? p.x[j[q]] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if ((unsigned)j[q] < (unsigned)p.n) {
+          ax += a[q] * xj[q];
+          atomicAdd(g_na.aty + j[q], a[q] * yi);
+        } else if (k + q * G < e) {
+          atomicAdd(&g_na.bad, 1u);
+        }
       }
     }
 #pragma unroll
