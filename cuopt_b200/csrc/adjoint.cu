@@ -308,7 +308,9 @@ void solution_adjoint_batch(const std::vector<adjoint_job>& jobs)
       sys.push_back(active_operator(p, a, false, std::move(gR)));  // M mu = g_R
     }
   }
+  trace("adjoint: active sets");
   const std::vector<lsqr_result> res = solve_all(sys);
+  trace("adjoint: solves");
   for (size_t t = 0; t < jobs.size(); ++t) {
     const adjoint_job& J = jobs[t];
     const lp_problem& p  = *J.p;

@@ -8,8 +8,8 @@
 // boundaries and a reduction per system per iteration if each iteration were a grid-wide launch,
 // so instead every system gets one thread-block cluster that runs its whole LSQR loop:
 //   * every block of the cluster holds a copy of u (rows) and v (cols) in shared memory, gathers
-//     from it, and sends each new entry to every block's copy through distributed shared memory;
-//     x and w are kept by the block that owns their column;
+//     from it, and sends each new entry to every block's copy with st.async, whose bytes count
+//     towards the receiving block's mbarrier; x and w are kept by the block that owns their column;
 //   * the operator and its transpose are stored as 32-row sliced ELL (lane t of a warp owns row t
 //     of a slice and reads element k at base + 32 k + t), rows sorted by length; slice s belongs to
 //     block s % C, whose share is copied into its shared memory (16-bit indices) where it fits, so
@@ -17,13 +17,15 @@
 //   * the two norms of an iteration are sums of per-warp sums, sent to every block with the vector
 //     entries and added in a fixed order by every warp, so the scalar recurrence and the stopping
 //     decision are uniform, the result is deterministic, and an iteration costs two products and
-//     two cluster barriers (hardware, no spin loop);
+//     two exchanges.  Every warp sends its sums after its gathers, so a block that has all of one
+//     exchange knows that every warp is done reading the vector written next;
 //   * the x / w update of an iteration is applied in the next transpose product by the thread that
 //     owns the row.
 // One block per system, reading the operator from L2, took 33 us an iteration on the 5000 x 5000
 // systems.  Systems whose vectors do not fit (some 14 000 rows and columns) still run in one block
 // each, with u, v, x and w in global memory.
-// Each cluster stops at LSQR's tests or at its iteration limit: none waits for another.
+// Each cluster stops at LSQR's tests or at its iteration limit: none waits for another, and a wait
+// for an exchange is bounded (its end without one is reported as an error).
 #include "common.cuh"
 #include "lsqr.hpp"
 
@@ -39,7 +41,13 @@ namespace {
 
 constexpr int kLsqrThreads = 512;
 constexpr int kLsqrWarps   = kLsqrThreads / kWarp;
+// Blocks of a cluster: 8 warps, so that a thread has the registers for eight elements in flight, its
+// row's state and the remote addresses (with 16 warps some 500 bytes of it spilled).
+constexpr int kClThreads = 256;
+constexpr int kClWarps   = kClThreads / kWarp;
 constexpr int kEquilibrationPasses = 10;
+constexpr int kLsqrPolls = 1 << 22;   // polls of one exchange
+constexpr int kLsqrFailed = -1;       // flag of a system whose exchange did not complete
 
 struct lsqr_desc {
   int rows, cols;           // u has `rows` entries, v / x / w have `cols`
@@ -66,7 +74,7 @@ struct lsqr_out {
 };
 
 // Sum over the block of K per-thread values; every thread gets the same totals (fixed order).
-template <int K>
+template <int K, int WARPS = kLsqrWarps>
 __device__ __forceinline__ void block_sums(const double (&v)[K], double* part, double (&out)[K])
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -79,7 +87,7 @@ __device__ __forceinline__ void block_sums(const double (&v)[K], double* part, d
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     double s = 0.0;
-    for (int w = 0; w < kLsqrWarps; ++w) s += part[w * K + q];
+    for (int w = 0; w < WARPS; ++w) s += part[w * K + q];
     out[q] = s;
   }
 }
@@ -229,7 +237,7 @@ struct lsqr_smem {
   B200_HD lsqr_smem(int rows, int cols, int slices_p, int slices_q, int64_t elems_p,
                     int64_t elems_q, int C, bool cached)
   {
-    size_t at    = pad((size_t)rows * 8);
+    size_t at    = 16 + pad((size_t)rows * 8);  // two barriers, u
     auto take    = [&](size_t b) {
       const size_t here = at;
       at += pad(b);
@@ -239,8 +247,8 @@ struct lsqr_smem {
     v      = take((size_t)cols * 8);
     x      = take(nq * kWarp * 8);
     w      = take(nq * kWarp * 8);
-    part_a = take((size_t)C * kLsqrWarps * 8);
-    part_b = take((size_t)C * kLsqrWarps * 16);
+    part_a = take((size_t)C * kClWarps * 8);
+    part_b = take((size_t)C * kClWarps * 16);
     tab[0] = take(cached ? np * 8 : 0);
     tab[1] = take(cached ? nq * 8 : 0);
     val[0] = take(cached ? (size_t)elems_p * 8 : 0);
@@ -265,27 +273,54 @@ __device__ __forceinline__ void lsqr_barrier()
     "barrier.cluster.wait.acquire.aligned;\n" ::
       : "memory");
 }
-// Stores v at `p`'s place in block c of the cluster.
-__device__ __forceinline__ void send(const double* p, unsigned c, double v)
+// The phase of `bar` that ends once `bytes` more have arrived (one call a phase, by one thread).
+__device__ __forceinline__ void expect_bytes(unsigned bar, unsigned bytes)
 {
-  unsigned remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-               : "=r"(remote)
-               : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(c));
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool wait_bytes(unsigned bar, unsigned parity)
+{
+  for (int i = 0; i < kLsqrPolls; ++i) {
+    unsigned ok;
+    asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void send_bytes(unsigned to, unsigned bar, double v)
+{
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(
+                 to),
+               "d"(v), "r"(bar)
+               : "memory");
+}
+// Stores v at offset `off` of every block, counted by its barrier at offset `bar`.
+template <int C>
+__device__ __forceinline__ void send_all(const unsigned (&base)[C], unsigned off, unsigned bar, double v)
+{
+#pragma unroll
+  for (int c = 0; c < C; ++c) send_bytes(base[c] + off, base[c] + bar, v);
 }
 
-// Sends this warp's sums of K per-thread values to every block (lane c to block c of C <= 16); after
-// the next cluster barrier, cluster_totals adds them in one order everywhere.
-template <int K>
-__device__ __forceinline__ void send_sums(const double (&v)[K], const double* part, unsigned rank,
-                                          int C)
+// Sends this warp's sums of K per-thread values to every block (lane c to block c; `mine`: that
+// block's base address); once they are in, cluster_totals adds them in one order everywhere.
+template <int K, int C>
+__device__ __forceinline__ void send_sums(const double (&v)[K], unsigned mine, unsigned part,
+                                          unsigned bar, unsigned rank)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     const double s = warp_sum(v[q]);
-    if (lane < C) send(part + ((size_t)q * C + rank) * kLsqrWarps + warp, lane, s);
+    if (lane < C)
+      send_bytes(mine + part + 8u * ((q * C + rank) * kClWarps + warp), mine + bar, s);
   }
 }
 template <int K>
@@ -295,23 +330,23 @@ __device__ __forceinline__ void cluster_totals(const double* part, int C, double
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     double s = 0.0;
-    for (int i = lane; i < C * kLsqrWarps; i += kWarp) s += part[q * C * kLsqrWarps + i];
+    for (int i = lane; i < C * kClWarps; i += kWarp) s += part[q * C * kClWarps + i];
     out[q] = warp_sum(s);
   }
 }
 
-template <bool CACHED>
-__global__ void __launch_bounds__(kLsqrThreads, 1)
-  lsqr_cluster_kernel(const lsqr_desc* __restrict__ descs, lsqr_out* __restrict__ outs, int C)
+template <int C, bool CACHED>
+__global__ void __launch_bounds__(kClThreads, 1)
+  lsqr_cluster_kernel(const lsqr_desc* __restrict__ descs, lsqr_out* __restrict__ outs)
 {
   extern __shared__ __align__(16) unsigned char dyn[];
   const unsigned rank = lsqr_rank();
   const int system    = (int)blockIdx.x / C;
   const lsqr_desc d   = descs[system];
   const lsqr_smem S(d.rows, d.cols, d.slices_p, d.slices_q, d.share_p, d.share_q, C, CACHED);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = kLsqrThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, T = kClThreads;
   auto at        = [&](size_t o) { return reinterpret_cast<double*>(dyn + o); };
-  double *u = at(0), *v = at(S.v), *x = at(S.x), *w = at(S.w);
+  double *u = at(16), *v = at(S.v), *x = at(S.x), *w = at(S.w);
   double *part_a = at(S.part_a), *part_b = at(S.part_b);
   const int np = (d.slices_p + C - 1) / C, nq = (d.slices_q + C - 1) / C;
 
@@ -334,7 +369,7 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
         }
       }
       __syncthreads();
-      for (int i = warp; i < n; i += kLsqrWarps) {
+      for (int i = warp; i < n; i += kClWarps) {
         const int s = (int)rank + C * i;
         if (s >= slices) break;
         const int64_t base = so[s];
@@ -350,27 +385,40 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
   auto products = [&](int m, const double* vec, auto&& f) {
     const int n = m == 0 ? np : nq, slices = m == 0 ? d.slices_p : d.slices_q;
     const int rows = m == 0 ? d.rows : d.cols;
-    for (int i = warp; i < n; i += kLsqrWarps) {
+    for (int i = warp; i < n; i += kClWarps) {
       const int s = (int)rank + C * i;
       if (s >= slices) break;
-      double acc = 0.0;
-      if constexpr (CACHED) {
-        const int2 t             = reinterpret_cast<const int2*>(dyn + S.tab[m])[i];
-        const double* vp         = at(S.val[m]) + t.x + lane;
-        const unsigned short* ip = reinterpret_cast<const unsigned short*>(dyn + S.idx[m]) + t.x +
-                                   lane;
-#pragma unroll 4
-        for (int k = 0; k < t.y; ++k) acc += vp[kWarp * k] * vec[ip[kWarp * k]];
-      } else {
-        const int64_t* so  = m == 0 ? d.p_slice : d.q_slice;
-        const int64_t base = so[s];
-        const int len      = (int)((so[s + 1] - base) >> 5);
-        const int* ip      = (m == 0 ? d.p_idx : d.q_idx) + base + lane;
-        const double* vp   = (m == 0 ? d.p_val : d.q_val) + base + lane;
-#pragma unroll 4
-        for (int k = 0; k < len; ++k) acc += vp[kWarp * k] * vec[ip[kWarp * k]];
-      }
       const int r = s * kWarp + lane;
+      double acc  = 0.0;
+      // Eight elements at a time, so that their loads, then their gathers, are in flight together.
+      auto sum = [&](const double* vp, const auto* ip, int len) {
+        for (int k = 0; k < len; k += 8) {
+          int j[8];
+          double a[8], g[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (k + e < len) {
+              j[e] = ip[kWarp * (k + e)];
+              a[e] = vp[kWarp * (k + e)];
+            }
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (k + e < len) g[e] = vec[j[e]];
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (k + e < len) acc += a[e] * g[e];
+        }
+      };
+      if constexpr (CACHED) {
+        const int2 t = reinterpret_cast<const int2*>(dyn + S.tab[m])[i];
+        sum(at(S.val[m]) + t.x + lane,
+            reinterpret_cast<const unsigned short*>(dyn + S.idx[m]) + t.x + lane, t.y);
+      } else {
+        const int64_t base = (m == 0 ? d.p_slice : d.q_slice)[s];
+        const int len      = (int)(((m == 0 ? d.p_slice : d.q_slice)[s + 1] - base) >> 5);
+        sum((m == 0 ? d.p_val : d.q_val) + base + lane, (m == 0 ? d.p_idx : d.q_idx) + base + lane,
+            len);
+      }
       if (r < rows) f(i, r, acc);
     }
   };
@@ -382,7 +430,7 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
     u[r]            = bv;
     t1[0] += bv * bv;
   }
-  block_sums<1>(t1, part_a, r1);
+  block_sums<1, kClWarps>(t1, part_a, r1);
   __syncthreads();  // part_a is read before other blocks write it
   double beta        = sqrt(r1[0]);
   const double bnorm = beta;
@@ -393,20 +441,46 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
     }
     return;
   }
-  // Every block of the cluster is running before any stores into another's shared memory.
+  // Exchanges of u (after P's products) and of v (after Q's): every entry and every warp's sums, to
+  // every block.
+  const unsigned home = (unsigned)__cvta_generic_to_shared(dyn), bar_u = home, bar_v = home + 8;
+  unsigned base[C], mine = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(home), "r"(c));
+    if (lane == c) mine = base[c];
+  }
+  const unsigned bytes_u = 8u * (d.rows + C * kClWarps), bytes_v = 8u * (d.cols + 2 * C * kClWarps);
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_u) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_v) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    expect_bytes(bar_u, bytes_u);
+    expect_bytes(bar_v, bytes_v - 8u * C * kClWarps);  // the first one has a single sum
+  }
+  unsigned phase_u = 0, phase_v = 0;
+  bool ok          = true;
+  auto wait_v = [&]() {
+    if (!(ok = wait_bytes(bar_v, phase_v))) return false;
+    phase_v ^= 1;
+    if (threadIdx.x == 0) expect_bytes(bar_v, bytes_v);
+    return true;
+  };
+  // Every block of the cluster is running, with its barriers, before any stores into another's
+  // shared memory.
   lsqr_barrier();
   double us = 1.0 / beta;  // the normalised u is u * us
   // v = Op^T u / beta, alpha = |v|; x = w = 0 (w becomes v_1 in the first transpose product)
   t1[0] = 0.0;
   products(1, u, [&](int i, int j, double acc) {
     const double vj = acc * us;
-    for (int c = 0; c < C; ++c) send(v + j, c, vj);
+    send_all<C>(base, (unsigned)S.v + 8u * j, 8, vj);
     x[i * kWarp + lane] = 0.0;
     w[i * kWarp + lane] = 0.0;
     t1[0] += vj * vj;
   });
-  send_sums<1>(t1, part_b, rank, C);
-  lsqr_barrier();
+  send_sums<1, C>(t1, mine, (unsigned)S.part_b, 8, rank);
+  wait_v();
   cluster_totals<1>(part_b, C, r1);
   double alpha  = sqrt(r1[0]);
   double vs     = alpha > 0.0 ? 1.0 / alpha : 0.0;
@@ -414,7 +488,9 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
   double c1 = 0.0, c2 = 0.0;  // pending update: x += c1 w; w = v - c2 w
   double rnorm = beta, arnorm = alpha * beta;
   int flag = 3, it = 0;
-  if (!(alpha > 0.0)) {
+  if (!ok) {
+    flag = kLsqrFailed;
+  } else if (!(alpha > 0.0)) {
     flag = 2;  // Op^T b = 0: z = 0 is the least-squares solution
   } else {
     for (it = 1; it <= d.max_iter; ++it) {
@@ -422,11 +498,13 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
       t1[0] = 0.0;
       products(0, v, [&](int, int r, double acc) {
         const double un = acc * vs - alpha * (u[r] * us);
-        for (int c = 0; c < C; ++c) send(u + r, c, un);
+        send_all<C>(base, 16 + 8u * r, 0, un);
         t1[0] += un * un;
       });
-      send_sums<1>(t1, part_a, rank, C);
-      lsqr_barrier();
+      send_sums<1, C>(t1, mine, (unsigned)S.part_a, 0, rank);
+      if (!(ok = wait_bytes(bar_u, phase_u))) break;
+      phase_u ^= 1;
+      if (threadIdx.x == 0) expect_bytes(bar_u, bytes_u);
       cluster_totals<1>(part_a, C, r1);
       beta = sqrt(r1[0]);
       us   = beta > 0.0 ? 1.0 / beta : 0.0;
@@ -442,12 +520,12 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
         x[q]            = xj;
         w[q]            = wj;
         const double vn = acc * us - beta * vo;
-        for (int c = 0; c < C; ++c) send(v + j, c, vn);
+        send_all<C>(base, (unsigned)S.v + 8u * j, 8, vn);
         t2[0] += vn * vn;
         t2[1] += xj * xj;
       });
-      send_sums<2>(t2, part_b, rank, C);
-      lsqr_barrier();
+      send_sums<2, C>(t2, mine, (unsigned)S.part_b, 8, rank);
+      if (!wait_v()) break;
       cluster_totals<2>(part_b, C, r2);
       alpha = sqrt(r2[0]);
       vs    = alpha > 0.0 ? 1.0 / alpha : 0.0;
@@ -477,14 +555,20 @@ __global__ void __launch_bounds__(kLsqrThreads, 1)
         break;
       }
     }
+    if (!ok) flag = kLsqrFailed;
     if (it > d.max_iter) it = d.max_iter;
   }
+  // Every exchange that was sent to this block is in (each is waited for before the next); after a
+  // failed one, all blocks end theirs before any leaves.
+  __syncthreads();
+  lsqr_barrier();
   // The last pending x update, then the result.
-  for (int i = warp; i < nq; i += kLsqrWarps) {
+  for (int i = warp; i < nq; i += kClWarps) {
     const int j = ((int)rank + C * i) * kWarp + lane, q = i * kWarp + lane;
     if (j < d.cols) d.z[j] = x[q] + c1 * w[q];
   }
-  if (rank == 0 && threadIdx.x == 0) outs[system] = lsqr_out{it, flag, rnorm, arnorm};
+  if (threadIdx.x == 0 && (rank == 0 || flag == kLsqrFailed))
+    outs[system] = lsqr_out{it, flag, rnorm, arnorm};
 }
 
 // Host-side packing of one problem: equilibration, transposition, row sorting, sliced ELL.
@@ -642,7 +726,7 @@ struct cluster_plan {
   {
     cfg                      = cudaLaunchConfig_t{};
     cfg.gridDim              = dim3(systems * blocks);
-    cfg.blockDim             = dim3(kLsqrThreads);
+    cfg.blockDim             = dim3(kClThreads);
     cfg.dynamicSmemBytes     = smem;
     cfg.stream               = s;
     attr[0].id               = cudaLaunchAttributeClusterDimension;
@@ -654,23 +738,38 @@ struct cluster_plan {
   }
 };
 
+using cluster_kernel_t = void (*)(const lsqr_desc*, lsqr_out*);
+cluster_kernel_t cluster_kernel(int blocks, bool cached)
+{
+  switch (blocks) {
+    case 1: return cached ? lsqr_cluster_kernel<1, true> : lsqr_cluster_kernel<1, false>;
+    case 2: return cached ? lsqr_cluster_kernel<2, true> : lsqr_cluster_kernel<2, false>;
+    case 4: return cached ? lsqr_cluster_kernel<4, true> : lsqr_cluster_kernel<4, false>;
+    case 8: return cached ? lsqr_cluster_kernel<8, true> : lsqr_cluster_kernel<8, false>;
+    default: return cached ? lsqr_cluster_kernel<16, true> : lsqr_cluster_kernel<16, false>;
+  }
+}
+
 // The plan with the least estimated time: waves of clusters, each iteration of one taking about
-// 1.2 us for its barriers and sums plus the products, shared by its blocks (0.16 ns per non-zero
-// and product from shared memory, 0.4 ns from L2).
+// 0.9 us for its exchanges' latency and sums, 0.3 ns for each entry of u and v (a block takes them in
+// at some 16 bytes a cycle), and the products, shared by its blocks (0.16 ns per non-zero and product
+// from shared memory, 0.4 ns from L2).
 cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>& ids, size_t limit)
 {
   cluster_plan best;
   if (ids.empty()) return best;
-  double nnz = 0.0, best_us = 0.0;
-  for (int i : ids) nnz += (double)(pk[i].p_val.size() + pk[i].q_val.size()) / ids.size();
+  double nnz = 0.0, entries = 0.0, best_us = 0.0;
+  for (int i : ids) {
+    nnz += (double)(pk[i].p_val.size() + pk[i].q_val.size()) / ids.size();
+    entries += (double)(pk[i].rows + pk[i].cols) / ids.size();
+  }
   for (const bool cached : {true, false})
     for (const int c : {16, 8, 4, 2, 1}) {
       cluster_plan p;
       p.blocks = c;
       p.cached = cached;
       for (int i : ids) p.smem = std::max(p.smem, cluster_smem(pk[i], c, cached));
-      const void* fn = cached ? (const void*)lsqr_cluster_kernel<true>
-                              : (const void*)lsqr_cluster_kernel<false>;
+      const void* fn = (const void*)cluster_kernel(c, cached);
       if (p.smem > limit) continue;
       if (c > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
                      cudaSuccess) {
@@ -687,7 +786,8 @@ cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>
         continue;
       }
       const double waves = std::ceil((double)ids.size() / active);
-      const double us    = waves * (1.2 + nnz * (cached ? 1.6e-4 : 4e-4) / c);
+      const double us    = waves * (0.9 + (c > 1 ? entries * 3e-4 : 0.0) +
+                                 nnz * (cached ? 1.6e-4 : 4e-4) / c);
       if (best.smem == 0 || us < best_us) {
         best    = p;
         best_us = us;
@@ -714,10 +814,10 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
       if (p.idx[e] < 0 || p.idx[e] >= p.cols) throw std::invalid_argument("lsqr: column out of range");
   }
   parallel_for(count, [&](int i) { pack(*ps[i], pk[i]); });
+  trace("lsqr: packing");
 
   // Systems with work go to the device: those whose vectors fit in a cluster's blocks, and the rest.
-  const size_t limit = std::min(max_dynamic_smem((const void*)lsqr_cluster_kernel<true>),
-                                max_dynamic_smem((const void*)lsqr_cluster_kernel<false>));
+  const size_t limit = max_dynamic_smem((const void*)cluster_kernel(16, true));
   std::vector<int> clus_ids, glob_ids;
   size_t scratch_doubles = 0;
   for (int i = 0; i < count; ++i) {
@@ -818,19 +918,20 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   dbuf<lsqr_desc> d_desc(h_desc.size());
   dbuf<lsqr_out> d_out(h_desc.size());
   d_desc.upload(h_desc.data(), h_desc.size(), s);
+  trace_sync(s, "lsqr: upload");
   const int n_clus = (int)clus_ids.size(), n_glob = (int)glob_ids.size();
   if (n_clus > 0) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
     plan.configure(cfg, attr, n_clus, s);
-    auto* fn = plan.cached ? lsqr_cluster_kernel<true> : lsqr_cluster_kernel<false>;
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, (const lsqr_desc*)d_desc.data(), d_out.data(),
-                                       plan.blocks));
+    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_kernel(plan.blocks, plan.cached),
+                                       (const lsqr_desc*)d_desc.data(), d_out.data()));
   }
   if (n_glob > 0) {
     lsqr_kernel<<<n_glob, kLsqrThreads, 0, s>>>(d_desc.data() + n_clus, d_out.data() + n_clus);
     B200_LAUNCH_CHECK();
   }
+  trace_sync(s, "lsqr: kernel");
   std::vector<double> h_z(n_z);
   std::vector<lsqr_out> h_out(h_desc.size());
   d_z.download(h_z.data(), n_z, s);
@@ -846,6 +947,8 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
     }
     r.iterations = h_out[k].iterations;
     r.flag       = h_out[k].flag;
+    if (r.flag == kLsqrFailed)
+      throw cuda_error("lsqr: an exchange between blocks passed its poll limit");
     r.rnorm      = h_out[k].rnorm;
     r.arnorm     = h_out[k].arnorm;
   }
