@@ -247,16 +247,40 @@ __device__ __forceinline__ T gather_load(const T* __restrict__ g, int i)
     return g[i];
 }
 
-// The strands of a wide row (elements [b, e)): this warp's, and all of them on one warp.
+// Sum over elements k = first, first + STRIDE, ... below `end` of a row, in that order: U of them
+// are loaded at a time (also the last, incomplete batch), so a row is a chain of ceil(count / U)
+// rounds of two dependent loads and not of one per element left over.
+template <int U, int STRIDE, bool COH, typename TM, typename TG>
+__device__ __forceinline__ double strided_product(const dev_sell<TM>& A, const TG* __restrict__ g,
+                                                  int64_t first, int64_t end)
+{
+  double acc = 0.0;
+  for (int64_t k = first; k < end; k += U * STRIDE) {
+    const int left = (int)(end - k);
+    int x[U];
+    TM v[U];
+    TG w[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) x[q] = q * STRIDE < left ? ld_stream(A.idx + k + q * STRIDE) : 0;
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (q * STRIDE < left) v[q] = ld_stream(A.val + k + q * STRIDE);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (q * STRIDE < left) w[q] = gather_load<COH>(g, x[q]);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (q * STRIDE < left) acc += (double)v[q] * (double)w[q];
+  }
+  return acc;
+}
+// The strands of a wide row: this warp's, and all of them on one warp.
 template <bool COH, typename TM, typename TG>
 __device__ __forceinline__ double wide_strand(const dev_sell<TM>& A, const TG* __restrict__ g,
                                               int64_t b, int64_t e, int strand)
 {
-  double acc = 0.0;
-#pragma unroll 4
-  for (int64_t k = b + strand * kWarp + (threadIdx.x & 31); k < e; k += kWideStrands * kWarp)
-    acc += (double)ld_stream(A.val + k) * (double)gather_load<COH>(g, ld_stream(A.idx + k));
-  return warp_sum(acc);
+  return warp_sum(strided_product<4, kWideStrands * kWarp, COH>(
+    A, g, b + strand * kWarp + (threadIdx.x & 31), e));
 }
 template <class Load>
 __device__ __forceinline__ double wide_row_by_warp(int len, Load&& term)
@@ -273,10 +297,14 @@ __device__ __forceinline__ double wide_row_by_warp(int len, Load&& term)
   for (int q = 0; q < kWideStrands; ++q) sum += warp_sum(acc[q]);
   return sum;
 }
-// Barrier of one group of kWideStrands warps of the block (group g of up to 15).
-__device__ __forceinline__ void wide_barrier(int g)
+// Barrier of one group (0 or 1) of kWideStrands warps of the block.  The barriers are named by
+// constants: with a register, the compiler reserves all 16 for the block.
+__device__ __forceinline__ void wide_barrier(int group)
 {
-  asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(kWideStrands* kWarp) : "memory");
+  if (group == 0)
+    asm volatile("bar.sync 1, %0;" ::"n"(kWideStrands* kWarp) : "memory");
+  else
+    asm volatile("bar.sync 2, %0;" ::"n"(kWideStrands* kWarp) : "memory");
 }
 
 // WPB: warps (rows or slices) per block.  Only the grouping of warps into blocks depends on it,
@@ -336,10 +364,7 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
     if (q < A.long_count() && !skip_rows(epi, row, row)) {
       const auto pre  = epi.load(row);
       const int64_t b = A.long_off[row], e = A.long_off[row + 1];
-      double acc      = 0.0;
-      for (int64_t k = b + lane; k < e; k += kWarp)
-        acc += (double)ld_stream(A.val + k) * (double)gather_load<COH>(g, ld_stream(A.idx + k));
-      acc = warp_sum(acc);
+      const double acc = warp_sum(strided_product<4, kWarp, COH>(A, g, b + lane, e));
       if (lane == 0) epi(row, acc, pre, red);
     }
   } else {
@@ -355,9 +380,13 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
       const TM* v        = A.val + base + lane * kChunk;
       const int* ix      = A.idx + base + lane * kChunk;
       double acc         = 0.0;
-      int q              = 0;
+      // Two chunks at a time; the indices of the next two are loaded while these are gathered, so a
+      // round waits for its gathers alone.
+      int4 i0 = make_int4(0, 0, 0, 0), i1 = i0;
+      if (nchunk > 0) i0 = load_idx_chunk(ix);
+      if (nchunk > 1) i1 = load_idx_chunk(ix + 32 * kChunk);
+      int q = 0;
       for (; q + 2 <= nchunk; q += 2) {
-        const int4 i0 = load_idx_chunk(ix), i1 = load_idx_chunk(ix + 32 * kChunk);
         double v0[4], v1[4];
         load_chunk(v, v0);
         load_chunk(v + 32 * kChunk, v1);
@@ -365,6 +394,10 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
         const TG g2 = gather_load<COH>(g, i0.z), g3 = gather_load<COH>(g, i0.w);
         const TG g4 = gather_load<COH>(g, i1.x), g5 = gather_load<COH>(g, i1.y);
         const TG g6 = gather_load<COH>(g, i1.z), g7 = gather_load<COH>(g, i1.w);
+        v += 64 * kChunk;
+        ix += 64 * kChunk;
+        if (q + 2 < nchunk) i0 = load_idx_chunk(ix);
+        if (q + 3 < nchunk) i1 = load_idx_chunk(ix + 32 * kChunk);
         acc += v0[0] * (double)g0;
         acc += v0[1] * (double)g1;
         acc += v0[2] * (double)g2;
@@ -373,11 +406,8 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
         acc += v1[1] * (double)g5;
         acc += v1[2] * (double)g6;
         acc += v1[3] * (double)g7;
-        v += 64 * kChunk;
-        ix += 64 * kChunk;
       }
       if (q < nchunk) {
-        const int4 i0 = load_idx_chunk(ix);
         double v0[4];
         load_chunk(v, v0);
         const TG g0 = gather_load<COH>(g, i0.x), g1 = gather_load<COH>(g, i0.y);
@@ -393,8 +423,12 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
   block_reduce_store<K, has_max_red<Epi>::value>(red, partials, vb);
 }
 
+// Resident blocks of 256 threads the sweeps are compiled for: 5 an SM with FP32 matrices (48
+// registers), 4 with FP64 (64; at 48 some spill, and left alone they take up to 78).
+template <typename TM>
+constexpr int kSweepBlocks = sizeof(TM) == 4 ? 5 : 4;
 template <typename TM, typename TG, class Epi>
-__global__ void __launch_bounds__(kBlock) sell_map_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_kernel(const dev_sell<TM> A,
                                                           const TG* __restrict__ g, Epi epi,
                                                           double* partials)
 {
@@ -404,7 +438,7 @@ __global__ void __launch_bounds__(kBlock) sell_map_kernel(const dev_sell<TM> A,
 // Blocks vb0, vb0 + 1, ... of a sweep's grid only (measurement of one row-length class: the
 // long rows are blocks [0, long_blocks), the slices the rest).
 template <typename TM, typename TG, class Epi>
-__global__ void __launch_bounds__(kBlock) sell_map_range_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_range_kernel(const dev_sell<TM> A,
                                                                 const TG* __restrict__ g, Epi epi,
                                                                 double* partials, int vb0)
 {
@@ -413,7 +447,7 @@ __global__ void __launch_bounds__(kBlock) sell_map_range_kernel(const dev_sell<T
 
 // The same sweep with WPB warps per block (the plain sweeps' block shape is autotuned).
 template <typename TM, typename TG, class Epi, int WPB>
-__global__ void __launch_bounds__(WPB * kWarp) sell_map_wpb_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(WPB * kWarp, kSweepBlocks<TM> * kWarpsPerBlock / WPB) sell_map_wpb_kernel(const dev_sell<TM> A,
                                                                   const TG* __restrict__ g,
                                                                   Epi epi, double* partials)
 {
@@ -537,7 +571,7 @@ struct advance_active {
 };
 
 template <typename TX, class PE, class DE, class ADV>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 3)
   persistent_plain_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, const TX* y, const TX* xbar,
                           PE pe, DE de, ADV adv, int L, int grid_p, int grid_d, persist_ctl* ctl,
                           unsigned long long budget_ns)
@@ -1247,7 +1281,7 @@ struct term_dual_epi {
 // (with the two error flags behind them, see enqueue_conv).  As two sweeps, two one-block sums and
 // a copy this took five stream operations per check; on a 2000 x 5000 LP they were the longer part
 // of it.  arrived must be 0 before the launch and is 0 after it.
-static __global__ void __launch_bounds__(kBlock)
+static __global__ void __launch_bounds__(kBlock, kSweepBlocks<double>)
   term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
               const double* __restrict__ yu, term_primal_epi ep, term_dual_epi ed, int gp, int gd,
               double* partials, unsigned* arrived, double* out, double* host, const int* flag_a,
@@ -1422,7 +1456,7 @@ static __global__ void gk_start_kernel(gk_state* st, const double* sumsq, double
 // A step is two launches; with the sum and its recording as kernels of their own it was six, and
 // on a 12k x 30k LP those four one-block kernels were the larger part of it.
 template <int FIELD, typename TM, class Epi>
-__global__ void __launch_bounds__(kBlock) gk_sweep_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) gk_sweep_kernel(const dev_sell<TM> A,
                                                           const double* __restrict__ g, Epi epi,
                                                           double* partials, gk_state* st,
                                                           double* hist)
