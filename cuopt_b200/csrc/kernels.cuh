@@ -621,13 +621,12 @@ struct no_sink {
   __device__ __forceinline__ void operator()(int, double) const {}
 };
 
+// w: the Halpern weight of the step (used with HALPERN).
 template <typename TX, bool MAJOR, bool HALPERN, bool SAVE_ATY, class P, class Sink = no_sink>
-__device__ __forceinline__ void primal_row_step(int j, double acc, const P& p,
-                                                const pdlp_scalars* st, int it_off, TX* xbar,
-                                                TX* xout, TX* xhat, TX* slack, TX* aty,
+__device__ __forceinline__ void primal_row_step(int j, double acc, const P& p, double tau, double w,
+                                                TX* xbar, TX* xout, TX* xhat, TX* slack, TX* aty,
                                                 const Sink& sink = Sink{})
 {
-  const double tau  = st->tau;
   const double xj   = (double)p.x;
   const double next = xj - tau * ((double)p.c - acc);
   const double cl   = fmax(fmin(next, (double)p.up), (double)p.lo);
@@ -638,30 +637,28 @@ __device__ __forceinline__ void primal_row_step(int j, double acc, const P& p,
   const double xb = 2.0 * cl - xj;
   if constexpr (SAVE_ATY) aty[j] = (TX)acc;
   if constexpr (HALPERN) {
-    const double w = halpern_weight(st, it_off);
-    xbar[j]        = (TX)xb;
-    xout[j]        = (TX)halpern_mix(w, xb, (double)p.xa);
+    xbar[j] = (TX)xb;
+    xout[j] = (TX)halpern_mix(w, xb, (double)p.xa);
   } else {
     xbar[j] = (TX)xb;
   }
   sink(j, (double)(TX)xb);
 }
 
-// The dual update of one constraint i; returns (y_bar_i - y_i)^2 for the fixed-point error.
+// The dual update of one constraint i (ratio: y_i / sigma); returns (y_bar_i - y_i)^2 for the
+// fixed-point error.
 template <typename TX, bool MAJOR, bool HALPERN, class P, class Sink = no_sink>
-__device__ __forceinline__ double dual_row_step(int i, double acc, const P& p,
-                                                const pdlp_scalars* st, int it_off, TX* ybar,
-                                                TX* yout, TX* yhat, const Sink& sink = Sink{})
+__device__ __forceinline__ double dual_row_step(int i, double acc, const P& p, double sigma,
+                                                double ratio, double w, TX* ybar, TX* yout,
+                                                TX* yhat, const Sink& sink = Sink{})
 {
-  const double sigma = st->sigma;
   const double yi    = (double)p.y;
-  const double t     = yi / sigma - acc;
+  const double t     = ratio - acc;
   const double tp    = fmax(-(double)p.up, fmin(t, -(double)p.lo));
   const double ny    = (t - tp) * sigma;
   if constexpr (MAJOR) yhat[i] = (TX)ny;
   const double yb = 2.0 * ny - yi;
   if constexpr (HALPERN) {
-    const double w  = halpern_weight(st, it_off);
     const TX y_next = (TX)halpern_mix(w, yb, (double)p.ya);
     yout[i]         = y_next;
     sink(i, (double)y_next);
@@ -670,6 +667,28 @@ __device__ __forceinline__ double dual_row_step(int i, double acc, const P& p,
   }
   const double d = yb - yi;
   return d * d;
+}
+
+// The same with the step's scalars read from `st`.
+template <typename TX, bool MAJOR, bool HALPERN, bool SAVE_ATY, class P, class Sink = no_sink>
+__device__ __forceinline__ void primal_row_step(int j, double acc, const P& p,
+                                                const pdlp_scalars* st, int it_off, TX* xbar,
+                                                TX* xout, TX* xhat, TX* slack, TX* aty,
+                                                const Sink& sink = Sink{})
+{
+  primal_row_step<TX, MAJOR, HALPERN, SAVE_ATY>(j, acc, p, st->tau,
+                                                HALPERN ? halpern_weight(st, it_off) : 0.0, xbar,
+                                                xout, xhat, slack, aty, sink);
+}
+template <typename TX, bool MAJOR, bool HALPERN, class P, class Sink = no_sink>
+__device__ __forceinline__ double dual_row_step(int i, double acc, const P& p,
+                                                const pdlp_scalars* st, int it_off, TX* ybar,
+                                                TX* yout, TX* yhat, const Sink& sink = Sink{})
+{
+  const double sigma = st->sigma;
+  return dual_row_step<TX, MAJOR, HALPERN>(i, acc, p, sigma, (double)p.y / sigma,
+                                           HALPERN ? halpern_weight(st, it_off) : 0.0, ybar, yout,
+                                           yhat, sink);
 }
 
 // Row j of A^T:  x_next = x - tau (c - A^T y);  x_hat = clamp(x_next, l, u);
@@ -810,11 +829,12 @@ struct resident_dims {
   B200_HD static size_t pad(size_t b) { return (b + 15) & ~(size_t)15; }
   // The image of a block's constant data (device memory, copied to shared memory by each launch):
   // {start, length} of the units of A^T and A, the operands c, l, u and l_c, u_c per unit lane,
-  // values and indices of A^T and A.
+  // values and indices of A^T and A, the blocks that need the entry of each unit lane of A^T and A
+  // (resident_needs_kernel), and the numbers of x_bar and y entries that this block needs.
   template <typename TX>
   B200_HD size_t image_at(int part) const
   {
-    const size_t bytes[9] = {(size_t)units[0] * 8,
+    const size_t bytes[11] = {(size_t)units[0] * 8,
                              (size_t)units[1] * 8,
                              (size_t)units[0] * 3 * kWarp * sizeof(TX),
                              (size_t)units[1] * 2 * kWarp * sizeof(TX),
@@ -822,7 +842,9 @@ struct resident_dims {
                              (size_t)elems[1] * sizeof(TX),
                              (size_t)elems[0] * 2,
                              (size_t)elems[1] * 2,
-                             0};
+                             (size_t)units[0] * kWarp * 2,
+                             (size_t)units[1] * kWarp * 2,
+                             8};
     size_t at = 0;
     for (int q = 0; q < part; ++q) at += pad(bytes[q]);
     return at;
@@ -830,7 +852,7 @@ struct resident_dims {
   template <typename TX>
   B200_HD size_t image_bytes() const
   {
-    return image_at<TX>(8);
+    return image_at<TX>(11);
   }
   // Shared memory of a launch: y, x_bar, then (CACHED) the iterates x, x_anchor, y, y_anchor per
   // unit lane and the image.
@@ -843,11 +865,6 @@ struct resident_dims {
   B200_HD size_t state_bytes() const
   {
     return (size_t)(units[0] + units[1]) * 2 * kWarp * sizeof(TX);
-  }
-  template <typename TX>
-  size_t smem(int m, int n) const
-  {
-    return vector_bytes<TX>(m, n) + state_bytes<TX>() + image_bytes<TX>();
   }
 };
 
@@ -863,34 +880,71 @@ __device__ __forceinline__ void unit_range(const dev_sell<TX>& M, int u, int64_t
   }
 }
 
+// Which blocks need an entry of x_bar or y: bit r of needs[j] for column j of block r's share of A,
+// of needs[n + i] for column i (row of A) of its share of A^T; and the first entry of every unit goes
+// to every block that has units of the other sweep, so that a block which has all the entries that it
+// needs also knows that every unit of the sweep before has read its own (see resident_unit_kernel).
+// needs must be zeroed first.  One block per block of the cluster.
+template <typename TX>
+__global__ void __launch_bounds__(kResidentThreads)
+  resident_needs_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, resident_dims D, int n,
+                        unsigned* needs)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int w = 0; w < 2; ++w) {
+    const dev_sell<TX>&M = w == 0 ? AT : A, &O = w == 0 ? A : AT;
+    const int total = M.n_long + M.n_slices, other = O.n_long + O.n_slices;
+    unsigned* read  = needs + (w == 0 ? n : 0);  // the vector that M's rows gather
+    unsigned* own   = needs + (w == 0 ? 0 : n);  // the vector of M's rows
+    const unsigned all = other >= 32 ? ~0u : (1u << min(other, D.blocks)) - 1u;
+    for (int u = (int)blockIdx.x + D.blocks * warp; u < total; u += D.blocks * kResidentWarps) {
+      int64_t b, e;
+      unit_range(M, u, b, e);
+      for (int64_t k = b + lane; k < e; k += kWarp) atomicOr(read + M.idx[k], 1u << blockIdx.x);
+      if (lane == 0)
+        atomicOr(own + (u < M.n_long ? u : M.n_long + (u - M.n_long) * kWarp),
+                 all & ((1u << D.blocks) - 1u));
+    }
+  }
+}
+
 // Builds the image of block blockIdx.x (once per solve).
 template <typename TX>
 __global__ void __launch_bounds__(kResidentThreads)
   resident_image_kernel(const dev_sell<TX> AT, const dev_sell<TX> A, const TX* c, const TX* lo,
-                        const TX* up, const TX* lc, const TX* uc, resident_dims D,
-                        unsigned char* images)
+                        const TX* up, const TX* lc, const TX* uc, resident_dims D, int m, int n,
+                        const unsigned* needs, unsigned char* images)
 {
   unsigned char* img = images + blockIdx.x * D.image_bytes<TX>();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ int count[2];
+  if (threadIdx.x < 2) count[threadIdx.x] = 0;
   for (int w = 0; w < 2; ++w) {
     const dev_sell<TX>& M = w == 0 ? AT : A;
     const int total       = M.n_long + M.n_slices;
     int2* table           = reinterpret_cast<int2*>(img + D.image_at<TX>(w));
+    for (int i = threadIdx.x; i < D.units[w]; i += kResidentThreads) {
+      const int u = (int)blockIdx.x + D.blocks * i;
+      int64_t b = 0, e = 0;
+      if (u < total) unit_range(M, u, b, e);
+      table[i] = make_int2(0, (int)(e - b));
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
       int at = 0;
       for (int i = 0; i < D.units[w]; ++i) {
-        const int u = (int)blockIdx.x + D.blocks * i;
-        int64_t b = 0, e = 0;
-        if (u < total) unit_range(M, u, b, e);
-        table[i] = make_int2(at, (int)(e - b));
-        at += ((int)(e - b) + 3) & ~3;
+        const int len = table[i].y;
+        table[i].x    = at;
+        at += (len + 3) & ~3;
       }
     }
     __syncthreads();
-    TX* ops           = reinterpret_cast<TX*>(img + D.image_at<TX>(2 + w));
-    TX* val           = reinterpret_cast<TX*>(img + D.image_at<TX>(4 + w));
-    unsigned short* x = reinterpret_cast<unsigned short*>(img + D.image_at<TX>(6 + w));
-    const int slots   = D.units[w] * kWarp;
+    TX* ops              = reinterpret_cast<TX*>(img + D.image_at<TX>(2 + w));
+    TX* val              = reinterpret_cast<TX*>(img + D.image_at<TX>(4 + w));
+    unsigned short* x    = reinterpret_cast<unsigned short*>(img + D.image_at<TX>(6 + w));
+    unsigned short* mask = reinterpret_cast<unsigned short*>(img + D.image_at<TX>(8 + w));
+    const unsigned* need = needs + (w == 0 ? 0 : n);
+    const int slots      = D.units[w] * kWarp;
     for (int i = warp; i < D.units[w]; i += kResidentWarps) {
       const int u  = (int)blockIdx.x + D.blocks * i;
       const int2 t = table[i];
@@ -910,6 +964,7 @@ __global__ void __launch_bounds__(kResidentThreads)
         ops[s]         = row >= 0 ? lc[row] : TX(0);
         ops[slots + s] = row >= 0 ? uc[row] : TX(0);
       }
+      mask[s] = row >= 0 ? (unsigned short)need[row] : (unsigned short)0;
       int64_t b = 0, e = 0;
       if (u < total) unit_range(M, u, b, e);
       for (int k = lane; k < t.y; k += kWarp) {
@@ -917,8 +972,14 @@ __global__ void __launch_bounds__(kResidentThreads)
         x[t.x + k]   = (unsigned short)M.idx[b + k];
       }
     }
+    // Entries of this sweep's vector that this block needs.
+    int mine = 0;
+    for (int j = threadIdx.x; j < (w == 0 ? n : m); j += kResidentThreads)
+      mine += (need[j] >> blockIdx.x) & 1u;
+    atomicAdd(count + w, mine);
     __syncthreads();
   }
+  if (threadIdx.x < 2) reinterpret_cast<int*>(img + D.image_at<TX>(10))[threadIdx.x] = count[threadIdx.x];
 }
 
 __device__ __forceinline__ void shared_chunk(const float* p, double (&v)[4])
@@ -1015,7 +1076,7 @@ __global__ void __launch_bounds__(kResidentThreads)
   resident_plain_kernel(const dev_sell<TX> AT, const dev_sell<TX> A,
                         primal_epi<TX, false, true, false> pe, dual_epi<TX, false, true, false> de,
                         int L, int keep, int m, int n, resident_dims D,
-                        const unsigned char* images, pdlp_scalars* st)
+                        const unsigned char* images, pdlp_scalars* st, int*)
 {
   extern __shared__ __align__(16) unsigned char cl_smem[];
   TX* ys  = reinterpret_cast<TX*>(cl_smem);
@@ -1155,6 +1216,279 @@ __global__ void __launch_bounds__(kResidentThreads)
       cluster_barrier();
     }
   }
+  if (rank == 0 && threadIdx.x == 0) st->t0 += L;
+}
+
+// The CACHED form where no warp takes more than one slice of either sweep and no row is long (up to
+// 16 x 10 slices, that is 5 120 rows of each matrix, with clusters of 16).  What bounds an iteration
+// here is the exchange of x_bar and y (a block sends some 16 bytes a cycle), the chain of a row's
+// products, and the latency of each.  A cluster barrier behind posted stores waits for every store
+// to be acknowledged: 2 300 (2048 entries, 16 blocks) and 4 300 cycles (5120) of a phase.  So:
+//   * an entry goes, only to the blocks that gather it, with st.async, whose bytes count towards the
+//     receiving block's mbarrier: no barrier at all (1 480 and 2 960 cycles for all entries);
+//   * the first entry of every slice goes to every block of the other sweep.  A warp sends after its
+//     gathers, so a block that has its bytes of one sweep knows that every warp of that sweep is done
+//     reading the vector that the block is about to write next;
+//   * the cluster is the smallest of 4, 8 and 16 blocks whose warps suffice: every further block is
+//     one more store for every entry;
+//   * a row's gathers run two chunks ahead of its sum (1 870 cycles for 9 chunks without);
+//   * a row's operands and the remote addresses stay in registers, and the Halpern weight and
+//     y / sigma (two FP64 divisions) are formed between sending and waiting.
+// Waits are bounded: one that runs out sets the launch's status, and every block leaves through the
+// closing cluster barrier.
+constexpr int kClusterBlocks = 16;
+constexpr int kUnitWarps     = 10;
+constexpr int kExchangePolls = 1 << 22;
+
+__device__ __forceinline__ void exchange_init(unsigned bar)
+{
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// The phase that ends once `bytes` more have arrived (one call a phase, by one thread).
+__device__ __forceinline__ void exchange_expect(unsigned bar, unsigned bytes)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool exchange_wait(unsigned bar, unsigned parity)
+{
+  for (int i = 0; i < kExchangePolls; ++i) {
+    unsigned ok;
+    asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+// Stores v at offset `off` from the mapped base addresses in the blocks of `mask`, counted by the
+// barrier at offset `bar` there.  Predicated, not branched over: with sixteen branches a warp's step
+// and sends took 1 200 to 2 300 cycles.
+template <int C>
+__device__ __forceinline__ void exchange_send(const unsigned (&base)[C], unsigned mask, unsigned off,
+                                              unsigned bar, double v)
+{
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    asm volatile(
+      "{\n .reg .pred p;\n"
+      " setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];\n}" ::"r"(
+        base[c] + off),
+      "d"(v), "r"(base[c] + bar), "r"(mask & (1u << c))
+      : "memory");
+}
+template <int C>
+__device__ __forceinline__ void exchange_send(const unsigned (&base)[C], unsigned mask, unsigned off,
+                                              unsigned bar, float v)
+{
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    asm volatile(
+      "{\n .reg .pred p;\n"
+      " setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];\n}" ::"r"(
+        base[c] + off),
+      "f"(v), "r"(base[c] + bar), "r"(mask & (1u << c))
+      : "memory");
+}
+
+// This lane's row (-1: none) of a warp's slice, and its elements (first chunk in registers).
+template <typename TX>
+struct held_unit {
+  int row    = -1;
+  int chunks = -1;  // -1: the warp has no slice
+  TX v0[4];
+  ushort4 x0, x1;
+  const TX* val;
+  const unsigned short* idx;
+  __device__ __forceinline__ void load(const dev_sell<TX>& M, int s, const int2& t, const TX* vals,
+                                       const unsigned short* idxs)
+  {
+    const int lane = threadIdx.x & 31;
+    x0 = x1 = make_ushort4(0, 0, 0, 0);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v0[e] = TX(0);
+    val = vals + t.x + lane * kChunk;
+    idx = idxs + t.x + lane * kChunk;
+    if (s >= M.n_slices) return;
+    row = s * kWarp + lane;
+    if (row >= M.rows) row = -1;
+    chunks = t.y >> 7;
+    if (chunks > 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v0[e] = val[e];
+      x0 = *reinterpret_cast<const ushort4*>(idx);
+    }
+    if (chunks > 1) x1 = *reinterpret_cast<const ushort4*>(idx + kWarp * kChunk);
+  }
+  // The row's product, in sell_map_block's order: while chunk q is added, the entries of chunk q + 1
+  // and the indices of chunk q + 2 are on their way.
+  __device__ __forceinline__ double product(const TX* g) const
+  {
+    double acc = 0.0;
+    if (chunks <= 0) return acc;
+    TX gq[4] = {g[x0.x], g[x0.y], g[x0.z], g[x0.w]};
+    double vq[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) vq[e] = (double)v0[e];
+    ushort4 x = x1;
+    for (int q = 0; q < chunks; ++q) {
+      TX gn[4]     = {TX(0), TX(0), TX(0), TX(0)};
+      double vn[4] = {0.0, 0.0, 0.0, 0.0};
+      if (q + 1 < chunks) {
+        gn[0] = g[x.x];
+        gn[1] = g[x.y];
+        gn[2] = g[x.z];
+        gn[3] = g[x.w];
+        shared_chunk(val + (q + 1) * kWarp * kChunk, vn);
+        if (q + 2 < chunks) x = *reinterpret_cast<const ushort4*>(idx + (q + 2) * kWarp * kChunk);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc += vq[e] * (double)gq[e];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        gq[e] = gn[e];
+        vq[e] = vn[e];
+      }
+    }
+    return acc;
+  }
+};
+
+// Shared memory: the barriers of x_bar and y, y, x_bar, the image.
+constexpr unsigned kUnitBars = 16;
+template <typename TX, int C>
+__global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
+  resident_unit_kernel(const dev_sell<TX> AT, const dev_sell<TX> A,
+                       primal_epi<TX, false, true, false> pe, dual_epi<TX, false, true, false> de,
+                       int L, int keep, int m, int n, resident_dims D, const unsigned char* images,
+                       pdlp_scalars* st, int* status)
+{
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  const unsigned xb_0 = kUnitBars + (unsigned)resident_dims::pad((size_t)m * sizeof(TX));
+  TX* ys              = reinterpret_cast<TX*>(cl_smem + kUnitBars);
+  TX* xbs             = reinterpret_cast<TX*>(cl_smem + xb_0);
+  unsigned char* img  = cl_smem + kUnitBars + resident_dims::vector_bytes<TX>(m, n);
+  const unsigned rank = cluster_rank();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned bar_x = (unsigned)__cvta_generic_to_shared(cl_smem), bar_y = bar_x + 8;
+  if (threadIdx.x == 0) {
+    exchange_init(bar_x);
+    exchange_init(bar_y);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  {
+    const size_t bytes       = D.image_bytes<TX>();
+    const unsigned char* src = images + rank * bytes;
+    for (size_t b = (size_t)threadIdx.x * 16; b < bytes; b += (size_t)blockDim.x * 16)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(img + b)),
+                   "l"(src + b)
+                   : "memory");
+  }
+  for (int i = threadIdx.x; i < m; i += blockDim.x) ys[i] = de.y[i];
+  const pdlp_scalars sc = *st;
+  unsigned base[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(bar_x), "r"(c));
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const int slice = (int)rank + D.blocks * warp;
+  held_unit<TX> P, Q;
+  typename primal_epi<TX, false, true, false>::pre_t px{};
+  typename dual_epi<TX, false, true, false>::pre_t dy{};
+  unsigned to_p = 0, to_d = 0;  // blocks that need this lane's x_bar, y
+  if (warp < D.units[0]) {
+    P.load(AT, slice, reinterpret_cast<const int2*>(img + D.image_at<TX>(0))[warp],
+           reinterpret_cast<const TX*>(img + D.image_at<TX>(4)),
+           reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(6)));
+    const TX* op = reinterpret_cast<const TX*>(img + D.image_at<TX>(2)) + warp * kWarp + lane;
+    to_p = reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(8))[warp * kWarp + lane];
+    if (P.row >= 0)
+      px = {pe.x[P.row], op[0], op[D.units[0] * kWarp], op[2 * D.units[0] * kWarp], pe.xa[P.row]};
+  }
+  if (warp < D.units[1]) {
+    Q.load(A, slice, reinterpret_cast<const int2*>(img + D.image_at<TX>(1))[warp],
+           reinterpret_cast<const TX*>(img + D.image_at<TX>(5)),
+           reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(7)));
+    const TX* op = reinterpret_cast<const TX*>(img + D.image_at<TX>(3)) + warp * kWarp + lane;
+    to_d = reinterpret_cast<const unsigned short*>(img + D.image_at<TX>(9))[warp * kWarp + lane];
+    if (Q.row >= 0) dy = {de.y[Q.row], op[0], op[D.units[1] * kWarp], de.ya[Q.row]};
+  }
+  const int2 need = *reinterpret_cast<const int2*>(img + D.image_at<TX>(10));
+  const unsigned bytes_x = need.x * (unsigned)sizeof(TX), bytes_y = need.y * (unsigned)sizeof(TX);
+  if (threadIdx.x == 0) {
+    exchange_expect(bar_x, bytes_x);
+    exchange_expect(bar_y, bytes_y);
+  }
+  double w = halpern_weight(&sc, 0), ratio = (double)dy.y / sc.sigma;
+  // Every block of the cluster is running, with its copy of y and its barriers, before any block
+  // stores into another's shared memory.
+  cluster_barrier();
+  unsigned phase_x = 0, phase_y = 0;
+  bool ok = true;
+  for (int it = 0; it < L; ++it) {
+    const bool last = it == L - 1;
+    if (P.chunks >= 0) {
+      if (it > 0) {
+        if (!(ok = exchange_wait(bar_y, phase_y))) break;
+        phase_y ^= 1;
+        if (threadIdx.x == 0) exchange_expect(bar_y, bytes_y);
+      }
+      const double acc = P.product(ys);
+      if (P.row >= 0) {
+        const auto send = [&](int, double v) {
+          exchange_send(base, to_p, xb_0 + (unsigned)P.row * (unsigned)sizeof(TX), 0, (TX)v);
+        };
+        TX xb, xn;
+        if (last && keep)
+          primal_row_step<TX, true, true, false>(0, acc, px, sc.tau, w, &xb, &xn,
+                                                 pe.xhat + P.row, pe.slack + P.row, (TX*)nullptr,
+                                                 send);
+        else
+          primal_row_step<TX, false, true, false>(0, acc, px, sc.tau, w, &xb, &xn, (TX*)nullptr,
+                                                  (TX*)nullptr, (TX*)nullptr, send);
+        px.x = xn;
+        if (last) {
+          pe.xout[P.row] = xn;
+          pe.xbar[P.row] = xb;
+        }
+      }
+    }
+    if (Q.chunks >= 0) {
+      if (!(ok = exchange_wait(bar_x, phase_x))) break;
+      phase_x ^= 1;
+      if (threadIdx.x == 0) exchange_expect(bar_x, bytes_x);
+      const double acc = Q.product(xbs);
+      if (Q.row >= 0) {
+        const auto send = [&](int, double v) {
+          exchange_send(base, to_d, kUnitBars + (unsigned)Q.row * (unsigned)sizeof(TX), 8, (TX)v);
+        };
+        TX yn;
+        if (last && keep)
+          dual_row_step<TX, true, true>(0, acc, dy, sc.sigma, ratio, w, (TX*)nullptr, &yn,
+                                        de.yhat + Q.row, send);
+        else
+          dual_row_step<TX, false, true>(0, acc, dy, sc.sigma, ratio, w, (TX*)nullptr, &yn,
+                                         (TX*)nullptr, send);
+        dy.y = yn;
+        if (last) de.yout[Q.row] = yn;
+      }
+    }
+    w     = halpern_weight(&sc, it + 1);
+    ratio = (double)dy.y / sc.sigma;
+  }
+  // No block leaves while entries of the last sweep are on their way to it.
+  if (ok && P.chunks >= 0) ok = exchange_wait(bar_y, phase_y);
+  if (!ok) atomicCAS(status, 0, kBarrierPollLimit);
+  __syncthreads();
+  cluster_barrier();
   if (rank == 0 && threadIdx.x == 0) st->t0 += L;
 }
 

@@ -132,6 +132,7 @@ class engine {
   {
     // A check may still read buffers that are released, in the order of s_, after this.
     if (es_) cudaStreamSynchronize(es_);
+    if (!graphs_.empty()) cudaStreamSynchronize(s_);  // no graph is destroyed while it runs
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
     if (kept_) cudaEventDestroy(kept_);
     if (checked_) cudaEventDestroy(checked_);
@@ -524,7 +525,7 @@ class engine {
       if (cluster) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
-        cluster_config(cfg, attr, smem);
+        cluster_config(cfg, attr, kResidentThreads, smem);
         B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_gk_kernel<TX>, ATs, As, u.data(), v.data(),
                                            st.data(), alphas.data(), betas.data(), c, m, n,
                                            resident_, (const unsigned char*)images_.data()));
@@ -566,7 +567,7 @@ class engine {
     allow_max_dynamic_smem(fn);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
-    cluster_config(cfg, attr, smem);
+    cluster_config(cfg, attr, kResidentThreads, smem);
     int clusters  = 0;
     const bool ok = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
                     clusters > 0;
@@ -888,16 +889,25 @@ class engine {
   }
 
   // ------------------------------------------------------------------ cluster plain iterations
-  static const void* resident_fn(bool cached)
+  // Variants of the cluster form: one slice a warp, shares in shared memory, matrices read from L2.
+  enum { kUnit, kCached, kUncached };
+  using resident_kernel_t = void (*)(const dev_sell<TX>, const dev_sell<TX>, persist_pe, persist_de,
+                                     int, int, int, int, resident_dims, const unsigned char*,
+                                     pdlp_scalars*, int*);
+  static resident_kernel_t resident_kernel(int variant, int blocks = kClusterBlocks)
   {
-    return cached ? (const void*)resident_plain_kernel<TX, true>
-                  : (const void*)resident_plain_kernel<TX, false>;
+    return variant == kUnit     ? (blocks == 4   ? resident_unit_kernel<TX, 4>
+                                   : blocks == 8 ? resident_unit_kernel<TX, 8>
+                                                 : resident_unit_kernel<TX, kClusterBlocks>)
+           : variant == kCached ? resident_plain_kernel<TX, true>
+                                : resident_plain_kernel<TX, false>;
   }
-  void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1], size_t smem) const
+  void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute (&attr)[1], int threads,
+                      size_t smem) const
   {
     cfg                              = cudaLaunchConfig_t{};
     cfg.gridDim                      = dim3(resident_.blocks);
-    cfg.blockDim                     = dim3(kResidentThreads);
+    cfg.blockDim                     = dim3(threads);
     cfg.dynamicSmemBytes             = smem;
     cfg.stream                       = s_;
     attr[0].id                       = cudaLaunchAttributeClusterDimension;
@@ -913,7 +923,9 @@ class engine {
   bool prepare_resident()
   {
     const int m = in_.m, n = in_.n;
-    if (resident_dims::vector_bytes<TX>(m, n) > max_dynamic_smem(resident_fn(true))) return false;
+    if (resident_dims::vector_bytes<TX>(m, n) >
+        max_dynamic_smem((const void*)resident_kernel(kUncached)))
+      return false;
     const auto AT = ATs_view(), A = As_view();
     std::vector<int64_t> off[4];
     const dbuf<int64_t>* src[4] = {&L_.AT.long_off, &L_.AT.slice_off, &L_.A.long_off,
@@ -923,8 +935,10 @@ class engine {
       src[q]->download(off[q].data(), off[q].size(), s_);
     }
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    for (const bool cached : {true, false})
-      for (const int c : {16, 8}) {
+    for (const int variant : {kUnit, kCached, kUncached})
+      for (const int c : variant == kUnit ? std::vector<int>{4, 8, kClusterBlocks}
+                                          : std::vector<int>{kClusterBlocks, 8}) {
+        const bool cached = variant != kUncached;
         resident_dims d;
         d.blocks = c;
         for (int w = 0; cached && w < 2; ++w) {
@@ -940,8 +954,15 @@ class engine {
           if (most > INT_MAX / 2) return false;
           d.elems[w] = (int)((most + 7) & ~int64_t(7));
         }
-        const void* fn    = resident_fn(cached);
-        const size_t smem = cached ? d.smem<TX>(m, n) : resident_dims::vector_bytes<TX>(m, n);
+        const void* fn    = (const void*)resident_kernel(variant, c);
+        const int most    = std::max(d.units[0], d.units[1]);
+        if (variant == kUnit &&
+            (most > kUnitWarps || AT.n_long > 0 || A.n_long > 0))
+          continue;
+        const size_t smem = (variant == kUnit ? kUnitBars : 0) +
+                            resident_dims::vector_bytes<TX>(m, n) +
+                            (cached ? d.image_bytes<TX>() : 0) +
+                            (variant == kCached ? d.state_bytes<TX>() : 0);
         if (smem > max_dynamic_smem(fn)) continue;
         if (c > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
                        cudaSuccess) {
@@ -949,12 +970,14 @@ class engine {
           continue;
         }
         allow_max_dynamic_smem(fn);
-        resident_        = d;
-        resident_cached_ = cached;
-        cluster_smem_    = smem;
+        resident_         = d;
+        resident_variant_ = variant;
+        resident_cached_  = cached;
+        resident_threads_ = variant == kUnit ? std::max(4, most) * kWarp : kResidentThreads;
+        cluster_smem_     = smem;
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
-        cluster_config(cfg, attr, smem);
+        cluster_config(cfg, attr, resident_threads_, smem);
         int clusters  = 0;
         const bool ok = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
                         clusters > 0;
@@ -962,9 +985,13 @@ class engine {
         if (!ok) continue;
         if (cached) {
           images_.resize(c * d.image_bytes<TX>());
+          dbuf<unsigned> needs((size_t)n + m);
+          needs.zero(s_);
+          resident_needs_kernel<TX><<<c, kResidentThreads, 0, s_>>>(AT, A, d, n, needs.data());
           resident_image_kernel<TX><<<c, kResidentThreads, 0, s_>>>(
-            AT, A, cs_.data(), ls_.data(), us_.data(), lcs_.data(), ucs_.data(), d, images_.data());
-          ++launches_;
+            AT, A, cs_.data(), ls_.data(), us_.data(), lcs_.data(), ucs_.data(), d, m, n,
+            needs.data(), images_.data());
+          launches_ += 2;
           B200_LAUNCH_CHECK();
         }
         for (auto* v : {&xhat2_, &slack2_}) v->resize(n);
@@ -986,11 +1013,11 @@ class engine {
                   y_.data(),    kept_yhat(), scalars_.data(), 0};
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr[1];
-    cluster_config(cfg, attr, cluster_smem_);
-    auto* fn = resident_cached_ ? resident_plain_kernel<TX, true> : resident_plain_kernel<TX, false>;
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, AT, A, pe, de, L, (int)keep, in_.m, in_.n,
+    cluster_config(cfg, attr, resident_threads_, cluster_smem_);
+    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, resident_kernel(resident_variant_, resident_.blocks),
+                                       AT, A, pe, de, L, (int)keep, in_.m, in_.n,
                                        resident_, (const unsigned char*)images_.data(),
-                                       scalars_.data()));
+                                       scalars_.data(), &pctl_.data()->status));
     ++launches_;
     return cluster_launches_++ == 0;
   }
@@ -1144,8 +1171,9 @@ class engine {
   }
 
   // ------------------------------------------------------------------ termination
-  // A termination check runs on its own stream beside the plain iterations that follow the step it
-  // looks at: it reads x_hat, y_hat and the slack, which only the next step that keeps them
+  // A termination check of an LP whose iterations do not fill the GPU runs on its own stream beside the
+  // plain iterations that follow the step it looks at; beside a large LP's (whose matrices and
+  // vectors fill L2) it slowed both down, so it goes in their stream there.  It reads x_hat, y_hat and the slack, which only the next step that keeps them
   // overwrites, and that step is not launched before the check's results are in (resolve).
   void post_check()
   {
@@ -1201,8 +1229,8 @@ class engine {
     const int* flags = reinterpret_cast<const int*>(h + 8);
     if (flags[0] != 0)
       throw cuda_error(flags[0] == kBarrierTimedOut
-                         ? "persistent iterations: a grid barrier passed its deadline"
-                         : "persistent iterations: a grid barrier passed its poll limit");
+                         ? "plain iterations: a grid barrier passed its deadline"
+                         : "plain iterations: a barrier or an exchange passed its poll limit");
     if (flags[1] != 0)
       throw cuda_error("tiled sweep: a panel copy did not complete within its wait limit");
     conv_info cv;
@@ -1358,7 +1386,8 @@ class engine {
     // about 40 us from its launch to the host's decision; the 8 iterations of a run between two
     // checks are launched in one piece while that wastes little.
     const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
-    ahead_ = est_us <= 16.0 ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    const bool small    = est_us <= 16.0;
+    ahead_              = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
     const auto A = As_view(), AT = ATs_view();
 
     for (;;) {
@@ -1622,6 +1651,7 @@ class engine {
   size_t cluster_smem_ = 0;         // dynamic shared memory of the cluster form
   resident_dims resident_;          // its blocks and their shares (none without resident_cached_)
   bool resident_ok_ = false, resident_cached_ = false;
+  int resident_variant_ = kUncached, resident_threads_ = kResidentThreads;
   dbuf<unsigned char> images_;
   // x_hat, y_hat and the slack of the last keeping step are in buffer kept_in_: 0 is xhat_, yhat_,
   // slack_; the cluster form alternates with these.

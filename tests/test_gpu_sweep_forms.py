@@ -53,6 +53,18 @@ def test_forms_are_bit_identical(kind, m, n, k, precision):
         _same(ref, _solve(lp, GRAPHS, 230, precision, wpb))
 
 
+@pytest.mark.parametrize("m,n,k", [(300, 1280, 4), (300, 1281, 4),     # 4 blocks of 10 slices; 8
+                                   (2560, 700, 5), (2561, 700, 5),     # 8 blocks of 10 slices; 16
+                                   (2000, 5120, 5), (2000, 5121, 5)])  # 16 of 10; several a warp
+def test_cluster_sizes_at_their_last_slice(m, n, k):
+    """One slice a warp while a side has at most 10 per block, in the smallest cluster that holds it."""
+    lp = gen.constructed_lp(m, n, k, seed=m + n)
+    for precision in (0, 1):
+        c = _solve(lp, CLUSTER, 230, precision)
+        assert c.stats["plain_iteration_form"] == CLUSTER
+        _same(_solve(lp, GRAPHS, 230, precision), c)
+
+
 @pytest.mark.parametrize("limit", [1200, 1300])
 def test_cluster_form_checks_every_hundred_iterations(limit):
     lp = gen.constructed_lp(150, 333, 5, seed=4)
