@@ -29,23 +29,17 @@ __device__ __forceinline__ void gather_group(const double* __restrict__ p, doubl
   }
 }
 
-// acc[b] = sum_k A[r,k] g[idx[r,k] * ld + g0 + b] for the kGroup climbers of a group, then
-// epi(r, acc, pre, red).  One launch covers the n_groups groups listed in `groups`: block
-// q * n_groups + i sweeps matrix block q for group groups[i] (its g0 replaces the epilogue's), so
-// the blocks that read one stretch of the matrix run side by side and share it through L2.  The
-// block sums of group g go to partials + g * pstride.
+// acc[b] = sum_k A[r,k] g[idx[r,k] * ld + g0 + b] for the kGroup climbers of group grp (g0 its first),
+// then epi(r, acc, pre, red), for matrix block xb of the sweep; the block sums go to partials at
+// block xb.  The next chunk's indices and values are loaded while this one's are gathered.
 template <class Epi>
-__global__ void __launch_bounds__(kBlock) mm_sweep_kernel(const dev_sell<double> A,
-                                                          const double* __restrict__ g, int ld,
-                                                          const int* __restrict__ groups,
-                                                          int n_groups, Epi epi, double* partials,
-                                                          size_t pstride)
+__device__ __forceinline__ void mm_sweep_block(const dev_sell<double>& A,
+                                               const double* __restrict__ g, int ld, int grp,
+                                               int xb, Epi epi, double* partials)
 {
   constexpr int K = Epi::kRed;
-  const int grp = groups[blockIdx.x % n_groups];
-  const int xb  = (int)(blockIdx.x / n_groups);
-  const int g0  = grp * kGroup;
-  epi.ctx.g0    = g0;
+  const int g0    = grp * kGroup;
+  epi.ctx.g0      = g0;
   red_t<K> red;
 #pragma unroll
   for (int q = 0; q < (K > 0 ? K : 1); ++q) red.v[q] = 0.0;
@@ -79,35 +73,72 @@ __global__ void __launch_bounds__(kBlock) mm_sweep_kernel(const dev_sell<double>
       const int nchunk   = (int)((A.slice_off[s + 1] - base) >> 7);
       const double* v    = A.val + base + lane * kChunk;
       const int* ix      = A.idx + base + lane * kChunk;
-      for (int q = 0; q < nchunk; ++q) {
-        const int4 i4 = load_idx_chunk(ix);
-        double v4[4];
+      int4 i4            = make_int4(0, 0, 0, 0);
+      double v4[4]       = {0.0, 0.0, 0.0, 0.0};
+      if (nchunk > 0) {
+        i4 = load_idx_chunk(ix);
         load_chunk(v, v4);
+      }
+      for (int q = 0; q < nchunk; ++q) {
         const int id[4] = {i4.x, i4.y, i4.z, i4.w};
+        double gv[4][kGroup];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          double gv[kGroup];
-          gather_group(g + (size_t)id[e] * ld + g0, gv);
-#pragma unroll
-          for (int b = 0; b < kGroup; ++b) acc[b] += v4[e] * gv[b];
-        }
+        for (int e = 0; e < 4; ++e) gather_group(g + (size_t)id[e] * ld + g0, gv[e]);
+        const double w[4] = {v4[0], v4[1], v4[2], v4[3]};
         v += kWarp * kChunk;
         ix += kWarp * kChunk;
+        if (q + 1 < nchunk) {
+          i4 = load_idx_chunk(ix);
+          load_chunk(v, v4);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int b = 0; b < kGroup; ++b) acc[b] += w[e] * gv[e][b];
       }
       if (valid) epi(row, acc, pre, red);
     }
   }
-  block_reduce_store<K>(red, partials + (size_t)grp * pstride, xb);
+  block_reduce_store<K>(red, partials, xb);
 }
 
-// out[g * stride + q] = the ordered sum of group g's block sums, one block per listed group.
+// One launch covers the n_groups groups listed in `groups`: block q * n_groups + i sweeps matrix
+// block q for group groups[i], so the blocks that read one stretch of the matrix run side by side
+// and share it through L2.  The block sums of group g go to partials + g * pstride.
+template <class Epi>
+__global__ void __launch_bounds__(kBlock) mm_sweep_kernel(const dev_sell<double> A,
+                                                          const double* __restrict__ g, int ld,
+                                                          const int* __restrict__ groups,
+                                                          int n_groups, Epi epi, double* partials,
+                                                          size_t pstride)
+{
+  const int grp = groups[blockIdx.x % n_groups];
+  mm_sweep_block(A, g, ld, grp, (int)(blockIdx.x / n_groups), epi, partials + (size_t)grp * pstride);
+}
+
+// out[g * stride + q] = the ordered sum of value q of K of group g's block sums, one block for each
+// listed group and value (as one block per group, K = 24 values took 190 block barriers).
+template <int K>
+__device__ __forceinline__ void mm_ordered_sum(const double* partials, int nblocks, int q, double* out)
+{
+  __shared__ double sm[kBlock];
+  ksum acc;
+  for (int b = threadIdx.x; b < nblocks; b += kBlock) acc.add(partials[(size_t)b * K + q]);
+  sm[threadIdx.x] = acc.value();
+  __syncthreads();
+  for (int h = kBlock / 2; h > 0; h >>= 1) {
+    if (threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = sm[0];
+}
 template <int K>
 __global__ void __launch_bounds__(kBlock) mm_finalize_kernel(const double* partials, size_t pstride,
                                                              int nblocks, const int* groups,
                                                              double* out, int stride)
 {
-  const int grp = groups[blockIdx.x];
-  ordered_block_sum<K>(partials + (size_t)grp * pstride, nblocks, out + (size_t)grp * stride);
+  const int grp = groups[blockIdx.x / K], q = (int)(blockIdx.x % K);
+  mm_ordered_sum<K>(partials + (size_t)grp * pstride, nblocks, q, out + (size_t)grp * stride + q);
 }
 
 // Per-climber state shared by the climber epilogues.
@@ -287,6 +318,36 @@ struct mm_term_dual_epi {
   }
 };
 
+// Both termination sweeps of every listed group in one launch (blocks of the rows of A first), and
+// the sums of both in another, written to the pinned host buffer that the host reads when the
+// launch's event has completed: 5 kGroup values per group.
+static __global__ void __launch_bounds__(kBlock)
+  mm_term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
+                 const double* __restrict__ yu, int ld, const int* __restrict__ groups,
+                 int n_groups, mm_term_primal_epi ep, mm_term_dual_epi ed, int gp, double* partials,
+                 size_t pstride)
+{
+  const int grp = groups[blockIdx.x % n_groups], xb = (int)(blockIdx.x / n_groups);
+  double* part  = partials + (size_t)grp * pstride;
+  if (xb < gp)
+    mm_sweep_block(A, xu, ld, grp, xb, ep, part);
+  else
+    mm_sweep_block(AT, yu, ld, grp, xb - gp, ed, part + (size_t)gp * 2 * kGroup);
+}
+static __global__ void __launch_bounds__(kBlock)
+  mm_term_sums_kernel(const double* partials, size_t pstride, int gp, int gd, const int* groups,
+                      double* host)
+{
+  constexpr int K   = 5 * kGroup;
+  const int grp     = groups[blockIdx.x / K], q = (int)(blockIdx.x % K);
+  const double* p   = partials + (size_t)grp * pstride;
+  double* out       = host + (size_t)grp * K + q;
+  if (q < 2 * kGroup)
+    mm_ordered_sum<2 * kGroup>(p, gp, q, out);
+  else
+    mm_ordered_sum<3 * kGroup>(p + (size_t)gp * 2 * kGroup, gd, q - 2 * kGroup, out);
+}
+
 // Element-wise kernels over climber-interleaved vectors (element e = row * ld + climber).
 __global__ void mm_halpern_kernel(double* x, const double* xbar, const double* xa, size_t nx,
                                   double* y, const double* ybar, const double* ya, size_t ny,
@@ -403,6 +464,18 @@ __global__ void mm_broadcast_kernel(const double* src, int rows, int ld, double*
   }
 }
 
+// out[b * rows + new2old[i]] = sign * v[i * ld + b] for the first B climbers.
+__global__ void mm_output_kernel(const double* v, const int* new2old, int rows, int ld, int B,
+                                 double sign, double* out)
+{
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < (size_t)rows * ld;
+       e += (size_t)gridDim.x * blockDim.x) {
+    const int b = (int)(e % ld);
+    const size_t i = e / ld;
+    if (b < B) out[(size_t)b * rows + new2old[i]] = sign * v[e];
+  }
+}
+
 class climber_engine {
  public:
   // base: an engine<double> whose setup ran on the LP; var / lo / up: per climber the user-order
@@ -420,6 +493,7 @@ class climber_engine {
   }
   ~climber_engine()
   {
+    cudaStreamSynchronize(e_.es_);  // an outstanding check reads buffers that are released now
     drop_graphs();
     cudaFreeHost(hbuf_);
   }
@@ -430,9 +504,12 @@ class climber_engine {
     t_start_ = e_.t_start_;
     results_.assign(B_, pdlp_result{});
     setup();
+    trace("climbers: setup");
     t_loop_ = now_s();
     loop();
+    trace("climbers: loop");
     write_outputs(x_out, y_out, rc_out);
+    trace("climbers: outputs");
     for (int b = 0; b < B_; ++b) {
       results_[b].setup_time       = t_loop_ - t_start_;
       results_[b].loop_time        = results_[b].solve_time - (t_loop_ - t_start_);
@@ -505,6 +582,9 @@ class climber_engine {
       std::max({sell_grid(view64(e_.L_.A)), sell_grid(view64(e_.L_.AT)), e_.vgrid_});
     pstride_ = (size_t)g * 3 * kGroup;
     partials_.resize(pstride_ * groups_);
+    tstride_ = ((size_t)2 * sell_grid(view64(e_.L_.A)) + (size_t)3 * sell_grid(view64(e_.L_.AT))) *
+               kGroup;
+    tpartials_.resize(tstride_ * groups_);
     dres_.resize((size_t)6 * ld_);
     B200_LAUNCH_CHECK();
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
@@ -613,7 +693,7 @@ class climber_engine {
   void finalize(int nblocks, size_t off, int stride)
   {
     if (n_act() == 0) return;
-    mm_finalize_kernel<K><<<n_act(), kBlock, 0, s_>>>(partials_.data(), pstride_, nblocks,
+    mm_finalize_kernel<K><<<n_act() * K, kBlock, 0, s_>>>(partials_.data(), pstride_, nblocks,
                                                       groups_d_.data(), dres_.data() + off, stride);
     ++launches_;
   }
@@ -633,22 +713,34 @@ class climber_engine {
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
   }
 
-  // Residuals and objectives of every active climber (unscaled x_hat, y_hat, slack).
-  std::vector<conv_info> evaluate()
+  // Residuals and objectives of every active climber (unscaled x_hat, y_hat, slack), on the checks'
+  // stream (see engine::post_check).
+  void post_check()
   {
     const int m = e_.in_.m, n = e_.in_.n;
-    mm_unscale_kernel<<<e_.vgrid_, kBlock, 0, s_>>>(
-      xhat_.data(), yhat_.data(), slack_.data(), e_.dc_.data(), e_.dr_.data(), 1.0 / e_.beta_,
-      1.0 / e_.gamma_, n, m, ld_, active_d_.data(), xu_.data(), yu_.data(), su_.data());
-    ++launches_;
-    const auto A = view64(e_.L_.A), AT = view64(e_.L_.AT);
+    B200_CUDA_CHECK(cudaStreamWaitEvent(e_.es_, e_.kept_, 0));
+    if (n_act() > 0) {
+      mm_unscale_kernel<<<e_.vgrid_, kBlock, 0, e_.es_>>>(
+        xhat_.data(), yhat_.data(), slack_.data(), e_.dc_.data(), e_.dr_.data(), 1.0 / e_.beta_,
+        1.0 / e_.gamma_, n, m, ld_, active_d_.data(), xu_.data(), yu_.data(), su_.data());
+      const auto A = view64(e_.L_.A), AT = view64(e_.L_.AT);
+      const int gp = sell_grid(A), gd = sell_grid(AT);
+      mm_term_kernel<<<(gp + gd) * n_act(), kBlock, 0, e_.es_>>>(
+        A, AT, xu_.data(), yu_.data(), ld_, groups_d_.data(), n_act(),
+        mm_term_primal_epi{e_.lc64_.data(), e_.uc64_.data(), yu_.data(), ctx()},
+        mm_term_dual_epi{e_.c64_.data(), xu_.data(), su_.data(), ctx()}, gp, tpartials_.data(),
+        tstride_);
+      mm_term_sums_kernel<<<n_act() * 5 * kGroup, kBlock, 0, e_.es_>>>(
+        tpartials_.data(), tstride_, gp, gd, groups_d_.data(), hbuf_);
+      launches_ += 3;
+      B200_LAUNCH_CHECK();
+    }
+    B200_CUDA_CHECK(cudaEventRecord(e_.checked_, e_.es_));
+  }
+  std::vector<conv_info> wait_check()
+  {
+    B200_CUDA_CHECK(cudaEventSynchronize(e_.checked_));
     std::vector<conv_info> cv(ld_);
-    sweep(A, xu_.data(), mm_term_primal_epi{e_.lc64_.data(), e_.uc64_.data(), yu_.data(), ctx()});
-    finalize<2 * kGroup>(sell_grid(A), 0, 5 * kGroup);
-    sweep(AT, yu_.data(), mm_term_dual_epi{e_.c64_.data(), xu_.data(), su_.data(), ctx()});
-    finalize<3 * kGroup>(sell_grid(AT), 2 * kGroup, 5 * kGroup);
-    B200_LAUNCH_CHECK();
-    fetch(5 * (size_t)ld_);
     for (int g : groups_h_) {
       const double* h = hbuf_ + (size_t)g * 5 * kGroup;
       for (int q = 0; q < kGroup; ++q) {
@@ -710,41 +802,60 @@ class climber_engine {
     std::vector<int> groups_seen(groups_);
     for (int g = 0; g < groups_; ++g) groups_seen[g] = group_active(g);
 
+    B200_CUDA_CHECK(cudaEventRecord(e_.kept_, s_));
+    const double est_us = 9.0 + 2.0 * (double)e_.L_.nnz * groups_ / 5e4;
+    const bool small    = est_us <= 16.0;
+    const long ahead    = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    std::vector<conv_info> cv;
+    // Reads the outstanding check; false when no climber is left.  Climbers that end are taken out of
+    // the iterations from here on (their solution is the check's, which is not written again).
+    auto resolve = [&]() {
+      const long kc = posted_;
+      posted_       = -1;
+      cv            = wait_check();
+      const bool out_of_time = now_s() - t_start_ >= p_.time_limit;
+      bool ended             = false;
+      for (int b = 0; b < B_; ++b) {
+        if (!active_h_[b]) continue;
+        const conv_info& c   = cv[b];
+        const bool primal_ok = c.l2_primal <= p_.abs_primal + p_.rel_primal * e_.b_norm_;
+        const bool optimal   = c.l2_dual <= p_.abs_dual + p_.rel_dual * e_.c_norm_ && primal_ok &&
+                             c.gap <= p_.abs_gap + p_.rel_gap * c.abs_obj;
+        if (kc > 1 && optimal)
+          finish(b, kOptimal, c, kc);
+        else if (out_of_time)
+          finish(b, kTimeLimit, c, kc);
+        else if (kc >= p_.iteration_limit)
+          finish(b, kIterationLimit, c, kc);
+        else if (!std::isfinite(c.l2_primal) || !std::isfinite(c.l2_dual))
+          finish(b, kNumericalError, c, kc);
+        ended |= !active_h_[b];
+      }
+      if (std::count(active_h_.begin(), active_h_.end(), 1) == 0) return false;
+      bool groups_changed = false;
+      for (int g = 0; g < groups_; ++g)
+        if (groups_seen[g] && !group_active(g)) {
+          groups_seen[g] = 0;
+          groups_changed = true;
+        }
+      if (groups_changed) {
+        B200_CUDA_CHECK(cudaStreamSynchronize(s_));  // no graph is destroyed while it runs
+        drop_graphs();
+        refresh_groups();
+      }
+      if (ended) active_d_.upload(active_h_.data(), ld_, s_);
+      return true;
+    };
+
     for (long k = 0;;) {
       const bool major = (k % kMajor == 0 && k > 0) || k <= 0;
       const bool cond  = (k % conditional_major(k)) == 0;
       std::fill(restarted.begin(), restarted.end(), 0);
       bool any_restart = false;
       if (major || cond) {
-        const std::vector<conv_info> cv = evaluate();
-        const bool out_of_time = now_s() - t_start_ >= p_.time_limit;
-        for (int b = 0; b < B_; ++b) {
-          if (!active_h_[b]) continue;
-          const conv_info& c   = cv[b];
-          const bool primal_ok = c.l2_primal <= p_.abs_primal + p_.rel_primal * e_.b_norm_;
-          const bool optimal   = c.l2_dual <= p_.abs_dual + p_.rel_dual * e_.c_norm_ &&
-                               primal_ok && c.gap <= p_.abs_gap + p_.rel_gap * c.abs_obj;
-          if (k > 1 && optimal)
-            finish(b, kOptimal, c, k);
-          else if (out_of_time)
-            finish(b, kTimeLimit, c, k);
-          else if (k >= p_.iteration_limit)
-            finish(b, kIterationLimit, c, k);
-          else if (!std::isfinite(c.l2_primal) || !std::isfinite(c.l2_dual))
-            finish(b, kNumericalError, c, k);
-        }
-        if (std::count(active_h_.begin(), active_h_.end(), 1) == 0) break;
-        bool groups_changed = false;
-        for (int g = 0; g < groups_; ++g)
-          if (groups_seen[g] && !group_active(g)) {
-            groups_seen[g] = 0;
-            groups_changed = true;
-          }
-        if (groups_changed) {
-          drop_graphs();
-          refresh_groups();
-        }
-        active_d_.upload(active_h_.data(), ld_, s_);
+        post_check();
+        posted_ = k;
+        if (major && !resolve()) break;
 
         if (major) {
           sqdiff(xa_.data(), xhat_.data(), n, 0);
@@ -804,8 +915,8 @@ class climber_engine {
                                                             yhat_.data(), ny, ld_, flags_.data());
             ++launches_;
           }
+          if (any_restart) upload_state(since);
         }
-        upload_state(since);
         B200_LAUNCH_CHECK();
       }
 
@@ -818,12 +929,15 @@ class climber_engine {
           if (is_check(kk) || is_major_step(kk) || ((kk + 1) % kMajor == 0)) break;
           ++R;
         }
+        if (posted_ >= 0) R = std::min(R, ahead);
         run_plain(R);
         k += R;
         for (int b = 0; b < B_; ++b)
           if (active_h_[b]) since[b] += R;
+        if (posted_ >= 0 && !resolve()) break;
         continue;
       }
+      if (posted_ >= 0 && !resolve()) break;
 
       if (fpe_all || any_restart) {
         const auto A = view_of<double>(e_.L_.A, e_.As_.data());
@@ -831,6 +945,7 @@ class climber_engine {
         if (mstep) {
           launch_primal<true, false, true>(0);
           launch_dual<true, false, true>(0);
+          B200_CUDA_CHECK(cudaEventRecord(e_.kept_, s_));
         } else {
           launch_primal<false, false, true>(0);
           launch_dual<false, false, true>(0);
@@ -858,6 +973,7 @@ class climber_engine {
       } else {
         launch_primal<true, true, false>(0);
         launch_dual<true, true, false>(0);
+        B200_CUDA_CHECK(cudaEventRecord(e_.kept_, s_));
         advance(1);
         B200_LAUNCH_CHECK();
       }
@@ -870,24 +986,21 @@ class climber_engine {
   // Climber-interleaved unscaled solutions to the user's order, climber-major (B x n, B x m).
   void write_outputs(double* x_out, double* y_out, double* rc_out)
   {
-    const int m = e_.in_.m, n = e_.in_.n;
     const double sgn = e_.in_.maximize ? -1.0 : 1.0;
-    std::vector<int> c2o(n), r2o(m);
-    e_.L_.col_new2old.download(c2o.data(), n, s_);
-    e_.L_.row_new2old.download(r2o.data(), m, s_);
-    std::vector<double> hx((size_t)n * ld_), hs((size_t)n * ld_), hy((size_t)m * ld_);
-    xu_.download(hx.data(), hx.size(), s_);
-    su_.download(hs.data(), hs.size(), s_);
-    yu_.download(hy.data(), hy.size(), s_);
-    B200_CUDA_CHECK(cudaStreamSynchronize(s_));
-    for (int b = 0; b < B_; ++b) {
-      for (int j = 0; j < n; ++j) {
-        if (x_out) x_out[(size_t)b * n + c2o[j]] = hx[(size_t)j * ld_ + b];
-        if (rc_out) rc_out[(size_t)b * n + c2o[j]] = sgn * hs[(size_t)j * ld_ + b];
-      }
-      if (y_out)
-        for (int i = 0; i < m; ++i) y_out[(size_t)b * m + r2o[i]] = sgn * hy[(size_t)i * ld_ + b];
-    }
+    B200_CUDA_CHECK(cudaStreamSynchronize(e_.es_));
+    dbuf<double> ordered((size_t)B_ * std::max(e_.in_.m, e_.in_.n));
+    auto write = [&](const dbuf<double>& v, const dbuf<int>& new2old, int rows, double sign,
+                     double* out) {
+      if (!out || rows == 0) return;
+      mm_output_kernel<<<e_.vgrid_, kBlock, 0, s_>>>(v.data(), new2old.data(), rows, ld_, B_, sign,
+                                                     ordered.data());
+      ++launches_;
+      B200_LAUNCH_CHECK();
+      staged_download(out, ordered.data(), (size_t)B_ * rows * sizeof(double), s_);
+    };
+    write(xu_, e_.L_.col_new2old, e_.in_.n, 1.0, x_out);
+    write(su_, e_.L_.col_new2old, e_.in_.n, sgn, rc_out);
+    write(yu_, e_.L_.row_new2old, e_.in_.m, sgn, y_out);
   }
 
   engine<double>& e_;
@@ -904,9 +1017,10 @@ class climber_engine {
   dbuf<climber_bound> ovr_;
   dbuf<int> active_d_, flags_, groups_d_;
   std::vector<int> groups_h_;
-  size_t pstride_ = 0;
+  size_t pstride_ = 0, tstride_ = 0;  // block sums per group: the steps', the checks'
+  long posted_ = -1;                  // the check that has been launched but not read yet
   dbuf<pdlp_scalars> sc_d_;
   dbuf<double> x_, xhat_, slack_, xbar_, xa_, aty_, y_, yhat_, ybar_, ya_, xu_, yu_, su_;
-  dbuf<double> partials_, dres_;
+  dbuf<double> partials_, tpartials_, dres_;
   std::map<int, cudaGraphExec_t> graphs_;
 };
