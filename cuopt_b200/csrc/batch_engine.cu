@@ -245,6 +245,81 @@ __global__ void instance_reduce_kernel(const double* part, const int* chunk_off,
   }
 }
 
+// Both termination sweeps of a check in one launch (blocks [0, gp) the rows of A, the others the rows
+// of A^T; each writes planes of its own), and the per-instance sums of both in another: block c sums
+// the planes of its chunk (chunks of rows, then chunks of columns), and the block that finishes last of
+// its instance and side adds the instance's chunks in order into the pinned host buffer that the
+// host reads once the launch's event has completed (2 values per instance, then 3).
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<double>)
+  b_term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
+                const double* __restrict__ yu, b_term_primal_epi ep, b_term_dual_epi ed, int gp)
+{
+  if ((int)blockIdx.x < gp)
+    sell_map_block(A, xu, ep, nullptr, (int)blockIdx.x);
+  else
+    sell_map_block(AT, yu, ed, nullptr, (int)blockIdx.x - gp);
+}
+
+// Fixed-order block sum of per-thread values (compensated per thread, then a fixed tree).
+__device__ __forceinline__ double block_sum(const ksum& acc, double* sm)
+{
+  sm[threadIdx.x] = acc.value();
+  __syncthreads();
+  for (int h = kBlock / 2; h > 0; h >>= 1) {
+    if (threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
+    __syncthreads();
+  }
+  const double v = sm[0];
+  __syncthreads();
+  return v;
+}
+
+struct b_side {  // one side (rows or columns) of a check's sums
+  const int4* chunks;
+  const int* offsets;
+  int count;            // chunks
+  const double* planes;
+  double* part;
+  unsigned* arrived;    // per instance; 0 before and after
+  double* host;
+};
+template <int K>
+__device__ __forceinline__ void b_term_side(const b_side& S, int c, size_t stride, const int* want)
+{
+  const int4 ch = S.chunks[c];
+  if (!want[ch.x]) return;
+  __shared__ double sm[kBlock];
+  ksum acc[K];
+  for (int i = ch.y + threadIdx.x; i < ch.z; i += kBlock)
+#pragma unroll
+    for (int q = 0; q < K; ++q) acc[q].add(S.planes[q * stride + i]);
+  double t[K];
+#pragma unroll
+  for (int q = 0; q < K; ++q) t[q] = block_sum(acc[q], sm);
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int q = 0; q < K; ++q) S.part[(size_t)c * K + q] = t[q];
+  const int c0 = S.offsets[ch.x], c1 = S.offsets[ch.x + 1];
+  __threadfence();
+  if (atomicAdd(S.arrived + ch.x, 1u) != (unsigned)(c1 - c0 - 1)) return;
+  __threadfence();
+  double sum[K] = {};
+  for (int d = c0; d < c1; ++d)
+#pragma unroll
+    for (int q = 0; q < K; ++q) sum[q] += __ldcg(S.part + (size_t)d * K + q);
+#pragma unroll
+  for (int q = 0; q < K; ++q) S.host[(size_t)ch.x * K + q] = sum[q];
+  S.arrived[ch.x] = 0;
+}
+__global__ void __launch_bounds__(kBlock) b_term_sums_kernel(b_side rows, b_side cols, size_t stride,
+                                                             const int* want)
+{
+  if ((int)blockIdx.x < rows.count)
+    b_term_side<2>(rows, (int)blockIdx.x, stride, want);
+  else
+    b_term_side<3>(cols, (int)blockIdx.x - rows.count, stride, want);
+}
+
 // Elementwise fills of the row buffer.
 template <typename TA>
 __global__ void sq_diff_kernel(const TA* a, const TA* b, int n, double* out)
@@ -422,20 +497,6 @@ __global__ void b_advance_kernel(pdlp_scalars* sc, const int* active, int count,
     if (active[b]) sc[b].t0 += steps;
 }
 
-// Fixed-order block sum of per-thread values (compensated per thread, then a fixed tree).
-__device__ __forceinline__ double block_sum(const ksum& acc, double* sm)
-{
-  sm[threadIdx.x] = acc.value();
-  __syncthreads();
-  for (int h = kBlock / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
-    __syncthreads();
-  }
-  const double v = sm[0];
-  __syncthreads();
-  return v;
-}
-
 // Golub-Kahan-Lanczos bidiagonalisation per instance (the step size), the single engine's
 // run on every instance at once: u and v hold the unnormalised Lanczos vectors, st[b] their
 // norms (and the row chunks of the running sum that have been added), and rowbuf the squares of
@@ -588,9 +649,21 @@ class batch_engine {
     B200_CUDA_CHECK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev));
     B200_CUDA_CHECK(cudaMallocHost(&hbuf_, sizeof(double) * 8 * (size_t)std::max(B_, 1)));
     B200_CUDA_CHECK(cudaMallocHost(&hstatus_, sizeof(int)));
+    B200_CUDA_CHECK(cudaStreamCreateWithFlags(&es_, cudaStreamNonBlocking));
+    B200_CUDA_CHECK(cudaEventCreateWithFlags(&kept_, cudaEventDisableTiming));
+    B200_CUDA_CHECK(cudaEventCreateWithFlags(&checked_, cudaEventDisableTiming));
   }
+  batch_engine(const batch_engine&)            = delete;
+  batch_engine& operator=(const batch_engine&) = delete;
   ~batch_engine()
   {
+    // A check may still read buffers that are released, in the order of s_, after this; and no graph
+    // is destroyed while it runs.
+    if (es_) cudaStreamSynchronize(es_);
+    if (!graphs_.empty()) cudaStreamSynchronize(s_);
+    if (kept_) cudaEventDestroy(kept_);
+    if (checked_) cudaEventDestroy(checked_);
+    if (es_) cudaStreamDestroy(es_);
     for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
     cudaFreeHost(hbuf_);
     cudaFreeHost(hstatus_);
@@ -663,6 +736,10 @@ class batch_engine {
     cr_d_.upload(cranges_.data(), B_, s_);
     build_chunks(rranges_, rows_);
     build_chunks(cranges_, cols_);
+    tplanes_.resize(5 * stride_);
+    tpart_.resize(2 * (size_t)rows_.count + 3 * (size_t)cols_.count + 1);
+    tarrived_.resize(2 * (size_t)B_);
+    tarrived_.zero(s_);
 
     // Per-instance sign (maximisation) and objective scale / offset.
     std::vector<double> sgn(B_);
@@ -869,12 +946,16 @@ class batch_engine {
     B200_CUDA_CHECK(cudaStreamSynchronize(s_));
     if (persist_used_) {
       persist_used_ = false;
-      if (*hstatus_ != 0)
-        throw cuda_error(*hstatus_ == kBarrierTimedOut
-                           ? "persistent batch iterations: a grid barrier passed its deadline"
-                           : "persistent batch iterations: a grid barrier passed its poll limit");
+      check_status();
     }
     collect_form_timing();
+  }
+  void check_status() const
+  {
+    if (*hstatus_ != 0)
+      throw cuda_error(*hstatus_ == kBarrierTimedOut
+                         ? "persistent batch iterations: a grid barrier passed its deadline"
+                         : "persistent batch iterations: a grid barrier passed its poll limit");
   }
 
   void prepare_vectors()
@@ -1296,7 +1377,8 @@ class batch_engine {
       pctl_.zero(s_);
     }
     form_active_ = n_active;
-    cycle_open_  = false;
+    if (cycle_open_) form_.end(s_, cycle_form_, 0, true);  // a cycle cut short is not counted
+    cycle_open_ = false;
     ++form_epochs_;
     const bool avail[plain_form_tuner::kForms] = {true, coop && persist_grid_ > 0, false};
     form_key_   = tune_key(p_.persistent, set_hash);
@@ -1431,29 +1513,52 @@ class batch_engine {
   }
 
   // Unscaled residuals / objectives of every active instance (x_hat, y_hat, slack of the last
-  // major step), like the single-LP evaluation.
-  std::vector<inst_conv> evaluate()
+  // major step), like the single-LP evaluation; where the iterations do not fill the GPU, on a stream
+  // of its own beside the plain iterations that follow, which do not write what it reads.
+  void post_check()
   {
     const int m = in_.m, n = in_.n;
-    b_unscale_kernel<TX><<<vgrid_, kBlock, 0, s_>>>(
+    B200_CUDA_CHECK(cudaStreamWaitEvent(es_, kept_, 0));
+    b_unscale_kernel<TX><<<vgrid_, kBlock, 0, es_>>>(
       xhat_.data(), yhat_.data(), slack_.data(), dc_.data(), dr_.data(), beta_d_.data(),
       gamma_d_.data(), cinst_.data(), rinst_.data(), active_d_.data(), n, m, xu_.data(), yu_.data(),
       su_.data());
     const auto A = wview<double>(true, L_.A.val.data()), AT = wview<double>(false, L_.AT.val.data());
-    sell_map_kernel<double, double, b_term_primal_epi><<<sell_grid(A), kBlock, 0, s_>>>(
-      A, xu_.data(),
-      b_term_primal_epi{lc64_.data(), uc64_.data(), yu_.data(), rowbuf_.data(), stride_,
+    const int gp = sell_grid(A), gd = sell_grid(AT);
+    double* col_planes = tplanes_.data() + 2 * stride_;
+    b_term_kernel<<<gp + gd, kBlock, 0, es_>>>(
+      A, AT, xu_.data(), yu_.data(),
+      b_term_primal_epi{lc64_.data(), uc64_.data(), yu_.data(), tplanes_.data(), stride_,
                         ctx_rows()},
-      partials_.data());
-    seg_reduce<2>(true, 0, true);
-    sell_map_kernel<double, double, b_term_dual_epi><<<sell_grid(AT), kBlock, 0, s_>>>(
-      AT, yu_.data(),
-      b_term_dual_epi{c64_.data(), xu_.data(), su_.data(), rowbuf_.data(), stride_, ctx_cols()},
-      partials_.data());
-    seg_reduce<3>(false, 2 * (size_t)B_, true);
+      b_term_dual_epi{c64_.data(), xu_.data(), su_.data(), col_planes, stride_, ctx_cols()}, gp);
+    const b_side rows{rows_.chunks.data(), rows_.offsets.data(), rows_.count, tplanes_.data(),
+                      tpart_.data(), tarrived_.data(), hbuf_};
+    const b_side cols{cols_.chunks.data(), cols_.offsets.data(), cols_.count, col_planes,
+                      tpart_.data() + 2 * (size_t)rows_.count, tarrived_.data() + B_,
+                      hbuf_ + 2 * (size_t)B_};
+    // Instances without rows or columns have no chunk that would write their sums.
+    for (int b = 0; b < B_; ++b) {
+      const int4 r = rranges_[b], c = cranges_[b];
+      if (r.x == r.y && r.z == r.w) std::fill_n(hbuf_ + 2 * (size_t)b, 2, 0.0);
+      if (c.x == c.y && c.z == c.w) std::fill_n(hbuf_ + 2 * (size_t)B_ + 3 * (size_t)b, 3, 0.0);
+    }
+    if (rows_.count + cols_.count > 0)
+      b_term_sums_kernel<<<rows_.count + cols_.count, kBlock, 0, es_>>>(rows, cols, stride_,
+                                                                       active_d_.data());
     launches_ += 3;
+    if (persist_used_)
+      B200_CUDA_CHECK(cudaMemcpyAsync(hstatus_, &pctl_.data()->status, sizeof(int),
+                                      cudaMemcpyDeviceToHost, es_));
+    status_posted_ = persist_used_;
+    persist_used_  = false;
     B200_LAUNCH_CHECK();
-    fetch(0, 5 * (size_t)B_, hbuf_);
+    B200_CUDA_CHECK(cudaEventRecord(checked_, es_));
+  }
+  std::vector<inst_conv> wait_check()
+  {
+    B200_CUDA_CHECK(cudaEventSynchronize(checked_));
+    if (status_posted_) check_status();
+    collect_form_timing();
     std::vector<inst_conv> cv(B_);
     for (int b = 0; b < B_; ++b) {
       if (!active_h_[b]) continue;
@@ -1509,6 +1614,58 @@ class batch_engine {
     std::vector<long> stall_k(B_, 0);
     int n_active = B_, listed = B_;
     upload_scalars(since);
+    B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
+    // As in the single engine: a check takes about 40 us until the host has read it.
+    const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
+    const bool small    = est_us <= 16.0;
+    const long ahead    = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    std::vector<inst_conv> cv;
+    // Reads the outstanding check; false when no instance is left.  Instances that end are taken out
+    // of the iterations from here on (their solution is the check's, which is not written again).
+    auto resolve = [&]() {
+      const long kc = posted_;
+      posted_       = -1;
+      cv            = wait_check();
+      const bool out_of_time = now_s() - t_start_ >= p_.time_limit;
+      const int before       = n_active;
+      for (int b = 0; b < B_; ++b) {
+        if (!active_h_[b]) continue;
+        const inst_conv& c   = cv[b];
+        const bool primal_ok = c.l2_primal <= p_.abs_primal + p_.rel_primal * b_norm_[b];
+        const bool optimal   = c.l2_dual <= p_.abs_dual + p_.rel_dual * c_norm_[b] && primal_ok &&
+                             c.gap <= p_.abs_gap + p_.rel_gap * c.abs_obj;
+        if (kc > 1 && optimal)
+          finish(b, kOptimal, c, kc);
+        else if (out_of_time)
+          finish(b, kTimeLimit, c, kc);
+        else if (kc >= p_.iteration_limit)
+          finish(b, kIterationLimit, c, kc);
+        else if (!std::isfinite(c.l2_primal) || !std::isfinite(c.l2_dual))
+          finish(b, kNumericalError, c, kc);
+        else if (std::is_same_v<TX, float>) {
+          const double q = termination_distance(
+            c.l2_primal, p_.abs_primal + p_.rel_primal * b_norm_[b], c.l2_dual,
+            p_.abs_dual + p_.rel_dual * c_norm_[b], c.gap, p_.abs_gap + p_.rel_gap * c.abs_obj);
+          if (q <= 0.5 * stall_ref[b]) {
+            stall_ref[b] = q;
+            stall_k[b]   = kc;
+          } else if (kc - stall_k[b] >= kStallWindow)
+            finish(b, kStalled, c, kc);
+        }
+      }
+      n_active = (int)std::count(active_h_.begin(), active_h_.end(), 1);
+      if (n_active == 0) return false;
+      if (n_active < before) active_d_.upload(active_h_.data(), B_, s_);
+      if (2 * n_active <= listed) {
+        B200_CUDA_CHECK(cudaStreamSynchronize(s_));  // no graph is destroyed while it runs
+        rebuild_work(active_h_);
+        listed = n_active;
+        char what[96];
+        std::snprintf(what, sizeof what, "batch: loop to %ld its, %d instances left", kc, n_active);
+        trace(what);
+      }
+      return true;
+    };
 
     for (long k = 0;;) {
       const bool major = (k % kMajor == 0 && k > 0) || k <= 0;
@@ -1517,49 +1674,14 @@ class batch_engine {
       bool any_restart = false;
       if (major || cond) {
         close_cycle(k);
-        const std::vector<inst_conv> cv = evaluate();
-        const bool out_of_time = now_s() - t_start_ >= p_.time_limit;
-        for (int b = 0; b < B_; ++b) {
-          if (!active_h_[b]) continue;
-          const inst_conv& c   = cv[b];
-          const bool primal_ok = c.l2_primal <= p_.abs_primal + p_.rel_primal * b_norm_[b];
-          const bool optimal   = c.l2_dual <= p_.abs_dual + p_.rel_dual * c_norm_[b] &&
-                               primal_ok && c.gap <= p_.abs_gap + p_.rel_gap * c.abs_obj;
-          if (k > 1 && optimal)
-            finish(b, kOptimal, c, k);
-          else if (out_of_time)
-            finish(b, kTimeLimit, c, k);
-          else if (k >= p_.iteration_limit)
-            finish(b, kIterationLimit, c, k);
-          else if (!std::isfinite(c.l2_primal) || !std::isfinite(c.l2_dual))
-            finish(b, kNumericalError, c, k);
-          else if (std::is_same_v<TX, float>) {
-            const double q = termination_distance(
-              c.l2_primal, p_.abs_primal + p_.rel_primal * b_norm_[b], c.l2_dual,
-              p_.abs_dual + p_.rel_dual * c_norm_[b], c.gap, p_.abs_gap + p_.rel_gap * c.abs_obj);
-            if (q <= 0.5 * stall_ref[b]) {
-              stall_ref[b] = q;
-              stall_k[b]   = k;
-            } else if (k - stall_k[b] >= kStallWindow)
-              finish(b, kStalled, c, k);
-          }
-        }
-        n_active = (int)std::count(active_h_.begin(), active_h_.end(), 1);
-        if (n_active == 0) break;
-        if (2 * n_active <= listed) {
-          rebuild_work(active_h_);
-          listed = n_active;
-          char what[96];
-          std::snprintf(what, sizeof what, "batch: loop to %ld its, %d instances left", k,
-                        n_active);
-          trace(what);
-        }
+        post_check();
+        posted_ = k;
+        if (major && !resolve()) break;
 
         if (major) {
           // Restart distances of every active instance.
           sq_diff_kernel<TX><<<vgrid_, kBlock, 0, s_>>>(xa_.data(), xhat_.data(), n,
                                                         rowbuf_.data());
-          active_d_.upload(active_h_.data(), B_, s_);
           seg_reduce<1>(false, 0, true);
           sq_diff_kernel<TX><<<vgrid_, kBlock, 0, s_>>>(ya_.data(), yhat_.data(), m,
                                                         rowbuf_.data());
@@ -1618,9 +1740,9 @@ class batch_engine {
               x_.data(), xa_.data(), xhat_.data(), n, y_.data(), ya_.data(), yhat_.data(), m,
               cinst_.data(), rinst_.data(), restart_flags_.data());
             ++launches_;
+            upload_scalars(since);
           }
         }
-        upload_scalars(since);
         B200_LAUNCH_CHECK();
       }
 
@@ -1633,12 +1755,15 @@ class batch_engine {
           if (is_check(kk) || is_major_step(kk) || ((kk + 1) % kMajor == 0)) break;
           ++R;
         }
+        if (posted_ >= 0) R = std::min(R, ahead);
         run_plain(R, k);
         k += R;
         for (int b = 0; b < B_; ++b)
           if (active_h_[b]) since[b] += R;
+        if (posted_ >= 0 && !resolve()) break;
         continue;
       }
+      if (posted_ >= 0 && !resolve()) break;
 
       if (fpe_all || any_restart) {
         // Every active instance takes the fixed-point-error form of the step (the same update
@@ -1646,6 +1771,7 @@ class batch_engine {
         if (mstep) {
           launch_primal<true, false, true>(0);
           launch_dual<true, false, true>(0);
+          B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
         } else {
           launch_primal<false, false, true>(0);
           launch_dual<false, false, true>(0);
@@ -1675,6 +1801,7 @@ class batch_engine {
       } else {
         launch_primal<true, true, false>(0);
         launch_dual<true, true, false>(0);
+        B200_CUDA_CHECK(cudaEventRecord(kept_, s_));
         advance(1);
         B200_LAUNCH_CHECK();
       }
@@ -1687,6 +1814,7 @@ class batch_engine {
   void write_outputs(double* x_out, double* y_out, double* rc_out)
   {
     const int m = in_.m, n = in_.n;
+    B200_CUDA_CHECK(cudaStreamSynchronize(es_));
     if (x_out)
       scatter_by_inst_kernel<<<vgrid_, kBlock, 0, s_>>>(xu_.data(), L_.col_new2old.data(),
                                                         cinst_.data(), nullptr, n, x_out);
@@ -1707,6 +1835,16 @@ class batch_engine {
   int B_;
   int sms_ = 148, vgrid_ = 592;
   double* hbuf_ = nullptr;
+  // Termination checks: their stream, the event of the last step that kept x_hat / y_hat / slack,
+  // the event of the last check's end, the check that has been launched but not read yet, and
+  // its planes and sums.
+  cudaStream_t es_     = nullptr;
+  cudaEvent_t kept_    = nullptr;
+  cudaEvent_t checked_ = nullptr;
+  long posted_         = -1;
+  bool status_posted_  = false;
+  dbuf<double> tplanes_, tpart_;
+  dbuf<unsigned> tarrived_;
   double t_start_ = 0, t_loop_ = 0;
   double launches_ = 0;
   size_t stride_ = 0;
