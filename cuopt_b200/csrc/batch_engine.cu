@@ -1518,15 +1518,15 @@ class batch_engine {
   void post_check()
   {
     const int m = in_.m, n = in_.n;
-    B200_CUDA_CHECK(cudaStreamWaitEvent(es_, kept_, 0));
-    b_unscale_kernel<TX><<<vgrid_, kBlock, 0, es_>>>(
+    if (cs_check_ != s_) B200_CUDA_CHECK(cudaStreamWaitEvent(cs_check_, kept_, 0));
+    b_unscale_kernel<TX><<<vgrid_, kBlock, 0, cs_check_>>>(
       xhat_.data(), yhat_.data(), slack_.data(), dc_.data(), dr_.data(), beta_d_.data(),
       gamma_d_.data(), cinst_.data(), rinst_.data(), active_d_.data(), n, m, xu_.data(), yu_.data(),
       su_.data());
     const auto A = wview<double>(true, L_.A.val.data()), AT = wview<double>(false, L_.AT.val.data());
     const int gp = sell_grid(A), gd = sell_grid(AT);
     double* col_planes = tplanes_.data() + 2 * stride_;
-    b_term_kernel<<<gp + gd, kBlock, 0, es_>>>(
+    b_term_kernel<<<gp + gd, kBlock, 0, cs_check_>>>(
       A, AT, xu_.data(), yu_.data(),
       b_term_primal_epi{lc64_.data(), uc64_.data(), yu_.data(), tplanes_.data(), stride_,
                         ctx_rows()},
@@ -1543,16 +1543,16 @@ class batch_engine {
       if (c.x == c.y && c.z == c.w) std::fill_n(hbuf_ + 2 * (size_t)B_ + 3 * (size_t)b, 3, 0.0);
     }
     if (rows_.count + cols_.count > 0)
-      b_term_sums_kernel<<<rows_.count + cols_.count, kBlock, 0, es_>>>(rows, cols, stride_,
+      b_term_sums_kernel<<<rows_.count + cols_.count, kBlock, 0, cs_check_>>>(rows, cols, stride_,
                                                                        active_d_.data());
     launches_ += 3;
     if (persist_used_)
       B200_CUDA_CHECK(cudaMemcpyAsync(hstatus_, &pctl_.data()->status, sizeof(int),
-                                      cudaMemcpyDeviceToHost, es_));
+                                      cudaMemcpyDeviceToHost, cs_check_));
     status_posted_ = persist_used_;
     persist_used_  = false;
     B200_LAUNCH_CHECK();
-    B200_CUDA_CHECK(cudaEventRecord(checked_, es_));
+    B200_CUDA_CHECK(cudaEventRecord(checked_, cs_check_));
   }
   std::vector<inst_conv> wait_check()
   {
@@ -1619,6 +1619,7 @@ class batch_engine {
     const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
     const bool small    = est_us <= 16.0;
     const long ahead    = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    cs_check_           = small ? es_ : s_;
     std::vector<inst_conv> cv;
     // Reads the outstanding check; false when no instance is left.  Instances that end are taken out
     // of the iterations from here on (their solution is the check's, which is not written again).
@@ -1838,7 +1839,7 @@ class batch_engine {
   // Termination checks: their stream, the event of the last step that kept x_hat / y_hat / slack,
   // the event of the last check's end, the check that has been launched but not read yet, and
   // its planes and sums.
-  cudaStream_t es_     = nullptr;
+  cudaStream_t es_     = nullptr, cs_check_ = nullptr;  // cs_check_: es_, or s_ for large batches
   cudaEvent_t kept_    = nullptr;
   cudaEvent_t checked_ = nullptr;
   long posted_         = -1;

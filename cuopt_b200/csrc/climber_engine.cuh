@@ -718,24 +718,24 @@ class climber_engine {
   void post_check()
   {
     const int m = e_.in_.m, n = e_.in_.n;
-    B200_CUDA_CHECK(cudaStreamWaitEvent(e_.es_, e_.kept_, 0));
+    if (cs_check_ != s_) B200_CUDA_CHECK(cudaStreamWaitEvent(cs_check_, e_.kept_, 0));
     if (n_act() > 0) {
-      mm_unscale_kernel<<<e_.vgrid_, kBlock, 0, e_.es_>>>(
+      mm_unscale_kernel<<<e_.vgrid_, kBlock, 0, cs_check_>>>(
         xhat_.data(), yhat_.data(), slack_.data(), e_.dc_.data(), e_.dr_.data(), 1.0 / e_.beta_,
         1.0 / e_.gamma_, n, m, ld_, active_d_.data(), xu_.data(), yu_.data(), su_.data());
       const auto A = view64(e_.L_.A), AT = view64(e_.L_.AT);
       const int gp = sell_grid(A), gd = sell_grid(AT);
-      mm_term_kernel<<<(gp + gd) * n_act(), kBlock, 0, e_.es_>>>(
+      mm_term_kernel<<<(gp + gd) * n_act(), kBlock, 0, cs_check_>>>(
         A, AT, xu_.data(), yu_.data(), ld_, groups_d_.data(), n_act(),
         mm_term_primal_epi{e_.lc64_.data(), e_.uc64_.data(), yu_.data(), ctx()},
         mm_term_dual_epi{e_.c64_.data(), xu_.data(), su_.data(), ctx()}, gp, tpartials_.data(),
         tstride_);
-      mm_term_sums_kernel<<<n_act() * 5 * kGroup, kBlock, 0, e_.es_>>>(
+      mm_term_sums_kernel<<<n_act() * 5 * kGroup, kBlock, 0, cs_check_>>>(
         tpartials_.data(), tstride_, gp, gd, groups_d_.data(), hbuf_);
       launches_ += 3;
       B200_LAUNCH_CHECK();
     }
-    B200_CUDA_CHECK(cudaEventRecord(e_.checked_, e_.es_));
+    B200_CUDA_CHECK(cudaEventRecord(e_.checked_, cs_check_));
   }
   std::vector<conv_info> wait_check()
   {
@@ -806,6 +806,7 @@ class climber_engine {
     const double est_us = 9.0 + 2.0 * (double)e_.L_.nnz * groups_ / 5e4;
     const bool small    = est_us <= 16.0;
     const long ahead    = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    cs_check_           = small ? e_.es_ : s_;
     std::vector<conv_info> cv;
     // Reads the outstanding check; false when no climber is left.  Climbers that end are taken out of
     // the iterations from here on (their solution is the check's, which is not written again).
@@ -1018,6 +1019,7 @@ class climber_engine {
   dbuf<int> active_d_, flags_, groups_d_;
   std::vector<int> groups_h_;
   size_t pstride_ = 0, tstride_ = 0;  // block sums per group: the steps', the checks'
+  cudaStream_t cs_check_ = nullptr;   // the checks' stream (the iterations' for large batches)
   long posted_ = -1;                  // the check that has been launched but not read yet
   dbuf<pdlp_scalars> sc_d_;
   dbuf<double> x_, xhat_, slack_, xbar_, xa_, aty_, y_, yhat_, ybar_, ya_, xu_, yu_, su_;

@@ -1178,13 +1178,13 @@ class engine {
   void post_check()
   {
     const int m = in_.m, n = in_.n;
-    B200_CUDA_CHECK(cudaStreamWaitEvent(es_, kept_, 0));
-    unscale_kernel<TX><<<std::min(vgrid_, ceil_div((long)n + m, kBlock)), kBlock, 0, es_>>>(
+    if (cs_check_ != s_) B200_CUDA_CHECK(cudaStreamWaitEvent(cs_check_, kept_, 0));
+    unscale_kernel<TX><<<std::min(vgrid_, ceil_div((long)n + m, kBlock)), kBlock, 0, cs_check_>>>(
       kept_xhat(), kept_yhat(), kept_slack(), dc_.data(), dr_.data(), 1.0 / beta_, 1.0 / gamma_, n,
       m, xu_.data(), yu_.data(), su_.data());
     ++launches_;
     enqueue_conv(hres_);
-    B200_CUDA_CHECK(cudaEventRecord(checked_, es_));
+    B200_CUDA_CHECK(cudaEventRecord(checked_, cs_check_));
   }
   conv_info wait_check()
   {
@@ -1200,24 +1200,24 @@ class engine {
   {
     const auto A = view64(L_.A), AT = view64(L_.AT);
     const int gp = sweep_grid(A), gd = sweep_grid(AT);
-    term_kernel<<<gp + gd, kBlock, 0, es_>>>(
+    term_kernel<<<gp + gd, kBlock, 0, cs_check_>>>(
       A, AT, xu_.data(), yu_.data(), term_primal_epi{lc64_.data(), uc64_.data(), yu_.data()},
       term_dual_epi{c64_.data(), xu_.data(), su_.data()}, gp, gd, tpartials_.data(),
       tarrived_.data(), tres_.data(), h, &pctl_.data()->status,
       tile_primal_ || tile_dual_ ? terr_.data() : nullptr);
     ++launches_;
     if (p_.per_constraint_residual) {
-      sell_map_kernel<double, double, term_linf_primal_epi><<<gp, kBlock, 0, es_>>>(
+      sell_map_kernel<double, double, term_linf_primal_epi><<<gp, kBlock, 0, cs_check_>>>(
         A, xu_.data(), term_linf_primal_epi{lc64_.data(), uc64_.data(), p_.rel_primal},
         tpartials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, es_>>>(tpartials_.data(), gp, tres_.data() + 5);
-      sell_map_kernel<double, double, term_linf_dual_epi><<<gd, kBlock, 0, es_>>>(
+      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gp, tres_.data() + 5);
+      sell_map_kernel<double, double, term_linf_dual_epi><<<gd, kBlock, 0, cs_check_>>>(
         AT, yu_.data(), term_linf_dual_epi{c64_.data(), su_.data(), p_.rel_dual},
         tpartials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, es_>>>(tpartials_.data(), gd, tres_.data() + 6);
+      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gd, tres_.data() + 6);
       launches_ += 4;
       B200_CUDA_CHECK(cudaMemcpyAsync(h + 5, tres_.data() + 5, 2 * sizeof(double),
-                                      cudaMemcpyDeviceToHost, es_));
+                                      cudaMemcpyDeviceToHost, cs_check_));
     }
     B200_LAUNCH_CHECK();
   }
@@ -1388,6 +1388,7 @@ class engine {
     const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
     const bool small    = est_us <= 16.0;
     ahead_              = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
+    cs_check_           = small ? es_ : s_;
     const auto A = As_view(), AT = ATs_view();
 
     for (;;) {
@@ -1610,7 +1611,7 @@ class engine {
   cudaStream_t s_ = nullptr;
   // Termination checks: their stream, the event of the last step that kept x_hat / y_hat / slack,
   // the event of the last check's end, and the check that has been launched but not read yet.
-  cudaStream_t es_     = nullptr;
+  cudaStream_t es_     = nullptr, cs_check_ = nullptr;  // cs_check_: es_, or s_ for large LPs
   cudaEvent_t kept_    = nullptr;
   cudaEvent_t checked_ = nullptr;
   long posted_         = -1;
