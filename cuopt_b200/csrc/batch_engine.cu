@@ -774,23 +774,7 @@ class batch_engine {
     fill(dr_.data(), m, 1.0);
     fill(dc_.data(), n, 1.0);
     dbuf<double> rtmp(m), ctmp(n);
-    for (int it = 0; it < kRuizIterations; ++it) {
-      row_scaled_abs_kernel<0, false><<<sell_grid(A64), kBlock, 0, s_>>>(A64, dr_.data(),
-                                                                        dc_.data(), 0.0,
-                                                                        rtmp.data());
-      row_scaled_abs_kernel<0, true><<<sell_grid(AT64), kBlock, 0, s_>>>(AT64, dr_.data(),
-                                                                        dc_.data(), 0.0,
-                                                                        ctmp.data());
-      apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dr_.data(), rtmp.data(), m);
-      apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dc_.data(), ctmp.data(), n);
-    }
-    row_scaled_abs_kernel<1, false><<<sell_grid(A64), kBlock, 0, s_>>>(A64, dr_.data(), dc_.data(),
-                                                                      kPcAlpha, rtmp.data());
-    row_scaled_abs_kernel<1, true><<<sell_grid(AT64), kBlock, 0, s_>>>(
-      AT64, dr_.data(), dc_.data(), 2.0 - kPcAlpha, ctmp.data());
-    apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dr_.data(), rtmp.data(), m);
-    apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dc_.data(), ctmp.data(), n);
-    B200_LAUNCH_CHECK();
+    launches_ += scale_passes(A64, AT64, kRuizIterations, kPcAlpha, dr_, dc_, rtmp, ctmp, s_);
     As_.resize(L_.A.stored());
     ATs_.resize(L_.AT.stored());
     scale_values_kernel<TX, false><<<sell_grid(A64), kBlock, 0, s_>>>(A64, dr_.data(), dc_.data(),

@@ -1957,15 +1957,17 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
 // ---------------------------------------------------------------------------------------------
 // Scaling (reference initial_scaling.cu:152-569).
 
-// For every row r of layout A: out[r] = max_k |v (s_first) (s_second)| (MODE 0) or
-// sum_k |v s_first s_second|^alpha (MODE 1), where for A (TRANSPOSED=false) the product is
-// (a_ij dr_i) dc_j and for A^T (TRANSPOSED=true) it is (a_ij dr_i) dc_j with i = idx, j = row.
+// One pass of the scaling: for every row of A, drn_i = dr_i / sqrt(v_i) with v_i = max_k |a_ik dr_i
+// dc_k| (MODE 0) or sum_k |a_ik dr_i dc_k|^alpha_r (MODE 1), and for every row of A^T the same with
+// dc (a_divides_sqrt_b_bounded, utils.cuh:156-163: unchanged where v is 0).  Both sides read the old
+// factors, so they run in one launch (blocks [0, ga) the rows of A) that writes the new ones beside
+// them; as two sweeps and two vector steps a pass was four launches, and the 11 passes the longer
+// part of a small LP's scaling.
 template <int MODE, bool TRANSPOSED>
-__global__ void __launch_bounds__(kBlock) row_scaled_abs_kernel(const dev_sell<double> A,
-                                                                const double* dr,
-                                                                const double* dc, double alpha,
-                                                                double* out)
+__device__ __forceinline__ void scale_pass_block(const dev_sell<double>& A, const double* dr,
+                                                 const double* dc, double alpha, double* out, int vb)
 {
+  const double* own = TRANSPOSED ? dc : dr;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int lb   = long_blocks(A.n_long);
   auto term      = [&](double v, int row, int col) {
@@ -1973,8 +1975,12 @@ __global__ void __launch_bounds__(kBlock) row_scaled_abs_kernel(const dev_sell<d
     const double a = fabs(p);
     return MODE == 0 ? a : pow(a, alpha);
   };
-  if ((int)blockIdx.x < lb) {
-    const int row = blockIdx.x * kWarpsPerBlock + warp;
+  auto store = [&](int row, double v) {
+    const double d = own[row];
+    out[row]       = v > 0.0 ? d / sqrt(v) : d;
+  };
+  if (vb < lb) {
+    const int row = vb * kWarpsPerBlock + warp;
     if (row < A.n_long) {
       double acc = 0.0;
       for (int64_t k = A.long_off[row] + lane; k < A.long_off[row + 1]; k += kWarp) {
@@ -1982,36 +1988,59 @@ __global__ void __launch_bounds__(kBlock) row_scaled_abs_kernel(const dev_sell<d
         acc            = MODE == 0 ? fmax(acc, t) : acc + t;
       }
       acc = MODE == 0 ? warp_max(acc) : warp_sum(acc);
-      if (lane == 0) out[row] = acc;
+      if (lane == 0) store(row, acc);
     }
   } else {
-    const int s = (blockIdx.x - lb) * kWarpsPerBlock + warp;
+    const int s = (vb - lb) * kWarpsPerBlock + warp;
     if (s < A.n_slices) {
       const int64_t base = A.slice_off[s];
       const int len      = (int)((A.slice_off[s + 1] - base) >> 5);
       const int row      = A.n_long + s * kWarp + lane;
       if (row < A.rows) {
         double acc = 0.0;
-          for (int k = 0; k < len; ++k) {
+        for (int k = 0; k < len; ++k) {
           const int64_t p = sell_pos(base, k, lane);
           const double v  = A.val[p];
           if (v == 0.0) continue;  // padding (and explicit zeros, which contribute nothing)
           const double t = term(v, row, A.idx[p]);
           acc            = MODE == 0 ? fmax(acc, t) : acc + t;
         }
-        out[row] = acc;
+        store(row, acc);
       }
     }
   }
 }
-
-// d[i] <- d[i] / sqrt(v[i]) where v[i] > 0 (a_divides_sqrt_b_bounded, utils.cuh:156-163)
-static __global__ void apply_root_scaling_kernel(double* d, const double* v, int n)
+template <int MODE>
+__global__ void __launch_bounds__(kBlock)
+  scale_pass_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* dr,
+                    const double* dc, double alpha_r, double alpha_c, double* drn, double* dcn,
+                    int ga)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double b = v[i];
-    if (b > 0.0) d[i] = d[i] / sqrt(b);
+  if ((int)blockIdx.x < ga)
+    scale_pass_block<MODE, false>(A, dr, dc, alpha_r, drn, (int)blockIdx.x);
+  else
+    scale_pass_block<MODE, true>(AT, dr, dc, alpha_c, dcn, (int)blockIdx.x - ga);
+}
+
+// Ruiz (`ruiz` passes) then Pock-Chambolle (reference initial_scaling.cu:152-365) on factors that
+// start at 1 in dr / dc; rt / ct: buffers of the same lengths.  Returns the launches.
+inline int scale_passes(const dev_sell<double>& A, const dev_sell<double>& AT, int ruiz, double alpha,
+                        dbuf<double>& dr, dbuf<double>& dc, dbuf<double>& rt, dbuf<double>& ct,
+                        cudaStream_t s)
+{
+  const int ga = sell_grid(A), g = ga + sell_grid(AT);
+  for (int it = 0; it <= ruiz; ++it) {
+    if (it < ruiz)
+      scale_pass_kernel<0><<<g, kBlock, 0, s>>>(A, AT, dr.data(), dc.data(), 0.0, 0.0, rt.data(),
+                                               ct.data(), ga);
+    else
+      scale_pass_kernel<1><<<g, kBlock, 0, s>>>(A, AT, dr.data(), dc.data(), alpha, 2.0 - alpha,
+                                               rt.data(), ct.data(), ga);
+    std::swap(dr, rt);
+    std::swap(dc, ct);
   }
+  B200_LAUNCH_CHECK();
+  return ruiz + 1;
 }
 
 // Scaled copy of the matrix values: A_s = (a dr_i) dc_j, A^T_s = (a dc_j) dr_i.

@@ -229,21 +229,8 @@ class engine {
     fill(dr_.data(), m, 1.0);
     fill(dc_.data(), n, 1.0);
     dbuf<double> rtmp(m), ctmp(n);
-    for (int it = 0; it < kRuizIterations; ++it) {
-      row_scaled_abs_kernel<0, false><<<sell_grid(view64(L_.A)), kBlock, 0, s_>>>(
-        view64(L_.A), dr_.data(), dc_.data(), 0.0, rtmp.data());
-      row_scaled_abs_kernel<0, true><<<sell_grid(view64(L_.AT)), kBlock, 0, s_>>>(
-        view64(L_.AT), dr_.data(), dc_.data(), 0.0, ctmp.data());
-      apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dr_.data(), rtmp.data(), m);
-      apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dc_.data(), ctmp.data(), n);
-    }
-    row_scaled_abs_kernel<1, false><<<sell_grid(view64(L_.A)), kBlock, 0, s_>>>(
-      view64(L_.A), dr_.data(), dc_.data(), kPcAlpha, rtmp.data());
-    row_scaled_abs_kernel<1, true><<<sell_grid(view64(L_.AT)), kBlock, 0, s_>>>(
-      view64(L_.AT), dr_.data(), dc_.data(), 2.0 - kPcAlpha, ctmp.data());
-    apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dr_.data(), rtmp.data(), m);
-    apply_root_scaling_kernel<<<vgrid_, kBlock, 0, s_>>>(dc_.data(), ctmp.data(), n);
-    B200_LAUNCH_CHECK();
+    launches_ += scale_passes(view64(L_.A), view64(L_.AT), kRuizIterations, kPcAlpha, dr_, dc_, rtmp,
+                              ctmp, s_);
 
     // Scaled matrix values in the iterate precision.
     As_.resize(L_.A.stored());
