@@ -16,7 +16,7 @@
 // are the exact derivatives; otherwise lambda and mu are LSQR's minimum-norm least-squares
 // solutions (in the equilibrated variables), the derivatives of the minimum-norm response.
 //
-// Every solve with M or M^T is matrix-free: LSQR on the GPU with one thread block per system
+// Every solve with M or M^T is matrix-free: LSQR on the GPU with one cluster per system
 // (lsqr.cu), all the systems of a batch of instances in one launch.
 #include <algorithm>
 #include <cmath>

@@ -1,4 +1,4 @@
-// Batched LSQR on sm_100a: many small sparse least-squares systems, one thread block each.
+// Batched LSQR on sm_100a: many small sparse least-squares systems, one cluster each.
 //
 // The KKT adjoint and the vertex polish both need solves with the active-set matrix M = A_{R,F}
 // (rows held at a bound x variables strictly inside their bounds) or its transpose.  These are

@@ -29,8 +29,8 @@ struct lsqr_result {
 };
 
 // Solves every problem with LSQR (Paige and Saunders, ACM TOMS 8(1), 1982) after a two-sided
-// diagonal equilibration of each operator.  One thread block per problem runs the whole
-// iteration; nothing is launched per iteration.  `tol` is LSQR's atol = btol; `max_iter` <= 0
+// diagonal equilibration of each operator.  One thread-block cluster per problem runs the
+// whole iteration; nothing is launched per iteration.  `tol` is LSQR's atol = btol; `max_iter` <= 0
 // chooses 20 x (rows + cols), at most 200000.
 std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>& ps,
                                           cudaStream_t s, double tol = 1e-14, int max_iter = 0);

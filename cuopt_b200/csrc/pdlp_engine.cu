@@ -5,7 +5,8 @@
 // the host (restart decision, PID primal weight, fixed-point errors); all vector and matrix work
 // is in the kernels of kernels.cuh.  Iterations that need neither a termination test, a "major"
 // step nor a fixed-point error are replayed from cached CUDA graphs of 2^k iterations, or run by one
-// persistent cooperative launch, whichever form timed faster on the solve's first runs.
+// persistent cooperative launch or one cluster launch, whichever form timed faster on the solve's
+// first runs (small LPs always take the cluster).
 #include "device_layout.cuh"
 #include "host_io.hpp"
 #include "kernels.cuh"

@@ -3,9 +3,10 @@
 //   form 0: replays of cached CUDA graphs of 2^k iterations (two sweep kernels per iteration);
 //   form 1: one cooperative launch of the persistent kernel (persistent_plain_kernel), with a grid
 //           barrier after every sweep;
-//   form 2: one launch of a thread-block cluster that keeps the gathered vectors in the shared
-//           memory of each of its blocks (cluster_plain_kernel, small LPs only), with a cluster
-//           barrier after every sweep.
+//   form 2: one launch of a thread-block cluster that keeps the gathered vectors, and where they
+//           fit the matrices, in the shared memory of its blocks (resident_unit_kernel and
+//           resident_plain_kernel, small LPs only), with an exchange or a cluster barrier after
+//           every sweep.
 // All forms run the same per-row arithmetic, so the iterates do not depend on the choice, and the
 // choice can be made online: with pdlp_persistent_iterations = -1 the first cycles of a solve (a
 // cycle: the iterations from one termination check to the next, with their major steps and every

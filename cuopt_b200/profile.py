@@ -539,7 +539,7 @@ def run_adjoint(a) -> dict:
             solver_checked += 1
     return {"config": "c4", "count": count, "m": 5000, "n": 10000, "forward_s": forward_s,
             "backward_s": backward_s, "adjoint_ms_per_instance": backward_s * 1e3 / count,
-            "backward": "matrix-free LSQR on the GPU (cuOptSolutionAdjointBatch), one thread block "
+            "backward": "matrix-free LSQR on the GPU (cuOptSolutionAdjointBatch), one cluster "
                         "per active-set system; no dense factorisation",
             "crossover_vertex_max_rel_error": vertex_err,
             "grad_vs_exact_max_rel_error": basis_err, "exact_checked_instances": count,

@@ -6,7 +6,7 @@ solves  min c.x  s.t.  con_lo <= A x <= con_up,  var_lo <= x <= var_up  (A in CS
 column_indices, row_offsets; int32 indices) with the library's PDLP and returns the primal and
 dual solutions as float64 tensors on the device of `c`.  Backward is the KKT adjoint of the
 optimal solution (cuOptSolutionAdjointBatch: matrix-free LSQR solves with the active-set matrix
-on the GPU, one thread block per system): gradients flow to c, con_lo, con_up and values; the CSR
+on the GPU, one thread-block cluster per system): gradients flow to c, con_lo, con_up and values; the CSR
 structure and the variable bounds are constants.  At a non-degenerate vertex these are the exact
 derivatives of the solution map; elsewhere they are those of its minimum-norm response.
 

@@ -240,7 +240,7 @@ cuopt_int_t cuOptBatchPDLPStrongBranching(cuOptOptimizationProblem problem,
  * bounds are equal, the gradient with respect to its right-hand side is in dl_dlower.  At a
  * non-degenerate vertex these are the exact derivatives; otherwise those of the minimum-norm
  * response (in the equilibrated variables).  The active-set solves are matrix-free: LSQR on the
- * GPU, one thread block per system.  Any output pointer may be NULL.  Returns
+ * GPU, one cluster per system.  Any output pointer may be NULL.  Returns
  * CUOPT_INVALID_ARGUMENT if the solution is not Optimal. */
 cuopt_int_t cuOptSolutionAdjoint(cuOptOptimizationProblem problem,
                                  cuOptSolution solution,
@@ -254,7 +254,7 @@ cuopt_int_t cuOptSolutionAdjoint(cuOptOptimizationProblem problem,
 /* cuOptSolutionAdjoint for `count` (problem, solution) pairs at once (no counterpart in the
  * reference): every pointer argument is an array of `count` pointers with the meaning of the single
  * call's argument (dl_dx[i] required; dl_dy, the output arrays, or any of their entries may be
- * NULL).  All the active-set solves of the batch run in one launch, one thread block each.
+ * NULL).  All the active-set solves of the batch run in one launch, one cluster each.
  * Returns CUOPT_INVALID_ARGUMENT (and writes nothing) if any solution is not Optimal. */
 cuopt_int_t cuOptSolutionAdjointBatch(cuopt_int_t count,
                                       const cuOptOptimizationProblem* problems,
