@@ -3,7 +3,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <limits>
 #include <memory>
 #include <mutex>
@@ -128,43 +127,28 @@ class krylov_power_iteration {
     }
     const int J = (int)d_.size();
     if (J == 0) return false;
-    // T and q padded with zeros to whole groups of four (and one entry in front), so that the sums
-    // (four each: one per place in a group) are added two by two: 1 149 iterates of 16 to 176
-    // entries took 0.97 ms entry by entry and take 0.32 ms, with the same bits.
-    const int G = (J + 3) / 4 * 4;
-    if (q_.empty()) q_.assign(2, 1.0), q_[0] = 0.0;
-    d_.resize(G, 0.0);
-    e_.insert(e_.begin(), 0.0);
-    e_[J] = 0.0;
-    e_.resize(G + 1, 0.0);
-    q_.resize(G + 2, 0.0);
-    z_.resize(G);
-    const double *d = d_.data(), *e = e_.data();
-    double *q = q_.data() + 1, *z = z_.data();
+    if (q_.empty()) q_.assign(1, 1.0);
+    q_.resize(J, 0.0);
+    z_.resize(J);
     while (k_ < kPowerMaxIters) {
-      // z = T q and s2 = q . z, then |z - s2 q| and |z|.
-      pair s[2]{}, r[2]{}, w[2]{};
-      for (int j = 0; j < G; j += 4)
-        for (int h = 0; h < 2; ++h) {
-          const int i   = j + 2 * h;
-          const pair qi = get(q + i);
-          const pair zi = get(e + i) * get(q + i - 1) + get(d + i) * qi + get(e + i + 1) * get(q + i + 1);
-          put(z + i, zi);
-          s[h] += qi * zi;
-        }
-      const double s2 = sum(s);
-      if (!capped && !(std::fabs(next * q[J - 1]) <= kKrylovLeak * s2)) return false;
-      for (int j = 0; j < G; j += 4)
-        for (int h = 0; h < 2; ++h) {
-          const pair zi = get(z + j + 2 * h), t = zi - s2 * get(q + j + 2 * h);
-          r[h] += t * t;
-          w[h] += zi * zi;
-        }
+      // z = T q and s2 = q . z, then |z - s2 q| and |z| (four sums each, so the additions overlap).
+      double s[4] = {0, 0, 0, 0}, r[4] = {0, 0, 0, 0}, w[4] = {0, 0, 0, 0};
+      z_[0] = d_[0] * q_[0] + (J > 1 ? e_[0] * q_[1] : 0.0);
+      for (int j = 1; j < J - 1; ++j) z_[j] = e_[j - 1] * q_[j - 1] + d_[j] * q_[j] + e_[j] * q_[j + 1];
+      if (J > 1) z_[J - 1] = e_[J - 2] * q_[J - 2] + d_[J - 1] * q_[J - 1];
+      for (int j = 0; j < J; ++j) s[j & 3] += q_[j] * z_[j];
+      const double s2 = (s[0] + s[1]) + (s[2] + s[3]);
+      if (!capped && !(std::fabs(next * q_[J - 1]) <= kKrylovLeak * s2)) return false;
+      for (int j = 0; j < J; ++j) {
+        const double t = z_[j] - s2 * q_[j];
+        r[j & 3] += t * t;
+        w[j & 3] += z_[j] * z_[j];
+      }
       s2_ = s2;
       ++k_;
-      if (std::sqrt(sum(r)) < kPowerTol) return true;
-      const double scale = 1.0 / std::sqrt(sum(w));
-      for (int i = 0; i < G; i += 2) put(q + i, get(z + i) * scale);
+      if (std::sqrt((r[0] + r[1]) + (r[2] + r[3])) < kPowerTol) return true;
+      const double scale = 1.0 / std::sqrt((w[0] + w[1]) + (w[2] + w[3]));
+      for (int j = 0; j < J; ++j) q_[j] = z_[j] * scale;
     }
     return true;
   }
@@ -172,16 +156,6 @@ class krylov_power_iteration {
   int iterations() const { return k_; }
 
  private:
-  typedef double pair __attribute__((vector_size(16)));
-  static pair get(const double* p)
-  {
-    pair v;
-    std::memcpy(&v, p, sizeof v);
-    return v;
-  }
-  static void put(double* p, const pair& v) { std::memcpy(p, &v, sizeof v); }
-  static double sum(const pair (&v)[2]) { return (v[0][0] + v[0][1]) + (v[1][0] + v[1][1]); }
-
   std::vector<double> d_, e_, q_, z_;  // T, and the normalised iterate of step k_ + 1
   double s2_ = 0.0;
   int k_     = 0;
