@@ -1746,7 +1746,7 @@ __device__ __forceinline__ double gk_next_u(double acc, double u, double alpha, 
 struct gk_primal_epi {
   static constexpr int kRed = 1;
   double* v;
-  const gk_state* st;
+  double beta = 0.0, alpha = 0.0;  // set by the kernel
   struct pre_t {
     double v;
   };
@@ -1754,7 +1754,7 @@ struct gk_primal_epi {
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{v[j]}; }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<1>& r) const
   {
-    const double pj = gk_next_v(acc, p.v, st->beta, st->alpha);
+    const double pj = gk_next_v(acc, p.v, beta, alpha);
     v[j]            = pj;
     r.v[0] += pj * pj;
   }
@@ -1764,7 +1764,7 @@ struct gk_primal_epi {
 struct gk_dual_epi {
   static constexpr int kRed = 1;
   double* u;
-  const gk_state* st;
+  double beta = 0.0, alpha = 0.0;
   struct pre_t {
     double u;
   };
@@ -1772,7 +1772,7 @@ struct gk_dual_epi {
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{u[i]}; }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<1>& r) const
   {
-    const double qi = gk_next_u(acc, p.u, st->alpha, st->beta);
+    const double qi = gk_next_u(acc, p.u, alpha, beta);
     u[i]            = qi;
     r.v[0] += qi * qi;
   }
@@ -1795,6 +1795,8 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) gk_sweep_kernel(cons
                                                           double* partials, gk_state* st,
                                                           double* hist)
 {
+  epi.beta  = st->beta;
+  epi.alpha = st->alpha;
   sell_map_block(A, g, epi, partials, (int)blockIdx.x);
   __shared__ int last;
   if (threadIdx.x == 0) {  // the thread that wrote this block's partial
@@ -1818,6 +1820,56 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) gk_sweep_kernel(cons
       st->step    = k + 1;
     }
     st->arrived = 0;
+  }
+}
+
+// sqrt of the sum of at most kBlock block partials, in ordered_block_sum's tree, by every warp.
+__device__ __forceinline__ double gk_tree(double (&e)[kBlock / kWarp])
+{
+#pragma unroll
+  for (int h = kBlock / kWarp / 2; h > 0; h >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; ++j) e[j] += e[j + h];
+#pragma unroll
+  for (int h = kWarp / 2; h > 0; h >>= 1) e[0] += __shfl_down_sync(0xffffffffu, e[0], h);
+  return sqrt(__shfl_sync(0xffffffffu, e[0], 0));
+}
+__device__ __forceinline__ double gk_partials_norm(const double* partials, int blocks)
+{
+  double e[kBlock / kWarp];
+#pragma unroll
+  for (int j = 0; j < kBlock / kWarp; ++j) {
+    const int b = (threadIdx.x & 31) + j * kWarp;
+    e[j]        = b < blocks ? partials[b] : 0.0;
+  }
+  return gk_tree(e);
+}
+
+// The half step of an LP whose sweeps have at most kBlock blocks: the norm of the vector gathered
+// is formed at the start of the sweep, by every warp from the `nin` block partials of the sweep
+// before (nin 0: it is in st), instead of at the end of that sweep.  There, the fence, the count of
+// blocks and the sums of the last one follow one another: a half step on a 12 007 x 30 011 LP took
+// 7.7 us and takes 6.6 us.  With more partials every block would read more than one a thread.
+template <int FIELD, typename TM, class Epi>
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>)
+  gk_chain_kernel(const dev_sell<TM> A, const double* __restrict__ g, Epi epi, const double* pin,
+                  int nin, double* pout, gk_state* st, double* hist, int k)
+{
+  double& own = FIELD == 0 ? st->beta : st->alpha;  // written by block 0, read by later kernels
+  const double norm = nin > 0 ? gk_partials_norm(pin, nin) : own;
+  epi.beta          = FIELD == 0 ? norm : st->beta;
+  epi.alpha         = FIELD == 0 ? st->alpha : norm;
+  if (nin > 0 && blockIdx.x == 0 && threadIdx.x == 0) own = hist[k] = norm;
+  sell_map_block(A, g, epi, pout, (int)blockIdx.x);
+}
+// beta after the last step of a chain.
+static __global__ void gk_chain_end_kernel(const double* partials, int blocks, gk_state* st,
+                                           double* betas, int k)
+{
+  const double norm = gk_partials_norm(partials, blocks);
+  if (threadIdx.x == 0) {
+    st->beta = betas[k] = norm;
+    st->step = k;
   }
 }
 
@@ -1855,13 +1907,7 @@ __device__ __forceinline__ double cluster_gk_norm(const double* ws, int blocks)
       for (int w = 0; w < kWarpsPerBlock; ++w) t += ws[b * kWarpsPerBlock + w];
     e[j] = t;
   }
-#pragma unroll
-  for (int h = kBlock / kWarp / 2; h > 0; h >>= 1)
-#pragma unroll
-    for (int j = 0; j < h; ++j) e[j] += e[j + h];
-#pragma unroll
-  for (int h = kWarp / 2; h > 0; h >>= 1) e[0] += __shfl_down_sync(0xffffffffu, e[0], h);
-  return sqrt(__shfl_sync(0xffffffffu, e[0], 0));
+  return gk_tree(e);
 }
 
 template <typename TX>

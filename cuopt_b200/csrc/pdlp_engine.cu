@@ -506,6 +506,7 @@ class engine {
     const size_t smem  = cluster_gk_smem<TX>(m, n, sweep_grid(ATs), sweep_grid(As), resident_);
     const bool cluster = resident_ok_ && resident_cached_ && sweep_grid(ATs) <= kBlock &&
                          sweep_grid(As) <= kBlock && allow_cluster_gk(smem);
+    const bool chained = sweep_grid(ATs) <= kBlock && sweep_grid(As) <= kBlock;
     for (int k = 0, tested = 0; k < max_steps;) {
       // One cluster launch takes the steps that most small LPs need, then two chunks at a time.
       const int want = !cluster ? kLanczosChunk : k == 0 ? 6 * kLanczosChunk : 2 * kLanczosChunk;
@@ -519,12 +520,25 @@ class engine {
                                            resident_, (const unsigned char*)images_.data()));
         ++launches_;
       } else {
-        for (int i = 0; i < c; ++i) {
+        const int gp = sweep_grid(ATs), gd = sweep_grid(As);
+        for (int i = 0; chained && i < c; ++i) {
+          gk_chain_kernel<0, TX, gk_primal_epi><<<gp, kBlock, 0, s_>>>(
+            ATs, u.data(), gk_primal_epi{v.data()}, partials_.data() + kBlock, i ? gd : 0,
+            partials_.data(), st.data(), betas.data(), k + i);
+          gk_chain_kernel<1, TX, gk_dual_epi><<<gd, kBlock, 0, s_>>>(
+            As, v.data(), gk_dual_epi{u.data()}, partials_.data(), gp, partials_.data() + kBlock,
+            st.data(), alphas.data(), k + i);
+        }
+        if (chained)
+          gk_chain_end_kernel<<<1, kWarp, 0, s_>>>(partials_.data() + kBlock, gd, st.data(),
+                                                   betas.data(), k + c);
+        launches_ += chained;
+        for (int i = 0; !chained && i < c; ++i) {
           gk_sweep_kernel<0, TX, gk_primal_epi><<<sweep_grid(ATs), kBlock, 0, s_>>>(
-            ATs, u.data(), gk_primal_epi{v.data(), st.data()}, partials_.data(), st.data(),
+            ATs, u.data(), gk_primal_epi{v.data()}, partials_.data(), st.data(),
             alphas.data());
           gk_sweep_kernel<1, TX, gk_dual_epi><<<sweep_grid(As), kBlock, 0, s_>>>(
-            As, v.data(), gk_dual_epi{u.data(), st.data()}, partials_.data(), st.data(),
+            As, v.data(), gk_dual_epi{u.data()}, partials_.data(), st.data(),
             betas.data());
         }
         launches_ += 2.0 * c;
@@ -1159,10 +1173,11 @@ class engine {
   }
 
   // ------------------------------------------------------------------ termination
-  // A termination check of an LP whose iterations do not fill the GPU runs on its own stream beside the
-  // plain iterations that follow the step it looks at; beside a large LP's (whose matrices and
-  // vectors fill L2) it slowed both down, so it goes in their stream there.  It reads x_hat, y_hat and the slack, which only the next step that keeps them
-  // overwrites, and that step is not launched before the check's results are in (resolve).
+  // A termination check of an LP whose iterations do not fill the GPU runs on its own stream beside
+  // the plain iterations that follow the step it looks at; beside a larger LP's it slowed both down,
+  // so it goes in their stream there.  It reads x_hat, y_hat and the slack, which only the next step
+  // that keeps them overwrites, and that step is not launched before the check's results are in
+  // (resolve).
   void post_check()
   {
     const int m = in_.m, n = in_.n;

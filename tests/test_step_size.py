@@ -133,3 +133,16 @@ def test_step_size_and_power_iterations_match_the_oracle(lp):
     for sol in (single, batch[1]):
         assert rel(sol.stats["step_size"], want["step_size"]) <= SIGMA_RTOL
         assert sol.stats["power_iterations"] == want["power_iterations"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n", [(5000, 65536), (65537, 30000), (5000, 65537)])
+def test_step_size_where_the_norms_change_place(m, n):
+    """Sweeps of 256 blocks sum the norm in the sweep that follows, sweeps of 257 in their last."""
+    from oracle import oracle as O
+
+    lp = gen.constructed_lp(m, n, 3, seed=n)
+    want = O.solve(lp, tol=1e-12, iteration_limit=0)[0]
+    got = lpm.Solve(datamodel_from_lp(lp), settings(tol=1e-12, iteration_limit=0)).stats
+    assert rel(got["step_size"], want["step_size"]) <= SIGMA_RTOL
+    assert got["power_iterations"] == want["power_iterations"]
