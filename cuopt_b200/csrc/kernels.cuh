@@ -87,10 +87,16 @@ __device__ __forceinline__ double halpern_weight(const pdlp_scalars* st, int it_
 }
 
 // The Halpern step w v + (1 - w) anchor, rounded the same way in every form of the iterations (left
-// to the compiler, which of the two products was fused depended on the kernel).
+// to the compiler, which of the two products was fused depended on the kernel).  The fused step of y
+// takes the other product than the one of x: these are the roundings that the graphs' kernels always
+// had, and a mixed-precision solve of a million rows shows a difference in the last bit.
 __device__ __forceinline__ double halpern_mix(double w, double v, double anchor)
 {
   return fma(w, v, (1.0 - w) * anchor);
+}
+__device__ __forceinline__ double halpern_mix_y(double w, double v, double anchor)
+{
+  return fma(1.0 - w, anchor, w * v);
 }
 
 template <int K>
@@ -659,7 +665,7 @@ __device__ __forceinline__ double dual_row_step(int i, double acc, const P& p, d
   if constexpr (MAJOR) yhat[i] = (TX)ny;
   const double yb = 2.0 * ny - yi;
   if constexpr (HALPERN) {
-    const TX y_next = (TX)halpern_mix(w, yb, (double)p.ya);
+    const TX y_next = (TX)halpern_mix_y(w, yb, (double)p.ya);
     yout[i]         = y_next;
     sink(i, (double)y_next);
   } else {
