@@ -453,9 +453,8 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_range_kerne
 
 // The same sweep with WPB warps per block (the plain sweeps' block shape is autotuned).
 template <typename TM, typename TG, class Epi, int WPB>
-__global__ void __launch_bounds__(WPB * kWarp, kSweepBlocks<TM> * kWarpsPerBlock / WPB) sell_map_wpb_kernel(const dev_sell<TM> A,
-                                                                  const TG* __restrict__ g,
-                                                                  Epi epi, double* partials)
+__global__ void __launch_bounds__(WPB * kWarp, kSweepBlocks<TM> * kWarpsPerBlock / WPB)
+  sell_map_wpb_kernel(const dev_sell<TM> A, const TG* __restrict__ g, Epi epi, double* partials)
 {
   sell_map_block<TM, TG, Epi, false, WPB>(A, g, epi, partials, (int)blockIdx.x);
 }
@@ -1796,10 +1795,9 @@ static __global__ void gk_start_kernel(gk_state* st, const double* sumsq, double
 // A step is two launches; with the sum and its recording as kernels of their own it was six, and
 // on a 12k x 30k LP those four one-block kernels were the larger part of it.
 template <int FIELD, typename TM, class Epi>
-__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) gk_sweep_kernel(const dev_sell<TM> A,
-                                                          const double* __restrict__ g, Epi epi,
-                                                          double* partials, gk_state* st,
-                                                          double* hist)
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>)
+  gk_sweep_kernel(const dev_sell<TM> A, const double* __restrict__ g, Epi epi, double* partials,
+                  gk_state* st, double* hist)
 {
   epi.beta  = st->beta;
   epi.alpha = st->alpha;

@@ -1390,10 +1390,15 @@ class engine {
     const double est_us = 9.0 + 2.0 * (double)L_.nnz / 2.5e5;
     const bool small    = est_us <= 16.0;
     ahead_              = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));
-    // Up to about 3M non-zeros (the matrices of iterations and checks fit in L2 together) the check
-    // runs beside them: 44.5 -> 42.7 ms for 1000 iterations of a 20000 x 60000 LP with skewed rows
-    // (33 us each), no difference at 4M non-zeros, and a loss of 7 % at 16M.
-    cs_check_           = est_us <= 32.0 ? es_ : s_;
+    // While the matrices of the iterations and the values of the check's (FP64, of both layouts) fit
+    // in L2 together, the check runs beside the iterations: 44.5 -> 42.7 ms for 1000 iterations of a
+    // 20000 x 60000 LP with skewed rows (3.1M non-zeros), no difference at 4M non-zeros, and a loss
+    // of 7 % at 16M.
+    int dev = 0, l2 = 0;
+    B200_CUDA_CHECK(cudaGetDevice(&dev));
+    B200_CUDA_CHECK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+    const double bytes = 2.0 * (double)L_.nnz * (sizeof(TX) + sizeof(int) + sizeof(double));
+    cs_check_          = bytes <= (double)l2 ? es_ : s_;
     const auto A = As_view(), AT = ATs_view();
 
     for (;;) {
