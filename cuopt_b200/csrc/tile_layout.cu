@@ -172,6 +172,9 @@ bool build_tile_matrix(const dev_matrix& M, const float* vals, int sms, size_t s
   dbuf<uint64_t> keys(stored), keys_sorted(stored);
   dbuf<float> v(stored), v_sorted(stored);
   const tile_geom g{R, W, panels};
+  // The up to three elements between the long rows and the slices belong to no row: padding too.
+  B200_CUDA_CHECK(cudaMemsetAsync(keys.data(), 0xff, (size_t)stored * sizeof(uint64_t), s));
+  v.zero(s);
   tile_keys_kernel<<<grid_for((int64_t)(M.n_long + M.n_slices) * 32), kT, 0, s>>>(
     M.long_off.data(), M.slice_off.data(), M.n_long, M.n_slices, rows, M.idx.data(),
     M.src.data(), vals, g, keys.data(), v.data());

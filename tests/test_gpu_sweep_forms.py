@@ -98,3 +98,16 @@ def test_wide_rows_follow_the_oracle(m, n, cap):
         assert sol.get_lp_stats()["nb_iterations"] == res["iterations"]
         for got, want in ((sol.get_primal_solution(), x), (sol.get_dual_solution(), y)):
             assert np.max(np.abs(got - want)) <= ITERATE_RTOL * (1 + np.abs(want).max())
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_tiled_copy_with_a_gap_behind_the_long_rows(seed):
+    """Long rows whose elements end off a chunk leave a gap before the slices; the tiled copy takes
+    its elements for padding (tiles are refused or not, the FP32 iterates stay close)."""
+    lp = gen.skewed_lp(300, 2000 + seed, seed=20 + seed, zipf_a=0.7, cap=300)
+    out = []
+    for tiled in (0, 1):
+        s = settings(tol=1e-13, iteration_limit=20, precision=1)
+        s.set_parameter(lpm.CUOPT_PDLP_TILED_SWEEPS, tiled)
+        out.append(lpm.Solve(datamodel_from_lp(lp), s).get_primal_solution())
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-4 * np.linalg.norm(out[0])
