@@ -1231,8 +1231,9 @@ __global__ void __launch_bounds__(kResidentThreads)
 // to be acknowledged: 2 300 (2048 entries, 16 blocks) and 4 300 cycles (5120) of a phase.  So:
 //   * an entry goes, only to the blocks that gather it, with st.async, whose bytes count towards the
 //     receiving block's mbarrier: no barrier at all (1 480 and 2 960 cycles for all entries);
-//   * the first entry of every slice goes to every block of the other sweep.  A warp sends after its
-//     gathers, so a block that has its bytes of one sweep knows that every warp of that sweep is done
+//   * the first entry of every slice goes to every block of the other sweep.  A warp sends after the
+//     gathers of all its lanes (a warp barrier stands between: lanes leave the wait and the gathers one
+//     by one), so a block that has its bytes of one sweep knows that every warp of that sweep is done
 //     reading the vector that the block is about to write next;
 //   * the cluster is the smallest of 4, 8 and 16 blocks whose warps suffice: every further block is
 //     one more store for every entry;
@@ -1447,6 +1448,7 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
         if (threadIdx.x == 0) exchange_expect(bar_y, bytes_y);
       }
       const double acc = P.product(ys);
+      __syncwarp();  // lane 0's entry tells the receivers that all lanes have gathered
       if (P.row >= 0) {
         const auto send = [&](int, double v) {
           exchange_send(base, to_p, xb_0 + (unsigned)P.row * (unsigned)sizeof(TX), 0, (TX)v);
@@ -1471,6 +1473,7 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
       phase_x ^= 1;
       if (threadIdx.x == 0) exchange_expect(bar_x, bytes_x);
       const double acc = Q.product(xbs);
+      __syncwarp();
       if (Q.row >= 0) {
         const auto send = [&](int, double v) {
           exchange_send(base, to_d, kUnitBars + (unsigned)Q.row * (unsigned)sizeof(TX), 8, (TX)v);

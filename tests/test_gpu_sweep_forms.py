@@ -65,6 +65,18 @@ def test_cluster_sizes_at_their_last_slice(m, n, k):
         _same(_solve(lp, GRAPHS, 230, precision), c)
 
 
+@pytest.mark.parametrize("m,n,k", [(65, 161, 30), (33, 161, 14), (320, 1280, 15)])
+def test_cluster_exchange_behind_long_gathers(m, n, k):
+    """A slice's first entry releases the vector that its other lanes have just gathered: slices of
+    many chunks (long gathers between the wait and the sends), last slices of one row (lane 0 sends
+    alone) and of 32, over 590 iterations."""
+    lp = gen.constructed_lp(m, n, k, seed=m + n)
+    for precision in (0, 1):
+        c = _solve(lp, CLUSTER, 590, precision)
+        assert c.stats["plain_iteration_form"] == CLUSTER
+        _same(_solve(lp, GRAPHS, 590, precision), c)
+
+
 @pytest.mark.parametrize("limit", [1200, 1300])
 def test_cluster_form_checks_every_hundred_iterations(limit):
     lp = gen.constructed_lp(150, 333, 5, seed=4)
