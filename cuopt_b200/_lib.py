@@ -142,6 +142,7 @@ SIGNATURES = {
                                               C.POINTER(C.c_double), C.POINTER(cuopt_int_t)]),
     "cuOptProbeClusterBarrier": (cuopt_int_t, [cuopt_int_t, cuopt_int_t, cuopt_int_t, C.c_void_p,
                                                C.POINTER(C.c_double)]),
+    "cuOptProbeExchange": (cuopt_int_t, [cuopt_int_t, cuopt_int_t, C.c_void_p, _P_int, _P_float]),
     "cuOptProbeGridBarrier": (cuopt_int_t, [cuopt_int_t, cuopt_int_t, cuopt_int_t, C.c_double,
                                             C.c_void_p, C.POINTER(cuopt_int_t),
                                             C.POINTER(C.c_double)]),

@@ -4,6 +4,8 @@
 // it in a cooperative launch with no sweep around it, to measure what one barrier costs, and to
 // check that a barrier which cannot complete (a target above the grid's arrivals, which no block
 // will ever provide) ends at its deadline with a status that the host reads, instead of hanging.
+// Beside it: the barrier of the cluster-resident kernels, and the bounded wait (phase_wait) of the
+// kernels whose blocks exchange their vectors by counted bytes.
 #include <cuopt_b200.h>
 
 #include <cstdio>
@@ -111,6 +113,56 @@ extern "C" cuopt_int_t cuOptProbeClusterBarrier(cuopt_int_t blocks, cuopt_int_t 
     *elapsed_ms = (double)he * 1e-6;
   } catch (const std::exception& e) {
     std::fprintf(stderr, "cuOptProbeClusterBarrier: %s\n", e.what());
+    return CUOPT_RUNTIME_ERROR;
+  }
+  return CUOPT_SUCCESS;
+}
+
+namespace cuopt_b200 {
+namespace {
+// One phase, armed with no bytes to come, or with `unreachable` with 8 that nobody sends.
+__global__ void exchange_probe_kernel(int unreachable, int polls, int* status,
+                                      unsigned long long* elapsed)
+{
+  __shared__ __align__(8) unsigned long long bar;
+  const unsigned long long t0 = global_ns();
+  const unsigned at           = (unsigned)__cvta_generic_to_shared(&bar);
+  if (threadIdx.x == 0) {
+    phase_init(at);
+    phase_expect(at, unreachable ? 8 : 0);
+  }
+  __syncthreads();
+  if (!phase_wait(at, 0, polls)) atomicCAS(status, 0, kBarrierPollLimit);
+  __syncthreads();
+  if (threadIdx.x == 0) *elapsed = global_ns() - t0;
+}
+}  // namespace
+}  // namespace cuopt_b200
+
+extern "C" cuopt_int_t cuOptProbeExchange(cuopt_int_t unreachable, cuopt_int_t polls, void* stream,
+                                          cuopt_int_t* status, cuopt_float_t* elapsed_ms)
+{
+  using namespace cuopt_b200;
+  if (polls < 0 || polls > kPhasePolls || !status || !elapsed_ms) return CUOPT_INVALID_ARGUMENT;
+  try {
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    alloc_scope scope(s);
+    dbuf<int> st(1);
+    dbuf<unsigned long long> el(1);
+    st.zero(s);
+    el.zero(s);
+    exchange_probe_kernel<<<1, 2 * kWarp, 0, s>>>((int)unreachable, polls ? (int)polls : kPhasePolls,
+                                                  st.data(), el.data());
+    B200_LAUNCH_CHECK();
+    int hs                = 0;
+    unsigned long long he = 0;
+    B200_CUDA_CHECK(cudaMemcpyAsync(&hs, st.data(), sizeof(hs), cudaMemcpyDeviceToHost, s));
+    B200_CUDA_CHECK(cudaMemcpyAsync(&he, el.data(), sizeof(he), cudaMemcpyDeviceToHost, s));
+    B200_CUDA_CHECK(cudaStreamSynchronize(s));
+    *status     = hs;
+    *elapsed_ms = (double)he * 1e-6;
+  } catch (const std::exception& e) {
+    std::fprintf(stderr, "cuOptProbeExchange: %s\n", e.what());
     return CUOPT_RUNTIME_ERROR;
   }
   return CUOPT_SUCCESS;

@@ -237,6 +237,36 @@ struct ksum {
   __device__ __forceinline__ double value() const { return s + c; }
 };
 
+// Byte-counted exchanges between the blocks of a cluster: a phase of the receiver's mbarrier (count 1)
+// ends once one thread has armed it with the bytes to come (phase_expect, once a phase) and they have
+// arrived (st.async of the senders).  Waits are bounded: a poll of an unfinished phase suspends the warp
+// for some 4 us (B200), so kPhasePolls of them give up after about a second; phase_wait is then false.
+constexpr int kPhasePolls = 1 << 18;
+__device__ __forceinline__ void phase_init(unsigned bar)
+{
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void phase_expect(unsigned bar, unsigned bytes)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool phase_wait(unsigned bar, unsigned parity, int polls = kPhasePolls)
+{
+  for (int i = 0; i < polls; ++i) {
+    unsigned ok;
+    asm volatile(
+      "{\n .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
 // Streaming (evict-first) loads for matrix data that is read once per sweep, so the L2 keeps the
 // iterate vectors that the gathers reuse.
 __device__ __forceinline__ double ld_stream(const double* p) { return __ldcs(p); }

@@ -1244,33 +1244,7 @@ __global__ void __launch_bounds__(kResidentThreads)
 // closing cluster barrier.
 constexpr int kClusterBlocks = 16;
 constexpr int kUnitWarps     = 10;
-constexpr int kExchangePolls = 1 << 22;
 
-__device__ __forceinline__ void exchange_init(unsigned bar)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-}
-// The phase that ends once `bytes` more have arrived (one call a phase, by one thread).
-__device__ __forceinline__ void exchange_expect(unsigned bar, unsigned bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool exchange_wait(unsigned bar, unsigned parity)
-{
-  for (int i = 0; i < kExchangePolls; ++i) {
-    unsigned ok;
-    asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
 // Stores v at offset `off` from the mapped base addresses in the blocks of `mask`, counted by the
 // barrier at offset `bar` there.  Predicated, not branched over: with sixteen branches a warp's step
 // and sends took 1 200 to 2 300 cycles.
@@ -1384,8 +1358,8 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned bar_x = (unsigned)__cvta_generic_to_shared(cl_smem), bar_y = bar_x + 8;
   if (threadIdx.x == 0) {
-    exchange_init(bar_x);
-    exchange_init(bar_y);
+    phase_init(bar_x);
+    phase_init(bar_y);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   {
@@ -1430,8 +1404,8 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
   const int2 need = *reinterpret_cast<const int2*>(img + D.image_at<TX>(10));
   const unsigned bytes_x = need.x * (unsigned)sizeof(TX), bytes_y = need.y * (unsigned)sizeof(TX);
   if (threadIdx.x == 0) {
-    exchange_expect(bar_x, bytes_x);
-    exchange_expect(bar_y, bytes_y);
+    phase_expect(bar_x, bytes_x);
+    phase_expect(bar_y, bytes_y);
   }
   double w = halpern_weight(&sc, 0), ratio = (double)dy.y / sc.sigma;
   // Every block of the cluster is running, with its copy of y and its barriers, before any block
@@ -1443,9 +1417,9 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
     const bool last = it == L - 1;
     if (P.chunks >= 0) {
       if (it > 0) {
-        if (!(ok = exchange_wait(bar_y, phase_y))) break;
+        if (!(ok = phase_wait(bar_y, phase_y))) break;
         phase_y ^= 1;
-        if (threadIdx.x == 0) exchange_expect(bar_y, bytes_y);
+        if (threadIdx.x == 0) phase_expect(bar_y, bytes_y);
       }
       const double acc = P.product(ys);
       __syncwarp();  // lane 0's entry tells the receivers that all lanes have gathered
@@ -1469,9 +1443,9 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
       }
     }
     if (Q.chunks >= 0) {
-      if (!(ok = exchange_wait(bar_x, phase_x))) break;
+      if (!(ok = phase_wait(bar_x, phase_x))) break;
       phase_x ^= 1;
-      if (threadIdx.x == 0) exchange_expect(bar_x, bytes_x);
+      if (threadIdx.x == 0) phase_expect(bar_x, bytes_x);
       const double acc = Q.product(xbs);
       __syncwarp();
       if (Q.row >= 0) {
@@ -1493,7 +1467,7 @@ __global__ void __launch_bounds__(kUnitWarps * kWarp, 1)
     ratio = (double)dy.y / sc.sigma;
   }
   // No block leaves while entries of the last sweep are on their way to it.
-  if (ok && P.chunks >= 0) ok = exchange_wait(bar_y, phase_y);
+  if (ok && P.chunks >= 0) ok = phase_wait(bar_y, phase_y);
   if (!ok) atomicCAS(status, 0, kBarrierPollLimit);
   __syncthreads();
   cluster_barrier();

@@ -46,7 +46,6 @@ constexpr int kLsqrWarps   = kLsqrThreads / kWarp;
 constexpr int kClThreads = 256;
 constexpr int kClWarps   = kClThreads / kWarp;
 constexpr int kEquilibrationPasses = 10;
-constexpr int kLsqrPolls = 1 << 22;   // polls of one exchange
 constexpr int kLsqrFailed = -1;       // flag of a system whose exchange did not complete
 
 struct lsqr_desc {
@@ -273,27 +272,6 @@ __device__ __forceinline__ void lsqr_barrier()
     "barrier.cluster.wait.acquire.aligned;\n" ::
       : "memory");
 }
-// The phase of `bar` that ends once `bytes` more have arrived (one call a phase, by one thread).
-__device__ __forceinline__ void expect_bytes(unsigned bar, unsigned bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool wait_bytes(unsigned bar, unsigned parity)
-{
-  for (int i = 0; i < kLsqrPolls; ++i) {
-    unsigned ok;
-    asm volatile(
-      "{\n .reg .pred p;\n"
-      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
 __device__ __forceinline__ void send_bytes(unsigned to, unsigned bar, double v)
 {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(
@@ -452,18 +430,18 @@ __global__ void __launch_bounds__(kClThreads, 1)
   }
   const unsigned bytes_u = 8u * (d.rows + C * kClWarps), bytes_v = 8u * (d.cols + 2 * C * kClWarps);
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_u) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_v) : "memory");
+    phase_init(bar_u);
+    phase_init(bar_v);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    expect_bytes(bar_u, bytes_u);
-    expect_bytes(bar_v, bytes_v - 8u * C * kClWarps);  // the first one has a single sum
+    phase_expect(bar_u, bytes_u);
+    phase_expect(bar_v, bytes_v - 8u * C * kClWarps);  // the first one has a single sum
   }
   unsigned phase_u = 0, phase_v = 0;
   bool ok          = true;
   auto wait_v = [&]() {
-    if (!(ok = wait_bytes(bar_v, phase_v))) return false;
+    if (!(ok = phase_wait(bar_v, phase_v))) return false;
     phase_v ^= 1;
-    if (threadIdx.x == 0) expect_bytes(bar_v, bytes_v);
+    if (threadIdx.x == 0) phase_expect(bar_v, bytes_v);
     return true;
   };
   // Every block of the cluster is running, with its barriers, before any stores into another's
@@ -502,9 +480,9 @@ __global__ void __launch_bounds__(kClThreads, 1)
         t1[0] += un * un;
       });
       send_sums<1, C>(t1, mine, (unsigned)S.part_a, 0, rank);
-      if (!(ok = wait_bytes(bar_u, phase_u))) break;
+      if (!(ok = phase_wait(bar_u, phase_u))) break;
       phase_u ^= 1;
-      if (threadIdx.x == 0) expect_bytes(bar_u, bytes_u);
+      if (threadIdx.x == 0) phase_expect(bar_u, bytes_u);
       cluster_totals<1>(part_a, C, r1);
       beta = sqrt(r1[0]);
       us   = beta > 0.0 ? 1.0 / beta : 0.0;
@@ -729,6 +707,7 @@ struct cluster_plan {
     cfg.blockDim             = dim3(kClThreads);
     cfg.dynamicSmemBytes     = smem;
     cfg.stream               = s;
+    // Also for one block: st.async is an illegal instruction in a launch without a cluster size.
     attr[0].id               = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = blocks;
     attr[0].val.clusterDim.y = 1;

@@ -21,10 +21,6 @@ inline tile_view view_of(const tile_matrix& t)
                    t.panels, t.groups, t.tile_off.data(), t.key.data(), t.val.data()};
 }
 
-// Bounded number of mbarrier polls before a wait gives up (each poll may suspend the thread for a
-// short hardware-defined time); a copy of one panel completes within microseconds.
-constexpr long long kTileWaitPolls = 1ll << 22;
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p)
 {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -60,10 +56,11 @@ __device__ __forceinline__ bool tile_mbar_try_wait(uint64_t* bar, uint32_t parit
     : "memory");
   return ok != 0;
 }
-// Waits for phase `parity` of `bar`; false (and *err = 1) when the poll limit runs out.
+// Waits for phase `parity` of `bar`; false (and *err = 1) when kPhasePolls polls run out (a copy of
+// one panel completes within microseconds).
 __device__ __forceinline__ bool tile_mbar_wait(uint64_t* bar, uint32_t parity, int* err)
 {
-  for (long long i = 0; i < kTileWaitPolls; ++i)
+  for (int i = 0; i < kPhasePolls; ++i)
     if (tile_mbar_try_wait(bar, parity)) return true;
   atomicExch(err, 1);
   return false;

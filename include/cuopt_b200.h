@@ -128,6 +128,17 @@ cuopt_int_t cuOptProbeClusterBarrier(cuopt_int_t blocks,
                                      void* stream,
                                      cuopt_float_t* elapsed_ms);
 
+/* Test hook (no counterpart in the reference): the bounded wait of the kernels whose blocks exchange
+ * their vectors by counted bytes (cluster-resident iterations, LSQR), run alone by one block.  With
+ * `unreachable` != 0 it waits for bytes that nobody sends: the wait ends after `polls` polls (0: the limit that
+ * the kernels use, about a second) and records status 2 instead of hanging.  Returns the recorded
+ * status (0: the exchange completed) and the device time in milliseconds. */
+cuopt_int_t cuOptProbeExchange(cuopt_int_t unreachable,
+                               cuopt_int_t polls,
+                               void* stream,
+                               cuopt_int_t* status,
+                               cuopt_float_t* elapsed_ms);
+
 /* Measurement hook (no counterpart in the reference): the random-gather ceiling of the device.
  * Streams `gathers` random int32 indices into a vector of `vector_length` elements of
  * `element_bytes` (4 or 8) bytes, in the sliced-ELL sweeps' chunk shape (a warp reads 32 lanes x 4

@@ -224,6 +224,24 @@ def test_grid_barrier_deadline_ends_the_wait():
     assert sol.get_termination_status() == lpm.LPTerminationStatus.Optimal
 
 
+def _exchange(unreachable, polls=0):
+    st, ms = _lib.cuopt_int_t(), C.c_double()
+    rc = _lib.lib().cuOptProbeExchange(unreachable, polls, None, C.byref(st), C.byref(ms))
+    return rc, st.value, ms.value
+
+
+def test_exchange_wait_runs_out():
+    """An exchange between blocks whose bytes never come ends with status 2, within seconds at the
+    kernels' own limit; one that is complete has status 0, and the context stays usable."""
+    assert _exchange(0)[:2] == (0, 0)
+    rc, st, ms = _exchange(1, 16)
+    assert (rc, st) == (0, 2) and ms < 10.0
+    rc, st, ms = _exchange(1)
+    assert (rc, st) == (0, 2) and 100.0 <= ms < 5000.0
+    assert _exchange(0)[:2] == (0, 0)
+    assert _exchange(0, -1)[0] == 1  # CUOPT_INVALID_ARGUMENT
+
+
 def test_grid_barrier_rejects_oversized_grids():
     rc, _, _ = _probe(1_000_000, 1, 0, 10.0)
     assert rc == 1  # CUOPT_INVALID_ARGUMENT: more blocks than can be co-resident, nothing launched
