@@ -430,9 +430,11 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
 }
 
 // Resident blocks of 256 threads the sweeps are compiled for: 5 an SM with FP32 matrices (48
-// registers), 4 with FP64 (64; at 48 some spill, and left alone they take up to 78).
+// registers), 3 with FP64 (80).  FP64, 1M x 2M LP with 16M non-zeros, primal + dual sweep: 86.4 + 81.1
+// us at 4 blocks (64 registers), 86.5 + 78.9 at 3, 95.2 + 86.9 left alone; 400k x 1M: 45.1 + 45.8, 45.0
+// + 43.2, 48.3 + 47.0.  FP32, 1M x 2M: 71.8 + 73.3 at 5, 74.4 + 73.1 at 4.
 template <typename TM>
-constexpr int kSweepBlocks = sizeof(TM) == 4 ? 5 : 4;
+constexpr int kSweepBlocks = sizeof(TM) == 4 ? 5 : 3;
 template <typename TM, typename TG, class Epi>
 __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_kernel(const dev_sell<TM> A,
                                                           const TG* __restrict__ g, Epi epi,
