@@ -105,18 +105,19 @@ __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwar
   const int lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
   for (int i0 = warp0 * kRows; i0 < p.m; i0 += nwarps * kRows) {
     const int i = i0 + grp;
+    bool live   = i < p.m;
     int b = 0, e = 0;
     double yi = 0.0, l = 0.0, u = 0.0;
-    if (i < p.m) {
+    if (live) {
       b  = p.off[i];
       e  = p.off[i + 1];
       yi = p.y[i];
       l  = p.lo[i];
       u  = p.up[i];
-      if (b < 0 || e < b) {  // malformed offsets: counted, the row's entries are skipped
+      if (b < 0 || e < b) {  // malformed offsets: counted, the row is skipped
         if (sub == 0) atomicAdd(&g_na.bad, 1u);
+        live = false;
         b = e = 0;
-        l = u = CUDART_NAN;  // and it contributes nothing (below)
       }
     }
     // Four elements a lane at a time, so that their loads, then their gathers, are in flight together.
@@ -142,7 +143,7 @@ __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwar
     }
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
-    if (sub == 0 && i < p.m && !(isnan(l) && isnan(u))) {
+    if (sub == 0 && live) {
       const double rp   = ax - fmax(l, fmin(ax, u));
       const double yint = p.sgn * yi;  // the dual in minimisation form
       r[0] += rp * rp;

@@ -240,3 +240,33 @@ def test_no_alloc_sizes_against_numpy(m, n, length):
     other = {**d, "off": t([0] * (m + 1), torch.int32)}
     code, got = _no_alloc(L, torch, other, lp, 1, 0.0)  # no entries: A x = 0, A^T y = 0
     assert code == 0 and abs(got[1] - np.linalg.norm(c - rc)) <= 1e-12 * (1 + got[1])
+
+
+@pytest.mark.parametrize("n", [700, 5003])  # one cluster, two kernels
+def test_no_alloc_row_without_bounds_is_not_skipped(n):
+    """A row whose bounds are both NaN restricts nothing (residual 0 for a finite product), but one
+    whose product is not finite shows in the primal residual, and an infinite dual in the objective."""
+    torch = pytest.importorskip("torch")
+    L = lib()
+    m = 300
+    rng = np.random.default_rng(n)
+    t = lambda a, dt=torch.float64: torch.as_tensor(a, device="cuda", dtype=dt)
+    off, idx = np.arange(0, 2 * m + 1, 2), np.arange(2 * m) % n
+    lo = np.zeros(m)
+    up = np.full(m, 1.0)
+    lo[7] = up[7] = np.nan
+    x = np.zeros(n)
+    x[idx[14]] = 1.0
+    d = {"c": t(np.zeros(n)), "off": t(off, torch.int32), "idx": t(idx, torch.int32),
+         "val": t(rng.uniform(1.0, 2.0, 2 * m)), "lo": t(lo), "up": t(up), "x": t(x),
+         "y": t(np.zeros(m)), "rc": t(np.zeros(n))}
+    lp = type("Sizes", (), {"m": m, "n": n})
+    code, got = _no_alloc(L, torch, d, lp, 1, 0.0)
+    assert code == 0 and got[0] == 0.0 and got[8] == 0.0
+    x[idx[14]] = np.inf
+    code, got = _no_alloc(L, torch, {**d, "x": t(x)}, lp, 1, 0.0)
+    assert code == 0 and np.isnan(got[0]) and got[8] == 0.0
+    y = np.zeros(m)
+    y[7] = np.inf
+    code, got = _no_alloc(L, torch, {**d, "y": t(y)}, lp, 1, 0.0)
+    assert code == 0 and np.isnan(got[3]) and got[8] == 0.0
