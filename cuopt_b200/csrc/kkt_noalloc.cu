@@ -93,10 +93,44 @@ __device__ __forceinline__ void block_sum_store(const double (&v)[K], double* pa
   }
 }
 
+// Entries b + first, b + first + STRIDE, ... of one row: this lane's part of A x, and the scatter of
+// yi A[i, :] into the A^T y accumulator.  Four at a time, so that their loads, then their gathers, are
+// in flight together.  The count left is signed, the position is not: neither wraps near 2^31 entries.
+template <int STRIDE>
+__device__ __forceinline__ double na_row_part(const na_problem& p, int b, int e, int first, double yi)
+{
+  double ax = 0.0;
+  unsigned k = (unsigned)b + first;
+  for (int left = e - b - first; left > 0; left -= 4 * STRIDE, k += 4 * STRIDE) {
+    int j[4];
+    double a[4], xj[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) j[q] = q * STRIDE < left ? p.idx[k + q * STRIDE] : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) a[q] = q * STRIDE < left ? p.val[k + q * STRIDE] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) xj[q] = (unsigned)j[q] < (unsigned)p.n ? p.x[j[q]] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if ((unsigned)j[q] < (unsigned)p.n) {
+        ax += a[q] * xj[q];
+        atomicAdd(g_na.aty + j[q], a[q] * yi);
+      } else if (q * STRIDE < left) {
+        atomicAdd(&g_na.bad, 1u);
+      }
+    }
+  }
+  return ax;
+}
+
 // G lanes per constraint row: A x and the row's residual / dual-objective / |b| terms, and the
 // scatter of y_i A[i, :] into the A^T y accumulator.  Bound by the L1 request rate (one gather and
 // one reduction per non-zero), so rows shorter than a warp share one: with a whole warp per row of
-// 20 non-zeros 12 of 32 lanes issued nothing.
+// 20 non-zeros 12 of 32 lanes issued nothing.  A row of more than kNaLongRounds rounds of its G lanes
+// is left to the whole warp, which takes such rows of its groups one after another: the longest row
+// sets the time of the pass (one of 50 000 entries among 20 000 rows of 8: 1 730 us on 4 lanes, 227 us
+// on the warp).
+constexpr int kNaLongRounds = 8;
 template <int G>
 __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwarps,
                                         double (&r)[kNaRowRed])
@@ -120,29 +154,19 @@ __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwar
         b = e = 0;
       }
     }
-    // Four elements a lane at a time, so that their loads, then their gathers, are in flight together.
-    double ax = 0.0;
-    for (int k = b + sub; k < e; k += 4 * G) {
-      int j[4];
-      double a[4], xj[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) j[q] = k + q * G < e ? p.idx[k + q * G] : -1;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) a[q] = k + q * G < e ? p.val[k + q * G] : 0.0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) xj[q] = (unsigned)j[q] < (unsigned)p.n ? p.x[j[q]] : 0.0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if ((unsigned)j[q] < (unsigned)p.n) {
-          ax += a[q] * xj[q];
-          atomicAdd(g_na.aty + j[q], a[q] * yi);
-        } else if (k + q * G < e) {
-          atomicAdd(&g_na.bad, 1u);
-        }
-      }
-    }
+    const bool longer = G < kWarp && e - b > kNaLongRounds * 4 * G;
+    double ax         = longer ? 0.0 : na_row_part<G>(p, b, e, sub, yi);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) ax += __shfl_xor_sync(0xffffffffu, ax, o);
+    if constexpr (G < kWarp) {
+      for (unsigned left = __ballot_sync(0xffffffffu, longer && sub == 0); left; left &= left - 1) {
+        const int from  = __ffs(left) - 1;
+        const int lb    = __shfl_sync(0xffffffffu, b, from), le = __shfl_sync(0xffffffffu, e, from);
+        const double ly = __shfl_sync(0xffffffffu, yi, from);
+        const double t  = warp_sum(na_row_part<kWarp>(p, lb, le, lane, ly));
+        if (lane == from) ax = t;
+      }
+    }
     if (sub == 0 && live) {
       const double rp   = ax - fmax(l, fmin(ax, u));
       const double yint = p.sgn * yi;  // the dual in minimisation form

@@ -242,6 +242,77 @@ def test_no_alloc_sizes_against_numpy(m, n, length):
     assert code == 0 and abs(got[1] - np.linalg.norm(c - rc)) <= 1e-12 * (1 + got[1])
 
 
+def _kkt_us(L, torch, m, n, lens):
+    """Microseconds of one evaluation (best of seven times twenty)."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    off = np.concatenate([[0], np.cumsum(lens)])
+    f = lambda k: torch.randn(k, device="cuda", dtype=torch.float64, generator=g)
+    d = {"c": f(n), "x": f(n), "rc": f(n), "y": f(m), "lo": f(m), "val": f(int(off[-1])),
+         "off": torch.as_tensor(off, device="cuda", dtype=torch.int32),
+         "idx": torch.arange(int(off[-1]), device="cuda", dtype=torch.int32) % n}
+    d["up"] = d["lo"] + 1.0
+    lp = type("Sizes", (), {"m": m, "n": n})
+    out = torch.zeros(9, device="cuda", dtype=torch.float64)
+    best = np.inf
+    for _ in range(7):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        e0.record()
+        for _ in range(20):
+            assert L.cuOptComputeKKTErrorsNoAlloc(
+                m, n, 1, 0.0, _p(d["c"]), _p(d["off"]), _p(d["idx"]), _p(d["val"]), _p(d["lo"]),
+                _p(d["up"]), _p(d["x"]), _p(d["y"]), _p(d["rc"]),
+                C.c_void_p(torch.cuda.current_stream().cuda_stream), _p(out)) == 0
+        e1.record()
+        e1.synchronize()
+        best = min(best, e0.elapsed_time(e1) * 50.0)
+    assert out[8].item() == 0.0
+    return best
+
+
+@pytest.mark.parametrize("rest", [8, 20])  # 4 and 8 lanes for the other rows
+def test_no_alloc_long_row_among_short_ones_takes_a_warp(rest):
+    """One row over all variables among short ones costs what it costs alone, on a whole warp, and
+    not what the few lanes of its neighbours take for it."""
+    torch = pytest.importorskip("torch")
+    L = lib()
+    m, n = 20000, 50000
+    lens = np.full(m, rest)
+    short = _kkt_us(L, torch, m, n, lens)
+    lens[777] = n
+    assert _kkt_us(L, torch, m, n, lens) <= 1.25 * _kkt_us(L, torch, 1, n, [n]) + short
+
+
+@pytest.mark.parametrize("m,n,rest,longs", [
+    (300, 9000, 5, {0: 129, 1: 128, 2: 9000, 3: 257, 299: 130}),      # 4 lanes: from 129 on
+    (333, 9000, 20, {0: 257, 7: 256, 8: 9000, 15: 300, 332: 9000})])  # 8 lanes: from 257 on
+def test_no_alloc_long_rows_against_numpy(m, n, rest, longs):
+    torch = pytest.importorskip("torch")
+    L = lib()
+    rng = np.random.default_rng(m)
+    lens = np.full(m, rest)
+    for i, l in longs.items():
+        lens[i] = l
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    idx = rng.integers(0, n, off[-1]).astype(np.int32)
+    val = rng.standard_normal(off[-1])
+    c, x, rc = (rng.standard_normal(n) for _ in range(3))
+    y = rng.standard_normal(m)
+    rows = np.repeat(np.arange(m), lens)
+    ax = np.bincount(rows, weights=val * x[idx], minlength=m)
+    aty = np.bincount(idx, weights=val * y[rows], minlength=n)
+    t = lambda a, dt=torch.float64: torch.as_tensor(a, device="cuda", dtype=dt)
+    d = {"c": t(c), "off": t(off, torch.int32), "idx": t(idx, torch.int32), "val": t(val),
+         "lo": t(np.zeros(m)), "up": t(np.full(m, 0.5)), "x": t(x), "y": t(y), "rc": t(rc)}
+    code, got = _no_alloc(L, torch, d, type("Sizes", (), {"m": m, "n": n}), 1, 0.0)
+    assert code == 0 and got[8] == 0
+    # Sums of at most 9000 terms of order 1 in FP64, as in test_no_alloc_sizes_against_numpy.
+    for q, want in ((0, np.linalg.norm(ax - np.clip(ax, 0.0, 0.5))),
+                    (1, np.linalg.norm(c - aty - rc))):
+        assert abs(got[q] - want) <= 1e-12 * (1 + want)
+
+
 @pytest.mark.parametrize("n", [700, 5003])  # one cluster, two kernels
 def test_no_alloc_row_without_bounds_is_not_skipped(n):
     """A row whose bounds are both NaN restricts nothing (residual 0 for a finite product), but one
