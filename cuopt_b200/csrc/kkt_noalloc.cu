@@ -47,11 +47,15 @@ constexpr int kNaBlocks  = 1184;     // 148 SMs x 8 resident blocks of 256 threa
 constexpr int kNaRowRed  = 3;        // row pass: |r_p|^2, dual row term, |b|^2
 constexpr int kNaColRed  = 4;        // column pass: |r_d|^2, c.x, rc.x, |c|^2
 // Small LPs run in one cluster of kNaClusterBlocks blocks: one launch in place of a memset and two
-// kernels (300 x 700: see na_small_kernel).  The line is drawn on m n, which bounds the non-zeros
-// (the host does not know them), so that a dense LP does not end up on 8 SMs with more than 2^20.
-constexpr int kNaClusterBlocks  = 8;
-constexpr int kNaClusterThreads = 1024;
-constexpr int64_t kNaClusterArea = 1 << 20;
+// kernels.  The line is drawn on m n, which bounds the non-zeros (the host does not know them), and on
+// n / m, because few long rows leave most of the eight SMs idle.  One cluster / kernels / the memset
+// and three kernels of one warp per row that these replaced, us: 300 x 873 with 2 400 entries 10.5 /
+// 12.7 / 21.9, dense 29 / 23 / 36; 4096 x 64 with 32 768 17.7 / 20.8 / 28.8; dense 512 x 512 28 / 25 /
+// 36; beyond the line 64 x 4096 with 65 536 37 / 19 / 34, dense 1000 x 1000 68 / 44 / 57.
+constexpr int kNaClusterBlocks   = 8;
+constexpr int kNaClusterThreads  = 1024;
+constexpr int64_t kNaClusterArea = 1 << 18;
+constexpr int kNaClusterAspect   = 32;
 
 struct na_globals {
   unsigned bad, arrived;  // the clear of a call covers these and the first n entries of aty
@@ -177,20 +181,24 @@ __device__ __forceinline__ void na_rows(const na_problem& p, int warp0, int nwar
   }
 }
 
-// The row pass of block `block` of `nblocks`; the lanes per row follow the mean row length.
+// The row pass of block `block` of `nblocks`; the lanes per row follow the mean row length.  A block
+// takes neighbouring rows; in the one cluster, short rows are dealt to the blocks (300 x 873 with 2 400
+// entries: 12.6 -> 10.5 us), but long ones then meet in their atomics (dense: 29 -> 41 us).
 template <int THREADS>
 __device__ __forceinline__ void na_row_pass(const na_problem& p, int block, int nblocks)
 {
-  double r[kNaRowRed] = {};
-  const int warp0 = block * (THREADS / kWarp) + (threadIdx.x >> 5);
-  const int nw    = nblocks * (THREADS / kWarp);
-  const int mean  = p.off[p.m] / p.m;
+  constexpr int W      = THREADS / kWarp;
+  double r[kNaRowRed]  = {};
+  const int warp       = threadIdx.x >> 5;
+  const int mean       = p.off[p.m] / p.m;
+  const int neighbours = block * W + warp;
+  const int dealt      = THREADS == kNaClusterThreads ? warp * nblocks + block : neighbours;
   if (mean <= 12)
-    na_rows<4>(p, warp0, nw, r);
+    na_rows<4>(p, dealt, nblocks * W, r);
   else if (mean <= 48)
-    na_rows<8>(p, warp0, nw, r);
+    na_rows<8>(p, dealt, nblocks * W, r);
   else
-    na_rows<32>(p, warp0, nw, r);
+    na_rows<32>(p, neighbours, nblocks * W, r);
   block_sum_store<kNaRowRed, THREADS>(r, g_na.partials, block);
 }
 
@@ -314,7 +322,7 @@ extern "C" cuopt_int_t cuOptComputeKKTErrorsNoAlloc(
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   const double sgn      = sense == CUOPT_MAXIMIZE ? -1.0 : 1.0;
   const na_problem p{m, n, d_off, d_idx, d_val, d_c, d_lo, d_up, d_x, d_y, d_rc, sgn, offset, d_out};
-  if ((int64_t)m * n <= kNaClusterArea) {
+  if ((int64_t)m * n <= kNaClusterArea && n <= (int64_t)kNaClusterAspect * m) {
     na_small_kernel<<<kNaClusterBlocks, kNaClusterThreads, 0, st>>>(p);
   } else {
     // The scratch's address is looked up on every call (a host query that allocates nothing), so

@@ -190,7 +190,8 @@ def test_no_alloc_leaves_free_memory_unchanged():
 
 
 @pytest.mark.parametrize("m,n,length", [
-    (1, 1, 1), (1, 700, 700), (700, 1, 1), (1024, 1024, 5), (1024, 1025, 5),  # around m n = 2^20
+    (1, 1, 1), (1, 700, 700), (700, 1, 1), (1024, 1024, 5), (1024, 1025, 5),
+    (512, 512, 5), (512, 513, 5), (40, 1280, 9), (40, 1281, 9),                # m n = 2^18, n = 32 m
     (3001, 5003, 12), (3001, 5003, 13), (1200, 5003, 48), (1200, 5003, 49),   # lanes per row
     (37, 900, 900), (9001, 400, 33)])
 def test_no_alloc_sizes_against_numpy(m, n, length):
@@ -282,6 +283,16 @@ def test_no_alloc_long_row_among_short_ones_takes_a_warp(rest):
     short = _kkt_us(L, torch, m, n, lens)
     lens[777] = n
     assert _kkt_us(L, torch, m, n, lens) <= 1.25 * _kkt_us(L, torch, 1, n, [n]) + short
+
+
+@pytest.mark.parametrize("m,n,length", [(1000, 1000, 1000), (500, 520, 520), (64, 4096, 1024)])
+def test_no_alloc_small_dense_rows_use_the_chip(m, n, length):
+    """Entries of few rows and columns are spread over the SMs: about the time of as many in an LP of
+    more columns (1000 x 1000 on eight SMs took 68 us and not 44)."""
+    torch = pytest.importorskip("torch")
+    L = lib()
+    wide = _kkt_us(L, torch, m, (1 << 20) // m + n, np.full(m, length))
+    assert _kkt_us(L, torch, m, n, np.full(m, length)) <= 2.0 * wide
 
 
 @pytest.mark.parametrize("m,n,rest,longs", [
