@@ -14,11 +14,14 @@
 //     of a slice and reads element k at base + 32 k + t), rows sorted by length; slice s belongs to
 //     block s % C, whose share is copied into its shared memory (16-bit indices) where it fits, so
 //     that an iteration reads no global memory;
-//   * the two norms of an iteration are sums of per-warp sums, sent to every block with the vector
-//     entries and added in a fixed order by every warp, so the scalar recurrence and the stopping
-//     decision are uniform, the result is deterministic, and an iteration costs two products and
-//     two exchanges.  Every warp sends its sums after its gathers, so a block that has all of one
-//     exchange knows that every warp is done reading the vector written next;
+//   * the two norms of an iteration are sums of per-slice sums, sent to every block with the vector
+//     entries and added in the slices' order by every warp, so the scalar recurrence and the stopping
+//     decision are uniform, and an iteration costs two products and two exchanges.  A warp sends the
+//     sums of a slice after its gathers (a warp without slices sends zeros that nobody adds), so a
+//     block that has all of one exchange knows that every warp is done reading the vector written
+//     next, and has read the sums of the exchange before.  No sum depends on the number of blocks, and
+//     every product that the compiler could fuse or not is written out: a system's result is the
+//     same bits whatever cluster it runs in, that is, whatever else is in its batch;
 //   * the x / w update of an iteration is applied in the next transpose product by the thread that
 //     owns the row.
 // One block per system, reading the operator from L2, took 33 us an iteration on the 5000 x 5000
@@ -227,9 +230,15 @@ __global__ void __launch_bounds__(kLsqrThreads, 1) lsqr_kernel(const lsqr_desc* 
   if (threadIdx.x == 0) outs[blockIdx.x] = lsqr_out{it, flag, rnorm, arnorm};
 }
 
+// Entries of the sums of one exchange: one per slice, and one for every warp of the cluster that has
+// none (slice s is the first of warp s / C of block s % C).
+B200_HD inline size_t sum_slots(int slices, int C)
+{
+  return slices > C * kClWarps ? slices : C * kClWarps;
+}
 // Shared memory of one block of a cluster of C for a system: u, v, the x and w of the block's
-// columns, the per-warp sums of the two norms from every block, and with `cached` the block's
-// shares of P and Q: {start, length} per slice, values, 16-bit indices.
+// columns, the per-slice sums of the two norms, and with `cached` the block's shares of P and Q:
+// {start, length} per slice, values, 16-bit indices.
 struct lsqr_smem {
   size_t v, x, w, part_a, part_b, tab[2], val[2], idx[2], bytes;
   static B200_HD size_t pad(size_t b) { return (b + 15) & ~(size_t)15; }
@@ -246,8 +255,8 @@ struct lsqr_smem {
     v      = take((size_t)cols * 8);
     x      = take(nq * kWarp * 8);
     w      = take(nq * kWarp * 8);
-    part_a = take((size_t)C * kClWarps * 8);
-    part_b = take((size_t)C * kClWarps * 16);
+    part_a = take(sum_slots(slices_p, C) * 8);
+    part_b = take(sum_slots(slices_q, C) * 16);
     tab[0] = take(cached ? np * 8 : 0);
     tab[1] = take(cached ? nq * 8 : 0);
     val[0] = take(cached ? (size_t)elems_p * 8 : 0);
@@ -287,28 +296,29 @@ __device__ __forceinline__ void send_all(const unsigned (&base)[C], unsigned off
   for (int c = 0; c < C; ++c) send_bytes(base[c] + off, base[c] + bar, v);
 }
 
-// Sends this warp's sums of K per-thread values to every block (lane c to block c; `mine`: that
-// block's base address); once they are in, cluster_totals adds them in one order everywhere.
+// Sends the warp's sums of K per-thread values for slot `slot` of `slots` (planes of them) to every
+// block (lane c to block c; `mine`: that block's base address); once all are in, cluster_totals adds
+// those of the slices in one order everywhere.
 template <int K, int C>
 __device__ __forceinline__ void send_sums(const double (&v)[K], unsigned mine, unsigned part,
-                                          unsigned bar, unsigned rank)
+                                          unsigned bar, int slot, int slots)
 {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     const double s = warp_sum(v[q]);
-    if (lane < C)
-      send_bytes(mine + part + 8u * ((q * C + rank) * kClWarps + warp), mine + bar, s);
+    if (lane < C) send_bytes(mine + part + 8u * (q * slots + slot), mine + bar, s);
   }
 }
 template <int K>
-__device__ __forceinline__ void cluster_totals(const double* part, int C, double (&out)[K])
+__device__ __forceinline__ void cluster_totals(const double* part, int slices, int slots,
+                                               double (&out)[K])
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     double s = 0.0;
-    for (int i = lane; i < C * kClWarps; i += kWarp) s += part[q * C * kClWarps + i];
+    for (int i = lane; i < slices; i += kWarp) s += part[q * slots + i];
     out[q] = warp_sum(s);
   }
 }
@@ -359,10 +369,15 @@ __global__ void __launch_bounds__(kClThreads, 1)
       }
     }
   }
-  // The products of this block's rows of P (m = 0) or Q (m = 1) with `vec`: f(unit, row, product).
-  auto products = [&](int m, const double* vec, auto&& f) {
+  const int slots_p = (int)sum_slots(d.slices_p, C), slots_q = (int)sum_slots(d.slices_q, C);
+  unsigned base[C], mine = 0;  // addresses of the cluster's blocks, and of block `lane`
+  // The products of this block's rows of P (m = 0) or Q (m = 1) with `vec`: f(unit, row, product, t)
+  // fills the row's terms of the K sums, which go to the entries at `part` of every block.
+  auto products = [&](int m, const double* vec, auto& t, unsigned part, auto&& f) {
+    constexpr int K = (int)(sizeof(t) / sizeof(double));
     const int n = m == 0 ? np : nq, slices = m == 0 ? d.slices_p : d.slices_q;
-    const int rows = m == 0 ? d.rows : d.cols;
+    const int rows = m == 0 ? d.rows : d.cols, slots = m == 0 ? slots_p : slots_q;
+    const unsigned bar = 8u * m;
     for (int i = warp; i < n; i += kClWarps) {
       const int s = (int)rank + C * i;
       if (s >= slices) break;
@@ -384,20 +399,28 @@ __global__ void __launch_bounds__(kClThreads, 1)
             if (k + e < len) g[e] = vec[j[e]];
 #pragma unroll
           for (int e = 0; e < 8; ++e)
-            if (k + e < len) acc += a[e] * g[e];
+            if (k + e < len) acc = fma(a[e], g[e], acc);
         }
       };
       if constexpr (CACHED) {
-        const int2 t = reinterpret_cast<const int2*>(dyn + S.tab[m])[i];
-        sum(at(S.val[m]) + t.x + lane,
-            reinterpret_cast<const unsigned short*>(dyn + S.idx[m]) + t.x + lane, t.y);
+        const int2 at_s = reinterpret_cast<const int2*>(dyn + S.tab[m])[i];
+        sum(at(S.val[m]) + at_s.x + lane,
+            reinterpret_cast<const unsigned short*>(dyn + S.idx[m]) + at_s.x + lane, at_s.y);
       } else {
-        const int64_t base = (m == 0 ? d.p_slice : d.q_slice)[s];
-        const int len      = (int)(((m == 0 ? d.p_slice : d.q_slice)[s + 1] - base) >> 5);
-        sum((m == 0 ? d.p_val : d.q_val) + base + lane, (m == 0 ? d.p_idx : d.q_idx) + base + lane,
+        const int64_t first = (m == 0 ? d.p_slice : d.q_slice)[s];
+        const int len       = (int)(((m == 0 ? d.p_slice : d.q_slice)[s + 1] - first) >> 5);
+        sum((m == 0 ? d.p_val : d.q_val) + first + lane, (m == 0 ? d.p_idx : d.q_idx) + first + lane,
             len);
       }
-      if (r < rows) f(i, r, acc);
+#pragma unroll
+      for (int q = 0; q < K; ++q) t[q] = 0.0;
+      if (r < rows) f(i, r, acc, t);
+      send_sums<K, C>(t, mine, part, bar, s, slots);
+    }
+    if ((int)rank + C * warp >= slices) {  // a warp without slices
+#pragma unroll
+      for (int q = 0; q < K; ++q) t[q] = 0.0;
+      send_sums<K, C>(t, mine, part, bar, (int)rank + C * warp, slots);
     }
   };
 
@@ -406,7 +429,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
   for (int r = threadIdx.x; r < d.rows; r += T) {
     const double bv = d.b[r];
     u[r]            = bv;
-    t1[0] += bv * bv;
+    t1[0] = fma(bv, bv, t1[0]);
   }
   block_sums<1, kClWarps>(t1, part_a, r1);
   __syncthreads();  // part_a is read before other blocks write it
@@ -419,22 +442,20 @@ __global__ void __launch_bounds__(kClThreads, 1)
     }
     return;
   }
-  // Exchanges of u (after P's products) and of v (after Q's): every entry and every warp's sums, to
-  // every block.
+  // Exchanges of u (after P's products) and of v (after Q's): every entry and every sum, to every block.
   const unsigned home = (unsigned)__cvta_generic_to_shared(dyn), bar_u = home, bar_v = home + 8;
-  unsigned base[C], mine = 0;
 #pragma unroll
   for (int c = 0; c < C; ++c) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base[c]) : "r"(home), "r"(c));
     if (lane == c) mine = base[c];
   }
-  const unsigned bytes_u = 8u * (d.rows + C * kClWarps), bytes_v = 8u * (d.cols + 2 * C * kClWarps);
+  const unsigned bytes_u = 8u * (d.rows + slots_p), bytes_v = 8u * (d.cols + 2 * slots_q);
   if (threadIdx.x == 0) {
     phase_init(bar_u);
     phase_init(bar_v);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     phase_expect(bar_u, bytes_u);
-    phase_expect(bar_v, bytes_v - 8u * C * kClWarps);  // the first one has a single sum
+    phase_expect(bar_v, bytes_v - 8u * slots_q);  // the first one has a single sum
   }
   unsigned phase_u = 0, phase_v = 0;
   bool ok          = true;
@@ -449,17 +470,15 @@ __global__ void __launch_bounds__(kClThreads, 1)
   lsqr_barrier();
   double us = 1.0 / beta;  // the normalised u is u * us
   // v = Op^T u / beta, alpha = |v|; x = w = 0 (w becomes v_1 in the first transpose product)
-  t1[0] = 0.0;
-  products(1, u, [&](int i, int j, double acc) {
+  products(1, u, t1, (unsigned)S.part_b, [&](int i, int j, double acc, double (&t)[1]) {
     const double vj = acc * us;
     send_all<C>(base, (unsigned)S.v + 8u * j, 8, vj);
     x[i * kWarp + lane] = 0.0;
     w[i * kWarp + lane] = 0.0;
-    t1[0] += vj * vj;
+    t[0]                = vj * vj;
   });
-  send_sums<1, C>(t1, mine, (unsigned)S.part_b, 8, rank);
   wait_v();
-  cluster_totals<1>(part_b, C, r1);
+  cluster_totals<1>(part_b, d.slices_q, slots_q, r1);
   double alpha  = sqrt(r1[0]);
   double vs     = alpha > 0.0 ? 1.0 / alpha : 0.0;
   double rhobar = alpha, phibar = beta, anorm2 = 0.0, xnorm = 0.0;
@@ -473,43 +492,40 @@ __global__ void __launch_bounds__(kClThreads, 1)
   } else {
     for (it = 1; it <= d.max_iter; ++it) {
       // u <- Op v - alpha u  (normalised v = v * vs, normalised u = u * us)
-      t1[0] = 0.0;
-      products(0, v, [&](int, int r, double acc) {
-        const double un = acc * vs - alpha * (u[r] * us);
+      products(0, v, t1, (unsigned)S.part_a, [&](int, int r, double acc, double (&t)[1]) {
+        const double un = fma(acc, vs, -alpha * (u[r] * us));
         send_all<C>(base, 16 + 8u * r, 0, un);
-        t1[0] += un * un;
+        t[0] = un * un;
       });
-      send_sums<1, C>(t1, mine, (unsigned)S.part_a, 0, rank);
       if (!(ok = phase_wait(bar_u, phase_u))) break;
       phase_u ^= 1;
       if (threadIdx.x == 0) phase_expect(bar_u, bytes_u);
-      cluster_totals<1>(part_a, C, r1);
+      cluster_totals<1>(part_a, d.slices_p, slots_p, r1);
       beta = sqrt(r1[0]);
       us   = beta > 0.0 ? 1.0 / beta : 0.0;
-      anorm2 += alpha * alpha + beta * beta;
+      anorm2 = fma(alpha, alpha, fma(beta, beta, anorm2));
       // pending x / w update, then v <- Op^T u - beta v
-      double t2[2] = {0.0, 0.0}, r2[2];
-      products(1, u, [&](int i, int j, double acc) {
+      double t2[2], r2[2];
+      products(1, u, t2, (unsigned)S.part_b, [&](int i, int j, double acc, double (&t)[2]) {
         const int q     = i * kWarp + lane;
         const double vo = v[j] * vs;
         double wj       = w[q];
-        const double xj = x[q] + c1 * wj;
-        wj              = vo - c2 * wj;
+        const double xj = fma(c1, wj, x[q]);
+        wj              = fma(-c2, wj, vo);
         x[q]            = xj;
         w[q]            = wj;
-        const double vn = acc * us - beta * vo;
+        const double vn = fma(acc, us, -beta * vo);
         send_all<C>(base, (unsigned)S.v + 8u * j, 8, vn);
-        t2[0] += vn * vn;
-        t2[1] += xj * xj;
+        t[0] = vn * vn;
+        t[1] = xj * xj;
       });
-      send_sums<2, C>(t2, mine, (unsigned)S.part_b, 8, rank);
       if (!wait_v()) break;
-      cluster_totals<2>(part_b, C, r2);
+      cluster_totals<2>(part_b, d.slices_q, slots_q, r2);
       alpha = sqrt(r2[0]);
       vs    = alpha > 0.0 ? 1.0 / alpha : 0.0;
       xnorm = sqrt(r2[1]);
       // Plane rotation (no damping) and the new pending update.
-      const double rho = sqrt(rhobar * rhobar + beta * beta);
+      const double rho = sqrt(fma(rhobar, rhobar, beta * beta));
       const double cs = rhobar / rho, sn = beta / rho;
       const double theta = sn * alpha;
       rhobar             = -cs * alpha;
@@ -520,7 +536,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
       rnorm              = phibar;
       arnorm             = alpha * fabs(sn * phi);
       const double anorm = sqrt(anorm2);
-      if (rnorm <= d.tol * bnorm + d.tol * anorm * xnorm) {
+      if (rnorm <= fma(d.tol * anorm, xnorm, d.tol * bnorm)) {
         flag = 1;
         break;
       }
@@ -543,7 +559,7 @@ __global__ void __launch_bounds__(kClThreads, 1)
   // The last pending x update, then the result.
   for (int i = warp; i < nq; i += kClWarps) {
     const int j = ((int)rank + C * i) * kWarp + lane, q = i * kWarp + lane;
-    if (j < d.cols) d.z[j] = x[q] + c1 * w[q];
+    if (j < d.cols) d.z[j] = fma(c1, w[q], x[q]);
   }
   if (threadIdx.x == 0 && (rank == 0 || flag == kLsqrFailed))
     outs[system] = lsqr_out{it, flag, rnorm, arnorm};

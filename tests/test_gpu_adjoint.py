@@ -1,5 +1,5 @@
 """GPU tests of the matrix-free KKT adjoint (cuOptSolutionAdjointBatch: LSQR on the GPU, one
-thread block per active-set system), the torch layer over it, and the vertex crossover (the same
+cluster per active-set system), the torch layer over it, and the vertex crossover (the same
 LSQR solves).
 
 References: the constructed optimum of generators.vertex_lp (unique and non-degenerate, with a
@@ -160,9 +160,9 @@ def test_adjoint_requires_an_optimal_solution(vlp):
 
 
 def test_batched_backward_equals_single_backwards():
-    """lp_solve_batch back-propagates through one cuOptSolutionAdjointBatch call (every active-set
-    system in one launch); the gradients equal those of the instances solved and differentiated one
-    at a time (each system's LSQR runs alone in its thread block, so the batch does not change it)."""
+    """lp_solve_batch back-propagates through one cuOptSolutionAdjointBatch call; the gradients equal
+    those of the instances solved and differentiated one at a time, to 1e-9 (the solutions differ by
+    rounding)."""
     from cuopt_b200.torch_layer import LPInstance, lp_solve, lp_solve_batch
     lps = [gen.vertex_lp(150 + 50 * i, 300 + 100 * i, 6, seed=70 + i) for i in range(3)]
     rng = np.random.default_rng(12)
@@ -176,6 +176,25 @@ def test_batched_backward_equals_single_backwards():
         (torch.tensor(w, device="cuda") * x).sum().backward()
         for k in ("c", "con_lo", "con_up", "values"):
             _close(tb[k].grad.cpu().numpy(), ts[k].grad.cpu().numpy(), 1e-9)
+
+
+def test_gradients_do_not_depend_on_the_batch():
+    """The gradients of given solutions are the same bits alone, in pairs and in larger batches: the
+    clusters that the systems run in (their number, their size, what is kept in shared memory)
+    change no sum."""
+    from cuopt_b200 import torch_layer as tl
+    from cuopt_b200.torch_layer import LPInstance, lp_solve_batch
+    lps = [gen.vertex_lp(40 + 110 * i, 90 + 220 * i, 6, seed=70 + i) for i in range(8)]
+    out = lp_solve_batch([LPInstance(**_tensors(lp)) for lp in lps], _settings())
+    solved = out[0][0].grad_fn.solved
+    rng = np.random.default_rng(5)
+    t = lambda k: torch.tensor(rng.standard_normal(k), device="cuda")
+    pairs = [(t(lp.n), t(lp.m)) for lp in lps]
+    alone = [tl._adjoint_batch(solved[i:i + 1], pairs[i:i + 1])[0] for i in range(8)]
+    for order in ([0, 1], [6, 7], [3, 1, 4], list(range(8)), [7] * 20 + [0], [0] * 200):
+        got = tl._adjoint_batch([solved[i] for i in order], [pairs[i] for i in order])
+        for i, g in zip(order, got):
+            assert all(torch.equal(a, b) for a, b in zip(g, alone[i])), (order[:4], i)
 
 
 def test_c4_shape_adjoint_against_vertex_map():
