@@ -296,6 +296,17 @@ __device__ __forceinline__ void send_all(const unsigned (&base)[C], unsigned off
   for (int c = 0; c < C; ++c) send_bytes(base[c] + off, base[c] + bar, v);
 }
 
+// Warp sums of K values (as warp_sum, step by step together).
+template <int K>
+__device__ __forceinline__ void warp_sums(const double (&v)[K], double (&s)[K])
+{
+#pragma unroll
+  for (int q = 0; q < K; ++q) s[q] = v[q];
+#pragma unroll
+  for (int o = kWarp / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < K; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+}
 // Sends the warp's sums of K per-thread values for slot `slot` of `slots` (planes of them) to every
 // block (lane c to block c; `mine`: that block's base address); once all are in, cluster_totals adds
 // those of the slices in one order everywhere.
@@ -303,11 +314,11 @@ template <int K, int C>
 __device__ __forceinline__ void send_sums(const double (&v)[K], unsigned mine, unsigned part,
                                           unsigned bar, int slot, int slots)
 {
-  const int lane = threadIdx.x & 31;
+  double s[K];
+  warp_sums<K>(v, s);
+  if ((threadIdx.x & 31) < C) {
 #pragma unroll
-  for (int q = 0; q < K; ++q) {
-    const double s = warp_sum(v[q]);
-    if (lane < C) send_bytes(mine + part + 8u * (q * slots + slot), mine + bar, s);
+    for (int q = 0; q < K; ++q) send_bytes(mine + part + 8u * (q * slots + slot), mine + bar, s[q]);
   }
 }
 template <int K>
@@ -316,11 +327,20 @@ __device__ __forceinline__ void cluster_totals(const double* part, int slices, i
 {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int q = 0; q < K; ++q) {
-    double s = 0.0;
-    for (int i = lane; i < slices; i += kWarp) s += part[q * slots + i];
-    out[q] = warp_sum(s);
+  for (int q = 0; q < K; ++q) out[q] = 0.0;
+  for (int i = lane; i < slices; i += 4 * kWarp) {  // four at a time, so that their loads overlap
+    double e[K][4];
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        e[q][j] = i + j * kWarp < slices ? part[q * slots + i + j * kWarp] : 0.0;
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) out[q] += e[q][j];
   }
+  warp_sums<K>(out, out);
 }
 
 template <int C, bool CACHED>
