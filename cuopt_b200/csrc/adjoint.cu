@@ -17,7 +17,7 @@
 // solutions (in the equilibrated variables), the derivatives of the minimum-norm response.
 //
 // Every solve with M or M^T is matrix-free: LSQR on the GPU with one cluster per system
-// (lsqr.cu), all the systems of a batch of instances in one launch.
+// (lsqr.cu), all the systems of a batch of instances side by side.
 #include <algorithm>
 #include <cmath>
 #include <stdexcept>

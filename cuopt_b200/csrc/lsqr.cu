@@ -765,11 +765,18 @@ cluster_kernel_t cluster_kernel(int blocks, bool cached)
   }
 }
 
-// The plan with the least estimated time: waves of clusters, each iteration of one taking about
-// 0.9 us for its exchanges' latency and sums, 0.3 ns for each entry of u and v (a block takes them in
-// at some 16 bytes a cycle), and the products, shared by its blocks (0.16 ns per non-zero and product
-// from shared memory, 0.4 ns from L2).
-cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>& ids, size_t limit)
+// The plan with the least estimated time: waves of clusters, each iteration of one taking a latency,
+// a share for every block and, between blocks, for every entry of u and v, and the products, shared by
+// the blocks.  Fitted to these us an iteration with 1, 2, 4, 8 and 16 blocks, operators in shared
+// memory, then from L2 (stored elements of both operators, rows + columns):
+//      704,   66:  2.7  2.7  2.6  2.7  2.8    3.4  3.3  3.3  3.3  3.7
+//    4 704,  600:  3.6  2.6  2.5  2.5  2.7    4.8  3.5  3.5  3.5  3.9
+//   13 088, 1600:  5.8  3.8  2.8  2.7  2.9    7.9  5.1  3.7  3.6  4.1
+//   40 672, 5000:    -    -  4.8  4.0  4.1   18.3 10.2  7.2  5.8  4.9
+// (within 18 %, 7 % in the mean).
+// `share`: the part of the GPU that the systems have while others run beside them.
+cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>& ids, size_t limit,
+                           double share)
 {
   cluster_plan best;
   if (ids.empty()) return best;
@@ -800,9 +807,9 @@ cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>
         (void)cudaGetLastError();
         continue;
       }
-      const double waves = std::ceil((double)ids.size() / active);
-      const double us    = waves * (0.9 + (c > 1 ? entries * 3e-4 : 0.0) +
-                                 nnz * (cached ? 1.6e-4 : 4e-4) / c);
+      const double waves = std::ceil((double)ids.size() / std::max(1.0, active * share));
+      const double us    = waves * ((cached ? 2.3 : 3.0) + 0.03 * c + (c > 1 ? entries * 5e-5 : 0.0) +
+                                 nnz * (cached ? 2.2e-4 : 3.5e-4) / c);
       if (best.smem == 0 || us < best_us) {
         best    = p;
         best_us = us;
@@ -810,6 +817,68 @@ cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>
     }
   if (best.smem == 0) throw cuda_error("lsqr: no cluster shape can be launched");
   return best;
+}
+
+// Streams beside `s` for launches that may run at the same time: each begins after the work that is in
+// s when it is taken, and join() makes s wait for all of them.
+class side_streams {
+ public:
+  explicit side_streams(cudaStream_t s) : s_(s) {}
+  side_streams(const side_streams&)            = delete;
+  side_streams& operator=(const side_streams&) = delete;
+  ~side_streams()
+  {
+    for (auto& l : lanes_) {
+      cudaStreamSynchronize(l.stream);  // after an error too: the caller's buffers are freed in s
+      cudaStreamDestroy(l.stream);
+      cudaEventDestroy(l.event);
+    }
+  }
+  cudaStream_t take()
+  {
+    lane l{};
+    B200_CUDA_CHECK(cudaEventCreateWithFlags(&l.event, cudaEventDisableTiming));
+    const cudaError_t e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
+    if (e != cudaSuccess) cudaEventDestroy(l.event);
+    B200_CUDA_CHECK(e);
+    lanes_.push_back(l);
+    B200_CUDA_CHECK(cudaEventRecord(l.event, s_));
+    B200_CUDA_CHECK(cudaStreamWaitEvent(l.stream, l.event, 0));
+    return l.stream;
+  }
+  void join()
+  {
+    for (auto& l : lanes_) {
+      B200_CUDA_CHECK(cudaEventRecord(l.event, l.stream));
+      B200_CUDA_CHECK(cudaStreamWaitEvent(s_, l.event, 0));
+    }
+  }
+
+ private:
+  struct lane {
+    cudaStream_t stream;
+    cudaEvent_t event;
+  };
+  cudaStream_t s_;
+  std::vector<lane> lanes_;
+};
+
+// Systems of like size, launched together: those whose shares of the operators fit in the shared memory
+// of the same number of blocks (the last class: of no number).  A large system so neither takes
+// the cache from small ones nor gives them its cluster.
+struct size_class {
+  std::vector<int> ids;
+  cluster_plan plan;
+};
+constexpr int kClassBlocks[] = {1, 2, 4, 8, 16};
+int class_of(const packed& q, size_t limit)
+{
+  int k = 0;
+  for (const int c : kClassBlocks) {
+    if (cluster_smem(q, c, true) <= limit) break;
+    ++k;
+  }
+  return k;
 }
 
 }  // namespace
@@ -833,25 +902,38 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
 
   // Systems with work go to the device: those whose vectors fit in a cluster's blocks, and the rest.
   const size_t limit = max_dynamic_smem((const void*)cluster_kernel(16, true));
-  std::vector<int> clus_ids, glob_ids;
+  std::vector<size_class> classes(std::size(kClassBlocks) + 1);
+  std::vector<int> glob_ids;
   size_t scratch_doubles = 0;
   for (int i = 0; i < count; ++i) {
     res[i].z.assign(ps[i]->cols, 0.0);
     if (pk[i].rows == 0 || pk[i].cols == 0) continue;
     if (cluster_smem(pk[i], 1, false) <= limit) {
-      clus_ids.push_back(i);
+      classes[class_of(pk[i], limit)].ids.push_back(i);
     } else {
       glob_ids.push_back(i);
       scratch_doubles += (size_t)pk[i].rows + 3 * (size_t)pk[i].cols;
     }
   }
-  if (clus_ids.empty() && glob_ids.empty()) return res;
-  const cluster_plan plan = plan_clusters(pk, clus_ids, limit);
+  std::vector<int> order;              // systems as they are launched
+  std::vector<int> blocks(count, 1);   // of the cluster of each
+  // A class's share of the GPU is its share of the work: iterations grow with the rows and columns.
+  std::vector<double> work(classes.size(), 0.0);
+  for (size_t k = 0; k < classes.size(); ++k)
+    for (int i : classes[k].ids)
+      work[k] += (double)(pk[i].rows + pk[i].cols) *
+                 (2.3 + 2.2e-4 * (double)(pk[i].p_val.size() + pk[i].q_val.size()));
+  const double all = std::accumulate(work.begin(), work.end(), 0.0);
+  for (auto& k : classes) {
+    k.plan = plan_clusters(pk, k.ids, limit, work[&k - classes.data()] / std::max(all, 1e-300));
+    for (int i : k.ids) blocks[i] = k.plan.blocks;
+    order.insert(order.end(), k.ids.begin(), k.ids.end());
+  }
+  order.insert(order.end(), glob_ids.begin(), glob_ids.end());
+  if (order.empty()) return res;
 
   // One upload of every array: offsets, indices, values, right-hand sides; outputs z.
   size_t n_off = 0, n_idx = 0, n_val = 0, n_b = 0, n_z = 0;
-  auto order = clus_ids;
-  order.insert(order.end(), glob_ids.begin(), glob_ids.end());
   for (int i : order) {
     n_off += pk[i].p_slice.size() + pk[i].q_slice.size();
     n_idx += pk[i].p_idx.size() + pk[i].q_idx.size();
@@ -923,8 +1005,8 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
     d.b        = d_b.data() + w.b;
     d.z        = d_z.data() + w.z;
     d.scratch  = d_scratch.data() + w.scratch;
-    d.share_p  = most_elements(q.p_slice, plan.blocks);
-    d.share_q  = most_elements(q.q_slice, plan.blocks);
+    d.share_p  = most_elements(q.p_slice, blocks[i]);
+    d.share_q  = most_elements(q.q_slice, blocks[i]);
     d.tol      = tol;
     d.max_iter = default_iter > 0 ? default_iter
                                   : (int)std::min<long long>(200000, 20LL * (q.rows + q.cols));
@@ -934,18 +1016,31 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   dbuf<lsqr_out> d_out(h_desc.size());
   d_desc.upload(h_desc.data(), h_desc.size(), s);
   trace_sync(s, "lsqr: upload");
-  const int n_clus = (int)clus_ids.size(), n_glob = (int)glob_ids.size();
-  if (n_clus > 0) {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    plan.configure(cfg, attr, n_clus, s);
-    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_kernel(plan.blocks, plan.cached),
-                                       (const lsqr_desc*)d_desc.data(), d_out.data()));
-  }
-  if (n_glob > 0) {
-    lsqr_kernel<<<n_glob, kLsqrThreads, 0, s>>>(d_desc.data() + n_clus, d_out.data() + n_clus);
+  // Launched from the largest systems down, which take the longest; the last launch is in s itself.
+  side_streams side(s);
+  size_t first = order.size();
+  int launches = !glob_ids.empty();
+  for (const auto& k : classes) launches += !k.ids.empty();
+  auto next = [&](size_t systems) {
+    first -= systems;
+    return --launches > 0 ? side.take() : s;
+  };
+  if (!glob_ids.empty()) {
+    const cudaStream_t ls = next(glob_ids.size());
+    lsqr_kernel<<<(int)glob_ids.size(), kLsqrThreads, 0, ls>>>(d_desc.data() + first,
+                                                               d_out.data() + first);
     B200_LAUNCH_CHECK();
   }
+  for (auto k = classes.rbegin(); k != classes.rend(); ++k) {
+    if (k->ids.empty()) continue;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    k->plan.configure(cfg, attr, (int)k->ids.size(), next(k->ids.size()));
+    B200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cluster_kernel(k->plan.blocks, k->plan.cached),
+                                       (const lsqr_desc*)d_desc.data() + first,
+                                       d_out.data() + first));
+  }
+  side.join();
   trace_sync(s, "lsqr: kernel");
   std::vector<double> h_z(n_z);
   std::vector<lsqr_out> h_out(h_desc.size());

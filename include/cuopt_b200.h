@@ -265,7 +265,8 @@ cuopt_int_t cuOptSolutionAdjoint(cuOptOptimizationProblem problem,
 /* cuOptSolutionAdjoint for `count` (problem, solution) pairs at once (no counterpart in the
  * reference): every pointer argument is an array of `count` pointers with the meaning of the single
  * call's argument (dl_dx[i] required; dl_dy, the output arrays, or any of their entries may be
- * NULL).  All the active-set solves of the batch run in one launch, one cluster each.
+ * NULL).  The active-set solves of the batch run side by side, one
+ * cluster each (one launch per size class); a system's result does not depend on the others.
  * Returns CUOPT_INVALID_ARGUMENT (and writes nothing) if any solution is not Optimal. */
 cuopt_int_t cuOptSolutionAdjointBatch(cuopt_int_t count,
                                       const cuOptOptimizationProblem* problems,
