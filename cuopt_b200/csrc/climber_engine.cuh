@@ -51,16 +51,23 @@ __device__ __forceinline__ void mm_sweep_block(const dev_sell<double>& A,
   if (xb < lb) {
     const int row = xb * kWarpsPerBlock + warp;
     if (row < A.n_long) {
-      const auto pre = epi.load(row);
-      for (int64_t k = A.long_off[row] + lane; k < A.long_off[row + 1]; k += kWarp) {
-        const double v = ld_stream(A.val + k);
-        double gv[kGroup];
-        gather_group(g + (size_t)ld_stream(A.idx + k) * ld + g0, gv);
+      const auto pre    = epi.load(row);
+      const int64_t end = A.long_off[row + 1];
+      const int strands = row < A.n_wide ? kWideStrands : 1;  // as in the single solve's sweeps
+      for (int q = 0; q < strands; ++q) {
+        double part[kGroup];
 #pragma unroll
-        for (int b = 0; b < kGroup; ++b) acc[b] += v * gv[b];
+        for (int b = 0; b < kGroup; ++b) part[b] = 0.0;
+        for (int64_t k = A.long_off[row] + q * kWarp + lane; k < end; k += strands * kWarp) {
+          const double v = ld_stream(A.val + k);
+          double gv[kGroup];
+          gather_group(g + (size_t)ld_stream(A.idx + k) * ld + g0, gv);
+#pragma unroll
+          for (int b = 0; b < kGroup; ++b) part[b] += v * gv[b];
+        }
+#pragma unroll
+        for (int b = 0; b < kGroup; ++b) acc[b] += warp_sum(part[b]);
       }
-#pragma unroll
-      for (int b = 0; b < kGroup; ++b) acc[b] = warp_sum(acc[b]);
       if (lane == 0) epi(row, acc, pre, red);
     }
   } else {

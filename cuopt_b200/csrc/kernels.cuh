@@ -51,8 +51,9 @@ inline int sell_grid(const dev_sell<T>& a, int wpb = kWarpsPerBlock)
 // rounds, which a sweep waits for when the rest of it is done (20k x 60k LP, Zipf rows up to 5000
 // long: 38 of 50 us an iteration).  So rows longer than kWideRow elements (a sixteenth of such a
 // chain) are cut into kWideStrands strands, lane l of strand s taking elements 256 t + 32 s + l,
-// whose sums are added in strand order: by the 8 warps of a block (or half block of 16 warps), or
-// by one warp where a block has fewer.  Every form of the sweeps adds them in the same order.
+// whose sums are added in strand order: by the 8 warps of a block (or half block of 16 warps), or by
+// one warp (where a block has fewer, in the cluster-resident form, in batches and for climbers).  Every
+// form of the sweeps adds them in the same order, so iterates do not depend on the form.
 constexpr int kWideStrands = 8;
 B200_HD inline int wide_blocks(int n_wide, int wpb = kWarpsPerBlock)
 {
@@ -370,7 +371,12 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
     if (q < A.long_count() && !skip_rows(epi, row, row)) {
       const auto pre  = epi.load(row);
       const int64_t b = A.long_off[row], e = A.long_off[row + 1];
-      const double acc = warp_sum(strided_product<4, kWarp, COH>(A, g, b + lane, e));
+      double acc = 0.0;
+      // In batches the wide rows are not the first ones: one warp takes each, strand after strand.
+      if (has_skip_range<Epi>::value && e - b > kWideRow)
+        for (int q = 0; q < kWideStrands; ++q) acc += wide_strand<COH>(A, g, b, e, q);
+      else
+        acc = warp_sum(strided_product<4, kWarp, COH>(A, g, b + lane, e));
       if (lane == 0) epi(row, acc, pre, red);
     }
   } else {

@@ -112,6 +112,23 @@ def test_wide_rows_follow_the_oracle(m, n, cap):
             assert np.max(np.abs(got - want)) <= ITERATE_RTOL * (1 + np.abs(want).max())
 
 
+@pytest.mark.parametrize("kind", ["plain", "long", "wide"])
+@pytest.mark.parametrize("limit", [10, 190])
+def test_climbers_and_batches_follow_single_solves_bit_by_bit(kind, limit):
+    """Before the first restart nothing but the rows' sums can differ: climbers and batch instances
+    have a single solve's iterates, also with rows of more than 512 elements."""
+    lp = {"plain": lambda: gen.constructed_lp(300, 700, 6, seed=3),
+          "long": lambda: gen.skewed_lp(60, 400, seed=9, zipf_a=0.7, cap=400),
+          "wide": lambda: gen.skewed_lp(60, 2500, seed=9, zipf_a=0.7, cap=2500)}[kind]()
+    s = settings(tol=1e-13, iteration_limit=limit)
+    single = lpm.Solve(datamodel_from_lp(lp), s)
+    var = np.array([0, lp.n // 2, lp.n - 1], np.int32)
+    for sol in (lpm.SolveClimbers(datamodel_from_lp(lp), var, lp.var_lo[var], lp.var_up[var], s)[0] +
+                lpm.BatchSolve([datamodel_from_lp(lp)] * 2, s)[0]):
+        _same(single, sol)
+        assert sol.stats["step_size"] == single.stats["step_size"]
+
+
 @pytest.mark.parametrize("seed", range(4))
 def test_tiled_copy_with_a_gap_behind_the_long_rows(seed):
     """Long rows whose elements end off a chunk leave a gap before the slices; the tiled copy takes
