@@ -1037,7 +1037,6 @@ class batch_engine {
   void bidiagonalise(int max_steps, Test&& test)
   {
     const int m = in_.m, n = in_.n;
-    const int ld = max_steps + 2;  // history rows (steps), each B_ wide
     // Every instance starts from the first m_b values of the std::mt19937(1) normal sequence.
     std::vector<double> z0(m);
     int max_rows = 0;
@@ -1046,14 +1045,14 @@ class batch_engine {
     for (int b = 0; b < B_; ++b)
       std::copy(seq->begin(), seq->begin() + (in_.row_start[b + 1] - in_.row_start[b]),
                 z0.begin() + in_.row_start[b]);
-    dbuf<double> u(m), v(n), tmp(m), alphas((size_t)B_ * ld), betas((size_t)B_ * ld);
+    dbuf<double> u(m), v(n), tmp(m);
+    // The coefficients of one chunk, a row of B_ a step; row 0 of betas is the norm of the start.
+    dbuf<double> alphas((size_t)B_ * kLanczosChunk), betas((size_t)B_ * (kLanczosChunk + 1));
     dbuf<b_gk_state> st(B_);
     tmp.upload(z0.data(), m, s_);
     permute_gather(tmp.data(), L_.row_new2old.data(), m, 1.0, u.data(), s_);
     v.zero(s_);
     st.zero(s_);
-    alphas.zero(s_);  // an instance without rows or columns records nothing
-    betas.zero(s_);
     dbuf<int> pact(B_);
     std::vector<int> pact_h(B_, 1);
     pact.upload(pact_h.data(), B_, s_);
@@ -1082,37 +1081,38 @@ class batch_engine {
         rows_.chunks.data(), rows_.offsets.data(), B_, pact.data(), rowbuf_.data(), part.data(),
         st.data(), betas.data(), k);
     };
-    std::vector<double> ha((size_t)B_ * ld), hb((size_t)B_ * ld);
+    // On the host, each instance's own from its first step to its last.
+    std::vector<double> ha((size_t)B_ * kLanczosChunk), hb((size_t)B_ * kLanczosChunk);
+    std::vector<std::vector<double>> diag(B_), sub(B_);
     std::vector<char> done(B_, 0);
     eta_.assign(B_, 0.0);
     power_iters_.assign(B_, 0);
     int left = B_, listed = B_, k = 0;
     while (left > 0 && k < max_steps) {
       const int c = std::min(kLanczosChunk, max_steps - k);
-      for (int i = 0; i < c; ++i) step(k + i);
+      for (int i = 0; i < c; ++i) step(i);
       launches_ += 4.0 * c;
       B200_LAUNCH_CHECK();
-      // The new rows of the histories.
-      B200_CUDA_CHECK(cudaMemcpyAsync(ha.data() + (size_t)k * B_, alphas.data() + (size_t)k * B_,
-                                      (size_t)c * B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
-      B200_CUDA_CHECK(cudaMemcpyAsync(hb.data() + (size_t)(k + 1) * B_,
-                                      betas.data() + (size_t)(k + 1) * B_,
-                                      (size_t)c * B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
+      alphas.download(ha.data(), (size_t)c * B_, s_);
+      B200_CUDA_CHECK(cudaMemcpyAsync(hb.data(), betas.data() + B_, (size_t)c * B_ * sizeof(double),
+                                      cudaMemcpyDeviceToHost, s_));
       B200_CUDA_CHECK(cudaStreamSynchronize(s_));
       k += c;
       // Each instance's test (the host's share of the step) is independent of the others:
       // instances are split over host threads, each writing only its own entries, so the results
       // do not depend on the split.
       parallel_ranges(B_, [&](int b0, int b1) {
-        std::vector<double> a(k), bb(k);
         for (int b = b0; b < b1; ++b) {
           if (!pact_h[b]) continue;
-          // betas[0] holds |z0|; the recurrence coefficients are betas[1..].
-          for (int j = 0; j < k; ++j) {
-            a[j]  = ha[(size_t)j * B_ + b];
-            bb[j] = hb[(size_t)(j + 1) * B_ + b];
+          for (int j = 0; j < c; ++j) {
+            diag[b].push_back(ha[(size_t)j * B_ + b]);
+            sub[b].push_back(hb[(size_t)j * B_ + b]);
           }
-          done[b] = test(b, k, a.data(), bb.data());
+          done[b] = test(b, k, diag[b].data(), sub[b].data());
+          if (done[b]) {
+            diag[b] = {};
+            sub[b]  = {};
+          }
         }
       });
       for (int b = 0; b < B_; ++b)

@@ -176,3 +176,22 @@ def test_c3_subset_mixed_refined_meets_objective_bound():
         assert relative_kkt(sol) <= REFINED_TOL
         assert rel(sol.get_primal_objective(), lp.optimal_objective) <= OBJ_RTOL, i
         assert rel(sol.get_primal_objective(), fx[i]["1e-08"]["primal_objective"]) <= OBJ_RTOL, i
+
+
+def test_step_sizes_of_many_instances_keep_no_history_on_the_device():
+    """The step sizes' recurrence may take 1 024 steps; its coefficients leave the device chunk by
+    chunk.  4 000 tiny LPs: histories of all steps would be 65 MB, the rest of the batch is a few."""
+    from cuda.bindings import driver, runtime as rt
+
+    lp = gen.constructed_lp(3, 5, 2, seed=1)
+    models = [datamodel_from_lp(lp)] * 4000
+    s = settings(tol=1e-6, iteration_limit=10, precision=0)
+    lpm.BatchSolve(models[:10], s)
+    err, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    assert err == rt.cudaError_t.cudaSuccess
+    used = lambda a: int(rt.cudaMemPoolGetAttribute(pool, a)[1])
+    A = rt.cudaMemPoolAttr
+    rt.cudaMemPoolSetAttribute(pool, A.cudaMemPoolAttrUsedMemHigh, driver.cuuint64_t(0))
+    before = used(A.cudaMemPoolAttrUsedMemCurrent)
+    lpm.BatchSolve(models, s)
+    assert 0 < used(A.cudaMemPoolAttrUsedMemHigh) - before < 40e6
