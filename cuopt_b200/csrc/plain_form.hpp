@@ -35,10 +35,7 @@ class plain_form_tuner {
   plain_form_tuner& operator=(const plain_form_tuner&) = delete;
   ~plain_form_tuner()
   {
-    for (auto& p : pending_) {
-      cudaEventDestroy(p.e0);
-      cudaEventDestroy(p.e1);
-    }
+    drop_all();
     for (auto& p : spare_) {
       cudaEventDestroy(p.e0);
       cudaEventDestroy(p.e1);
@@ -50,7 +47,7 @@ class plain_form_tuner {
   // timing).  `available[f]` tells whether form f can run on this problem and device.
   void reset(int mode, int known, const bool (&available)[kForms])
   {
-    collect_all_dropped();
+    drop_all();
     for (auto& u : us_) u.clear();
     for (int f = 0; f < kForms; ++f) avail_[f] = f == 0 || available[f];
     turn_ = 0;
@@ -70,18 +67,23 @@ class plain_form_tuner {
   // The form of the next cycle.
   int next() const { return decided() ? chosen_ : turn_; }
 
-  // Brackets one cycle (only while tuning).
+  // Brackets one cycle (only while tuning).  The form may be decided between the two: results of
+  // earlier cycles are collected while this one runs.  Its events then go back unused.
   void begin(cudaStream_t s)
   {
     if (decided()) return;
-    cur_ = take();
+    drop_open();
+    cur_  = take();
+    open_ = true;
     B200_CUDA_CHECK(cudaEventRecord(cur_.e0, s));
   }
   // `one_time`: the cycle included work that later cycles of the form will not repeat; it is not
   // counted, and the same form runs again next.
   void end(cudaStream_t s, int form, long iters, bool one_time)
   {
-    if (decided()) return;
+    if (!open_) return;
+    if (decided()) return drop_open();
+    open_         = false;
     cur_.form     = form;
     cur_.iters    = iters;
     cur_.one_time = one_time;
@@ -162,14 +164,21 @@ class plain_form_tuner {
     B200_CUDA_CHECK(cudaEventCreate(&r.e1));
     return r;
   }
-  void collect_all_dropped()
+  void drop_open()
   {
+    if (open_) spare_.push_back(cur_);
+    open_ = false;
+  }
+  void drop_all()
+  {
+    drop_open();
     for (auto& p : pending_) spare_.push_back(p);
     pending_.clear();
   }
 
   std::vector<run> pending_, spare_;
-  run cur_;
+  run cur_;            // the cycle that has begun and not ended, while open_
+  bool open_ = false;
   std::vector<double> us_[kForms];  // microseconds per iteration of each counted cycle, per form
   bool avail_[kForms] = {true, false, false};
   int turn_           = 0;
