@@ -77,7 +77,6 @@ struct b_primal_epi {
     TX x, c, lo, up, xa;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int j) const
   {
@@ -104,7 +103,6 @@ struct b_dual_epi {
     TX y, lo, up, ya;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int i) const
   {
@@ -131,7 +129,6 @@ struct b_fpe_epi {
     TX aty, xbar, x;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int j) const
   {
@@ -158,7 +155,6 @@ struct b_term_primal_epi {
     double l, u, y;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int i) const
   {
@@ -185,7 +181,6 @@ struct b_term_dual_epi {
     double c, x, s;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int j) const
   {
@@ -519,7 +514,6 @@ struct b_gk_primal_epi {
     double v;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{v[j], ctx.inst[j]}; }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<0>&) const
@@ -542,7 +536,6 @@ struct b_gk_dual_epi {
     double u;
     int b;
   };
-  __device__ bool skip() const { return false; }
   __device__ bool skip_range(int r0, int r1) const { return ctx.all_frozen(r0, r1); }
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{u[i], ctx.inst[i]}; }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<0>&) const

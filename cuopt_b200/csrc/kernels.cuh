@@ -325,11 +325,6 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
   red_t<K> red;
 #pragma unroll
   for (int q = 0; q < (K > 0 ? K : 1); ++q) red.v[q] = 0.0;
-  if (epi.skip()) {
-    // Uniform early exit (e.g. converged power iteration): every block still stores zeros.
-    block_reduce_store<K, has_max_red<Epi>::value>(red, partials, vb);
-    return;
-  }
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) & (WPB - 1);
   const int wb   = wide_blocks(A.wide_count(), WPB);
   const int lb   = row_blocks(A, WPB);
@@ -725,7 +720,6 @@ struct primal_epi {
   struct pre_t {
     TX x, c, lo, up, xa;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const
   {
     return pre_t{x[j], c[j], lo[j], up[j], HALPERN ? xa[j] : TX(0)};
@@ -754,7 +748,6 @@ struct dual_epi {
   struct pre_t {
     TX y, lo, up, ya;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const
   {
     return pre_t{y[i], lo[i], up[i], HALPERN ? ya[i] : TX(0)};
@@ -1054,7 +1047,6 @@ struct cluster_primal_epi {
   using pre_t               = typename base_t::pre_t;
   base_t base;
   unsigned copy, blocks;
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return base.load(j); }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<0>&) const
   {
@@ -1070,7 +1062,6 @@ struct cluster_dual_epi {
   using pre_t               = typename base_t::pre_t;
   base_t base;
   unsigned copy, blocks;
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const { return base.load(i); }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<0>&) const
   {
@@ -1493,7 +1484,6 @@ struct fpe_epi {
   struct pre_t {
     TX aty, xbar, x;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{aty[j], xbar[j], x[j]}; }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<2>& r) const
   {
@@ -1565,7 +1555,6 @@ struct term_primal_epi {
   struct pre_t {
     double l, u, y;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{lc[i], uc[i], y[i]}; }
   __device__ __forceinline__ void operator()(int i, double ax, const pre_t& p, red_t<2>& r) const
   {
@@ -1587,7 +1576,6 @@ struct term_dual_epi {
   struct pre_t {
     double c, x, s;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{c[j], x[j], s[j]}; }
   __device__ __forceinline__ void operator()(int j, double aty, const pre_t& p, red_t<3>& r) const
   {
@@ -1600,16 +1588,15 @@ struct term_dual_epi {
 };
 
 // Both termination sweeps in one launch (blocks [0, gp) the rows of A, the others the rows of A^T),
-// and their sums by the block that finishes last, in finalize_sum_kernel's order, written to device
-// memory and to the pinned host buffer that the host reads once the launch's event has completed
-// (with the two error flags behind them, see enqueue_conv).  As two sweeps, two one-block sums and
-// a copy this took five stream operations per check; on a 2000 x 5000 LP they were the longer part
-// of it.  arrived must be 0 before the launch and is 0 after it.
+// and their sums by the block that finishes last, in finalize_sum_kernel's order, written to the pinned
+// host buffer that the host reads once the launch's event has completed (with the two error flags
+// behind them, see enqueue_conv).  As two sweeps, two one-block sums and a copy this took five stream
+// operations per check; on a 2000 x 5000 LP they were the longer part of it.  arrived must be 0
+// before the launch and is 0 after it.
 static __global__ void __launch_bounds__(kBlock, kSweepBlocks<double>)
   term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
               const double* __restrict__ yu, term_primal_epi ep, term_dual_epi ed, int gp, int gd,
-              double* partials, unsigned* arrived, double* out, double* host, const int* flag_a,
-              const int* flag_b)
+              double* partials, unsigned* arrived, double* host, const int* flag_a, const int* flag_b)
 {
   double* part_d = partials + 2 * (size_t)gp;
   if ((int)blockIdx.x < gp)
@@ -1628,7 +1615,7 @@ static __global__ void __launch_bounds__(kBlock, kSweepBlocks<double>)
   __shared__ double sums[5];
   ordered_block_sum<2, true>(partials, gp, sums);
   ordered_block_sum<3, true>(part_d, gd, sums + 2);
-  if (threadIdx.x < 5) out[threadIdx.x] = host[threadIdx.x] = sums[threadIdx.x];
+  if (threadIdx.x < 5) host[threadIdx.x] = sums[threadIdx.x];
   if (threadIdx.x == 0) {
     int* flags = reinterpret_cast<int*>(host + 8);
     flags[0]   = *flag_a;
@@ -1650,7 +1637,6 @@ struct term_linf_primal_epi {
   struct pre_t {
     double l, u;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{lc[i], uc[i]}; }
   __device__ __forceinline__ void operator()(int, double ax, const pre_t& p, red_t<1>& r) const
   {
@@ -1670,7 +1656,6 @@ struct term_linf_dual_epi {
   struct pre_t {
     double c, s;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{c[j], s[j]}; }
   __device__ __forceinline__ void operator()(int, double aty, const pre_t& p, red_t<1>& r) const
   {
@@ -1685,25 +1670,23 @@ struct term_linf_dual_epi {
 // mode 0: sum x^2 ; mode 1: sum (a-b)^2 ; mode 2: bound norm terms of (lo, up)
 template <int MODE, typename TA>
 __global__ void __launch_bounds__(kBlock) vec_reduce_kernel(const TA* a, const TA* b, int n,
-                                                            double* partials, const int* done)
+                                                            double* partials)
 {
   red_t<1> r;
   r.v[0] = 0.0;
-  if (!(done && *done)) {
-    for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-      if constexpr (MODE == 0) {
-        const double v = (double)a[i];
-        r.v[0] += v * v;
-      } else if constexpr (MODE == 1) {
-        const double d = (double)a[i] - (double)b[i];
-        r.v[0] += d * d;
-      } else {
-        const double l = (double)a[i], u = (double)b[i];
-        double s       = 0.0;
-        if (isfinite(l) && l != u) s += l * l;
-        if (isfinite(u)) s += u * u;
-        r.v[0] += s;
-      }
+  for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+    if constexpr (MODE == 0) {
+      const double v = (double)a[i];
+      r.v[0] += v * v;
+    } else if constexpr (MODE == 1) {
+      const double d = (double)a[i] - (double)b[i];
+      r.v[0] += d * d;
+    } else {
+      const double l = (double)a[i], u = (double)b[i];
+      double s       = 0.0;
+      if (isfinite(l) && l != u) s += l * l;
+      if (isfinite(u)) s += u * u;
+      r.v[0] += s;
     }
   }
   block_reduce_store<1>(r, partials);
@@ -1740,7 +1723,6 @@ struct gk_primal_epi {
   struct pre_t {
     double v;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int j) const { return pre_t{v[j]}; }
   __device__ __forceinline__ void operator()(int j, double acc, const pre_t& p, red_t<1>& r) const
   {
@@ -1758,7 +1740,6 @@ struct gk_dual_epi {
   struct pre_t {
     double u;
   };
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int i) const { return pre_t{u[i]}; }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t& p, red_t<1>& r) const
   {
@@ -2211,7 +2192,6 @@ struct ray_primal_epi {
   double inv_norm;
   double* out;
   struct pre_t {};
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int) const { return pre_t{}; }
   __device__ __forceinline__ void operator()(int i, double acc, const pre_t&, red_t<0>&) const
   {
@@ -2232,7 +2212,6 @@ struct ray_dual_epi {
   double* slack_term;
   double* violation;
   struct pre_t {};
-  __device__ bool skip() const { return false; }
   __device__ __forceinline__ pre_t load(int) const { return pre_t{}; }
   __device__ __forceinline__ void operator()(int j, double g, const pre_t&, red_t<0>&) const
   {

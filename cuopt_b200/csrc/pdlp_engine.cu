@@ -271,7 +271,7 @@ class engine {
   void prepare_checks()
   {
     tpartials_.resize(2 * (size_t)sweep_grid(view64(L_.A)) + 3 * (size_t)sweep_grid(view64(L_.AT)));
-    tres_.resize(8);
+    tres_.resize(2);  // the per-constraint maxima
     tarrived_.resize(1);
     tarrived_.zero(s_);
   }
@@ -430,7 +430,7 @@ class engine {
   template <int MODE, typename TA>
   double reduce(const TA* a, const TA* b, int n)
   {
-    vec_reduce_kernel<MODE, TA><<<vgrid_, kBlock, 0, s_>>>(a, b, n, partials_.data(), nullptr);
+    vec_reduce_kernel<MODE, TA><<<vgrid_, kBlock, 0, s_>>>(a, b, n, partials_.data());
     finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), vgrid_, dres_.data());
     launches_ += 2;
     B200_LAUNCH_CHECK();
@@ -496,8 +496,7 @@ class engine {
     permute_gather(tmp.data(), L_.row_new2old.data(), m, 1.0, u.data(), s_);
     v.zero(s_);
     st.zero(s_);
-    vec_reduce_kernel<0, double><<<vgrid_, kBlock, 0, s_>>>(u.data(), nullptr, m,
-                                                            partials_.data(), nullptr);
+    vec_reduce_kernel<0, double><<<vgrid_, kBlock, 0, s_>>>(u.data(), nullptr, m, partials_.data());
     finalize_sum_kernel<1><<<1, kBlock, 0, s_>>>(partials_.data(), vgrid_, dres_.data());
     gk_start_kernel<<<1, 1, 0, s_>>>(st.data(), dres_.data(), betas.data());
     launches_ += 3;
@@ -1205,20 +1204,20 @@ class engine {
     term_kernel<<<gp + gd, kBlock, 0, cs_check_>>>(
       A, AT, xu_.data(), yu_.data(), term_primal_epi{lc64_.data(), uc64_.data(), yu_.data()},
       term_dual_epi{c64_.data(), xu_.data(), su_.data()}, gp, gd, tpartials_.data(),
-      tarrived_.data(), tres_.data(), h, &pctl_.data()->status,
+      tarrived_.data(), h, &pctl_.data()->status,
       tile_primal_ || tile_dual_ ? terr_.data() : nullptr);
     ++launches_;
     if (p_.per_constraint_residual) {
       sell_map_kernel<double, double, term_linf_primal_epi><<<gp, kBlock, 0, cs_check_>>>(
         A, xu_.data(), term_linf_primal_epi{lc64_.data(), uc64_.data(), p_.rel_primal},
         tpartials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gp, tres_.data() + 5);
+      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gp, tres_.data());
       sell_map_kernel<double, double, term_linf_dual_epi><<<gd, kBlock, 0, cs_check_>>>(
         AT, yu_.data(), term_linf_dual_epi{c64_.data(), su_.data(), p_.rel_dual},
         tpartials_.data());
-      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gd, tres_.data() + 6);
+      finalize_max_kernel<1><<<1, kBlock, 0, cs_check_>>>(tpartials_.data(), gd, tres_.data() + 1);
       launches_ += 4;
-      B200_CUDA_CHECK(cudaMemcpyAsync(h + 5, tres_.data() + 5, 2 * sizeof(double),
+      B200_CUDA_CHECK(cudaMemcpyAsync(h + 5, tres_.data(), 2 * sizeof(double),
                                       cudaMemcpyDeviceToHost, cs_check_));
     }
     B200_LAUNCH_CHECK();
