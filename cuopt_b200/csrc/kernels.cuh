@@ -1241,6 +1241,10 @@ __global__ void __launch_bounds__(kResidentThreads)
 //     y / sigma (two FP64 divisions) are formed between sending and waiting.
 // Waits are bounded: one that runs out sets the launch's status, and every block leaves through the
 // closing cluster barrier.
+// At most kUnitWarps slices a block: with 10, an iteration of a 2000 x 5000 LP takes 5.20 us (FP64; 5.46
+// in the form of several slices a warp) and of 2400 x 6000, 12 slices a block, 6.22 in that form;
+// compiled for 12 it takes 5.94 here, but smaller LPs up to 0.07 us more, and 8000 columns with 16
+// lose (7.46, 7.26 there).
 constexpr int kClusterBlocks = 16;
 constexpr int kUnitWarps     = 10;
 

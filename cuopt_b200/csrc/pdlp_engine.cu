@@ -5,8 +5,8 @@
 // the host (restart decision, PID primal weight, fixed-point errors); all vector and matrix work
 // is in the kernels of kernels.cuh.  Iterations that need neither a termination test, a "major"
 // step nor a fixed-point error are replayed from cached CUDA graphs of 2^k iterations, or run by one
-// persistent cooperative launch or one cluster launch, whichever form timed faster on the solve's
-// first runs (small LPs always take the cluster).
+// persistent cooperative launch or, for small LPs, one cluster launch, whichever form timed faster on
+// the first cycles of the first solve of a shape (see plain_form.hpp).
 #include "device_layout.cuh"
 #include "host_io.hpp"
 #include "kernels.cuh"
@@ -458,7 +458,7 @@ class engine {
   // mixed precision (where the iterates are not expected to match the FP64 reference path): the
   // estimate sigma_max(B_k) of the bidiagonal B_k rises to sigma_max(A) within tens of matrix
   // pairs, where the reference's power iteration (kept for FP64) takes hundreds.  Same start vector
-  // as the power iteration; stops when the estimate changes by less than 1e-10 relative.
+  // as the power iteration; stops when the estimate changes by at most kLanczosTol (relative).
   void lanczos_step_size()
   {
     double sigma2 = 0.0, prev = -1.0;

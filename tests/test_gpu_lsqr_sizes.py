@@ -1,5 +1,6 @@
 """Active-set solves over the cluster shapes of the LSQR kernel: one system (the largest clusters),
-many at once (small ones), sizes around a slice, and operators that do not fit in shared memory;
+many at once (small ones), sizes around a slice, operators that do not fit in shared memory, and
+vectors that do not (one block, everything in global memory);
 the gradients are those of the constructed vertex's basis (SciPy), to the adjoint tests' 1e-7."""
 from __future__ import annotations
 
@@ -41,3 +42,8 @@ def test_one_system(m, n, k):
 def test_many_systems(count):
     sizes = [(9, 20, 3), (33, 70, 5), (130, 260, 6), (300, 640, 7)]
     _check([gen.vertex_lp(*sizes[i % 4], seed=100 + i) for i in range(count)])
+
+
+def test_vectors_beyond_shared_memory():
+    """15 000 rows and columns: u, v, x and w are in global memory, one block runs the system."""
+    _check([gen.vertex_lp(15000, 30100, 2, seed=9)])

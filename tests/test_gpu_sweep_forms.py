@@ -16,7 +16,7 @@ GRAPHS, PERSISTENT, CLUSTER = 0, 1, 2
 ITERATE_RTOL = 1e-9  # the repository's parity tolerance for iterates against the oracle
 
 
-def _solve(lp, form, limit, precision=0, wpb=0, refine=False):
+def _solve(lp, form, limit, precision=0, wpb=0):
     s = settings(tol=1e-13, iteration_limit=limit, precision=precision)
     s.set_parameter(lpm.CUOPT_PDLP_PERSISTENT_ITERATIONS, form)
     if wpb:
@@ -83,18 +83,23 @@ def test_cluster_form_checks_every_hundred_iterations(limit):
     _same(_solve(lp, GRAPHS, limit), _solve(lp, CLUSTER, limit))
 
 
-@pytest.mark.parametrize("form", [GRAPHS, CLUSTER])
-def test_refined_mixed_solve_takes_over_the_kept_iterates(form):
-    """The FP64 continuation starts from the iterates of the check that ended the mixed solve."""
+@pytest.mark.parametrize("form", [PERSISTENT, CLUSTER])
+@pytest.mark.parametrize("tol,refine", [(1e-5, True), (1e-10, False)])
+def test_fp64_continuation_takes_over_the_kept_iterates(form, tol, refine):
+    """The FP64 continuation starts from the iterates of the check that ended the mixed solve: one that
+    met its tolerance and is refined, and one that stalled (FP32 does not reach 1e-10)."""
     lp = gen.constructed_lp(300, 700, 6, seed=12)
     out = []
     for f in (GRAPHS, form):
-        s = settings(tol=1e-5, precision=1)
+        s = settings(tol=tol, precision=1)
         s.set_parameter(lpm.CUOPT_PDLP_PERSISTENT_ITERATIONS, f)
-        s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_PASSES, 1)
-        s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_TOLERANCE, 1e-8)
+        if refine:
+            s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_PASSES, 1)
+            s.set_parameter(lpm.CUOPT_PDLP_REFINEMENT_TOLERANCE, 1e-8)
         out.append(lpm.Solve(datamodel_from_lp(lp), s))
-    assert out[0].stats["refinement_passes"] == 1
+        assert out[-1].get_termination_status() == lpm.LPTerminationStatus.Optimal
+        assert out[-1].stats["refinement_passes"] == 1
+        assert out[-1].stats["plain_iteration_form"] == f
     _same(out[0], out[1])
 
 
