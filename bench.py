@@ -33,6 +33,9 @@ iterates, FP64 termination / restart / step ratio).  The same solve in plain FP6
             gradients checked against every instance's exact derivatives and central differences
             (h = 1e-6, 32 coordinates of each of c, b and A per instance).
 
+The one JSON line on stdout holds the result and each leg's main figures, short enough to be read from
+the tail of a log (headline()); the legs in full go to stderr, as one JSON object after "details: ".
+
 `--impl reference` times the CPU oracle alone (rank 0) on the same workload and metric.
 """
 from __future__ import annotations
@@ -281,6 +284,31 @@ def bench_config(args, lp, world):
                         "relative KKT", "replicas": world,
             "l2": "inputs larger than L2 (matrix 16M nnz, >= 190 MB per copy)",
             "parallelism": f"replicas x{world}"}
+
+
+def headline(line):
+    """The line printed on stdout: all scalars of `line`, the config, clocks, CPU baseline and
+    end-to-end figures whole, and of the other legs their scalars that name a time, a rate or an
+    error."""
+    scalar = lambda v: v is None or isinstance(v, (bool, int, float, str))
+    out = {k: v for k, v in line.items() if scalar(v) and k != "objective_bound"}
+    for k in ("config", "cpu_baseline", "clocks", "e2e"):
+        if line.get(k) is not None:
+            out[k] = dict(line[k])
+    if "status" in out.get("e2e", {}):
+        out["e2e"]["status"] = sorted(set(out["e2e"]["status"]))
+    legs = {"fp64": ("ms_per_step", "ms_per_solve", "pdhg_iter_per_s", "objective_rel_error"),
+            "mixed_refined_to_1e-8": ("ms_per_solve", "objective_rel_error"),
+            "c0": (), "batch_c3": ("batch_lps_per_s",), "batch_c3_mixed": ("batch_lps_per_s",),
+            "adjoint_c4": ("adjoint_ms_per_instance",),
+            "roofline": ("bound", "achieved", "peak", "unit", "frac", "peak_kind", "kernel",
+                         "traffic")}
+    for k, keys in legs.items():
+        leg = line.get(k) or {}
+        small = {q: leg[q] for q in keys if q in leg and scalar(leg[q])}
+        if small:
+            out[k] = small
+    return out
 
 
 def run_reference(args):
@@ -678,7 +706,8 @@ def run_b200(args):
         "clocks": clocks, "gpu_launches": int(sum(st["kernel_launches"] for _, st in st_mixed)),
     }
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print("details: " + json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     L.cuOptDestroySolverSettings(C.byref(s_mixed))
     L.cuOptDestroySolverSettings(C.byref(s_fp64))
     replicas.close()
