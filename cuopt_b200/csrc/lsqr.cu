@@ -25,8 +25,8 @@
 //   * the x / w update of an iteration is applied in the next transpose product by the thread that
 //     owns the row.
 // One block per system, reading the operator from L2, took 33 us an iteration on the 5000 x 5000
-// systems.  Systems whose vectors do not fit (some 14 000 rows and columns) still run in one block
-// each, with u, v, x and w in global memory.
+// systems.  Systems whose vectors do not fit in clusters of 8 (some 25 000 rows and columns together)
+// still run in one block each, with u, v, x and w in global memory.
 // Each cluster stops at LSQR's tests or at its iteration limit: none waits for another, and a wait
 // for an exchange is bounded (its end without one is reported as an error).
 #include "common.cuh"
@@ -784,7 +784,7 @@ cluster_kernel_t cluster_kernel(int blocks, bool cached)
   }
 }
 
-// The plan with the least estimated time: waves of clusters, each iteration of one taking a latency,
+// The plan with the least estimated time (smem 0: no shape can be launched): waves of clusters, each iteration of one taking a latency,
 // a share for every block and, between blocks, for every entry of u and v, and the products, shared by
 // the blocks.  Fitted to these us an iteration with 1, 2, 4, 8 and 16 blocks, operators in shared
 // memory, then from L2 (stored elements of both operators, rows + columns):
@@ -834,7 +834,6 @@ cluster_plan plan_clusters(const std::vector<packed>& pk, const std::vector<int>
         best_us = us;
       }
     }
-  if (best.smem == 0) throw cuda_error("lsqr: no cluster shape can be launched");
   return best;
 }
 
@@ -890,6 +889,7 @@ struct size_class {
   cluster_plan plan;
 };
 constexpr int kClassBlocks[] = {1, 2, 4, 8, 16};
+constexpr int kPortableBlocks = 8;  // the largest cluster that every launch may have
 int class_of(const packed& q, size_t limit)
 {
   int k = 0;
@@ -923,16 +923,13 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   const size_t limit = max_dynamic_smem((const void*)cluster_kernel(16, true));
   std::vector<size_class> classes(std::size(kClassBlocks) + 1);
   std::vector<int> glob_ids;
-  size_t scratch_doubles = 0;
   for (int i = 0; i < count; ++i) {
     res[i].z.assign(ps[i]->cols, 0.0);
     if (pk[i].rows == 0 || pk[i].cols == 0) continue;
-    if (cluster_smem(pk[i], 1, false) <= limit) {
+    if (cluster_smem(pk[i], kPortableBlocks, false) <= limit)
       classes[class_of(pk[i], limit)].ids.push_back(i);
-    } else {
+    else
       glob_ids.push_back(i);
-      scratch_doubles += (size_t)pk[i].rows + 3 * (size_t)pk[i].cols;
-    }
   }
   std::vector<int> order;              // systems as they are launched
   std::vector<int> blocks(count, 1);   // of the cluster of each
@@ -945,9 +942,15 @@ std::vector<lsqr_result> lsqr_solve_batch(const std::vector<const lsqr_problem*>
   const double all = std::accumulate(work.begin(), work.end(), 0.0);
   for (auto& k : classes) {
     k.plan = plan_clusters(pk, k.ids, limit, work[&k - classes.data()] / std::max(all, 1e-300));
+    if (k.plan.smem == 0) {
+      glob_ids.insert(glob_ids.end(), k.ids.begin(), k.ids.end());
+      k.ids.clear();
+    }
     for (int i : k.ids) blocks[i] = k.plan.blocks;
     order.insert(order.end(), k.ids.begin(), k.ids.end());
   }
+  size_t scratch_doubles = 0;
+  for (int i : glob_ids) scratch_doubles += (size_t)pk[i].rows + 3 * (size_t)pk[i].cols;
   order.insert(order.end(), glob_ids.begin(), glob_ids.end());
   if (order.empty()) return res;
 

@@ -44,6 +44,8 @@ def test_many_systems(count):
     _check([gen.vertex_lp(*sizes[i % 4], seed=100 + i) for i in range(count)])
 
 
-def test_vectors_beyond_shared_memory():
-    """15 000 rows and columns: u, v, x and w are in global memory, one block runs the system."""
-    _check([gen.vertex_lp(15000, 30100, 2, seed=9)])
+@pytest.mark.parametrize("m", [7200, 10000, 15000])
+def test_vectors_beyond_shared_memory(m):
+    """Rows and columns around what one block (7 100), then a cluster of 8 (12 500) holds; at 15 000,
+    u, v, x and w are in global memory and one block runs the system."""
+    _check([gen.vertex_lp(m, 2 * m + 100, 2, seed=9)])
