@@ -810,6 +810,7 @@ class climber_engine {
     for (int g = 0; g < groups_; ++g) groups_seen[g] = group_active(g);
 
     B200_CUDA_CHECK(cudaEventRecord(e_.kept_, s_));
+    // As in batches (by what fits in L2: 32 climbers of 2000 x 5000 41.4 ms instead of 40.9).
     const double est_us = 9.0 + 2.0 * (double)e_.L_.nnz * groups_ / 5e4;
     const bool small    = est_us <= 16.0;
     const long ahead    = small ? 8 : std::max(1L, (long)std::ceil(40.0 / est_us));

@@ -1597,7 +1597,9 @@ struct term_dual_epi {
 // behind them, see enqueue_conv).  As two sweeps, two one-block sums and a copy this took five stream
 // operations per check; on a 2000 x 5000 LP they were the longer part of it.  arrived must be 0
 // before the launch and is 0 after it.
-static __global__ void __launch_bounds__(kBlock, kSweepBlocks<double>)
+// At 5 resident blocks: 1M x 2M 192 us at 3, 178 at 4, 173 at 5, 187 at 6 (spills); the sums are 28 of them.
+constexpr int kCheckBlocks = 5;
+static __global__ void __launch_bounds__(kBlock, kCheckBlocks)
   term_kernel(const dev_sell<double> A, const dev_sell<double> AT, const double* __restrict__ xu,
               const double* __restrict__ yu, term_primal_epi ep, term_dual_epi ed, int gp, int gd,
               double* partials, unsigned* arrived, double* host, const int* flag_a, const int* flag_b)
