@@ -434,10 +434,12 @@ __device__ __forceinline__ void sell_map_block(const dev_sell<TM>& A, const TG* 
 // registers), 3 with FP64 (80).  FP64, 1M x 2M LP with 16M non-zeros, primal + dual sweep: 86.4 + 81.1
 // us at 4 blocks (64 registers), 86.5 + 78.9 at 3, 95.2 + 86.9 left alone; 400k x 1M: 45.1 + 45.8, 45.0
 // + 43.2, 48.3 + 47.0.  FP32, 1M x 2M: 71.8 + 73.3 at 5, 74.4 + 73.1 at 4.
-template <typename TM>
-constexpr int kSweepBlocks = sizeof(TM) == 4 ? 5 : 3;
+// Batches, whose gathers hit L1, want the warps instead: 4 in FP64 (512 LPs with 51.6M non-zeros,
+// primal sweep 215 us, 231 at 3).
+template <typename TM, class Epi>
+constexpr int kSweepBlocks = sizeof(TM) == 4 ? 5 : has_skip_range<Epi>::value ? 4 : 3;
 template <typename TM, typename TG, class Epi>
-__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM, Epi>) sell_map_kernel(const dev_sell<TM> A,
                                                           const TG* __restrict__ g, Epi epi,
                                                           double* partials)
 {
@@ -447,7 +449,7 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_kernel(cons
 // Blocks vb0, vb0 + 1, ... of a sweep's grid only (measurement of one row-length class: the
 // long rows are blocks [0, long_blocks), the slices the rest).
 template <typename TM, typename TG, class Epi>
-__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_range_kernel(const dev_sell<TM> A,
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM, Epi>) sell_map_range_kernel(const dev_sell<TM> A,
                                                                 const TG* __restrict__ g, Epi epi,
                                                                 double* partials, int vb0)
 {
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>) sell_map_range_kerne
 
 // The same sweep with WPB warps per block (the plain sweeps' block shape is autotuned).
 template <typename TM, typename TG, class Epi, int WPB>
-__global__ void __launch_bounds__(WPB * kWarp, kSweepBlocks<TM> * kWarpsPerBlock / WPB)
+__global__ void __launch_bounds__(WPB * kWarp, kSweepBlocks<TM, Epi> * kWarpsPerBlock / WPB)
   sell_map_wpb_kernel(const dev_sell<TM> A, const TG* __restrict__ g, Epi epi, double* partials)
 {
   sell_map_block<TM, TG, Epi, false, WPB>(A, g, epi, partials, (int)blockIdx.x);
@@ -1767,7 +1769,7 @@ static __global__ void gk_start_kernel(gk_state* st, const double* sumsq, double
 // A step is two launches; with the sum and its recording as kernels of their own it was six, and
 // on a 12k x 30k LP those four one-block kernels were the larger part of it.
 template <int FIELD, typename TM, class Epi>
-__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>)
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM, Epi>)
   gk_sweep_kernel(const dev_sell<TM> A, const double* __restrict__ g, Epi epi, double* partials,
                   gk_state* st, double* hist)
 {
@@ -1827,7 +1829,7 @@ __device__ __forceinline__ double gk_partials_norm(const double* partials, int b
 // blocks and the sums of the last one follow one another: a half step on a 12 007 x 30 011 LP took
 // 7.7 us and takes 6.6 us.  With more partials every block would read more than one a thread.
 template <int FIELD, typename TM, class Epi>
-__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM>)
+__global__ void __launch_bounds__(kBlock, kSweepBlocks<TM, Epi>)
   gk_chain_kernel(const dev_sell<TM> A, const double* __restrict__ g, Epi epi, const double* pin,
                   int nin, double* pout, gk_state* st, double* hist, int k)
 {
